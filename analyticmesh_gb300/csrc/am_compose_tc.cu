@@ -960,7 +960,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
             const int nchunks = (R * 64 + 4 * kSBuild - 1) / (4 * kSBuild);
             // The epilogue of a pass reads its accumulators (warp w: TMEM
             // lanes 32 (w % 4).., column blocks cgrp, cgrp + ngrp, ... of each
-            // M tile; at most four blocks of 16 columns) and stores their rows,
+            // M tile) and stores their rows,
             // except the last block, which stays in registers and is stored
             // during the next pass's first step, while the tensor core works
             // (a pass's 128 KB of rows take ~4 K cycles of the SM's store
@@ -1106,8 +1106,12 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                 def_ok = acc_ok;
                 def_nit = nit;
                 def_first = nit - nkeep;
+                // (every block of the pass: three M tiles of 80 columns give a
+                // warp six, so no fixed bound)
+                for (int it0 = 0; it0 < nit; it0 += 4)
 #pragma unroll
-                for (int it = 0; it < 4; ++it) {
+                for (int u = 0; u < 4; ++u) {
+                    const int it = it0 + u;
                     if (!acc_ok || it >= nit) break;
                     const int mt = mt0 + it / ncbw, cb = cgrp + (it % ncbw) * ngrp;
                     const int mm = mt * 128 + q4 * 32 + lane;

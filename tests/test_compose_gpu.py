@@ -127,3 +127,27 @@ def test_streamed_and_resident_operand_tiles_agree(factory):
     ref_rows, ref_eq = compose_fp64(net, out[2][2])
     assert rel_err(out[2][3], ref_rows) <= 1e-5
     assert rel_err(out[2][4], ref_eq) <= 1e-5
+
+
+@pytest.mark.parametrize("widths", [[260, 260], [300, 64, 384], [520, 48]], ids=["260", "300_64_384", "520"])
+def test_layers_of_three_and_five_m_tiles(widths):
+    """Widths whose M tiles (of 128 rows) are three or five: the streamed tile
+    then has more than four 16-column blocks per epilogue warp.  Rows of the
+    seed regions against FP64 (FP32-level: 1e-5 of a row's scale, the bound of
+    the tests above), in both streamed variants."""
+    m = wl.geometric(widths, 17, perturb=0.01)
+    net = wl.net_arrays(m)
+    st, pt = wl.seeds_for(m, init_num=1500, seed=7)
+    for tile in (2, 3):
+        eng = engine.Engine("mixed", net.nodes, net.arc_table, net.num_extra)
+        eng.set_option(_lib.AM_OPT_COMPOSE_TILE, tile)
+        eng.set_option(_lib.AM_OPT_MAX_REGIONS, 1600)
+        try:
+            eng.run_net(net, st, pt)
+        except _lib.AmError as ex:
+            assert ex.status == _lib.AM_ERR_CAPACITY
+        n = 1400  # (the seeds come first)
+        rows, eq = eng.region_rows(0, n)
+        ref_rows, ref_eq = compose_fp64(net, eng.regions().bits[:n])
+        assert rel_err(rows, ref_rows) <= 1e-5 and rel_err(eq, ref_eq) <= 1e-5, tile
+        eng.close()
