@@ -34,8 +34,9 @@ struct Acc {
 // X = diag(s) rows [src, src+K) of the region's constraint block, negated
 // (C = -A for active units, so s * A = -s * C).
 template <typename T>
-__device__ __forceinline__ void accumulate(vec4_t<T> (*X)[kR], const T *cons, size_t rstride, const uint32_t *keys, int W,
-                                           int nreg, int src, int K, const T *Wt, int Mp, int m0, Acc<T> &acc)
+__device__ __forceinline__ void accumulate(vec4_t<T> (*X)[kR], const T *cons, size_t rstride, const int4 *ri, int jend,
+                                           const uint32_t *const *keys, int nreg, int src, int K, const T *Wt, int Mp,
+                                           int m0, Acc<T> &acc)
 {
     const int tid = threadIdx.x;
     const int r = tid & (kR - 1);
@@ -49,8 +50,8 @@ __device__ __forceinline__ void accumulate(vec4_t<T> (*X)[kR], const T *cons, si
             x.x = x.y = x.z = x.w = T(0);
             if (kk < kc && rr < nreg) {
                 const int row = src + k0 + kk;
-                if (key_bit(keys + (size_t)rr * W, row)) {
-                    const vec4_t<T> c = ld4<T>(cons + (size_t)rr * rstride + (size_t)row * 4);
+                if (key_bit(keys[rr], row)) {
+                    const vec4_t<T> c = tile_row<T>(cons, rstride, ri[rr], row, jend);
                     x.x = -c.x;
                     x.y = -c.y;
                     x.z = -c.z;
@@ -83,6 +84,9 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) compose_kernel(NetDev net, RegionsDev reg, ChunkDev ch, T iso)
 {
     __shared__ vec4_t<T> X[kKC][kR];
+    __shared__ WavePlan plan;
+    __shared__ int4 ri[kR];
+    __shared__ const uint32_t *keys[kR];
     const int tid = threadIdx.x;
     const int r = tid & (kR - 1);
     const int g = tid >> 4;
@@ -90,27 +94,40 @@ __global__ void __launch_bounds__(kThreads) compose_kernel(NetDev net, RegionsDe
     int count;
     chunk_range(ch, head, count);
     const size_t rstride = (size_t)net.ALLP * 4;
-    // tiles of kR regions, strided over the grid (the graph-driven loop
-    // launches a fixed grid; the host-driven one a tile per CTA)
-    for (long long rl0 = (long long)blockIdx.x * kR; rl0 < count; rl0 += (long long)gridDim.x * kR) {
-        const int nreg = (int)min((long long)kR, (long long)count - rl0);
-        T *cons = (T *)ch.cons + (size_t)rl0 * rstride;
-        const uint32_t *keys = reg.keys + (size_t)(head + rl0) * net.W;
+    T *cons = (T *)ch.cons;
+    if (tid == 0) {
+        plan_counts(plan, ch, net.n_lin - 1, count);
+        plan_finish(plan, kR);
+    }
+    __syncthreads();
+    const int rounds = plan_rounds(plan, (int)gridDim.x);
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+        if (t < 0) continue;
+        const int cls = plan_class(plan, t);
+        const int jend = cls > 1 ? net.hoff[cls + 1] : 0;
+        const int nreg = tile_nreg(plan, t, cls);
+        __syncthreads(); // the previous tile is done with ri, keys
+        if (tid < nreg) {
+            ri[tid] = tile_region(plan, reg, ch, head, t, cls, tid);
+            keys[tid] = reg.keys + (size_t)(head + ri[tid].w) * net.W;
+        }
+        __syncthreads();
 
-        // hidden layer 1 = linear 0 rows, sign-flipped; extra constraints as given
+        // class 1: hidden layer 1 = linear 0 rows, sign-flipped; extra constraints as given
         {
             const T *W0 = (const T *)net.W0;
             const T *b0 = (const T *)net.bias[0];
-            const int n1 = net.nodes[1];
+            const int n1 = cls == 1 ? net.nodes[1] : 0;
             for (int q = tid; q < nreg * n1; q += kThreads) {
                 const int rr = q / n1, m = q % n1;
-                const T sg = key_bit(keys + (size_t)rr * net.W, m) ? T(-1) : T(1);
+                const T sg = key_bit(keys[rr], m) ? T(-1) : T(1);
                 vec4_t<T> c;
                 c.x = sg * W0[3 * m + 0];
                 c.y = sg * W0[3 * m + 1];
                 c.z = sg * W0[3 * m + 2];
                 c.w = sg * b0[m];
-                st4<T>(cons + (size_t)rr * rstride + (size_t)m * 4, c);
+                st4<T>(cons + (size_t)ri[rr].x * rstride + (size_t)m * 4, c);
             }
             const T *we = (const T *)net.w_extra;
             const T *be = (const T *)net.b_extra;
@@ -121,11 +138,11 @@ __global__ void __launch_bounds__(kThreads) compose_kernel(NetDev net, RegionsDe
                 c.y = we[3 * e + 1];
                 c.z = we[3 * e + 2];
                 c.w = be[e];
-                st4<T>(cons + (size_t)rr * rstride + (size_t)(net.N + e) * 4, c);
+                st4<T>(cons + (size_t)ri[rr].x * rstride + (size_t)(net.N + e) * 4, c);
             }
         }
 
-        for (int i = 1; i < net.n_lin; ++i) {
+        for (int i = cls; i < net.n_lin; ++i) {
             const int M = net.nodes[i + 1];
             const int K = net.nodes[i];
             const bool last = (i == net.n_lin - 1);
@@ -133,21 +150,22 @@ __global__ void __launch_bounds__(kThreads) compose_kernel(NetDev net, RegionsDe
             for (int mb = 0; mb < M; mb += kRowsPerPass) {
                 const int m0 = mb + 4 * g;
                 Acc<T> acc;
-    #pragma unroll
+#pragma unroll
                 for (int j = 0; j < 4; ++j)
-    #pragma unroll
+#pragma unroll
                     for (int c = 0; c < 4; ++c) acc.v[j][c] = T(0);
-                accumulate<T>(X, cons, rstride, keys, net.W, nreg, net.hoff[i], K, (const T *)net.Wt[i], net.Mp[i], m0, acc);
+                accumulate<T>(X, cons, rstride, ri, jend, keys, nreg, net.hoff[i], K, (const T *)net.Wt[i], net.Mp[i], m0,
+                              acc);
                 for (int s = 0; s < net.nskip[i]; ++s) {
                     const SkipDev &sk = net.skip[i][s];
                     if (sk.kind == 1 && sk.from >= 1)
-                        accumulate<T>(X, cons, rstride, keys, net.W, nreg, net.hoff[sk.from], net.nodes[sk.from],
+                        accumulate<T>(X, cons, rstride, ri, jend, keys, nreg, net.hoff[sk.from], net.nodes[sk.from],
                                       (const T *)sk.tmt, sk.Mp, m0, acc);
                 }
                 if (r < nreg) {
-                    const uint32_t *key = keys + (size_t)r * net.W;
-                    T *cr = cons + (size_t)r * rstride;
-    #pragma unroll
+                    const uint32_t *key = keys[r];
+                    T *cr = cons + (size_t)ri[r].x * rstride;
+#pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int m = m0 + j;
                         if (m >= M) continue;
@@ -160,7 +178,7 @@ __global__ void __launch_bounds__(kThreads) compose_kernel(NetDev net, RegionsDe
                                 } else {
                                     const int row = net.hoff[sk.from] + m;
                                     if (key_bit(key, row)) {
-                                        const vec4_t<T> c = ld4<T>(cr + (size_t)row * 4);
+                                        const vec4_t<T> c = tile_row<T>(cons, rstride, ri[r], row, jend);
                                         v[0] -= c.x;
                                         v[1] -= c.y;
                                         v[2] -= c.z;
@@ -188,7 +206,7 @@ __global__ void __launch_bounds__(kThreads) compose_kernel(NetDev net, RegionsDe
                             o.y = v[1];
                             o.z = v[2];
                             o.w = v[3] - iso;
-                            st4<T>((T *)ch.eq + (size_t)(rl0 + r) * 4, o);
+                            st4<T>((T *)ch.eq + (size_t)ri[r].w * 4, o);
                         }
                     }
                 }
@@ -238,7 +256,8 @@ void launch_check_finite(int prec, const FiniteList &list, int *d_err, cudaStrea
 void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso, cudaStream_t st)
 {
     if (!ch.ctl && ch.count <= 0) return;
-    const int grid = ch.ctl ? device_sms() * 4 : (ch.count + kR - 1) / kR;
+    int grid = device_sms() * 4;
+    if (!ch.ctl) grid = std::min(grid, (ch.count + kR - 1) / kR + (ch.order ? net.n_lin : 0));
     if (prec == kFloat64)
         compose_kernel<double><<<grid, kThreads, 0, st>>>(net, reg, ch, iso);
     else

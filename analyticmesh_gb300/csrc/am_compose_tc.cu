@@ -155,23 +155,53 @@ struct XOp {
     __device__ __forceinline__ uint32_t jstep() const { return mn ? (uint32_t)natoms * 128u : 2u; }
 };
 
+// Operand items (region r, row k of a 64-deep block) in the order the warps take
+// them: a warp item is two regions x sixteen rows, so that its loads are two runs
+// of 256 bytes and its stores fill whole 128-byte rows of the swizzled operand
+// (measured on GB300 with a lane per region instead: 32 lines per load, and the
+// block's loads took longer than its 48 products).
+struct Items {
+    int half, shift; // region pairs; their log2, or -1
+    __device__ __forceinline__ explicit Items(int R)
+    {
+        half = R / 2;
+        shift = -1;
+        for (int b = 0; b < 8; ++b)
+            if (half == 1 << b) shift = b;
+    }
+    // item `idx` of 2 R per block: false beyond the last
+    __device__ __forceinline__ bool at(int idx, int lane, int &r, int &k) const
+    {
+        const int kg = shift >= 0 ? idx >> shift : idx / half;
+        const int pair = idx - kg * half;
+        r = 2 * pair + (lane & 1);
+        k = kg * 16 + (lane >> 1);
+        return kg < 4;
+    }
+};
+
 // X[n = 4r + c][k] = s_k(r) ? -C[r][src + k][c] : 0 for k < K, 0 up to Kp
-__device__ void stage_x_from_rows(const XOp &X, const float *cons, size_t rstride, const uint32_t *keys, int W, int nreg,
-                                  int src, int K, int Kp)
+__device__ void stage_x_from_rows(const XOp &X, const float *cons, size_t rstride, const int4 *ri, int jend,
+                                  const uint32_t *keys, int W, int nreg, int src, int K, int Kp)
 {
-    const int R = X.ncols / 4;
-    for (int q = threadIdx.x; q < R * Kp; q += kThreads) {
-        const int r = q / Kp, k = q % Kp;
+    const Items items(X.ncols / 4);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool par = src < jend;
+    const int per = X.ncols / 2; // items per block
+    for (int q = warp; q < per * (Kp / 64); q += kThreads / 32) {
+        int r, k;
+        items.at(q % per, lane, r, k);
+        k += q / per * 64;
         float x[4] = {0.f, 0.f, 0.f, 0.f};
-        if (r < nreg && k < K) {
-            const int row = src + k;
-            if (key_bit(keys + (size_t)r * W, row)) {
-                const float4 c = ld4<float>(cons + (size_t)r * rstride + (size_t)row * 4);
-                x[0] = -c.x;
-                x[1] = -c.y;
-                x[2] = -c.z;
-                x[3] = -c.w;
-            }
+        const int row = src + k;
+        if (r < nreg && k < K && key_bit(keys + (size_t)r * W, row)) {
+            const int4 g = ri[r];
+            const float4 c = ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)row * 4);
+            const float sg = row == g.z ? 1.f : -1.f;
+            x[0] = sg * c.x;
+            x[1] = sg * c.y;
+            x[2] = sg * c.z;
+            x[3] = sg * c.w;
         }
         X.put<2>(4 * r, k, x);
     }
@@ -198,10 +228,11 @@ __device__ const uint8_t *block_ptr(const NetDev &net, const TcNet &tc, int g)
     return nullptr;
 }
 
-__device__ int total_blocks(const NetDev &net, const TcNet &tc)
+// blocks of the linears before `end` (total: end = n_lin - 1)
+__device__ int blocks_before(const NetDev &net, const TcNet &tc, int end)
 {
     int n = 0;
-    for (int i = 1; i <= net.n_lin - 2; ++i) {
+    for (int i = 1; i < end; ++i) {
         n += mat_blocks(tc.lin[i]);
         for (int s = 0; s < net.nskip[i]; ++s)
             if (tc_skip(net.skip[i][s])) n += mat_blocks(tc.skip[i][s]);
@@ -230,9 +261,8 @@ __device__ int total_blocks(const NetDev &net, const TcNet &tc)
 struct WPipe {
     uint64_t *full, *done;
     uint8_t *ws;
-    int nstage, total;
+    int nstage;
     int *err;
-    int per_tile;          // blocks one tile consumes; the sequence repeats per tile
     int consumed;          // (thread 0) blocks whose products were issued
     volatile int *abort;   // the CTA's abort flag (shared memory)
 };
@@ -246,18 +276,24 @@ __device__ __forceinline__ bool wp_wait(WPipe &p, uint64_t *bar, uint32_t parity
 }
 
 // (the copy warp's lane 0) every weight block of the CTA's tiles, nstage
-// blocks ahead of the products at most
-__device__ void wp_produce(WPipe &p, const NetDev &net, const TcNet &tc)
+// blocks ahead of the products at most; a tile of class c consumes the blocks
+// of linear c on
+__device__ void wp_produce(WPipe &p, const NetDev &net, const TcNet &tc, const WavePlan &plan, int rounds)
 {
     int last[4] = {-1, -1, -1, -1}; // the last block copied into each stage
-    for (int h = 0; h < p.total; ++h) {
-        const int s = h % p.nstage;
-        if (*p.abort) break;
-        if (h >= p.nstage && !wp_wait(p, p.done + s, (uint32_t)((h - p.nstage) / p.nstage) & 1u)) break;
-        umma::mbar_expect_tx(p.full + s, (uint32_t)kWBlockBytes);
-        umma::bulk_g2s(p.ws + (size_t)s * kWBlockBytes, block_ptr(net, tc, h % p.per_tile), (uint32_t)kWBlockBytes,
-                       p.full + s);
-        last[s] = h;
+    const int total = blocks_before(net, tc, net.n_lin - 1);
+    int h = 0;
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+        if (t < 0) continue;
+        for (int b = blocks_before(net, tc, plan_class(plan, t)); b < total; ++b, ++h) {
+            const int s = h % p.nstage;
+            if (*p.abort) continue;
+            if (h >= p.nstage && !wp_wait(p, p.done + s, (uint32_t)((h - p.nstage) / p.nstage) & 1u)) continue;
+            umma::mbar_expect_tx(p.full + s, (uint32_t)kWBlockBytes);
+            umma::bulk_g2s(p.ws + (size_t)s * kWBlockBytes, block_ptr(net, tc, b), (uint32_t)kWBlockBytes, p.full + s);
+            last[s] = h;
+        }
     }
     // nothing lands in shared memory after the CTA has left (bounded)
     for (int s = 0; s < p.nstage; ++s)
@@ -337,13 +373,18 @@ __device__ __forceinline__ void bar_main() { asm volatile("bar.sync 2, %0;" ::"r
 // reading consecutive regions' bits hit distinct banks
 __host__ __device__ __forceinline__ int key_stride(int W) { return W | 1; }
 
-// tile width for a wave of `count` regions: one tile per resident slot
-// while the wave is small, the widest tile otherwise
-__host__ __device__ __forceinline__ int tile_cols(int count, int slots, int ncols_max)
+// (one thread) tile width of the wave: one tile per resident slot while the
+// wave is small, the widest tile otherwise; the plan's tiles.  Returns the
+// tile's columns.
+__device__ int plan_wave(WavePlan &plan, const ChunkDev &ch, int layers, int count, int slots, int ncols_max)
 {
+    plan_counts(plan, ch, layers, count);
     const int per = (count + slots - 1) / slots;
-    const int ncols = (4 * per + 15) / 16 * 16;
-    return ncols < 16 ? 16 : (ncols > ncols_max ? ncols_max : ncols);
+    int ncols = (4 * per + 15) / 16 * 16;
+    ncols = ncols < 16 ? 16 : (ncols > ncols_max ? ncols_max : ncols);
+    while (ncols < ncols_max && plan_tiles(plan, ncols / 4) > slots) ncols += 16;
+    plan_finish(plan, ncols / 4);
+    return ncols;
 }
 
 __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net, TcNet tc, RegionsDev reg, ChunkDev ch,
@@ -355,16 +396,20 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
     __shared__ int s_last;
     __shared__ int s_abort; // a pipeline wait ran out (thread 0 or the copy warp)
     __shared__ int s_stop;  // thread 0's view of it, published before a tile barrier: uniform
+    __shared__ WavePlan plan;
+    __shared__ int s_ncols;
+    __shared__ int4 ri[64]; // the tile's regions (at most 256 columns)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     long long head;
     int count;
     chunk_range(ch, head, count);
     if (count <= 0) return;
-    const int ncols = tile_cols(count, slots, tc.ncols_max);
+    if (tid == 0) s_ncols = plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max);
+    __syncthreads();
+    const int ncols = s_ncols;
     const int R = ncols / 4;
-    const int ntiles = (count + R - 1) / R;
-    const int mytiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    if (mytiles == 0) return;
+    if ((int)blockIdx.x >= plan.tile0[plan.layers]) return;
+    const int rounds = plan_rounds(plan, (int)gridDim.x);
     int tmem_cols = 32;
     while (tmem_cols < 2 * tc.mtiles_max * ncols) tmem_cols <<= 1;
     const size_t rstride = (size_t)net.ALLP * 4;
@@ -385,9 +430,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
     float *wls = reinterpret_cast<float *>(w0s + net.nodes[1]);
     float *fsum = reinterpret_cast<float *>(reinterpret_cast<uintptr_t>(wls + net.nodes[net.n_lin - 1] + 3) & ~(uintptr_t)15);
 
-    WPipe pp{bars, bars + 2, ws, tc.nstage, 0, err, 1, 0, &s_abort};
-    pp.per_tile = total_blocks(net, tc);
-    pp.total = pp.per_tile * mytiles;
+    WPipe pp{bars, bars + 2, ws, tc.nstage, err, 0, &s_abort};
     if (tid == 0) {
         s_abort = 0;
         s_stop = 0;
@@ -406,7 +449,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
     }
     __syncthreads(); // barriers initialised, for the copy warp too
     if (warp == kThreads / 32) { // the copy warp: the weight blocks of every tile
-        if (lane == 0) wp_produce(pp, net, tc);
+        if (lane == 0) wp_produce(pp, net, tc, plan, rounds);
         __syncwarp();
         __syncthreads(); // the tile threads' last barrier
         return;
@@ -415,32 +458,45 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
     // epilogue: warp w reads TMEM lanes 32 (w % 4).. and every (kThreads / 128)-th column block
     const int q4 = warp & 3, cgrp = warp >> 2, ngrp = kThreads / 128;
 
-    for (int j = 0; j < mytiles; ++j) {
-        const long long rl0 = (long long)(blockIdx.x + (long long)j * gridDim.x) * R;
-        const int nreg = (int)min((long long)R, (long long)count - rl0);
-        float *cons = (float *)ch.cons + (size_t)rl0 * rstride;
-        const uint32_t *gkeys = reg.keys + (size_t)(head + rl0) * net.W;
+    float *cons = (float *)ch.cons;
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+        if (t < 0) continue;
+        const int cls = plan_class(plan, t);
+        const int jend = cls > 1 ? net.hoff[cls + 1] : 0; // rows before this are in the parent's slot
+        const int nreg = tile_nreg(plan, t, cls);
         bar_main(); // the previous tile is done with the keys and the operand
-        for (int q = tid; q < R * net.W; q += kThreads)
-            keys[(q / net.W) * KW + q % net.W] = q < nreg * net.W ? gkeys[q] : 0u;
+        if (tid < nreg) ri[tid] = tile_region(plan, reg, ch, head, t, cls, tid);
+        bar_main();
+        for (int q = tid; q < R * net.W; q += kThreads) {
+            const int rr = q / net.W, w = q % net.W;
+            keys[rr * KW + w] = rr < nreg ? reg.keys[(size_t)(head + ri[rr].w) * net.W + w] : 0u;
+        }
         bar_main(); // every thread reads every region's bits below
 
-        // hidden layer 1 = linear 0 rows (sign-flipped) and the extra constraints
+        // class 1: hidden layer 1 = linear 0 rows (sign-flipped); the extra constraints
         {
             const int n1 = net.nodes[1];
-            for (int q = tid; q < nreg * n1; q += kThreads) {
+            for (int q = tid; cls == 1 && q < nreg * n1; q += kThreads) {
                 const int rr = q / n1, m = q % n1;
                 const float sg = key_bit(keys + (size_t)rr * KW, m) ? -1.f : 1.f;
                 const float4 w = w0s[m];
-                st4<float>(cons + (size_t)rr * rstride + (size_t)m * 4, make_float4(sg * w.x, sg * w.y, sg * w.z, sg * w.w));
+                st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)m * 4,
+                           make_float4(sg * w.x, sg * w.y, sg * w.z, sg * w.w));
             }
             const float *we = (const float *)net.w_extra;
             const float *be = (const float *)net.b_extra;
             for (int q = tid; q < nreg * net.E; q += kThreads) {
                 const int rr = q / net.E, e = q % net.E;
-                st4<float>(cons + (size_t)rr * rstride + (size_t)(net.N + e) * 4,
+                st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)(net.N + e) * 4,
                            make_float4(we[3 * e], we[3 * e + 1], we[3 * e + 2], be[e]));
             }
+        }
+        if (cls > 1) { // the operand of linear cls, from the parent's rows
+            stage_x_from_rows(X, cons, rstride, ri, jend, keys, KW, nreg, net.hoff[cls], net.nodes[cls],
+                              (net.nodes[cls] + 63) / 64 * 64);
+        } else {
+            const int n1 = net.nodes[1];
             // X_1 = diag(s_1) [W0 | b0]; regions fastest across the lanes:
             // consecutive regions' columns share a 128-byte operand row
             const int Kp = (n1 + 63) / 64 * 64;
@@ -463,7 +519,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
         umma::fence_after();
         const uint32_t tmem = tslot;
 
-        for (int i = 1; i <= net.n_lin - 2; ++i) {
+        for (int i = cls; i <= net.n_lin - 2; ++i) {
             const int M = net.nodes[i + 1];
             const int mtiles = (M + 127) / 128;
             if (tid == 0) gemm_issue(pp, tc.lin[i], mtiles, X, tmem, true, g);
@@ -477,7 +533,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                     }
                     bar_main();
                     if (s_stop) break; // written by thread 0 before the barrier: uniform
-                    stage_x_from_rows(X, cons, rstride, keys, KW, nreg, net.hoff[sk.from],
+                    stage_x_from_rows(X, cons, rstride, ri, jend, keys, KW, nreg, net.hoff[sk.from],
                                       net.nodes[sk.from], tc.skip[i][s].Kp);
                     umma::fence_proxy_async();
                     bar_main();
@@ -521,7 +577,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                         x[4 * qq] = x[4 * qq + 1] = x[4 * qq + 2] = x[4 * qq + 3] = 0.f;
                         if (r < nreg) {
                             const uint32_t *key = keys + (size_t)r * KW;
-                            float *cr = cons + (size_t)r * rstride;
+                            float *cr = cons + (size_t)(uint32_t)ri[r].x * rstride;
                             float o[4] = {v[4 * qq] + vc[4 * qq], v[4 * qq + 1] + vc[4 * qq + 1],
                                           v[4 * qq + 2] + vc[4 * qq + 2], v[4 * qq + 3] + vc[4 * qq + 3] + bm};
                             for (int s = 0; s < net.nskip[i]; ++s) {
@@ -532,7 +588,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                                     } else {
                                         const int srow = net.hoff[sk.from] + m;
                                         if (key_bit(key, srow)) {
-                                            const float4 c = ld4<float>(cr + (size_t)srow * 4);
+                                            const float4 c = tile_row<float>(cons, rstride, ri[r], srow, jend);
                                             o[0] -= c.x;
                                             o[1] -= c.y;
                                             o[2] -= c.z;
@@ -597,23 +653,26 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                     for (int w = 0; w < kWarps; ++w) a += fsum[(w * 32 + rr) * 4 + c];
                     if (rg < nreg) {
                         const uint32_t *key = keys + (size_t)rg * KW;
-                        const float *cr = cons + (size_t)rg * rstride;
+                        auto crow = [&](int row) { // component c of a constraint row
+                            const float v = cons[(size_t)(uint32_t)(row < jend ? ri[rg].y : ri[rg].x) * rstride + (size_t)row * 4 + c];
+                            return row == ri[rg].z ? -v : v;
+                        };
                         for (int s = 0; s < net.nskip[i]; ++s) {
                             const SkipDev &sk = net.skip[i][s];
                             if (sk.kind == 0) {
                                 if (sk.from >= 1 && net.nodes[sk.from] == 1 && key_bit(key, net.hoff[sk.from]))
-                                    a -= cr[(size_t)net.hoff[sk.from] * 4 + c];
+                                    a -= crow(net.hoff[sk.from]);
                             } else if (sk.from == 0) {
                                 if (c < 3) a += ((const float *)sk.tmt)[(size_t)c * sk.Mp];
                             } else {
                                 const float *tt = (const float *)sk.tmt; // [dec][Mp]
                                 const int hs = net.hoff[sk.from];
                                 for (int k = 0; k < net.nodes[sk.from]; ++k)
-                                    if (key_bit(key, hs + k)) a -= tt[(size_t)k * sk.Mp] * cr[(size_t)(hs + k) * 4 + c];
+                                    if (key_bit(key, hs + k)) a -= tt[(size_t)k * sk.Mp] * crow(hs + k);
                             }
                         }
                         if (c == 3) a += bl - iso;
-                        ((float *)ch.eq)[(size_t)(rl0 + rg) * 4 + c] = a;
+                        ((float *)ch.eq)[(size_t)ri[rg].w * 4 + c] = a;
                     }
                 }
                 bar_main();
@@ -700,15 +759,17 @@ __device__ __forceinline__ bool swait(uint64_t *bar, uint32_t parity, int *err, 
 // products before its refill (about as long as the 24 products themselves),
 // so the tensor pipe was idle most of the time.
 __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, uint64_t *wfull, uint64_t *wdone,
-                                 int tiles, int *err, volatile int *abort)
+                                 const WavePlan &plan, int rounds, int *err, volatile int *abort)
 {
     const int nst = tc.nstage;
     int h = 0;
     int ps = 0;        // stage of block h (h % nst) ...
     uint32_t pph = 0u; // ... and (h / nst) & 1, kept incrementally
     int last[4] = {-1, -1, -1, -1}; // the last block copied into each stage
-    for (int t = 0; t < tiles; ++t)
-        for (int i = 1; i <= net.n_lin - 2; ++i) {
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+        if (t < 0) continue;
+        for (int i = plan_class(plan, t); i <= net.n_lin - 2; ++i) {
             const int mtl = (net.nodes[i + 1] + 127) / 128, mper = (mtl + tc.mgroups - 1) / tc.mgroups;
             for (int mt0 = 0; mt0 < mtl; mt0 += mper) {
             const int njobs = jobs_of(net, i);
@@ -735,6 +796,7 @@ __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws
             }
             }
         }
+    }
     // nothing lands in shared memory after the CTA has left: the last copy of
     // every stage (bounded)
     for (int s = 0; s < nst; ++s)
@@ -749,7 +811,7 @@ __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws
 // gave up.
 __device__ void issue_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, uint64_t *wfull, uint64_t *wdone,
                                const XOp *XS, uint64_t *xfull, uint64_t *xdone, uint64_t *accdone, uint32_t tmem,
-                               int ncols, int tiles, int *err, volatile int *abort)
+                               int ncols, const WavePlan &plan, int rounds, int *err, volatile int *abort)
 {
     const int nst = tc.nstage;
     int h = 0, xb = 0, consumed = 0;
@@ -762,8 +824,10 @@ __device__ void issue_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, 
     const uint64_t xd0 = XS[0].desc(0, 0, 0), xd1 = XS[1].desc(0, 0, 0);
     const uint64_t xu = XS[0].ustep(), xj = XS[0].jstep();
     const uint32_t idesc = XS[0].idesc();
-    for (int t = 0; t < tiles; ++t)
-        for (int i = 1; i <= net.n_lin - 2; ++i) {
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+        if (t < 0) continue;
+        for (int i = plan_class(plan, t); i <= net.n_lin - 2; ++i) {
             const int mtl = (net.nodes[i + 1] + 127) / 128, mper = (mtl + tc.mgroups - 1) / tc.mgroups;
             for (int mt0 = 0; mt0 < mtl; mt0 += mper) { // a group of M tiles, its own accumulators
             const int njobs = jobs_of(net, i);
@@ -812,6 +876,7 @@ __device__ void issue_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, 
             umma::commit(umma::smem_addr(accdone)); // the group's accumulators are complete
             }
         }
+    }
     // the last products have completed before TMEM is released
     if (consumed > 0 &&
         !umma::mbar_wait(wdone + (consumed - 1) % nst, (uint32_t)((consumed - 1) / nst) & 1u, kWaitIters))
@@ -826,16 +891,20 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
     __shared__ uint64_t bars[11];
     __shared__ uint32_t tslot;
     __shared__ int s_abort; // a wait ran out: nothing more is issued, epilogues are skipped
+    __shared__ WavePlan plan;
+    __shared__ int s_ncols;
+    __shared__ int4 ri[64]; // the tile's regions (at most 256 columns)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     long long head;
     int count;
     chunk_range(ch, head, count);
     if (count <= 0) return;
-    const int ncols = tile_cols(count, slots, tc.ncols_max);
+    if (tid == 0) s_ncols = plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max);
+    __syncthreads();
+    const int ncols = s_ncols;
     const int R = ncols / 4;
-    const int ntiles = (count + R - 1) / R;
-    const int tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    if (tiles == 0) return;
+    if ((int)blockIdx.x >= plan.tile0[plan.layers]) return;
+    const int rounds = plan_rounds(plan, (int)gridDim.x);
     int tmem_cols = 32;
     const int mper_max = (tc.mtiles_max + tc.mgroups - 1) / tc.mgroups;
     while (tmem_cols < 2 * mper_max * ncols) tmem_cols <<= 1;
@@ -890,74 +959,92 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
 
     if (warp == kSBuild / 32) {
         if (lane == 0)
-            issue_streamed(net, tc, ws, wfull, wdone, XS, xfull, xdone, accdone, tmem, ncols, tiles, err, abort);
+            issue_streamed(net, tc, ws, wfull, wdone, XS, xfull, xdone, accdone, tmem, ncols, plan, rounds, err,
+                           abort);
         __syncwarp(); // the warp reaches the block barrier below converged
     } else if (warp == kSBuild / 32 + 1) {
-        if (lane == 0) produce_streamed(net, tc, ws, wfull, wdone, tiles, err, abort);
+        if (lane == 0) produce_streamed(net, tc, ws, wfull, wdone, plan, rounds, err, abort);
         __syncwarp();
     } else {
         // epilogue: warp w reads TMEM lanes 32 (w % 4).. and every fourth column block
         const int q4 = warp & 3, cgrp = warp >> 2, ngrp = kSBuild / 128;
         int xb = 0, accph = 0;
-        for (int j = 0; j < tiles; ++j) {
-            const long long rl0 = (long long)(blockIdx.x + (long long)j * gridDim.x) * R;
-            const int nreg = (int)min((long long)R, (long long)count - rl0);
-            float *cons = (float *)ch.cons + (size_t)rl0 * rstride;
-            const uint32_t *gkeys = reg.keys + (size_t)(head + rl0) * net.W;
+        float *cons = (float *)ch.cons;
+        for (int rd = 0; rd < rounds; ++rd) {
+            const int tile = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+            if (tile < 0) continue;
+            const int cls = plan_class(plan, tile);
+            const int jend = cls > 1 ? net.hoff[cls + 1] : 0; // rows before this are in the parent's slot
+            const int nreg = tile_nreg(plan, tile, cls);
             bar_builders(); // the previous tile is done with the keys
-            for (int q = tid; q < R * net.W; q += kSBuild)
-                keys[(q / net.W) * KW + q % net.W] = q < nreg * net.W ? gkeys[q] : 0u;
+            if (tid < nreg) ri[tid] = tile_region(plan, reg, ch, head, tile, cls, tid);
             bar_builders();
-            // hidden layer 1 = linear 0 rows (sign-flipped) and the extra constraints
+            for (int q = tid; q < R * net.W; q += kSBuild) {
+                const int rr = q / net.W, w = q % net.W;
+                keys[rr * KW + w] = rr < nreg ? reg.keys[(size_t)(head + ri[rr].w) * net.W + w] : 0u;
+            }
+            bar_builders();
+            // class 1: hidden layer 1 = linear 0 rows (sign-flipped); the extra constraints
             const int n1 = net.nodes[1];
-            for (int q = tid; q < nreg * n1; q += kSBuild) {
+            for (int q = tid; cls == 1 && q < nreg * n1; q += kSBuild) {
                 const int rr = q / n1, m = q % n1;
                 const float sg = key_bit(keys + (size_t)rr * KW, m) ? -1.f : 1.f;
                 const float4 w = w0s[m];
-                st4<float>(cons + (size_t)rr * rstride + (size_t)m * 4, make_float4(sg * w.x, sg * w.y, sg * w.z, sg * w.w));
+                st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)m * 4,
+                           make_float4(sg * w.x, sg * w.y, sg * w.z, sg * w.w));
             }
             const float *we = (const float *)net.w_extra;
             const float *be = (const float *)net.b_extra;
             for (int q = tid; q < nreg * net.E; q += kSBuild) {
                 const int rr = q / net.E, e = q % net.E;
-                st4<float>(cons + (size_t)rr * rstride + (size_t)(net.N + e) * 4,
+                st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)(net.N + e) * 4,
                            make_float4(we[3 * e], we[3 * e + 1], we[3 * e + 2], be[e]));
             }
             bar_builders(); // layer-1 rows written by every builder
 
             // X[4r + c][k] = s_k(r) ? -C[r][k][c] : 0 (layer 1: +W0 rows from
             // shared memory), one 64-deep K block at a time; every pass of a
-            // layer streams the same blocks.  Thread tid owns the items q = tid
-            // + u kSBuild (region q % R, row q / R of the block): regions
-            // fastest across the lanes.  The first four items of the next
-            // block are loaded one step ahead, so that their latency hides
-            // behind the stage wait; raw values are kept and signed when
-            // stored.
+            // layer streams the same blocks.  Warp w owns the items w, w + 16,
+            // ... of a block (Items).  The first four items of the next block
+            // are loaded one step ahead, so that their latency hides behind
+            // the stage wait; raw values are kept and signed when stored (no
+            // use of a loaded value between the loads: they overlap).  The
+            // returned mask marks the items whose sign is the other one.
+            const Items items(R);
             auto load_items = [&](int li, int job, int kb, int c, float4 *v) {
                 int src;
                 job_mat(net, tc, li, job, src);
                 const int K = net.nodes[src], rows0 = net.hoff[src];
+                const bool par = rows0 < jend;
+                unsigned other = 0u;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const int q = tid + (4 * c + u) * kSBuild;
-                    const int r = q % R, k = kb * 64 + q / R;
+                    int r, kk;
+                    const bool in = items.at(warp + 16 * (4 * c + u), lane, r, kk);
+                    const int k = kb * 64 + kk;
                     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (q < R * 64 && r < nreg && k < K && key_bit(keys + (size_t)r * KW, rows0 + k))
-                        x = src == 1 ? w0s[k] : ld4<float>(cons + (size_t)r * rstride + (size_t)(rows0 + k) * 4);
+                    if (in && r < nreg && k < K && key_bit(keys + (size_t)r * KW, rows0 + k)) {
+                        const int4 g = ri[r];
+                        if (rows0 + k == g.z) other |= 1u << u;
+                        x = src == 1 ? w0s[k]
+                                     : ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)(rows0 + k) * 4);
+                    }
                     v[u] = x;
                 }
+                return src == 1 ? 0u : other;
             };
-            auto put_items = [&](const XOp &X, int c, const float4 *v, float sg) {
+            auto put_items = [&](const XOp &X, int c, const float4 *v, float sg, unsigned other) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const int q = tid + (4 * c + u) * kSBuild;
-                    if (q < R * 64) {
-                        const float x[4] = {sg * v[u].x, sg * v[u].y, sg * v[u].z, sg * v[u].w};
-                        X.put<2>(4 * (q % R), q / R, x);
+                    int r, kk;
+                    if (items.at(warp + 16 * (4 * c + u), lane, r, kk)) {
+                        const float s1 = (other >> u) & 1u ? -sg : sg;
+                        const float x[4] = {s1 * v[u].x, s1 * v[u].y, s1 * v[u].z, s1 * v[u].w};
+                        X.put<2>(4 * r, kk, x);
                     }
                 }
             };
-            const int nchunks = (R * 64 + 4 * kSBuild - 1) / (4 * kSBuild);
+            const int nchunks = (2 * R + 63) / 64;
             // The epilogue of a pass reads its accumulators (warp w: TMEM
             // lanes 32 (w % 4).., column blocks cgrp, cgrp + ngrp, ... of each
             // M tile) and stores their rows,
@@ -999,7 +1086,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                     const int r = cb * 4 + qq;
                     if (r >= nreg) continue;
                     const uint32_t *key = keys + (size_t)r * KW;
-                    float *cr = cons + (size_t)r * rstride;
+                    float *cr = cons + (size_t)(uint32_t)ri[r].x * rstride;
                     float v4[4] = {o[0][4 * qq], o[0][4 * qq + 1], o[0][4 * qq + 2], o[0][4 * qq + 3]};
                     for (int s = 0; s < net.nskip[li]; ++s) {
                         const SkipDev &sk = net.skip[li][s];
@@ -1009,7 +1096,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                             } else {
                                 const int srow = net.hoff[sk.from] + m;
                                 if (key_bit(key, srow)) {
-                                    const float4 c = ld4<float>(cr + (size_t)srow * 4);
+                                    const float4 c = tile_row<float>(cons, rstride, ri[r], srow, jend);
                                     v4[0] -= c.x;
                                     v4[1] -= c.y;
                                     v4[2] -= c.z;
@@ -1028,12 +1115,13 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                 }
             };
             float4 pre[4];
-            for (int i = 1; i <= net.n_lin - 2; ++i) {
+            unsigned pre_other = 0u;
+            for (int i = cls; i <= net.n_lin - 2; ++i) {
                 const int M = net.nodes[i + 1];
                 const int mtiles = (M + 127) / 128;
                 const int mper = (mtiles + tc.mgroups - 1) / tc.mgroups;
                 const int njobs = jobs_of(net, i);
-                load_items(i, 0, 0, 0, pre);
+                pre_other = load_items(i, 0, 0, 0, pre);
                 for (int mt0 = 0; mt0 < mtiles; mt0 += mper) { // the products of this group of M tiles
                 const int mt1 = min(mtiles, mt0 + mper);
                 int t = 0; // step of the pass
@@ -1060,11 +1148,11 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                         const bool ok = fill < 1 ? !*abort : swait(xdone + xs, (uint32_t)((fill - 1) & 1), err, abort);
                         const XOp &X = XS[xs];
                         if (ok) {
-                            put_items(X, 0, pre, sg);
+                            put_items(X, 0, pre, sg, pre_other);
                             for (int c = 1; c < nchunks; ++c) {
                                 float4 t4[4];
-                                load_items(i, job, kb, c, t4);
-                                put_items(X, c, t4, sg);
+                                const unsigned other = load_items(i, job, kb, c, t4);
+                                put_items(X, c, t4, sg, other);
                             }
                         }
                         umma::fence_proxy_async(); // generic-proxy stores -> the tensor cores
@@ -1075,7 +1163,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                             shift_o();
                             if (t == nd - 1) bar_builders();
                         }
-                        if (more) load_items(i, njob, nkb2, 0, pre);
+                        if (more) pre_other = load_items(i, njob, nkb2, 0, pre);
                     }
                 }
                 if (t < nd) { // a pass shorter than the deferred blocks
@@ -1170,20 +1258,27 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                 constexpr int kWarps = kSBuild / 32;
                 const bool live = !*abort; // per thread: the barriers below are kept either way
                 for (int r0 = 0; r0 < R; r0 += 32) {
-                    const int r = r0 + lane;
+                    // thread (region fr of these 32, K residue fw): sixteen
+                    // consecutive rows of two regions per warp and step
+                    const int fr = 2 * warp + (lane & 1), fw = lane >> 1, r = r0 + fr;
                     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                    if (live && r < nreg)
-                        for (int k = warp; k < K; k += kWarps) {
+                    if (live && r < nreg) {
+                        const int4 g = ri[r];
+                        const float *cr = cons + (size_t)(uint32_t)(rows0 < jend ? g.y : g.x) * rstride + (size_t)rows0 * 4;
+#pragma unroll 4
+                        for (int k = fw; k < K; k += kWarps) {
                             const float w = wls[k];
                             float x[4] = {0.f, 0.f, 0.f, 0.f};
                             if (key_bit(keys + (size_t)r * KW, rows0 + k)) {
-                                const float4 c = ld4<float>(cons + (size_t)r * rstride + (size_t)(rows0 + k) * 4);
+                                const float4 c = ld4<float>(cr + (size_t)k * 4);
                                 x[0] = -c.x, x[1] = -c.y, x[2] = -c.z, x[3] = -c.w;
                             }
+                            const float wk = rows0 + k == g.z ? -w : w; // (the parent's sign)
 #pragma unroll
-                            for (int c = 0; c < 4; ++c) acc[c] = fmaf(w, x[c], acc[c]);
+                            for (int c = 0; c < 4; ++c) acc[c] = fmaf(wk, x[c], acc[c]);
                         }
-                    reinterpret_cast<float4 *>(fsum)[warp * 32 + lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                    }
+                    reinterpret_cast<float4 *>(fsum)[fw * 32 + fr] = make_float4(acc[0], acc[1], acc[2], acc[3]);
                     bar_builders();
                     if (live && tid < 128) {
                         const int rr = tid >> 2, c = tid & 3, rg = r0 + rr;
@@ -1191,23 +1286,26 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                         for (int w = 0; w < kWarps; ++w) a += fsum[(w * 32 + rr) * 4 + c];
                         if (rg < nreg) {
                             const uint32_t *key = keys + (size_t)rg * KW;
-                            const float *cr = cons + (size_t)rg * rstride;
+                            auto crow = [&](int row) { // component c of a constraint row
+                                const float v = cons[(size_t)(uint32_t)(row < jend ? ri[rg].y : ri[rg].x) * rstride + (size_t)row * 4 + c];
+                                return row == ri[rg].z ? -v : v;
+                            };
                             for (int s = 0; s < net.nskip[i]; ++s) {
                                 const SkipDev &sk = net.skip[i][s];
                                 if (sk.kind == 0) {
                                     if (sk.from >= 1 && net.nodes[sk.from] == 1 && key_bit(key, net.hoff[sk.from]))
-                                        a -= cr[(size_t)net.hoff[sk.from] * 4 + c];
+                                        a -= crow(net.hoff[sk.from]);
                                 } else if (sk.from == 0) {
                                     if (c < 3) a += ((const float *)sk.tmt)[(size_t)c * sk.Mp];
                                 } else {
                                     const float *tt = (const float *)sk.tmt; // [dec][Mp]
                                     const int hs = net.hoff[sk.from];
                                     for (int k = 0; k < net.nodes[sk.from]; ++k)
-                                        if (key_bit(key, hs + k)) a -= tt[(size_t)k * sk.Mp] * cr[(size_t)(hs + k) * 4 + c];
+                                        if (key_bit(key, hs + k)) a -= tt[(size_t)k * sk.Mp] * crow(hs + k);
                                 }
                             }
                             if (c == 3) a += bl - iso;
-                            ((float *)ch.eq)[(size_t)(rl0 + rg) * 4 + c] = a;
+                            ((float *)ch.eq)[(size_t)ri[rg].w * 4 + c] = a;
                         }
                     }
                     bar_builders();
@@ -1275,30 +1373,15 @@ void launch_compose_tc(const NetDev &net, const TcNet &tc, const RegionsDev &reg
 {
     if (!ch.ctl && ch.count <= 0) return;
     const int sms = device_sms();
-    const size_t smem_max = tc_smem_bytes(tc, tc.ncols_max, net.W);
-    const int slots = sms; // one resident tile per SM
+    const size_t smem = tc_smem_bytes(tc, tc.ncols_max, net.W);
+    const int slots = sms; // one resident tile per SM, the wave's tiles strided over them
     if (tc.streamed) {
-        cudaFuncSetAttribute(compose_tcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
-        if (ch.ctl) {
-            compose_tcs_kernel<<<slots, kSThreads, smem_max, st>>>(net, tc, reg, ch, (float)iso, slots, d_err);
-            return;
-        }
-        const int ncols = tile_cols(ch.count, slots, tc.ncols_max);
-        const int R = ncols / 4;
-        compose_tcs_kernel<<<(ch.count + R - 1) / R, kSThreads, tc_smem_bytes(tc, ncols, net.W), st>>>(
-            net, tc, reg, ch, (float)iso, slots, d_err);
+        cudaFuncSetAttribute(compose_tcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        compose_tcs_kernel<<<slots, kSThreads, smem, st>>>(net, tc, reg, ch, (float)iso, slots, d_err);
         return;
     }
-    cudaFuncSetAttribute(compose_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
-    if (ch.ctl) { // wave size known on the device only: every resident tile slot, tiles strided
-        compose_tc_kernel<<<slots, kThreads + 32, smem_max, st>>>(net, tc, reg, ch, (float)iso, slots, d_err);
-        return;
-    }
-    const int ncols = tile_cols(ch.count, slots, tc.ncols_max);
-    const int R = ncols / 4;
-    const int grid = (ch.count + R - 1) / R;
-    compose_tc_kernel<<<grid, kThreads + 32, tc_smem_bytes(tc, ncols, net.W), st>>>(net, tc, reg, ch, (float)iso, slots,
-                                                                              d_err);
+    cudaFuncSetAttribute(compose_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    compose_tc_kernel<<<slots, kThreads + 32, smem, st>>>(net, tc, reg, ch, (float)iso, slots, d_err);
 }
 
 void launch_pack_weights(const float *src, int M, int K, int Mp, int Kp, void *dst, cudaStream_t st)

@@ -65,6 +65,93 @@ __device__ __forceinline__ unsigned long long slot_value(uint32_t fp, int cand, 
     return ((unsigned long long)fp << 32) | ((unsigned long long)(cand ? 1u : 0u) << 31) | (id & 0x7fffffffu);
 }
 
+// ---------------------------------------------------------------- tiles of a wave
+// The composition's tiles of R regions, the classes (ChunkDev) one after the
+// other from the longest (class 1) to the shortest, so that the CTAs' rounds
+// hold tiles of about the same length.  Every second round runs backwards over
+// the CTAs: the CTA with the longest tile of one round gets the shortest of the
+// next.
+struct WavePlan {
+    int cnt[kMaxLayers];        // regions per class
+    int tile0[kMaxLayers + 1];  // first tile of each class
+    int R, layers;
+};
+
+__device__ __forceinline__ int plan_tiles(const WavePlan &w, int R)
+{
+    int n = 0;
+    for (int c = 0; c < w.layers; ++c) n += (w.cnt[c] + R - 1) / R;
+    return n;
+}
+// (one thread) the class counts; then, R chosen, the tiles
+__device__ __forceinline__ void plan_counts(WavePlan &w, const ChunkDev &ch, int layers, int count)
+{
+    w.layers = ch.order ? layers : 1;
+    for (int c = 0; c < w.layers; ++c) w.cnt[c] = ch.order ? ch.ccount[c] : count;
+}
+__device__ __forceinline__ void plan_finish(WavePlan &w, int R)
+{
+    w.R = R;
+    int n = 0;
+    for (int c = 0; c < w.layers; ++c) {
+        w.tile0[c] = n;
+        n += (w.cnt[c] + R - 1) / R;
+    }
+    w.tile0[w.layers] = n;
+}
+// the tile of round j on CTA b of G, -1 when there is none
+__device__ __forceinline__ int plan_tile(const WavePlan &w, int j, int b, int G)
+{
+    const long long t = (long long)j * G + ((j & 1) ? G - 1 - b : b);
+    return t < w.tile0[w.layers] ? (int)t : -1;
+}
+__device__ __forceinline__ int plan_rounds(const WavePlan &w, int G) { return (w.tile0[w.layers] + G - 1) / G; }
+__device__ __forceinline__ int plan_class(const WavePlan &w, int t)
+{
+    int c = 0;
+    while (t >= w.tile0[c + 1]) ++c;
+    return c + 1;
+}
+
+// One region of a tile: x its own rows' slot, y its parent's, z the plane it
+// was entered through (its row changes sign between the two; -1 for class 1),
+// w its wave position.
+__device__ __forceinline__ int4 tile_region(const WavePlan &w, const RegionsDev &reg, const ChunkDev &ch, long long head,
+                                            int t, int c, int r)
+{
+    const int idx = (t - w.tile0[c - 1]) * w.R + r;
+    const int rl = ch.order ? ch.order[(size_t)(c - 1) * ch.order_cap + idx] : idx;
+    int4 o;
+    o.x = (int)row_slot(ch, head, rl);
+    o.y = o.x;
+    o.z = -1;
+    o.w = rl;
+    if (c > 1) {
+        o.y = (int)ring_slot(ch, reg.parent[head + rl]);
+        o.z = reg.start[head + rl];
+    }
+    return o;
+}
+__device__ __forceinline__ int tile_nreg(const WavePlan &w, int t, int c)
+{
+    return min(w.R, w.cnt[c - 1] - (t - w.tile0[c - 1]) * w.R);
+}
+// a region's constraint row: the rows before jend from its parent's slot
+// (rewritten by no region of this wave), the plane it was entered through with
+// the other sign; the rest from its own
+template <typename T>
+__device__ __forceinline__ vec4_t<T> tile_row(const T *cons, size_t rstride, const int4 &ri, int row, int jend)
+{
+    vec4_t<T> v = ld4<T>(cons + (size_t)(uint32_t)(row < jend ? ri.y : ri.x) * rstride + (size_t)row * 4);
+    if (row == ri.z) {
+        v.x = -v.x;
+        v.y = -v.y;
+        v.z = -v.z;
+        v.w = -v.w;
+    }
+    return v;
+}
+
 // ---------------------------------------------------------------- warp
 __device__ __forceinline__ int warp_sum(int v)
 {

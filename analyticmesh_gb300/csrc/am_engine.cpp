@@ -206,13 +206,17 @@ struct am_engine {
     DevBuf tc_lin[kMaxLayers], tc_skip[kMaxLayers][kMaxSkips];
     TcNet tcnet{};
     // regions
-    DevBuf keys, hash, mid, start, nv, status, verts, edges;
+    DevBuf keys, hash, mid, start, parent, nv, status, verts, edges;
     long long cap = 0;
     DevBuf table;
     unsigned long long hcap = 0;
     // chunk
-    DevBuf cons, eq, rec, blocksum;
+    DevBuf cons, eq, rec, blocksum, order, split;
     int chunk_cap = 0;
+    int ring = 0;             // slots of cons (ChunkDev)
+    long long ring_target = 0; // what ensure_ring last asked for
+    bool ring_min = false;    // memory is short: no slots beyond a wave's
+    long long rows_from = 0;  // regions before this have no rows in the ring
     // seeds
     DevBuf s_states, s_keys, s_hash, s_pts, s_rec;
     // counters
@@ -291,6 +295,7 @@ struct am_engine {
         r.hash = hash.as<uint64_t>();
         r.mid = mid.p;
         r.start = start.as<int32_t>();
+        r.parent = parent.as<int32_t>();
         r.nv = nv.as<int32_t>();
         r.status = status.as<int8_t>();
         r.verts = verts.p;
@@ -304,8 +309,11 @@ struct am_engine {
     void release_run_buffers()
     {
         drop_graph();
-        for (DevBuf *b : {&keys, &hash, &mid, &start, &nv, &status, &verts, &edges, &table, &cons, &eq, &rec, &blocksum})
+        for (DevBuf *b : {&keys, &hash, &mid, &start, &parent, &nv, &status, &verts, &edges, &table, &cons, &eq, &rec,
+                          &blocksum, &order, &split})
             b->reset();
+        ring = 0;
+        ring_target = 0;
         cap = 0;
         hcap = 0;
         chunk_cap = 0;
@@ -321,6 +329,7 @@ struct am_engine {
         AM_CUDA(hash.grow(sizeof(uint64_t) * nc, sizeof(uint64_t) * keep, st));
         AM_CUDA(mid.grow(ts * 4 * nc, ts * 4 * keep, st));
         AM_CUDA(start.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
+        AM_CUDA(parent.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
         AM_CUDA(nv.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
         AM_CUDA(status.grow(sizeof(int8_t) * nc, sizeof(int8_t) * keep, st));
         AM_CUDA(verts.grow(ts * 3 * kVMax * nc, ts * 3 * kVMax * keep, st));
@@ -355,11 +364,91 @@ struct am_engine {
     void ensure_chunk(int count)
     {
         if (count <= chunk_cap) return;
-        AM_CUDA(cons.alloc(tc * 4 * (size_t)ALLP * count, st));
+        if (classes()) {
+            AM_CUDA(order.alloc(sizeof(int32_t) * (size_t)(n_lin - 1) * count, st));
+            AM_CUDA(split.alloc(sizeof(int32_t) * (size_t)count, st));
+        }
         AM_CUDA(eq.alloc(tc * 4 * (size_t)count, st));
         AM_CUDA(rec.alloc(sizeof(int32_t) * (size_t)kVMax * count, st));
         AM_CUDA(blocksum.alloc(sizeof(int) * ((size_t)count * kVMax / 1024 + 6), st));
         chunk_cap = count;
+    }
+
+    // a network with no layer product has nothing to take from a parent
+    bool classes() const { return n_lin >= 3; }
+
+    // the ring of constraint rows: a wave's slots and the history in which
+    // its regions find their parents.  A parent is at most about one level of
+    // the breadth-first queue away, and a level held 28 to 39 regions per
+    // hidden unit on the benchmark networks (N = 512 .. 4,096): 48 N, at most
+    // an eighth of the free memory.  A batch member's ring grows with its
+    // waves: two waves, which always reach the parents while a wave holds a
+    // whole level.  Slots never hold less than a wave.
+    void ensure_ring(int wave, long long head)
+    {
+        const size_t per = tc * 4 * (size_t)ALLP;
+        long long target = wave;
+        if (classes() && !ring_min) target = run.lean ? 2ll * wave : std::max(run.chunk, wave) + 48ll * N;
+        if (wave <= ring && target <= ring_target) return;
+        long long want = target;
+        if (want > wave) {
+            size_t fr = 0, all = 0;
+            AM_CUDA(cudaMemGetInfo(&fr, &all));
+            want = std::min<long long>(want, (long long)((fr + cons.bytes) / 8 / per));
+            want = std::max<long long>(std::min<long long>(want, INT_MAX), wave);
+        }
+        ring_target = target;
+        if (want <= ring) return;
+        ring = 0;
+        cudaError_t rc = cons.alloc(per * (size_t)want, st);
+        if (rc == cudaErrorMemoryAllocation && want > wave) {
+            cudaGetLastError();
+            want = wave;
+            rc = cons.alloc(per * (size_t)want, st);
+        }
+        AM_CUDA(rc);
+        ring = (int)want;
+        rows_from = head;
+    }
+    ChunkDev wave_chunk(long long head, int count) const
+    {
+        ChunkDev ch;
+        ch.head = head;
+        ch.count = count;
+        ch.cons = cons.p;
+        ch.eq = eq.p;
+        ch.rec = rec.as<int32_t>();
+        ch.ring = ring;
+        if (classes()) {
+            ch.order_cap = chunk_cap;
+            ch.order = order.as<int32_t>();
+            ch.split = split.as<int32_t>();
+            ch.ccount = (int32_t *)((char *)d_tail.p + offsetof(WaveCtl, ccount));
+            ch.rows_from = rows_from;
+        }
+        return ch;
+    }
+    // room for a wave of `count` more regions' children; where memory runs
+    // out, the ring gives its history back first
+    void ensure_wave(int wave, long long head, long long tail, int count, bool fit_cap)
+    {
+        ensure_chunk(wave);
+        auto stores = [&] {
+            ensure_regions(tail + (long long)count * kVMax);
+            ensure_table(std::max<long long>(tail + (long long)count * kVMax, fit_cap ? cap : 0), true);
+        };
+        try {
+            stores();
+        } catch (const Failure &x) {
+            if (x.code != AM_ERR_OUT_OF_MEMORY || ring <= wave) throw;
+            cudaGetLastError();
+            cons.reset();
+            ring = 0;
+            ring_target = 0;
+            ring_min = true;
+            stores();
+        }
+        ensure_ring(wave, head);
     }
 
     int default_chunk() const
@@ -427,7 +516,8 @@ struct am_engine {
         auto add = [&](const void *p, size_t n) {
             sig.insert(sig.end(), (const unsigned char *)p, (const unsigned char *)p + n);
         };
-        const void *bufs[6] = {cons.p, eq.p, rec.p, blocksum.p, d_tail.p, (const void *)blocksum.bytes};
+        const void *bufs[9] = {cons.p,   eq.p,    rec.p, blocksum.p, d_tail.p, (const void *)blocksum.bytes,
+                               order.p, split.p, (const void *)(size_t)ring};
         add(&prec, sizeof(prec));
         add(&chunk, sizeof(chunk));
         add(&face_warps, sizeof(face_warps));
@@ -454,13 +544,9 @@ struct am_engine {
                 AM_CUDA(cudaGraphAddNode(&node, wgraph, nullptr, nullptr, 0, &np));
                 cudaGraph_t body = np.conditional.phGraph_out[0];
                 AM_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-                ChunkDev ch;
-                ch.head = 0;
-                ch.count = chunk;
-                ch.cons = cons.p;
-                ch.eq = eq.p;
-                ch.rec = rec.as<int32_t>();
+                ChunkDev ch = wave_chunk(0, chunk);
                 ch.ctl = ctl();
+                if (classes()) launch_wave_classes(net, reg, ch, st);
                 if (prec == kMixed)
                     launch_compose_tc(net, tcnet, reg, ch, iso, d_err.as<int>(), st);
                 else
@@ -683,7 +769,7 @@ void run_begin(am_engine *e, const RunArgs &a)
         // widest tile: three operand terms (3 x ncols x kp_max x 2 bytes)
         // beside two weight blocks in flight (one if that leaves no room),
         // two accumulators (main + correction) per M tile in 512 TMEM columns
-        const size_t smem_cap = 227u * 1024u;
+        const size_t smem_cap = 227u * 1024u - 2048u; // less the kernels' static shared memory
         // preference: MN-major operand (whole 64-column atoms), two weight
         // stages, then one; then the K-major operand (any 16 columns)
         tc.ncols_max = 0;
@@ -775,6 +861,8 @@ void run_begin(am_engine *e, const RunArgs &a)
     AM_CUDA(cudaMemsetAsync(e->d_tail.p, 0, sizeof(long long), st));
     AM_CUDA(cudaMemsetAsync(e->fp64_counter(), 0, sizeof(unsigned long long), st));
     const int chunk = e->default_chunk();
+    e->ring_min = false;
+    e->rows_from = 0;
     e->ensure_chunk(std::min(chunk, std::max(S, 1024)));
     // the first stores hold the seeds' children of a first wave (a batch
     // member's, or a small network's, grow on demand from there)
@@ -841,11 +929,11 @@ void run_graph_launch(am_engine *e, int max_waves)
         while (w < pending && w < r.chunk) w *= 2;
         wave = (int)std::min<long long>(w, r.chunk);
     }
-    e->ensure_chunk(wave);
     const int count = (int)std::min<long long>(pending, wave);
-    e->ensure_regions(r.tail + (long long)count * kVMax);
-    e->ensure_table(std::max<long long>(r.tail + (long long)count * kVMax, e->cap), true);
+    e->ensure_wave(wave, r.head, r.tail, count, true);
     WaveCtl *h = e->h_ctl;
+    h->rows_from = e->rows_from;
+    memset(h->ccount, 0, sizeof(h->ccount));
     h->head = r.head;
     h->count = count;
     h->waves = 0;
@@ -871,7 +959,7 @@ bool run_graph_done(am_engine *e)
     AM_CHECK(h->waves < kMaxWaves, "wave bound reached");
     r.tail = h->tail;
     r.chunks += h->waves;
-    r.launches += 5ll * h->waves;
+    r.launches += (e->classes() ? 6ll : 5ll) * h->waves;
     r.head = h->head;
     e->num_regions = r.tail;
     if (e->over_limit(r.tail)) return false; // stop: the regions so far stay
@@ -894,19 +982,17 @@ void run_host_loop(am_engine *e)
     cudaEvent_t pa = e->pa, pb = e->pb;
     while (head < tail) {
         const int count = (int)std::min<long long>(tail - head, chunk);
-        e->ensure_chunk(count);
-        e->ensure_regions(tail + (long long)count * kVMax);
-        e->ensure_table(tail + (long long)count * kVMax, true);
-        ChunkDev ch;
-        ch.head = head;
-        ch.count = count;
-        ch.cons = e->cons.p;
-        ch.eq = e->eq.p;
-        ch.rec = e->rec.as<int32_t>();
+        e->ensure_wave(count, head, tail, count, false);
+        const ChunkDev ch = e->wave_chunk(head, count);
         const RegionsDev reg = e->regions();
         const HashDev hs = e->hashdev();
         float ms = 0;
         if (e->phase_timing) AM_CUDA(cudaEventRecord(pa, st));
+        if (e->classes()) {
+            AM_CUDA(cudaMemsetAsync(ch.ccount, 0, sizeof(WaveCtl::ccount), st));
+            launch_wave_classes(net, reg, ch, st);
+            ++launches;
+        }
         if (prec == kMixed)
             launch_compose_tc(net, e->tcnet, reg, ch, iso, e->d_err.as<int>(), st);
         else
@@ -1666,6 +1752,10 @@ int am_region_rows(am_engine *e, int64_t first, int count, double *rows, double 
         cudaStream_t st = e->st;
         if (count == 0) return;
         e->ensure_chunk(count);
+        if (count > e->ring) {
+            AM_CUDA(e->cons.alloc(e->tc * 4 * (size_t)e->ALLP * (size_t)count, st));
+            e->ring = count;
+        }
         ChunkDev ch;
         ch.head = first;
         ch.count = count;

@@ -206,6 +206,7 @@ __device__ void append_one(const AppendArgs &a, int q, long long rid, long long 
         mid[2] = pt[2];
         mid[3] = TS(0);
         a.reg.start[rid] = -1;
+        a.reg.parent[rid] = -1;
     } else {
         const long long parent = head + q / kVMax;
         const int i = q % kVMax;
@@ -222,6 +223,7 @@ __device__ void append_one(const AppendArgs &a, int q, long long rid, long long 
         mid[2] = (v0[2] + v1[2]) / TS(2);
         mid[3] = TS(0);
         a.reg.start[rid] = k;
+        a.reg.parent[rid] = (int32_t)parent;
     }
     a.reg.hash[rid] = h;
     a.reg.nv[rid] = 0;
@@ -256,6 +258,40 @@ __global__ void __launch_bounds__(kScanBlock) append_write_kernel(AppendArgs a)
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *a.tail = base;
 }
 
+// Class of every region of the wave (ChunkDev): class j's list gets the wave
+// position, split[position] the number of leading rows that come from the
+// parent's slot (0 for class 1, whose layer-1 rows are the network's own).
+// The order within a class does not matter: a region's rows do not depend on
+// the tile it is composed in.
+__global__ void wave_classes_kernel(NetDev net, RegionsDev reg, ChunkDev ch)
+{
+    long long head;
+    int count;
+    chunk_range(ch, head, count);
+    const long long rows_from = ch.ctl ? *(volatile const long long *)&ch.ctl->rows_from : ch.rows_from;
+    // a slot that this wave writes holds no parent any more
+    const long long oldest = max(rows_from, head + count - (long long)ch.ring);
+    const int lane = threadIdx.x & 31;
+    const int layers = net.n_lin - 1;
+    for (int r0 = (int)(blockIdx.x * blockDim.x + threadIdx.x) - lane; r0 < count; r0 += (int)(gridDim.x * blockDim.x)) {
+        const int rl = r0 + lane;
+        int c = 0;
+        if (rl < count) {
+            const int par = reg.parent[head + rl], k = reg.start[head + rl];
+            c = 1;
+            if (par >= oldest && par >= 0 && k >= 0)
+                while (c < layers && k >= net.hoff[c + 1]) ++c;
+            ch.split[rl] = c > 1 ? net.hoff[c + 1] : 0;
+        }
+        const unsigned peers = __match_any_sync(0xffffffffu, c);
+        const int first = __ffs(peers) - 1;
+        int base = 0;
+        if (c > 0 && lane == first) base = atomicAdd(ch.ccount + c - 1, __popc(peers));
+        base = __shfl_sync(0xffffffffu, base, first);
+        if (c > 0) ch.order[(size_t)(c - 1) * ch.order_cap + base + __popc(peers & ((1u << lane) - 1u))] = rl;
+    }
+}
+
 // graph-driven loop: retire the wave, take the next one from the queue and
 // go on while it is non-empty, no error bit is set, its children fit and the
 // queue has not outgrown the wave buffers of a batch member
@@ -267,6 +303,7 @@ __global__ void wave_step_kernel(WaveCtl *ctl, cudaGraphConditionalHandle cond)
     const long long rem = c.tail - c.head;
     c.count = (int)(rem < (long long)c.chunk_cap ? (rem > 0 ? rem : 0) : (long long)c.chunk_cap);
     c.work = 0u;
+    for (int i = 0; i < kMaxLayers; ++i) c.ccount[i] = 0;
     const bool go = c.count > 0 && c.err == 0 &&
                     c.tail + (long long)c.count * kVMax <= c.limit && c.waves < c.max_waves &&
                     c.tail <= c.stop_tail && rem <= (long long)c.grow_at;
@@ -370,6 +407,12 @@ void launch_append(int mode, int prec, const NetDev &net, const RegionsDev &reg,
         append_write_kernel<float><<<nb, kScanBlock, 0, st>>>(a);
     else
         append_write_kernel<double><<<nb, kScanBlock, 0, st>>>(a);
+}
+
+void launch_wave_classes(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, cudaStream_t st)
+{
+    const int grid = std::min((ch.count + 255) / 256, 2 * device_sms());
+    if (grid > 0) wave_classes_kernel<<<grid, 256, 0, st>>>(net, reg, ch);
 }
 
 void launch_wave_step(WaveCtl *ctl, cudaGraphConditionalHandle cond, cudaStream_t st)

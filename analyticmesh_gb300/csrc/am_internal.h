@@ -56,6 +56,7 @@ struct RegionsDev {
     uint64_t *hash;     // [cap]
     void *mid;          // [cap][4] TS: seed point / edge midpoint
     int32_t *start;     // [cap] start plane (-1 = seed)
+    int32_t *parent;    // [cap] the region it was entered from (-1 = seed)
     int32_t *nv;        // [cap] polygon vertex count
     int8_t *status;     // [cap]
     void *verts;        // [cap][kVMax][3] TS
@@ -85,6 +86,8 @@ struct WaveCtl {
     int max_waves;      // waves one graph launch may run
     int grow_at;        // stop while more regions than this wait (a batch member's wave buffers grow with its queue)
     long long stop_tail; // stop after the wave that takes tail past this (a region limit)
+    long long rows_from; // regions before this have no rows in the ring (it was reallocated)
+    int ccount[kMaxLayers]; // regions of the wave per class (see ChunkDev)
 };
 
 // the control block's device / pinned allocation: WaveCtl, then the run's
@@ -96,13 +99,28 @@ constexpr int kFp64Slot = kStatsCount;
 constexpr size_t kStatsOff = (sizeof(WaveCtl) + 15) / 16 * 16;
 constexpr size_t kCtlBytes = kStatsOff + (kStatsCount + 1) * sizeof(unsigned long long);
 
+// A wave of regions.  The constraint rows live in a ring: region id r's rows
+// are at slot r % ring until a later wave takes the slot, so that a region
+// finds its parent's rows there.  A region entered through a plane of hidden
+// layer j has its parent's activations in layers 1 .. j - 1 and so its
+// parent's affine maps in layers 1 .. j, bit for bit; only the layers after j
+// are composed (class j), and the rows of the layers up to j come from the
+// parent's slot (the polygon kernel, which reads every row anyway, copies them
+// into the region's own).  Class 1 is composed from layer 1 on: seeds, regions
+// entered through layer 1, and regions whose parent's rows have been overwritten.
 struct ChunkDev {
     long long head;     // first rid of the chunk
     int count;          // regions in the chunk
-    void *cons;         // [count][ALLP][4] TC constraint rows
+    void *cons;         // [ring or count][ALLP][4] TC constraint rows
     void *eq;           // [count][4] TC face plane (b already offset by iso)
     int32_t *rec;       // [count * kVMax] hash slot claimed by each child, -1 none
     WaveCtl *ctl = nullptr; // set: head and count come from the device (graph-driven loop)
+    int ring = 0;       // slots of cons; 0: no ring, rows at the wave position, every region class 1
+    int order_cap = 0;  // wave positions per class list
+    int32_t *order = nullptr;  // [n_lin - 1][order_cap] wave positions by class (class c's list at c - 1)
+    int32_t *split = nullptr;  // [count] leading rows that come from the parent's slot
+    int32_t *ccount = nullptr; // [n_lin - 1] regions per class
+    long long rows_from = 0;   // host-driven loop: WaveCtl::rows_from
 };
 
 #ifdef __CUDACC__
@@ -117,6 +135,12 @@ __device__ __forceinline__ void chunk_range(const ChunkDev &ch, long long &head,
         count = ch.count;
     }
 }
+// slot of a region's rows: of the region at wave position rl, and of region rid
+__device__ __forceinline__ uint32_t row_slot(const ChunkDev &ch, long long head, int rl)
+{
+    return ch.ring ? (uint32_t)(head + rl) % (uint32_t)ch.ring : (uint32_t)rl;
+}
+__device__ __forceinline__ uint32_t ring_slot(const ChunkDev &ch, int rid) { return (uint32_t)rid % (uint32_t)ch.ring; }
 #endif
 
 struct Tolerances {
@@ -146,6 +170,8 @@ void launch_rehash(const RegionsDev &reg, long long n, const HashDev &hs, int *d
 // graph-driven loop: advance ctl to the next wave and set the loop condition
 void launch_region_stats(const int32_t *nv, const int8_t *status, long long n, unsigned long long *out,
                          cudaStream_t st);
+// class lists and splits of a wave (ChunkDev); ccount must be zero
+void launch_wave_classes(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, cudaStream_t st);
 void launch_wave_step(WaveCtl *ctl, cudaGraphConditionalHandle cond, cudaStream_t st);
 int device_sms();
 // the network's parameter buffers, checked for NaN / infinity in one launch

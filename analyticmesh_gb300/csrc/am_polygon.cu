@@ -105,6 +105,17 @@ __device__ __forceinline__ bool warp_solve(const vec4_t<TC> *rows, int a, int b,
     return finite_bits(V[0]) && finite_bits(V[1]) && finite_bits(V[2]);
 }
 
+// |w|^2 with the roundings fixed (not left to the compiler's contraction, which
+// depends on the code around it): the normalised rows decide the walk
+__device__ __forceinline__ float norm2(float x, float y, float z)
+{
+    return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y)));
+}
+__device__ __forceinline__ double norm2(double x, double y, double z)
+{
+    return __fma_rn(z, z, __fma_rn(x, x, __dmul_rn(y, y)));
+}
+
 // L1 distance test |V - P|_1 < eps.  With TS wider than TC it is decided on
 // the scan-precision copies when the rounding margin allows -- Vc and Pc are
 // V and P rounded to nearest, so the TC sum is within 2^-23 (|Vc|_1 + |Pc|_1)
@@ -911,17 +922,27 @@ __global__ void __launch_bounds__(256, 3) polygon_kernel(NetDev net, RegionsDev 
         }
         if (rl >= count) break;
         const long long rid = head + rl;
-        const vec4_t<TC> *grows = reinterpret_cast<const vec4_t<TC> *>((const TC *)ch.cons + (size_t)rl * net.ALLP * 4);
-        // the region's rows into shared memory by one bulk copy (the leader
-        // issues it once every warp of the group is done with the previous
-        // face's rows), then normalised in place
+        // the region's rows into shared memory by bulk copies (the leader
+        // issues them once every warp of the group is done with the previous
+        // face's rows), then normalised in place.  The first nsplit rows come
+        // from the parent's slot; they are the region's own but for the sign
+        // of the plane it was entered through, and are copied into its slot
+        // for its children.
+        vec4_t<TC> *grows = reinterpret_cast<vec4_t<TC> *>((TC *)ch.cons + (size_t)row_slot(ch, head, (int)rl) * net.ALLP * 4);
+        const int nsplit = ch.split ? ch.split[rl] : 0;
+        const int flip = nsplit ? reg.start[rid] : -1;
         {
             const uint32_t rbytes = (uint32_t)ALL * (uint32_t)sizeof(vec4_t<TC>);
             if (!kGroup) __syncwarp(); // (a group has met at its barrier above)
             if (g.gw == 0 && lane == 0) {
                 umma::fence_proxy_async(); // earlier generic reads of the rows before the copy's writes
                 umma::mbar_expect_tx(&g.sh->rbar, rbytes);
-                umma::bulk_g2s(rows, grows, rbytes, &g.sh->rbar);
+                const uint32_t pbytes = (uint32_t)nsplit * (uint32_t)sizeof(vec4_t<TC>);
+                if (nsplit) {
+                    const TC *pr = (const TC *)ch.cons + (size_t)ring_slot(ch, reg.parent[rid]) * net.ALLP * 4;
+                    umma::bulk_g2s(rows, pr, pbytes, &g.sh->rbar);
+                }
+                if (rbytes > pbytes) umma::bulk_g2s(rows + nsplit, grows + nsplit, rbytes - pbytes, &g.sh->rbar);
             }
             if (!umma::mbar_wait(&g.sh->rbar, rphase & 1u, kRowWaitIters)) {
                 atomicOr(err, kErrWait);
@@ -931,7 +952,14 @@ __global__ void __launch_bounds__(256, 3) polygon_kernel(NetDev net, RegionsDev 
         }
         for (int q = 32 * g.gw + lane; q < ALL; q += 32 * G) {
             vec4_t<TC> v = rows[q];
-            const TC n2 = v.x * v.x + v.y * v.y + v.z * v.z;
+            if (q == flip) {
+                v.x = -v.x;
+                v.y = -v.y;
+                v.z = -v.z;
+                v.w = -v.w;
+            }
+            if (q < nsplit) grows[q] = v;
+            const TC n2 = norm2(v.x, v.y, v.z);
             if (n2 > TC(0)) {
                 const TC inv = rsqrt(n2); // as the reference's distance normalisation
                 v.x *= inv;
