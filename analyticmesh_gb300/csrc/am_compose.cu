@@ -4,214 +4,401 @@
 // under the region's activation state and write the sign-flipped constraint
 // rows C_k = (1 - 2 s_k) [w_k | b_k] plus the face plane (w_eq, b_eq - iso).
 // Same mathematics as the reference's fill_constraints + offset_b_equ
-// (backend/inc/process.h:18-203), organised GB300-first: one CTA composes 16
-// regions through every layer, the layer product W_l . diag(s_l) A_l runs as
-// a 64-row x 64-column register-tiled product with the masked operand
-// diag(s_l) A_l = -s_l * C_l staged in shared memory, and skip connections
-// accumulate into the same tile.  Connections into the output layer are
-// composed too (the reference's loop stops before them, process.h:42).
+// (backend/inc/process.h:18-203), organised GB300-first.  Connections into the
+// output layer are composed too (the reference's loop stops before them,
+// process.h:42).
+//
+// One warp owns a region: its lanes hold 32 x RPL output units x 4 columns in
+// registers and walk over the *active* units of the operand only (an inactive
+// unit's column of W meets an all-zero row of X: skipping it changes no bit of
+// the sums, about half the units are inactive, and each region has its own).
+// The weights stream through shared memory once per tile of up to 16 regions: a
+// copy warp brings [32 units x up to 256 rows] blocks into a four-stage ring
+// with bulk copies, and the regions' warps pass through the ring on their own,
+// up to four blocks apart, because their active counts differ (a block barrier
+// per 32 units would cost the slowest of 16 each time).  A warp reads only rows
+// it has written itself (or its parent's), so nothing else is shared.
+//
+// What bounds it: the FMA pipe and the issue slots in fp32 (per active unit
+// 4 RPL FMAs, RPL + 1 shared loads), the FP64 pipe in fp64.  Measured on GB300:
+// see compose_kernel.
 #include <algorithm>
 #include <cuda_runtime.h>
 
 #include "am_device.cuh"
 #include "am_internal.h"
+#include "am_umma.cuh"
 
 namespace am {
 
 namespace {
 
-constexpr int kR = 16;        // regions per CTA
-constexpr int kThreads = 256; // 16 regions x 16 row groups of 4 rows
-constexpr int kKC = 32;       // k rows staged per pass
-constexpr int kRowsPerPass = 64;
+constexpr int kWarps = 16;              // regions per tile at most
+constexpr int kThreads = 32 * kWarps + 32; // + the copy warp
+constexpr int kKC = 32;                 // operand units per block
+constexpr int kStages = 4;
+constexpr int kWait = 1 << 22;
+constexpr int kStageBytes = 32 * 1024;  // kKC units x pass rows
+constexpr int kPadBytes = 2048;         // lanes beyond a pass's last row read past the block's end
 
 template <typename T>
-struct Acc {
-    T v[4][4];
+constexpr int pass_rows() { return kStageBytes / (kKC * (int)sizeof(T)); } // 256 fp32, 128 fp64
+
+template <typename T>
+constexpr size_t compose_smem()
+{
+    return (size_t)kStages * kStageBytes + kPadBytes + (size_t)kWarps * kKC * sizeof(vec4_t<T>);
+}
+
+struct Ring {
+    uint64_t full[kStages], empty[kStages];
+    int abort;
 };
 
-// acc[j][c] += sum_k Wt[k][m0 + j] * X[k][c] for the thread's region, where
-// X = diag(s) rows [src, src+K) of the region's constraint block, negated
-// (C = -A for active units, so s * A = -s * C).
-template <typename T>
-__device__ __forceinline__ void accumulate(vec4_t<T> (*X)[kR], const T *cons, size_t rstride, const int4 *ri, int jend,
-                                           const uint32_t *const *keys, int nreg, int src, int K, const T *Wt, int Mp,
-                                           int m0, Acc<T> &acc)
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+__device__ __forceinline__ bool ring_wait(uint64_t *bar, uint32_t parity, int *err, volatile int *abort)
 {
-    const int tid = threadIdx.x;
-    const int r = tid & (kR - 1);
-    const bool has_w = m0 < Mp;
-    for (int k0 = 0; k0 < K; k0 += kKC) {
-        const int kc = min(kKC, K - k0);
-        __syncthreads();
-        for (int q = tid; q < kKC * kR; q += kThreads) {
-            const int rr = q / kKC, kk = q % kKC;
-            vec4_t<T> x;
-            x.x = x.y = x.z = x.w = T(0);
-            if (kk < kc && rr < nreg) {
-                const int row = src + k0 + kk;
-                if (key_bit(keys[rr], row)) {
-                    const vec4_t<T> c = tile_row<T>(cons, rstride, ri[rr], row, jend);
-                    x.x = -c.x;
-                    x.y = -c.y;
-                    x.z = -c.z;
-                    x.w = -c.w;
-                }
-            }
-            X[kk][rr] = x;
-        }
-        __syncthreads();
-        if (has_w) {
-            const T *wp = Wt + (size_t)k0 * Mp + m0;
-#pragma unroll 4
-            for (int kk = 0; kk < kc; ++kk) {
-                const vec4_t<T> x = X[kk][r];
-                const vec4_t<T> w = ld4<T>(wp + (size_t)kk * Mp);
-                const T wj[4] = {w.x, w.y, w.z, w.w};
+    if (*abort) return false;
+    if (umma::mbar_wait(bar, parity, kWait)) return true;
+    if (err) atomicOr(err, kErrWait);
+    *abort = 1;
+    return false;
+}
+
+// The products of linear i: job 0 is the linear on hidden layer i, the others
+// its transforms from earlier hidden layers.
+struct Job {
+    const void *wt;
+    int Mp, src;
+};
+__device__ __forceinline__ int jobs_of(const NetDev &net, int i)
+{
+    int n = 1;
+    for (int s = 0; s < net.nskip[i]; ++s) n += net.skip[i][s].kind == 1 && net.skip[i][s].from >= 1;
+    return n;
+}
+__device__ __forceinline__ Job job_of(const NetDev &net, int i, int job)
+{
+    if (job > 0)
+        for (int s = 0, q = 0; s < net.nskip[i]; ++s)
+            if (net.skip[i][s].kind == 1 && net.skip[i][s].from >= 1 && ++q == job)
+                return Job{net.skip[i][s].tmt, net.skip[i][s].Mp, net.skip[i][s].from};
+    return Job{net.Wt[i], net.Mp[i], i};
+}
+
+// (the copy warp) the weight blocks of every tile of the CTA, in the order the
+// regions' warps consume them
+template <typename T>
+__device__ void produce(const NetDev &net, const WavePlan &plan, int rounds, unsigned char *ws, Ring &ring, int *err)
+{
+    const int lane = threadIdx.x & 31;
+    volatile int *abort = &ring.abort;
+    int h = 0;
+    int last[kStages]; // (lane 0's view, the same in every lane) the last block copied into each stage
+    for (int s = 0; s < kStages; ++s) last[s] = -1;
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+        if (t < 0) continue;
+        for (int i = plan_class(plan, t); i < net.n_lin; ++i)
+            for (int mb = 0; mb < net.nodes[i + 1]; mb += pass_rows<T>())
+                for (int job = 0, nj = jobs_of(net, i); job < nj; ++job) {
+                    const Job jb = job_of(net, i, job);
+                    const int K = net.nodes[jb.src], ld = min(pass_rows<T>(), jb.Mp - mb);
+                    for (int k0 = 0; k0 < K; k0 += kKC, ++h) {
+                        const int s = h % kStages;
+                        int go = 1;
+                        if (lane == 0)
+                            go = h < kStages || ring_wait(ring.empty + s, (uint32_t)(h / kStages - 1) & 1u, err, abort);
+                        if (!__shfl_sync(0xffffffffu, go, 0)) continue;
+                        const int kc = min(kKC, K - k0);
+                        const uint32_t row = (uint32_t)(ld * sizeof(T));
+                        const T *src = (const T *)jb.wt + (size_t)k0 * jb.Mp + mb;
+                        unsigned char *dst = ws + (size_t)s * kStageBytes;
+                        if (lane == 0) umma::mbar_expect_tx(ring.full + s, row * (uint32_t)kc);
+                        __syncwarp();
+                        if (ld == jb.Mp) { // whole rows of W^T: one contiguous run
+                            if (lane == 0) umma::bulk_g2s(dst, src, row * (uint32_t)kc, ring.full + s);
+                        } else if (lane < kc) {
+                            umma::bulk_g2s(dst + (size_t)lane * row, src + (size_t)lane * jb.Mp, row, ring.full + s);
+                        }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc.v[j][0] += wj[j] * x.x;
-                    acc.v[j][1] += wj[j] * x.y;
-                    acc.v[j][2] += wj[j] * x.z;
-                    acc.v[j][3] += wj[j] * x.w;
+                        for (int q = 0; q < kStages; ++q)
+                            if (q == s) last[q] = h;
+                    }
+                }
+    }
+    // nothing lands in shared memory after the CTA has left (bounded)
+    if (lane == 0)
+#pragma unroll
+        for (int s = 0; s < kStages; ++s)
+            if (last[s] >= 0) umma::mbar_wait(ring.full + s, (uint32_t)(last[s] / kStages) & 1u, kWait);
+    __syncwarp();
+}
+
+// A region's state in its warp.
+template <typename T>
+struct Region {
+    T *cons;
+    size_t rstride;
+    int4 ri;
+    int jend, lane;
+    const uint32_t *key;
+    vec4_t<T> *xs; // the warp's operand block
+    bool dense;
+};
+
+// one pass (32 RPL units of linear i from mb on) over every job's blocks
+template <typename T, int RPL>
+__device__ void pass(const NetDev &net, int i, int mb, const Region<T> &g, const unsigned char *ws, Ring &ring, int &h,
+                     int *err, T acc[RPL][4])
+{
+    volatile int *abort = &ring.abort;
+    for (int job = 0, nj = jobs_of(net, i); job < nj; ++job) {
+        const Job jb = job_of(net, i, job);
+        const int K = net.nodes[jb.src], rows0 = net.hoff[jb.src], ld = min(pass_rows<T>(), jb.Mp - mb);
+        const T *src = g.cons + (size_t)(uint32_t)(rows0 < g.jend ? g.ri.y : g.ri.x) * g.rstride + (size_t)rows0 * 4;
+        auto load = [&](int k0, bool &on) {
+            const int k = k0 + g.lane;
+            on = k < K && key_bit(g.key, rows0 + k);
+            vec4_t<T> c;
+            c.x = c.y = c.z = c.w = T(0);
+            if (on) c = ld4<T>(src + (size_t)k * 4);
+            return c;
+        };
+        bool on;
+        vec4_t<T> c = load(0, on);
+        for (int k0 = 0; k0 < K; k0 += kKC, ++h) {
+            const T sg = rows0 + k0 + g.lane == g.ri.z ? T(1) : T(-1); // (C = -A where active)
+            vec4_t<T> x;
+            x.x = sg * c.x;
+            x.y = sg * c.y;
+            x.z = sg * c.z;
+            x.w = sg * c.w;
+            unsigned mask = __ballot_sync(0xffffffffu, on);
+            if (g.dense) {
+                mask = K - k0 >= 32 ? 0xffffffffu : (1u << (K - k0)) - 1u;
+                if (!on) x.x = x.y = x.z = x.w = T(0);
+            }
+            g.xs[g.lane] = x;
+            __syncwarp();
+            if (k0 + kKC < K) c = load(k0 + kKC, on);
+            const int s = h % kStages;
+            // (the warp decides as one: after an abort nobody reads the ring)
+            const bool ok = __all_sync(0xffffffffu, ring_wait(ring.full + s, (uint32_t)(h / kStages) & 1u, err, abort));
+            if (ok) {
+                const T *w = reinterpret_cast<const T *>(ws + (size_t)s * kStageBytes) + g.lane;
+                while (mask) { // two active units at a time, in order
+                    const int ka = __ffs(mask) - 1;
+                    mask &= mask - 1u;
+                    const int kb = mask ? __ffs(mask) - 1 : -1;
+                    const vec4_t<T> xa = g.xs[ka];
+                    T wa[RPL];
+#pragma unroll
+                    for (int j = 0; j < RPL; ++j) wa[j] = w[ka * ld + 32 * j];
+                    if (kb >= 0) {
+                        mask &= mask - 1u;
+                        const vec4_t<T> xb = g.xs[kb];
+                        T wb[RPL];
+#pragma unroll
+                        for (int j = 0; j < RPL; ++j) wb[j] = w[kb * ld + 32 * j];
+#pragma unroll
+                        for (int j = 0; j < RPL; ++j) {
+                            acc[j][0] = fma_t(wa[j], xa.x, acc[j][0]);
+                            acc[j][1] = fma_t(wa[j], xa.y, acc[j][1]);
+                            acc[j][2] = fma_t(wa[j], xa.z, acc[j][2]);
+                            acc[j][3] = fma_t(wa[j], xa.w, acc[j][3]);
+                        }
+#pragma unroll
+                        for (int j = 0; j < RPL; ++j) {
+                            acc[j][0] = fma_t(wb[j], xb.x, acc[j][0]);
+                            acc[j][1] = fma_t(wb[j], xb.y, acc[j][1]);
+                            acc[j][2] = fma_t(wb[j], xb.z, acc[j][2]);
+                            acc[j][3] = fma_t(wb[j], xb.w, acc[j][3]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < RPL; ++j) {
+                            acc[j][0] = fma_t(wa[j], xa.x, acc[j][0]);
+                            acc[j][1] = fma_t(wa[j], xa.y, acc[j][1]);
+                            acc[j][2] = fma_t(wa[j], xa.z, acc[j][2]);
+                            acc[j][3] = fma_t(wa[j], xa.w, acc[j][3]);
+                        }
+                    }
                 }
             }
+            __syncwarp();
+            if (g.lane == 0) umma::mbar_arrive(ring.empty + s);
         }
     }
 }
 
+// bias, connections without a product (identities, the input), the output
 template <typename T>
-__global__ void __launch_bounds__(kThreads) compose_kernel(NetDev net, RegionsDev reg, ChunkDev ch, T iso)
+__device__ __forceinline__ void store_unit(const NetDev &net, int i, int m, const Region<T> &g, const T *acc, T iso,
+                                           T *eq)
 {
-    __shared__ vec4_t<T> X[kKC][kR];
+    T v[4] = {acc[0], acc[1], acc[2], acc[3] + ((const T *)net.bias[i])[m]};
+    for (int s = 0; s < net.nskip[i]; ++s) {
+        const SkipDev &sk = net.skip[i][s];
+        if (sk.kind == 0) {
+            if (sk.from == 0) {
+                if (m < 3) v[m] += T(1);
+            } else {
+                const int row = net.hoff[sk.from] + m;
+                if (key_bit(g.key, row)) {
+                    const vec4_t<T> c = tile_row<T>(g.cons, g.rstride, g.ri, row, g.jend);
+                    v[0] -= c.x;
+                    v[1] -= c.y;
+                    v[2] -= c.z;
+                    v[3] -= c.w;
+                }
+            }
+        } else if (sk.from == 0) {
+            const T *tt = (const T *)sk.tmt; // [3][Mp]
+            v[0] += tt[m];
+            v[1] += tt[(size_t)sk.Mp + m];
+            v[2] += tt[2 * (size_t)sk.Mp + m];
+        }
+    }
+    vec4_t<T> o;
+    if (i < net.n_lin - 1) {
+        const int row = net.hoff[i + 1] + m;
+        const T sg = key_bit(g.key, row) ? T(-1) : T(1);
+        o.x = sg * v[0];
+        o.y = sg * v[1];
+        o.z = sg * v[2];
+        o.w = sg * v[3];
+        st4<T>(g.cons + (size_t)(uint32_t)g.ri.x * g.rstride + (size_t)row * 4, o);
+    } else {
+        o.x = v[0];
+        o.y = v[1];
+        o.z = v[2];
+        o.w = v[3] - iso;
+        st4<T>(eq, o);
+    }
+}
+
+template <typename T, int RPL>
+__device__ void linear_pass(const NetDev &net, int i, int mb, const Region<T> &g, const unsigned char *ws, Ring &ring,
+                            int &h, int *err, T iso, T *eq)
+{
+    T acc[RPL][4];
+#pragma unroll
+    for (int j = 0; j < RPL; ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[j][c] = T(0);
+    pass<T, RPL>(net, i, mb, g, ws, ring, h, err, acc);
+#pragma unroll
+    for (int j = 0; j < RPL; ++j) {
+        const int m = mb + 32 * j + g.lane;
+        if (m < net.nodes[i + 1]) store_unit<T>(net, i, m, g, acc[j], iso, eq);
+    }
+}
+
+// Measured on GB300, composition of all 265 K regions of 3-[128]x4-1 in waves of
+// 7 K (parents' rows on both sides): fp32 3.1 ms, fp64 33 ms; a 16-region x
+// 64-row register tile per CTA over every unit, operand staged behind two block
+// barriers per 32 units, took 6.6 and 71 ms.  8,192 given states, every layer
+// (weights transposed and keys packed in the same call): 131 us against 238.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 1) compose_kernel(NetDev net, RegionsDev reg, ChunkDev ch, T iso,
+                                                              const int *nonfinite, int *err)
+{
+    extern __shared__ __align__(128) unsigned char ws[]; // the weight ring, then the warps' operand blocks
+    __shared__ Ring ring;
     __shared__ WavePlan plan;
-    __shared__ int4 ri[kR];
-    __shared__ const uint32_t *keys[kR];
-    const int tid = threadIdx.x;
-    const int r = tid & (kR - 1);
-    const int g = tid >> 4;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     long long head;
     int count;
     chunk_range(ch, head, count);
-    const size_t rstride = (size_t)net.ALLP * 4;
-    T *cons = (T *)ch.cons;
+    if (count <= 0) return;
     if (tid == 0) {
+        // as few regions per tile as fill the grid: a small wave spreads over every SM
         plan_counts(plan, ch, net.n_lin - 1, count);
-        plan_finish(plan, kR);
+        int R = min(kWarps, (count + (int)gridDim.x - 1) / (int)gridDim.x);
+        while (R < kWarps && plan_tiles(plan, R) > (int)gridDim.x) ++R;
+        plan_finish(plan, R);
+        ring.abort = 0;
+        for (int s = 0; s < kStages; ++s) {
+            umma::mbar_init(ring.full + s, 1);
+            umma::mbar_init(ring.empty + s, kWarps);
+        }
+        umma::fence_mbar_init();
     }
     __syncthreads();
     const int rounds = plan_rounds(plan, (int)gridDim.x);
+    if (warp == kWarps) {
+        produce<T>(net, plan, rounds, ws, ring, err);
+        return;
+    }
+    Region<T> g;
+    g.cons = (T *)ch.cons;
+    g.rstride = (size_t)net.ALLP * 4;
+    g.lane = lane;
+    g.xs = reinterpret_cast<vec4_t<T> *>(ws + (size_t)kStages * kStageBytes + kPadBytes) + warp * kKC;
+    // a weight that is not finite meets the zeros of inactive units too (NaN,
+    // as in a dense product): then no unit is skipped
+    g.dense = nonfinite && *nonfinite != 0;
+    int h = 0;
     for (int rd = 0; rd < rounds; ++rd) {
         const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
         if (t < 0) continue;
         const int cls = plan_class(plan, t);
-        const int jend = cls > 1 ? net.hoff[cls + 1] : 0;
-        const int nreg = tile_nreg(plan, t, cls);
-        __syncthreads(); // the previous tile is done with ri, keys
-        if (tid < nreg) {
-            ri[tid] = tile_region(plan, reg, ch, head, t, cls, tid);
-            keys[tid] = reg.keys + (size_t)(head + ri[tid].w) * net.W;
+        const bool live = warp < tile_nreg(plan, t, cls);
+        if (!live) { // no region for this warp: it gives its share of every block back
+            for (int i = cls; i < net.n_lin; ++i)
+                for (int mb = 0; mb < net.nodes[i + 1]; mb += pass_rows<T>())
+                    for (int job = 0, nj = jobs_of(net, i); job < nj; ++job)
+                        for (int k0 = 0, K = net.nodes[job_of(net, i, job).src]; k0 < K; k0 += kKC, ++h) {
+                            const int s = h % kStages;
+                            __all_sync(0xffffffffu, ring_wait(ring.full + s, (uint32_t)(h / kStages) & 1u, err, &ring.abort));
+                            if (lane == 0) umma::mbar_arrive(ring.empty + s);
+                        }
+            continue;
         }
-        __syncthreads();
-
+        g.ri = tile_region(plan, reg, ch, head, t, cls, warp);
+        g.jend = cls > 1 ? net.hoff[cls + 1] : 0;
+        g.key = reg.keys + (size_t)(head + g.ri.w) * net.W;
+        T *own = g.cons + (size_t)(uint32_t)g.ri.x * g.rstride;
+        T *eq = (T *)ch.eq + (size_t)g.ri.w * 4;
         // class 1: hidden layer 1 = linear 0 rows, sign-flipped; extra constraints as given
-        {
+        if (cls == 1) {
             const T *W0 = (const T *)net.W0;
             const T *b0 = (const T *)net.bias[0];
-            const int n1 = cls == 1 ? net.nodes[1] : 0;
-            for (int q = tid; q < nreg * n1; q += kThreads) {
-                const int rr = q / n1, m = q % n1;
-                const T sg = key_bit(keys[rr], m) ? T(-1) : T(1);
+            for (int m = lane; m < net.nodes[1]; m += 32) {
+                const T sg = key_bit(g.key, m) ? T(-1) : T(1);
                 vec4_t<T> c;
                 c.x = sg * W0[3 * m + 0];
                 c.y = sg * W0[3 * m + 1];
                 c.z = sg * W0[3 * m + 2];
                 c.w = sg * b0[m];
-                st4<T>(cons + (size_t)ri[rr].x * rstride + (size_t)m * 4, c);
-            }
-            const T *we = (const T *)net.w_extra;
-            const T *be = (const T *)net.b_extra;
-            for (int q = tid; q < nreg * net.E; q += kThreads) {
-                const int rr = q / net.E, e = q % net.E;
-                vec4_t<T> c;
-                c.x = we[3 * e + 0];
-                c.y = we[3 * e + 1];
-                c.z = we[3 * e + 2];
-                c.w = be[e];
-                st4<T>(cons + (size_t)ri[rr].x * rstride + (size_t)(net.N + e) * 4, c);
+                st4<T>(own + (size_t)m * 4, c);
             }
         }
-
+        const T *we = (const T *)net.w_extra;
+        const T *be = (const T *)net.b_extra;
+        for (int e = lane; e < net.E; e += 32) {
+            vec4_t<T> c;
+            c.x = we[3 * e + 0];
+            c.y = we[3 * e + 1];
+            c.z = we[3 * e + 2];
+            c.w = be[e];
+            st4<T>(own + (size_t)(net.N + e) * 4, c);
+        }
+        __syncwarp(); // the rows written above are other lanes' operand
         for (int i = cls; i < net.n_lin; ++i) {
-            const int M = net.nodes[i + 1];
-            const int K = net.nodes[i];
-            const bool last = (i == net.n_lin - 1);
-            const T *bias = (const T *)net.bias[i];
-            for (int mb = 0; mb < M; mb += kRowsPerPass) {
-                const int m0 = mb + 4 * g;
-                Acc<T> acc;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc.v[j][c] = T(0);
-                accumulate<T>(X, cons, rstride, ri, jend, keys, nreg, net.hoff[i], K, (const T *)net.Wt[i], net.Mp[i], m0,
-                              acc);
-                for (int s = 0; s < net.nskip[i]; ++s) {
-                    const SkipDev &sk = net.skip[i][s];
-                    if (sk.kind == 1 && sk.from >= 1)
-                        accumulate<T>(X, cons, rstride, ri, jend, keys, nreg, net.hoff[sk.from], net.nodes[sk.from],
-                                      (const T *)sk.tmt, sk.Mp, m0, acc);
-                }
-                if (r < nreg) {
-                    const uint32_t *key = keys[r];
-                    T *cr = cons + (size_t)ri[r].x * rstride;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int m = m0 + j;
-                        if (m >= M) continue;
-                        T v[4] = {acc.v[j][0], acc.v[j][1], acc.v[j][2], acc.v[j][3] + bias[m]};
-                        for (int s = 0; s < net.nskip[i]; ++s) {
-                            const SkipDev &sk = net.skip[i][s];
-                            if (sk.kind == 0) {
-                                if (sk.from == 0) {
-                                    if (m < 3) v[m] += T(1);
-                                } else {
-                                    const int row = net.hoff[sk.from] + m;
-                                    if (key_bit(key, row)) {
-                                        const vec4_t<T> c = tile_row<T>(cons, rstride, ri[r], row, jend);
-                                        v[0] -= c.x;
-                                        v[1] -= c.y;
-                                        v[2] -= c.z;
-                                        v[3] -= c.w;
-                                    }
-                                }
-                            } else if (sk.from == 0) {
-                                const T *tt = (const T *)sk.tmt; // [3][Mp]
-                                v[0] += tt[m];
-                                v[1] += tt[(size_t)sk.Mp + m];
-                                v[2] += tt[2 * (size_t)sk.Mp + m];
-                            }
-                        }
-                        vec4_t<T> o;
-                        if (!last) {
-                            const int row = net.hoff[i + 1] + m;
-                            const T sg = key_bit(key, row) ? T(-1) : T(1);
-                            o.x = sg * v[0];
-                            o.y = sg * v[1];
-                            o.z = sg * v[2];
-                            o.w = sg * v[3];
-                            st4<T>(cr + (size_t)row * 4, o);
-                        } else {
-                            o.x = v[0];
-                            o.y = v[1];
-                            o.z = v[2];
-                            o.w = v[3] - iso;
-                            st4<T>((T *)ch.eq + (size_t)ri[r].w * 4, o);
-                        }
-                    }
-                }
+            for (int mb = 0; mb < net.nodes[i + 1]; mb += pass_rows<T>()) {
+                const int n = (min(pass_rows<T>(), net.nodes[i + 1] - mb) + 31) / 32;
+                if (n <= 1) linear_pass<T, 1>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                else if (n <= 2) linear_pass<T, 2>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                else if (n <= 3) linear_pass<T, 3>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                else if (n <= 4 || sizeof(T) == 8) linear_pass<T, 4>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                else if (n <= 6) linear_pass<T, sizeof(T) == 4 ? 6 : 4>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                else linear_pass<T, sizeof(T) == 4 ? 8 : 4>(net, i, mb, g, ws, ring, h, err, iso, eq);
             }
-            __syncthreads(); // layer i+1 rows written by this CTA become the next operand
+            __syncwarp(); // layer i + 1's rows become the next operand
         }
     }
 }
@@ -225,6 +412,22 @@ __global__ void prepare_weights_kernel(const T *src, int M, int K, int Mp, T *ds
         const int k = (int)(q / Mp), m = (int)(q % Mp);
         dst[q] = m < M ? src[(size_t)m * K + k] : T(0);
     }
+}
+
+// the same for every listed linear in one launch (blockIdx.y); *nonfinite set
+// where a value is not finite
+__global__ void prepare_list_kernel(PrepareList list, int *nonfinite)
+{
+    const PrepareList::Item &it = list.item[blockIdx.y];
+    const int n = it.K * it.Mp;
+    bool bad = false;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        const int k = q / it.Mp, m = q % it.Mp;
+        const float v = m < it.M ? it.src[(size_t)m * it.K + k] : 0.f;
+        bad |= !isfinite(v);
+        it.dst[q] = v;
+    }
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(nonfinite, 1);
 }
 
 // every value of the listed buffers finite; kErrNonFinite otherwise
@@ -253,15 +456,28 @@ void launch_check_finite(int prec, const FiniteList &list, int *d_err, cudaStrea
         check_finite_kernel<float><<<grid, 256, 0, st>>>(list, d_err);
 }
 
-void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso, cudaStream_t st)
+template <typename T>
+static void launch_one(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, T iso, const int *nonfinite,
+                       int *d_err, cudaStream_t st)
+{
+    cudaFuncSetAttribute(compose_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)compose_smem<T>());
+    const int grid = ch.ctl ? device_sms() : std::min(device_sms(), ch.count);
+    compose_kernel<T><<<grid, kThreads, compose_smem<T>(), st>>>(net, reg, ch, iso, nonfinite, d_err);
+}
+
+void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso, int *d_err,
+                    cudaStream_t st, const int *nonfinite)
 {
     if (!ch.ctl && ch.count <= 0) return;
-    int grid = device_sms() * 4;
-    if (!ch.ctl) grid = std::min(grid, (ch.count + kR - 1) / kR + (ch.order ? net.n_lin : 0));
     if (prec == kFloat64)
-        compose_kernel<double><<<grid, kThreads, 0, st>>>(net, reg, ch, iso);
+        launch_one<double>(net, reg, ch, iso, nonfinite, d_err, st);
     else
-        compose_kernel<float><<<grid, kThreads, 0, st>>>(net, reg, ch, (float)iso);
+        launch_one<float>(net, reg, ch, (float)iso, nonfinite, d_err, st);
+}
+
+void launch_prepare_list(const PrepareList &list, int *nonfinite, cudaStream_t st)
+{
+    if (list.count > 0) prepare_list_kernel<<<dim3(64, (unsigned)list.count), 256, 0, st>>>(list, nonfinite);
 }
 
 void launch_prepare_weights(int prec, const void *src, int M, int K, int Mp, void *dst, cudaStream_t st)

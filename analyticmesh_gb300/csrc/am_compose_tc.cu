@@ -727,11 +727,6 @@ __device__ const TcMat &job_mat(const NetDev &net, const TcNet &tc, int i, int j
 
 __device__ __forceinline__ void bar_builders() { asm volatile("bar.sync 1, %0;" ::"r"(kSBuild) : "memory"); }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_addr(bar)) : "memory");
-}
-
 // Bounded wait of the streamed kernel: false at once when the CTA is
 // aborting, and false -- with the error bit kErrWait and the abort flag set --
 // when the wait runs out.  An aborting CTA keeps its arrive / commit / barrier
@@ -1156,7 +1151,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                             }
                         }
                         umma::fence_proxy_async(); // generic-proxy stores -> the tensor cores
-                        mbar_arrive(xfull + xs);
+                        umma::mbar_arrive(xfull + xs);
                         ++xb;
                         if (t < nd) {
                             store_block(def_first + t);

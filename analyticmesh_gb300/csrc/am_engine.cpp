@@ -550,7 +550,7 @@ struct am_engine {
                 if (prec == kMixed)
                     launch_compose_tc(net, tcnet, reg, ch, iso, d_err.as<int>(), st);
                 else
-                    launch_compose(prec, net, reg, ch, iso, st);
+                    launch_compose(prec, net, reg, ch, iso, d_err.as<int>(), st);
                 launch_polygon(prec, net, reg, ch, hs, tol, face_warps, prune, fp64_counter(), d_err.as<int>(), st);
                 launch_append(0, prec, net, reg, ch, hs, nullptr, nullptr, nullptr, chunk * kVMax,
                               d_tail.as<long long>(), blocksum.as<int>(), (int)(blocksum.bytes / sizeof(int)),
@@ -996,7 +996,7 @@ void run_host_loop(am_engine *e)
         if (prec == kMixed)
             launch_compose_tc(net, e->tcnet, reg, ch, iso, e->d_err.as<int>(), st);
         else
-            launch_compose(prec, net, reg, ch, iso, st);
+            launch_compose(prec, net, reg, ch, iso, e->d_err.as<int>(), st);
         if (e->phase_timing) {
             AM_CUDA(cudaEventRecord(pb, st));
             AM_CUDA(cudaEventSynchronize(pb));
@@ -1489,7 +1489,7 @@ int am_error_report(am_engine *e, int64_t sample_regions, am_error_report_t *out
             ch.cons = e->v_rows.p;
             ch.eq = e->v_eq.p;
             ch.rec = nullptr;
-            launch_compose(kFloat64, n64, rr, ch, e->iso, st);
+            launch_compose(kFloat64, n64, rr, ch, e->iso, e->d_err.as<int>(), st);
             launch_verify((int)e->ts, reg, dids, cnt, e->v_rows.as<double>(), e->v_eq.as<double>(), e->ALLP, e->ALL,
                           e->v_out.as<unsigned long long>(), st);
             AM_CUDA(cudaGetLastError());
@@ -1766,7 +1766,7 @@ int am_region_rows(am_engine *e, int64_t first, int count, double *rows, double 
         if (e->prec == kMixed)
             launch_compose_tc(e->net, e->tcnet, e->regions(), ch, e->iso, e->d_err.as<int>(), st);
         else
-            launch_compose(e->prec, e->net, e->regions(), ch, e->iso, st);
+            launch_compose(e->prec, e->net, e->regions(), ch, e->iso, e->d_err.as<int>(), st);
         AM_CUDA(cudaGetLastError());
         const size_t nrow = (size_t)count * e->ALLP * 4;
         std::vector<unsigned char> rb(nrow * e->tc), eb((size_t)count * 4 * e->tc);

@@ -60,21 +60,33 @@ __device__ int block_exclusive_scan(int v, int *total)
     return before + x - v;
 }
 
-__global__ void seed_pack_kernel(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash)
+// a warp per state: a word is one coalesced 32-byte read and a ballot (a thread
+// per state read bytes N apart from its neighbours')
+__global__ void seed_pack_kernel(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, int *zeroed)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (zeroed && blockIdx.x == 0 && threadIdx.x == 0) *zeroed = 0;
+    const int lane = threadIdx.x & 31;
+    const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (s >= S) return;
     const uint8_t *row = states + (size_t)s * N;
     uint64_t h = 0;
-    for (int w = 0; w < W; ++w) {
-        uint32_t word = 0;
-        const int lim = min(32, N - 32 * w);
-        for (int b = 0; b < lim; ++b)
-            if (row[32 * w + b]) word |= 1u << b;
-        keys[(size_t)s * W + w] = word;
-        h += word_term(word, w);
+    for (int w0 = 0; w0 < W; w0 += 32) {
+        uint32_t mine = 0;
+#pragma unroll 8
+        for (int u = 0; u < 32; ++u) {
+            if (w0 + u >= W) break;
+            const int q = 32 * (w0 + u) + lane;
+            const uint32_t word = __ballot_sync(0xffffffffu, q < N && row[q] != 0);
+            if (lane == u) mine = word;
+        }
+        if (w0 + lane < W) {
+            keys[(size_t)s * W + w0 + lane] = mine;
+            h += word_term(mine, w0 + lane);
+        }
     }
-    hash[s] = h;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+    if (lane == 0) hash[s] = h;
 }
 
 __global__ void seed_insert_kernel(const uint32_t *keys, const uint64_t *hash, int S, int W, HashDev hs, int32_t *rec,
@@ -361,10 +373,11 @@ __global__ void rehash_kernel(RegionsDev reg, long long n, HashDev hs, int *err)
 
 } // namespace
 
-void launch_seed_pack(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, cudaStream_t st)
+void launch_seed_pack(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, cudaStream_t st,
+                      int *zeroed)
 {
     if (S <= 0) return;
-    seed_pack_kernel<<<(S + 127) / 128, 128, 0, st>>>(states, S, N, W, keys, hash);
+    seed_pack_kernel<<<(S + 7) / 8, 256, 0, st>>>(states, S, N, W, keys, hash, zeroed);
 }
 
 void launch_seed_insert(const uint32_t *keys, const uint64_t *hash, int S, int W, const HashDev &hs, int32_t *rec,

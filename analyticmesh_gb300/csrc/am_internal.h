@@ -150,8 +150,9 @@ struct Tolerances {
 };
 
 // launchers (stream-ordered, no synchronisation)
-void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso,
-                    cudaStream_t st);
+// nonfinite: device flag, non-zero when a weight may not be finite (null: all are)
+void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso, int *d_err,
+                    cudaStream_t st, const int *nonfinite = nullptr);
 // prune: 1 = the walk scans only the rows that can bound the face (see
 // prune_rows), 0 = every row (the same faces)
 // nfp64: counts the faces the mixed form walks again with FP64 predicates
@@ -159,7 +160,9 @@ void launch_polygon(int prec, const NetDev &net, const RegionsDev &reg, const Ch
                     const Tolerances &tol, int face_warps, int prune, unsigned long long *nfp64, int *d_err,
                     cudaStream_t st);
 int polygon_face_warps(int prec, int ALLP);
-void launch_seed_pack(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, cudaStream_t st);
+// zeroed: an int set to zero as well (optional)
+void launch_seed_pack(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, cudaStream_t st,
+                      int *zeroed = nullptr);
 void launch_seed_insert(const uint32_t *keys, const uint64_t *hash, int S, int W, const HashDev &hs, int32_t *rec,
                         int *d_err, cudaStream_t st);
 // flags + scan + append.  mode 0: children of a chunk, mode 1: seeds.
@@ -181,6 +184,15 @@ struct FiniteList {
     int count;
 };
 void launch_check_finite(int prec, const FiniteList &list, int *d_err, cudaStream_t st);
+struct PrepareList { // FP32 linears to transpose and pad
+    struct Item {
+        const float *src;
+        float *dst;
+        int M, K, Mp;
+    } item[kMaxLayers];
+    int count;
+};
+void launch_prepare_list(const PrepareList &list, int *nonfinite, cudaStream_t st);
 void launch_prepare_weights(int prec, const void *src, int M, int K, int Mp, void *dst, cudaStream_t st);
 
 // error report (am_verify.cu): out[0] max |f(v)| bits, out[1] max vertex

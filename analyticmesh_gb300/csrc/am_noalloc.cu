@@ -38,7 +38,8 @@ namespace am {
 namespace {
 
 constexpr size_t kScratchBytes = size_t(8) << 20;
-static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
+// (and, behind it, a flag: a weight that is not finite)
+static __device__ __align__(256) unsigned char g_scratch[kScratchBytes + 256];
 
 constexpr int kMaxDevices = 64;
 void *g_scratch_addr[kMaxDevices] = {};
@@ -116,15 +117,19 @@ extern "C" int am_compose_rows_noalloc(const int32_t *nodesnum, int num_nodes, c
     for (int h = 1; h < n_lin; ++h) net.hoff[h + 1] = net.hoff[h] + nodesnum[h];
     net.W0 = weights[0];
     for (int i = 0; i < n_lin; ++i) net.bias[i] = biases[i];
+    PrepareList prep;
+    prep.count = 0;
     for (int i = 1; i < n_lin; ++i) {
         const int M = nodesnum[i + 1], K = nodesnum[i], Mp = (M + 3) / 4 * 4;
-        launch_prepare_weights(kFloat32, weights[i], M, K, Mp, scratch + off[i], st);
+        prep.item[prep.count++] = {weights[i], (float *)(scratch + off[i]), M, K, Mp};
         net.Wt[i] = scratch + off[i];
         net.Mp[i] = Mp;
     }
     uint32_t *keys = (uint32_t *)(scratch + keys_off);
     uint64_t *hash = (uint64_t *)(scratch + hash_off);
-    launch_seed_pack(states, count, N, W, keys, hash, st);
+    int *nonfinite = (int *)(scratch + kScratchBytes);
+    launch_seed_pack(states, count, N, W, keys, hash, st, nonfinite);
+    launch_prepare_list(prep, nonfinite, st);
 
     RegionsDev reg;
     memset(&reg, 0, sizeof(reg));
@@ -137,7 +142,7 @@ extern "C" int am_compose_rows_noalloc(const int32_t *nodesnum, int num_nodes, c
     ch.cons = rows;
     ch.eq = eq;
     ch.rec = nullptr;
-    launch_compose(kFloat32, net, reg, ch, iso, st);
+    launch_compose(kFloat32, net, reg, ch, iso, nullptr, st, nonfinite);
     // nothing was pending at entry: an error now comes from these launches
     return cudaGetLastError() == cudaSuccess ? AM_OK : AM_ERR_CUDA;
 }
