@@ -206,7 +206,7 @@ struct am_engine {
     DevBuf tc_lin[kMaxLayers], tc_skip[kMaxLayers][kMaxSkips];
     TcNet tcnet{};
     // regions
-    DevBuf keys, hash, mid, start, parent, nv, status, verts, edges;
+    DevBuf keys, hash, mid, start, parent, reach, nv, status, verts, edges;
     long long cap = 0;
     DevBuf table;
     unsigned long long hcap = 0;
@@ -245,10 +245,9 @@ struct am_engine {
     bool lean = false; // batch member: region store and table start small and grow on demand
     long long max_regions = 0; // AM_OPT_MAX_REGIONS (0: no limit)
     int compose_tile = 0;      // AM_OPT_COMPOSE_TILE: 0 automatic, 1 resident operand, 2 streamed operand
-    int face_warps = 0;        // AM_OPT_FACE_WARPS: warps per face polygon, 0 automatic
+    int face_warps = 0;        // AM_OPT_FACE_WARPS: the rule between near-equal hits, 0 automatic
     long long table_slots = 0; // AM_OPT_TABLE_SLOTS: fixed region hash table size, 0 automatic
     int inject_err = 0;        // AM_OPT_INJECT_ERROR: error bits set in the control block after the seeds
-    int prune = 0;             // AM_OPT_PRUNE_ROWS: the walk scans only the rows that can bound the face
     bool limit_hit = false;    // the last run stopped at the region limit
     bool over_limit(long long tail)
     {
@@ -296,6 +295,7 @@ struct am_engine {
         r.mid = mid.p;
         r.start = start.as<int32_t>();
         r.parent = parent.as<int32_t>();
+        r.reach = reach.as<float>();
         r.nv = nv.as<int32_t>();
         r.status = status.as<int8_t>();
         r.verts = verts.p;
@@ -309,7 +309,7 @@ struct am_engine {
     void release_run_buffers()
     {
         drop_graph();
-        for (DevBuf *b : {&keys, &hash, &mid, &start, &parent, &nv, &status, &verts, &edges, &table, &cons, &eq, &rec,
+        for (DevBuf *b : {&keys, &hash, &mid, &start, &parent, &reach, &nv, &status, &verts, &edges, &table, &cons, &eq, &rec,
                           &blocksum, &order, &split})
             b->reset();
         ring = 0;
@@ -330,6 +330,7 @@ struct am_engine {
         AM_CUDA(mid.grow(ts * 4 * nc, ts * 4 * keep, st));
         AM_CUDA(start.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
         AM_CUDA(parent.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
+        AM_CUDA(reach.grow(sizeof(float) * nc, sizeof(float) * keep, st));
         AM_CUDA(nv.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
         AM_CUDA(status.grow(sizeof(int8_t) * nc, sizeof(int8_t) * keep, st));
         AM_CUDA(verts.grow(ts * 3 * kVMax * nc, ts * 3 * kVMax * keep, st));
@@ -521,7 +522,6 @@ struct am_engine {
         add(&prec, sizeof(prec));
         add(&chunk, sizeof(chunk));
         add(&face_warps, sizeof(face_warps));
-        add(&prune, sizeof(prune));
         add(&iso, sizeof(iso));
         add(&tol, sizeof(tol));
         add(&net, sizeof(net));
@@ -551,7 +551,7 @@ struct am_engine {
                     launch_compose_tc(net, tcnet, reg, ch, iso, d_err.as<int>(), st);
                 else
                     launch_compose(prec, net, reg, ch, iso, d_err.as<int>(), st);
-                launch_polygon(prec, net, reg, ch, hs, tol, face_warps, prune, fp64_counter(), d_err.as<int>(), st);
+                launch_polygon(prec, net, reg, ch, hs, tol, face_warps, fp64_counter(), d_err.as<int>(), st);
                 launch_append(0, prec, net, reg, ch, hs, nullptr, nullptr, nullptr, chunk * kVMax,
                               d_tail.as<long long>(), blocksum.as<int>(), (int)(blocksum.bytes / sizeof(int)),
                               d_err.as<int>(), st);
@@ -1004,8 +1004,7 @@ void run_host_loop(am_engine *e)
             t_comp += ms;
             AM_CUDA(cudaEventRecord(pa, st));
         }
-        launch_polygon(prec, net, reg, ch, hs, tol, e->face_warps, e->prune, e->fp64_counter(), e->d_err.as<int>(),
-                       st);
+        launch_polygon(prec, net, reg, ch, hs, tol, e->face_warps, e->fp64_counter(), e->d_err.as<int>(), st);
         if (e->phase_timing) {
             AM_CUDA(cudaEventRecord(pb, st));
             AM_CUDA(cudaEventSynchronize(pb));
@@ -1208,8 +1207,7 @@ int am_set_option(am_engine *e, int option, int64_t value)
     }
     if (option == AM_OPT_PRUNE_ROWS) {
         if (value != 0 && value != 1) return AM_ERR_INVALID_ARGUMENT;
-        e->prune = (int)value;
-        return AM_OK;
+        return AM_OK; // the walk always leaves out the rows that cannot bound the face (am_polygon.cu)
     }
     if (option == AM_OPT_INJECT_ERROR) {
         if (value < 0 || value > (kErrTableFull | kErrWait | kErrCapacity | kErrNonFinite)) return AM_ERR_INVALID_ARGUMENT;
@@ -1248,9 +1246,8 @@ int am_analytic_marching(am_engine *e, const void *const *weights, const void *c
     });
 }
 
-// Autotuner: the composition tile (resident or streamed operand, mixed form)
-// and the warps per face polygon, chosen for a network architecture by
-// marching a sample of it (the first sample_regions regions, the region limit
+// Autotuner: the composition tile (resident or streamed operand, mixed form),
+// chosen for a network architecture by marching a sample of it (the first sample_regions regions, the region limit
 // of AM_OPT_MAX_REGIONS) once per candidate with per-phase device timing,
 // after one untimed pass over the candidates (first launches load modules).
 // Every candidate produces the same regions (the options change the work
@@ -1310,18 +1307,14 @@ int am_autotune(am_engine *e, const am_run_args *x, int64_t sample_regions, int3
     };
     std::vector<int> cts = {0};
     if (e->prec == kMixed) cts = {1, 2, 3};
-    const int fws[] = {1, 2, 4, 8};
     double c = 0, p = 0;
     for (int ct : cts) sample(ct, 0, c, p); // untimed pass
-    for (int fw : fws) sample(0, fw, c, p);
     int best_ct = -1, best_fw = -1;
     double best = 1e300;
     for (int ct : cts)
         if (sample(ct, 0, c, p) && c < best) best = c, best_ct = ct;
-    best = 1e300;
-    if (best_ct >= 0)
-        for (int fw : fws)
-            if (sample(best_ct, fw, c, p) && p < best) best = p, best_fw = fw;
+    // (a face is one warp's whatever the option says: its automatic value)
+    if (best_ct >= 0) best_fw = polygon_face_warps(e->prec, e->ALLP);
     e->max_regions = keep_max;
     e->phase_timing = keep_pt;
     e->has_am = false; // the samples are not a result

@@ -57,6 +57,7 @@ struct RegionsDev {
     void *mid;          // [cap][4] TS: seed point / edge midpoint
     int32_t *start;     // [cap] start plane (-1 = seed)
     int32_t *parent;    // [cap] the region it was entered from (-1 = seed)
+    float *reach;       // [cap] radius of the near list for the region's children (am_polygon.cu)
     int32_t *nv;        // [cap] polygon vertex count
     int8_t *status;     // [cap]
     void *verts;        // [cap][kVMax][3] TS
@@ -153,11 +154,10 @@ struct Tolerances {
 // nonfinite: device flag, non-zero when a weight may not be finite (null: all are)
 void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso, int *d_err,
                     cudaStream_t st, const int *nonfinite = nullptr);
-// prune: 1 = the walk scans only the rows that can bound the face (see
-// prune_rows), 0 = every row (the same faces)
+// face_warps: sets the rule between near-equal hits (0: by the rows' size)
 // nfp64: counts the faces the mixed form walks again with FP64 predicates
 void launch_polygon(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
-                    const Tolerances &tol, int face_warps, int prune, unsigned long long *nfp64, int *d_err,
+                    const Tolerances &tol, int face_warps, unsigned long long *nfp64, int *d_err,
                     cudaStream_t st);
 int polygon_face_warps(int prec, int ALLP);
 // zeroed: an int set to zero as well (optional)

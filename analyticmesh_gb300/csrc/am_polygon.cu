@@ -1,4 +1,4 @@
-// am_polygon.cu -- face polygon of every region of a chunk, warp per face,
+// am_polygon.cu -- face polygon of every region of a wave, a warp per face,
 // plus the frontier insert of its neighbours.
 //
 // The face of a region is the polygon {x : w_eq.x + b_eq = 0, C_k(x) <= 0 for
@@ -6,36 +6,64 @@
 // in order of distance from a seed point, one 3x3 solve plus an N-row
 // feasibility scan per candidate, one candidate per region per round with a
 // host round trip between rounds (backend/inc/kernel.h:1258-1320).  Here one
-// warp owns a face: the region's constraint rows are staged in shared memory
-// and the walk is ray shooting along the current edge line -- a single pass
-// over the rows gives the first plane the line hits, and the vertex is the
+// warp owns a face and the walk is ray shooting along the current edge line: a
+// pass over the rows gives the first plane the line hits, and the vertex is the
 // 3x3 solve of (edge plane, hit plane, face plane).  The walk goes
 // counter-clockwise about w_eq, which is the orientation the reference's
 // correctNormalDirection enforces (kernel.h:1325-1370).  Zero-length edges
 // (vertices closer than FP_SAME_EPS in L1) are merged and spawn no neighbour,
 // as in cudaUpdateVert_kernel (kernel.h:1197-1205).
 //
+// The near list.  A face is small against the distance of most of its rows'
+// planes, so the warp streams the rows once from global memory, keeps the
+// normalised rows of the planes within a distance T of the walk's start point p
+// in shared memory (about kTarget of them, at most kList) and walks over those.
+// A row left out has a plane farther than T from p, so within the ball of
+// radius D < T around p it is neither violated, nor near zero, nor hit: every
+// decision of the walk is the one over all rows as long as the walk's points
+// stay in the ball, which is checked at every step (see ball_radius for the
+// margin).  T comes from the parent's count, scaled (a plane count in a ball
+// grows with its radius); a seed's from a first pass over the rows.  A walk that
+// leaves its ball is repeated with a larger T, and then over every row.
+//
+// Which of two rows that the line hits at nearly the same parameter comes first
+// is decided by rounding.  The rule is the scan's over all rows by `ways` lanes
+// with two interleaved chains each: within a chain fractions are compared by
+// cross products in row order, between lanes by quotient and row.  A scan over
+// the list takes the smallest quotient if no other is within 1e-5 of it (any
+// rule gives that row), the rule's quotient and row if the candidates within
+// 1e-5 belong to different lanes, and otherwise gives up: the face is walked
+// over all rows with the rule itself.
+//
 // Seed regions (start == -1) first find a polygon vertex exactly as the
 // reference's calcStartIdx does (kernel.h:799-856): planes ordered by signed
 // geometric distance from the seed point, pairs enumerated by get_i_j up to
 // x = min((ALL-1)(ALL-2), 812), the first pair whose vertex satisfies every
 // other constraint within FP_EPS wins.  Those pairs only involve the 57
-// nearest planes, so a partial selection replaces the reference's full sort.
+// nearest planes, which the list holds.
 //
 // Every edge on a hidden unit's plane gives a neighbour: the key with that
 // bit flipped.  Its hash is updated in O(1) and it is inserted into the
 // region hash set (full-key comparison on fingerprint match); among equal new
 // keys the smallest (parent, plane) id wins, so the result is deterministic.
+#include <algorithm>
 #include <cuda/atomic>
 #include <cuda_runtime.h>
 
 #include "am_device.cuh"
 #include "am_internal.h"
-#include "am_umma.cuh"
 
 namespace am {
 
 namespace {
+
+constexpr int kList = 128;      // rows of the near list (four per lane)
+constexpr int kTarget = 64;     // and how many it aims at (80 and 48 measured 1 to 7 % slower)
+constexpr int kFaceWarps = 4;   // faces per block
+constexpr int kBlocks = 8;      // blocks per SM
+constexpr int kUnroll = 4;      // FP32 rows per lane in flight (half as many FP64 ones)
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kNoHit = 0x7fffffff;
 
 template <typename T>
 __device__ __forceinline__ unsigned long long order_key(T d);
@@ -68,52 +96,125 @@ __device__ __forceinline__ bool finite_bits(double v)
     return ((uint32_t)(__double_as_longlong(v) >> 52) & 0x7ffu) != 0x7ffu;
 }
 
-// The vertex of planes a, b and the face plane, solved by the warp: lanes
-// 0-7 convert the two rows' components (one conversion instruction), lane
+// Products and sums with the roundings fixed, not left to the compiler's
+// contraction (which depends on the code around them): they decide the walk, and
+// the list and the scan over every row must agree.
+__device__ __forceinline__ float mul_t(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_t(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
+// a0 b0 + a1 b1 + a2 b2
+template <typename T>
+__device__ __forceinline__ T dot3(T a0, T b0, T a1, T b1, T a2, T b2)
+{
+    return fma_t(a2, b2, fma_t(a0, b0, mul_t(a1, b1)));
+}
+// a b - c d
+template <typename T>
+__device__ __forceinline__ T diff2(T a, T b, T c, T d)
+{
+    return fma_t(a, b, -mul_t(c, d));
+}
+
+// ---------------------------------------------------------------- rows
+// A region's constraint rows in global memory: the first nsplit in the parent's
+// slot (the plane the region was entered through with the other sign), the rest
+// in its own.
+template <typename TC>
+struct GlobalRows {
+    const vec4_t<TC> *par, *own;
+    int nsplit, flip, n;
+    __device__ __forceinline__ vec4_t<TC> raw(int k) const
+    {
+        vec4_t<TC> v = k < nsplit ? par[k] : own[k];
+        if (k == flip) {
+            v.x = -v.x;
+            v.y = -v.y;
+            v.z = -v.z;
+            v.w = -v.w;
+        }
+        return v;
+    }
+    __device__ __forceinline__ vec4_t<TC> get(int k) const;
+    __device__ __forceinline__ int name(int k) const { return k; }
+};
+
+// Normalised (|w| = 1, zero rows become 0.x + sign(b) inf): signed geometric
+// distances are then plain dot products, the same quantity the reference's
+// feasibility test computes as (w.x + b) * rsqrt(|w|^2) (kernel.h:729-795).
+template <typename TC>
+__device__ __forceinline__ vec4_t<TC> normalised(vec4_t<TC> v)
+{
+    const TC n2 = dot3(v.x, v.x, v.y, v.y, v.z, v.z);
+    if (n2 > TC(0)) {
+        const TC inv = rsqrt(n2); // as the reference's distance normalisation
+        v.x = mul_t(v.x, inv);
+        v.y = mul_t(v.y, inv);
+        v.z = mul_t(v.z, inv);
+        v.w = mul_t(v.w, inv);
+    } else {
+        v.w = v.w > TC(0) ? TC(INFINITY) : (v.w < TC(0) ? TC(-INFINITY) : TC(NAN));
+    }
+    return v;
+}
+template <typename TC>
+__device__ __forceinline__ vec4_t<TC> GlobalRows<TC>::get(int k) const
+{
+    return normalised<TC>(raw(k));
+}
+
+// The near list of a face (shared memory); rows are named by their position.
+template <typename TC>
+struct NearList {
+    vec4_t<TC> row[kList];
+    uint16_t idx[kList];
+};
+template <typename TC>
+struct ListRows {
+    const NearList<TC> *l;
+    int n;
+    __device__ __forceinline__ vec4_t<TC> get(int j) const { return l->row[j]; }
+    __device__ __forceinline__ int name(int j) const { return l->idx[j]; } // the row's plane
+};
+
+// The vertex of planes ra, rb and the face plane, solved by the warp: lane
 // L = 0..3 (and its copies L + 4, L + 8, ...) computes Cramer's determinant
 // with column L - 1 replaced by -b (L = 0: none), then divides by the lane-0
-// determinant -- the same arithmetic as solve3 on one lane, in three
-// dependent FP64 sequences (convert, determinant, divide) instead of forty,
-// which matters because the SM's FP64 pipe issues a warp instruction at the
-// same cost however few lanes are active.  Every lane returns the vertex in
-// the solve precision (V) and rounded to the scan precision (Vc); false if a
-// coordinate is not finite.
+// determinant -- the same arithmetic as solve3 on one lane, in two dependent
+// sequences (determinant, divide) instead of seven, which matters because the
+// SM's FP64 pipe issues a warp instruction at the same cost however few lanes
+// are active (for the same reason a conversion to FP64 is spread over eight
+// lanes).  Every lane returns the vertex in the solve precision (V) and rounded
+// to the scan precision (Vc); false if a coordinate is not finite.
+template <typename TC>
+__device__ __forceinline__ TC component(const vec4_t<TC> &v, int c)
+{
+    return c < 2 ? (c == 0 ? v.x : v.y) : (c == 2 ? v.z : v.w);
+}
 template <typename TC, typename TS>
-__device__ __forceinline__ bool warp_solve(const vec4_t<TC> *rows, int a, int b, const TS *eqv, TS *V, TC *Vc,
+__device__ __forceinline__ bool warp_solve(const vec4_t<TC> &ra, const vec4_t<TC> &rb, const TS *eqv, TS *V, TC *Vc,
                                            int lane)
 {
-    const TC *ra = reinterpret_cast<const TC *>(rows + a);
-    const TC *rb = reinterpret_cast<const TC *>(rows + b);
-    const int c = lane & 7;
-    const TS cs = (TS)(c < 4 ? ra[c] : rb[c - 4]);
-    TS m[8];
+    TS m[8] = {(TS)ra.x, (TS)ra.y, (TS)ra.z, (TS)ra.w, (TS)rb.x, (TS)rb.y, (TS)rb.z, (TS)rb.w};
+    if (sizeof(TS) > sizeof(TC)) {
+        const int c = lane & 7;
+        const TS cs = (TS)component<TC>(c < 4 ? ra : rb, c & 3);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) m[j] = __shfl_sync(0xffffffffu, cs, j);
+        for (int j = 0; j < 8; ++j) m[j] = __shfl_sync(kFull, cs, j);
+    }
     const int L = lane & 3;
     const TS a00 = L == 1 ? -m[3] : m[0], a01 = L == 2 ? -m[3] : m[1], a02 = L == 3 ? -m[3] : m[2];
     const TS a10 = L == 1 ? -m[7] : m[4], a11 = L == 2 ? -m[7] : m[5], a12 = L == 3 ? -m[7] : m[6];
     const TS a20 = L == 1 ? -eqv[3] : eqv[0], a21 = L == 2 ? -eqv[3] : eqv[1], a22 = L == 3 ? -eqv[3] : eqv[2];
     const TS d = det3<TS>(a00, a01, a02, a10, a11, a12, a20, a21, a22);
-    const TS d0 = __shfl_sync(0xffffffffu, d, 0);
+    const TS d0 = __shfl_sync(kFull, d, 0);
     const TS x = d / d0;
-    const TC xc = (TC)x;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-        V[j] = __shfl_sync(0xffffffffu, x, j + 1);
-        Vc[j] = __shfl_sync(0xffffffffu, xc, j + 1);
+        V[j] = __shfl_sync(kFull, x, j + 1);
+        Vc[j] = (TC)V[j];
     }
     return finite_bits(V[0]) && finite_bits(V[1]) && finite_bits(V[2]);
-}
-
-// |w|^2 with the roundings fixed (not left to the compiler's contraction, which
-// depends on the code around it): the normalised rows decide the walk
-__device__ __forceinline__ float norm2(float x, float y, float z)
-{
-    return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y)));
-}
-__device__ __forceinline__ double norm2(double x, double y, double z)
-{
-    return __fma_rn(z, z, __fma_rn(x, x, __dmul_rn(y, y)));
 }
 
 // L1 distance test |V - P|_1 < eps.  With TS wider than TC it is decided on
@@ -133,234 +234,300 @@ __device__ __forceinline__ int same_filter(const TC *Vc, TC px, TC py, TC pz, TS
     return -1;
 }
 
-__device__ __forceinline__ long long next_work(WaveCtl *ctl, int lane)
-{
-    unsigned int v = 0;
-    if (lane == 0) v = atomicAdd(&ctl->work, 1u);
-    return (long long)__shfl_sync(0xffffffffu, v, 0);
-}
-
-__device__ __forceinline__ unsigned long long load_slot(const unsigned long long *p)
-{
-    cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> a(*const_cast<unsigned long long *>(p));
-    return a.load(cuda::memory_order_relaxed);
-}
-
-// Does the key stored behind slot value `cur` equal parent_key ^ flip(k)?
-// Region entries (tag 0) point at the region store; candidate entries (tag 1)
-// carry (chunk-local parent, plane) and point at the parent's key.  The whole
-// warp compares: lane l takes words l, l + 32, ..., all loads issued at once.
-__device__ bool warp_key_matches(unsigned long long cur, const RegionsDev &reg, long long head, int ALL, int W,
-                                 const uint32_t *pkey, int k, int lane)
-{
-    const uint32_t id = (uint32_t)cur & 0x7fffffffu;
-    const bool cand = (cur >> 31) & 1ull;
-    const uint32_t *other;
-    int ok2 = -1;
-    if (cand) {
-        other = reg.keys + (size_t)(head + id / ALL) * W;
-        ok2 = (int)(id % ALL);
-    } else {
-        other = reg.keys + (size_t)id * W;
+// ---------------------------------------------------------------- the ball
+// A row left out has its plane farther than T from p, up to the rounding of the
+// FP32 test (a few 1e-7 of the coordinates' size).  For a point x with
+// |x - p| <= D its value is below -(T - D), and the edge line reaches its plane
+// beyond |x - p| = T; with T - D >= D / 16 + 1e-4 of the coordinates' size the
+// computed quotient of such a row is larger than that of any hit within the
+// ball, whatever the line's angle to the plane: with m = T - D, t the hit's
+// distance (<= 2 D) and a the row's slope, the computed quotient is at least
+// (a (t + m) - 1e-6) / (a + 5e-7) and (m - 1e-6) / (a + 5e-7), and m^2 > 4e-6 D
+// puts one of the two above t for every a.  The same margin keeps its value
+// away from the 1e-6 and 2e-6 of the near-zero predicates.
+struct Ball {
+    float x, y, z, d2; // centre, squared radius (< 0: nothing is inside, infinite: every row is in the list)
+    __device__ __forceinline__ bool in(float px, float py, float pz) const
+    {
+        const float dx = px - x, dy = py - y, dz = pz - z;
+        return d2 == INFINITY || dx * dx + dy * dy + dz * dz <= d2; // (NaN: outside)
     }
-    const int kw = k >> 5;
-    const uint32_t kb = 1u << (k & 31);
-    const int ow = ok2 >= 0 ? (ok2 >> 5) : -1;
-    const uint32_t ob = ok2 >= 0 ? (1u << (ok2 & 31)) : 0u;
-    bool differ = false;
-    for (int w = lane; w < W; w += 32) {
-        const uint32_t a = pkey[w] ^ (w == kw ? kb : 0u);
-        const uint32_t b = other[w] ^ (w == ow ? ob : 0u);
-        differ = differ || a != b;
-    }
-    return !__any_sync(0xffffffffu, differ);
+};
+__device__ __forceinline__ float coord_size(float x, float y, float z) { return 1.f + fabsf(x) + fabsf(y) + fabsf(z); }
+__device__ __forceinline__ float ball_radius2(float T, float size)
+{
+    if (T == INFINITY) return INFINITY;
+    const float D = (T - 1e-4f * size) * (16.f / 17.f);
+    return D > 0.f ? D * D : -1.f;
 }
 
-// Insert the neighbour across plane k (parent key pkey with bit k flipped)
-// into the region hash set; the whole warp works on it, lane 0 owning the
-// slot operations.  Returns the slot claimed for a new candidate (or the
-// candidate slot this one now shares), -1 when the key is a committed
-// region already.  Among equal candidate keys the smallest (parent, plane)
-// id stays in the slot, so the result does not depend on timing.
-__device__ int warp_insert(const RegionsDev &reg, const HashDev &hs, long long head, int ALL, int W, const uint32_t *pkey,
-                           uint64_t phash, long long rl, int k, int lane, int *err)
+// The rows within T of the ball's centre go into the list.  The test compares
+// squares, without the square root, the centre scaled by 1 / T: a row is left out
+// if g < 0 and (g / T)^2 > |w|^2 (NaN: kept).  n counts them all; at most kList
+// are stored (raw; finish_list normalises).
+template <typename TC>
+struct Sieve {
+    float bx, by, bz, bw;
+    NearList<TC> *list;
+    int n, lane;
+    __device__ __forceinline__ Sieve(const Ball &ball, float T, NearList<TC> *l, int ln) : list(l), n(0), lane(ln)
+    {
+        bw = 1.f / T; // (T infinite: 0, every row is kept)
+        bx = ball.x * bw;
+        by = ball.y * bw;
+        bz = ball.z * bw;
+    }
+    // this lane's row of a block of 32 (k: its plane; in: there is one)
+    __device__ __forceinline__ void take(const vec4_t<TC> &v, int k, bool in)
+    {
+        const float x = (float)v.x, y = (float)v.y, z = (float)v.z, w = (float)v.w;
+        const float g = fmaf(x, bx, fmaf(y, by, fmaf(z, bz, w * bw)));
+        const float n2 = fmaf(x, x, fmaf(y, y, z * z));
+        const bool keep = in && !(g < 0.f && g * g > n2);
+        const unsigned b = __ballot_sync(kFull, keep);
+        if (b) {
+            const int pos = n + __popc(b & ((1u << lane) - 1u));
+            if (keep && pos < kList) {
+                list->row[pos] = v;
+                list->idx[pos] = (uint16_t)k;
+            }
+            n += __popc(b);
+        }
+    }
+    __device__ __forceinline__ void finish() const
+    {
+        __syncwarp();
+        for (int j = lane; j < min(n, kList); j += 32) list->row[j] = normalised<TC>(list->row[j]);
+        __syncwarp();
+    }
+};
+
+// A pass over the rows by plain loads (a repeat with another T: rare)
+template <typename TC>
+__device__ int collect(const GlobalRows<TC> &g, float T, const Ball &ball, NearList<TC> *list, int lane)
 {
-    const unsigned full = 0xffffffffu;
-    const uint64_t h = flip_hash(phash, pkey[k >> 5], k);
-    const uint32_t fp = fp_of(h);
-    const uint32_t myid = (uint32_t)(rl * ALL + k);
-    const unsigned long long mine = slot_value(fp, 1, myid);
-    unsigned long long slot = h & hs.mask;
-    for (int probe = 0; probe < kMaxProbes; ++probe) {
-        unsigned long long cur = 0ull;
-        int claimed = 0;
-        if (lane == 0) {
-            cur = load_slot(hs.slots + slot);
-            if (cur == kEmpty) {
-                const unsigned long long old = atomicCAS(hs.slots + slot, kEmpty, mine);
-                claimed = old == kEmpty;
-                cur = old;
+    Sieve<TC> sv(ball, T, list, lane);
+    __syncwarp();
+    for (int k = lane; k - lane < g.n; k += 32) {
+        const bool in = k < g.n;
+        vec4_t<TC> v;
+        v.x = v.y = v.z = v.w = TC(0);
+        if (in) v = g.raw(k);
+        sv.take(v, k, in);
+    }
+    sv.finish();
+    return sv.n;
+}
+
+// The pass over a face's rows, straight from global memory, the parent's rows into
+// the region's slot as well: kUnroll rows per lane in flight.  Measured on GB300
+// (3-[512]x8-1, polygon phase): 4 rows and 32 warps per SM 146 ms, 8 rows and 24
+// warps 158, 2 rows 151, 40 warps 158; a per-warp ring of bulk copies into shared
+// memory with the next face's chunks under way, 226 (its state spilled).
+template <typename TC, bool kCopy>
+__device__ __forceinline__ void stream_part(const vec4_t<TC> *src, vec4_t<TC> *copy, int k0, int k1, int flip, Sieve<TC> &sv)
+{
+    constexpr int U = sizeof(TC) == 4 ? kUnroll : kUnroll / 2;
+    const int lane = sv.lane;
+    for (; k0 < k1; k0 += 32 * U) {
+        vec4_t<TC> v[U];
+        const vec4_t<TC> *s = src + k0 + lane;
+        if (k0 + 32 * U <= k1) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = s[32 * u];
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                v[u].x = v[u].y = v[u].z = v[u].w = TC(0);
+                if (k0 + 32 * u + lane < k1) v[u] = s[32 * u];
             }
         }
-        cur = __shfl_sync(full, cur, 0);
-        if (__shfl_sync(full, claimed, 0)) return (int)slot;
-        if ((uint32_t)(cur >> 32) == fp && warp_key_matches(cur, reg, head, ALL, W, pkey, k, lane)) {
-            if ((cur >> 31) & 1ull) {
-                if (lane == 0) atomicMin(hs.slots + slot, mine);
-                return (int)slot;
+        if (kCopy) { // (the plane the region was entered through is a parent's row)
+            if (flip >= k0 && flip < k0 + 32 * U) {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (k0 + 32 * u + lane == flip) {
+                        v[u].x = -v[u].x;
+                        v[u].y = -v[u].y;
+                        v[u].z = -v[u].z;
+                        v[u].w = -v[u].w;
+                    }
             }
-            return -1;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k0 + 32 * u + lane < k1) copy[k0 + 32 * u + lane] = v[u];
         }
-        slot = (slot + (unsigned long long)probe + 1ull) & hs.mask;
+#pragma unroll
+        for (int u = 0; u < U; ++u) sv.take(v[u], k0 + 32 * u + lane, k0 + 32 * u + lane < k1);
     }
-    if (lane == 0) atomicOr(err, kErrTableFull);
+}
+
+// the list position of plane k (in the list)
+template <typename TC>
+__device__ __forceinline__ int position(const NearList<TC> *list, int n, int k, int lane)
+{
+    for (int j = 0; j < n; j += 32) {
+        const unsigned b = __ballot_sync(kFull, j + lane < n && (int)list->idx[j + lane] == k);
+        if (b) return j + __ffs(b) - 1;
+    }
     return -1;
 }
 
-// A face belongs to a group of G warps (G = 1, 2, 4 or 8; wide networks use
-// more, so that a block holds fewer faces' rows and more warps).  The group
-// stages the rows together, and every warp of it runs the same walk on them:
-// each scans rows k = 32 gw + lane (mod 32 G), the partial (t, plane) minima
-// meet in shared memory (two slots, by step parity) behind one named barrier
-// per step, and every warp takes the same minimum, so the group stays in
-// step without further messages.  Warp 0 (the leader) alone re-solves the
-// vertices in the solve precision and writes the outputs.  G = 1 is the plain
-// warp per face with no barrier.
-constexpr int kListCap = 384;  // rows the pruned walk keeps at most (more: the walk scans every row)
-constexpr int kPruneMin = 96;  // fewer rows than this: no pruning
-constexpr int kRowWaitIters = 1 << 22; // bound of the wait for a face's rows (bulk copy)
-
+// A radius that holds about kTarget rows: every lane's rows in four groups, the
+// smallest distance of each; T is the distance that 60 of the 128 groups reach
+// (rows spread evenly over the groups: ln(1 / (1 - 60 / 128)) rows per group).
 template <typename TC>
-struct GroupShared {
-    long long rl;   // the group's region (chunk-local)
-    uint64_t rbar;  // the face's rows have landed (bulk copy)
-    int done, near; // the leader's refinement outcome; a warp met a row near a vertex
-    TC bt[2][8];    // partial minima per step parity and warp
-    double btd[2][8]; // the same for a scan in FP64 over FP32 rows
-    int bk[2][8];
-    int nlist;      // rows kept by the pruning
-    // phases of a face, one at a time (a barrier between any two): the seed
-    // start search; row pruning, first the sample's extreme rows per warp
-    // and direction, then (once every warp has read those) the list of the
-    // rows kept, read by the walk; the neighbour planes by edge after it
-    union {
-        struct {
-            unsigned long long sk[2][8]; // partial choices of a selection pass
-            double sv[3];                // the start vertex found ...
-            int sri;                     // ... and its plane
-        } seed;
-        struct {
-            TC v[8][8];
-            int16_t i[8][8];
-        } ext;
-        uint16_t list[kListCap];
-        int ve[kVMax]; // -1: no neighbour across the edge (from the leader)
-    };
-};
-
-template <typename TC>
-struct Grp {
-    int G, gw, bar;
-    GroupShared<TC> *sh;
-    // named barrier 1 + group (at most four groups per block when G > 1);
-    // constant ids, so that a block reserves five barriers, not sixteen
-    __device__ __forceinline__ void sync() const
-    {
-        const int n = 32 * G;
-        switch (bar) {
-        case 1: asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); break;
-        case 2: asm volatile("bar.sync 2, %0;" ::"r"(n) : "memory"); break;
-        case 3: asm volatile("bar.sync 3, %0;" ::"r"(n) : "memory"); break;
-        default: asm volatile("bar.sync 4, %0;" ::"r"(n) : "memory"); break;
-        }
-    }
-};
-
-template <typename TC>
-__host__ __device__ constexpr size_t group_shared_bytes()
+__device__ float seed_radius(const GlobalRows<TC> &g, const Ball &ball, int lane)
 {
-    return (sizeof(GroupShared<TC>) + 15) / 16 * 16;
+    unsigned m[4] = {0x7f800000u, 0x7f800000u, 0x7f800000u, 0x7f800000u};
+    const int per = (g.n + 127) / 128; // rows of a lane per group
+    for (int i = 0, k = lane; k < g.n; ++i, k += 32) {
+        const vec4_t<TC> v = g.raw(k);
+        const float x = (float)v.x, y = (float)v.y, z = (float)v.z, w = (float)v.w;
+        const float c = -(x * ball.x + y * ball.y + z * ball.z + w) * rsqrtf(x * x + y * y + z * z);
+        const unsigned key = c > 0.f ? __float_as_uint(c) : (c != c ? 0x7f800000u : 0u);
+        const int q = i / per;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j == q) m[j] = min(m[j], key);
+    }
+    unsigned lo = 0u, hi = 0x7f800000u;
+    for (int it = 0; it < 20; ++it) {
+        const unsigned mid = (lo + hi) / 2u;
+        int c = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c += m[j] <= mid;
+        if (__reduce_add_sync(kFull, c) >= 60) hi = mid;
+        else lo = mid;
+    }
+    return fmaxf(__uint_as_float(hi), 1e-30f);
 }
 
-// first hit along the edge line over rows k0, k0 + kstep, ... (of the kept
-// list, when the rows were pruned): min over crossing planes of
-// t = max(0, -g) / a, compared as fractions within a lane (two interleaved
-// candidates per lane halve the compare chain), then across the warp; every
-// lane returns the warp's (t, plane), plane 0x7fffffff if none.  The rows are
-// TR, the arithmetic TA (FP64 over FP32 rows for the mixed form's FP64
-// predicates).  kNear: `near` is set when a row other than the two the
-// current point lies on has |g| < 1e-6 there (the rows are normalised, so g
-// is a distance): a predicate near zero, which the mixed form takes again in
-// FP64.
-template <typename TR, typename TA, bool kNear>
-__device__ __forceinline__ void hit_scan(const vec4_t<TR> *rows, int ALL, const uint16_t *list, int nlist, int k0,
-                                         int kstep, TA d0, TA d1, TA d2, TA thr, TA c0, TA c1, TA c2, int e, int prev,
-                                         TA &bt_out, int &bk_out, bool &near)
+// ---------------------------------------------------------------- scans
+// What a scan along an edge line found: the first plane (position), or none, or
+// (list only) that the rule between near-equal hits needs every row.
+enum : int { kHit = 0, kNone = 1, kGiveUp = 2 };
+
+template <typename TC>
+struct Line {
+    TC d0, d1, d2, thr; // direction (not normalised), parallel threshold
+    TC c0, c1, c2;      // current point
+    int e, prev;        // the planes it lies on
+};
+// the same in FP64, for the mixed form's predicates near zero (the threshold is
+// worked out where a row is near zero: few steps)
+struct Line64 {
+    double d0, d1, d2, par_eps, c0, c1, c2;
+    __device__ __forceinline__ double thr() const { return par_eps * sqrt(dot3(d0, d0, d1, d1, d2, d2)); }
+};
+
+// The rule over the list, `t` exact quotients by candidate: the smallest
+// (quotient, row) unless two candidates share a lane of the rule.
+// tf[j]: approximate quotient of the lane's row j (infinite: no candidate).
+template <typename TC, typename Exact>
+__device__ __forceinline__ int choose(const ListRows<TC> &rows, const float (&tf)[kList / 32], int ways, int lane, int &bk,
+                                      float &bt, Exact exact)
 {
-    TA bnum = TA(1), bden = TA(0), bnum1 = TA(1), bden1 = TA(0);
-    int bk = 0x7fffffff, bk1 = 0x7fffffff;
-    bool nr = false;
-    // rows of one chain come in increasing k, so that a later row never
-    // wins a tie against the chain's earlier choice: the index test is only
-    // needed for the pruning list, whose rows come in any order
-    auto consider = [&](int k, TA &bn, TA &bd, int &bi, bool any_order) {
-        const vec4_t<TR> r = rows[k];
-        const TA rx = (TA)r.x, ry = (TA)r.y, rz = (TA)r.z, rw = (TA)r.w;
-        const TA a = rx * d0 + ry * d1 + rz * d2;
-        TA num;
-        if (kNear) {
-            num = -(rx * c0 + ry * c1 + rz * c2 + rw);
-            nr = nr || (fabs(num) < TA(1e-6) && k != e && k != prev);
-            if (!(a > thr) || k == e || k == prev) return;
-        } else {
-            if (!(a > thr) || k == e || k == prev) return;
-            num = -(rx * c0 + ry * c1 + rz * c2 + rw);
+    float lmin = tf[0];
+    int lj = 0;
+#pragma unroll
+    for (int j = 1; j < kList / 32; ++j)
+        if (tf[j] < lmin) {
+            lmin = tf[j];
+            lj = j;
         }
-        num = num > TA(0) ? num : TA(0);
-        const TA lhs = num * bd, rhs = bn * a;
-        if (lhs < rhs || (any_order && lhs == rhs && k < bi)) {
-            bn = num;
-            bd = a;
-            bi = k;
-        }
-    };
-    if (list) { // the rows that survived pruning
-        int j = k0;
-        for (; j + kstep < nlist; j += 2 * kstep) {
-            consider(list[j], bnum, bden, bk, true);
-            consider(list[j + kstep], bnum1, bden1, bk1, true);
-        }
-        if (j < nlist) consider(list[j], bnum, bden, bk, true);
-    } else {
-        int k = k0;
-#pragma unroll 2
-        for (; k + kstep < ALL; k += 2 * kstep) {
-            consider(k, bnum, bden, bk, false);
-            consider(k + kstep, bnum1, bden1, bk1, false);
-        }
-        if (k < ALL) consider(k, bnum, bden, bk, false);
+    const unsigned mb = __reduce_min_sync(kFull, __float_as_uint(lmin)); // (quotients are not negative)
+    if (mb >= 0x7f800000u) return kNone;
+    bt = __uint_as_float(mb);
+    const float lim = bt * 1.00001f;
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < kList / 32; ++j) c += tf[j] <= lim;
+    const unsigned any = __ballot_sync(kFull, c > 0);
+    if (__popc(any) == 1 && __ballot_sync(kFull, c > 1) == 0u) {
+        const int src = __ffs(any) - 1;
+        bk = __shfl_sync(kFull, lane + 32 * lj, src);
+        return kHit;
     }
-    {
-        const TA lhs = bnum1 * bden, rhs = bnum * bden1;
-        if (bk1 != 0x7fffffff && (lhs < rhs || (lhs == rhs && bk1 < bk))) {
-            bnum = bnum1;
-            bden = bden1;
-            bk = bk1;
+    // several hits within 1e-5: by the rule (rare)
+    int lane_of[kList / 32]; // the rule's lane of each of this lane's candidates
+    double bq = INFINITY;    // quotients in FP64 hold the FP32 ones exactly
+    int bi = kNoHit, bp = kNoHit;
+#pragma unroll
+    for (int j = 0; j < kList / 32; ++j) {
+        const bool cand = tf[j] <= lim;
+        const int pos = lane + 32 * j;
+        const int k = cand ? (int)rows.l->idx[pos] : -1;
+        lane_of[j] = cand ? k % ways : -1 - pos;
+        if (cand) {
+            const double q = exact(j);
+            if (q < bq || (q == bq && k < bi)) {
+                bq = q;
+                bi = k;
+                bp = pos;
+            }
         }
     }
-    TA bt = bk == 0x7fffffff ? TA(INFINITY) : bnum / bden;
+    bool clash = false;
+#pragma unroll
+    for (int j = 0; j < kList / 32; ++j) {
+        unsigned left = __ballot_sync(kFull, lane_of[j] >= 0);
+        while (left) {
+            const int src = __ffs(left) - 1;
+            left &= left - 1u;
+            const int w = __shfl_sync(kFull, lane_of[j], src);
+#pragma unroll
+            for (int i = 0; i < kList / 32; ++i)
+                if (lane_of[i] == w && !(i == j && lane == src)) clash = true;
+        }
+    }
+    if (__any_sync(kFull, clash)) return kGiveUp;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        const TA ot = __shfl_xor_sync(0xffffffffu, bt, o);
-        const int ok = __shfl_xor_sync(0xffffffffu, bk, o);
-        if (ot < bt || (ot == bt && ok < bk)) {
-            bt = ot;
-            bk = ok;
+        const double oq = __shfl_xor_sync(kFull, bq, o);
+        const int oi = __shfl_xor_sync(kFull, bi, o), op = __shfl_xor_sync(kFull, bp, o);
+        if (oq < bq || (oq == bq && oi < bi)) {
+            bq = oq;
+            bi = oi;
+            bp = op;
         }
     }
-    bt_out = bt;
-    bk_out = bk;
-    if (kNear) near = __any_sync(0xffffffffu, nr);
+    bk = bp;
+    return kHit;
+}
+
+// First hit along the edge line over the list: min over crossing planes of
+// t = max(0, -g) / a.  kNear: `near` is set when a row other than the two the
+// current point lies on has |g| < 1e-6 there (the rows are normalised, so g is
+// a distance): a predicate near zero, which the mixed form takes again in FP64.
+template <typename TC, bool kNear>
+__device__ __forceinline__ int scan(const ListRows<TC> &rows, const Line<TC> &ln, int ways, int lane, int &bk, float &bt,
+                                    bool &near)
+{
+    float tf[kList / 32];
+    TC num[kList / 32], den[kList / 32];
+    bool nr = false;
+#pragma unroll
+    for (int j = 0; j < kList / 32; ++j) {
+        const int pos = lane + 32 * j;
+        tf[j] = INFINITY;
+        num[j] = den[j] = TC(1);
+        if (32 * j < rows.n && pos < rows.n && pos != ln.e && pos != ln.prev) {
+            const vec4_t<TC> r = rows.get(pos);
+            const TC a = dot3(r.x, ln.d0, r.y, ln.d1, r.z, ln.d2);
+            TC g = -(dot3(r.x, ln.c0, r.y, ln.c1, r.z, ln.c2) + r.w);
+            if (kNear) nr = nr || fabs(g) < TC(1e-6);
+            if (a > ln.thr) {
+                g = g > TC(0) ? g : TC(0);
+                num[j] = g;
+                den[j] = a;
+                const float q = __fdividef((float)g, (float)a);
+                tf[j] = q <= 3.4e38f ? q : 3.4e38f; // (a candidate stays one)
+            }
+        }
+    }
+    if (kNear) near = near || __any_sync(kFull, nr);
+    return choose<TC>(rows, tf, ways, lane, bk, bt, [&](int j) { return (double)(num[j] / den[j]); });
 }
 
 // The mixed form's scan with FP64 predicates (over FP32 rows): every row is
@@ -369,215 +536,312 @@ __device__ __forceinline__ void hit_scan(const vec4_t<TR> *rows, int ALL, const 
 // a sign or feasibility decision near zero, taken in FP64.  The first hit is
 // the smaller of the FP32 candidates' best and the FP64 candidates' best,
 // compared in FP64, ties to the lower row.
-__device__ __forceinline__ void hit_scan_wide(const float4 *rows, int ALL, const uint16_t *list, int nlist, int k0,
-                                              int kstep, float d0, float d1, float d2, float thr, float c0, float c1,
-                                              float c2, double D0, double D1, double D2, double thr64, double C0,
-                                              double C1, double C2, int e, int prev, double &bt_out, int &bk_out)
+struct Cand64 {
+    double t;
+    bool ok;
+};
+__device__ __forceinline__ Cand64 near_zero64(const float4 &r, const Line64 &l)
 {
-    float bnum = 1.f, bden = 0.f;
-    int bk = 0x7fffffff;
-    double tn = INFINITY;
-    int tk = 0x7fffffff;
-    auto consider = [&](int k) {
-        if (k == e || k == prev) return;
-        const float4 r = rows[k];
-        const float g = r.x * c0 + r.y * c1 + r.z * c2 + r.w;
-        if (fabsf(g) < 2e-6f) {
-            const double a = (double)r.x * D0 + (double)r.y * D1 + (double)r.z * D2;
-            if (!(a > thr64)) return;
-            double num = -((double)r.x * C0 + (double)r.y * C1 + (double)r.z * C2 + (double)r.w);
-            num = num > 0.0 ? num : 0.0;
-            const double t = num / a;
-            if (t < tn || (t == tn && k < tk)) {
-                tn = t;
-                tk = k;
-            }
-            return;
-        }
-        const float a = r.x * d0 + r.y * d1 + r.z * d2;
-        if (!(a > thr)) return;
-        const float num = -g > 0.f ? -g : 0.f;
-        const float lhs = num * bden, rhs = bnum * a;
-        if (lhs < rhs || (lhs == rhs && k < bk)) {
-            bnum = num;
-            bden = a;
-            bk = k;
-        }
-    };
-    if (list) {
-        for (int j = k0; j < nlist; j += kstep) consider(list[j]);
-    } else {
-        for (int k = k0; k < ALL; k += kstep) consider(k);
-    }
-    double bt = bk == 0x7fffffff ? INFINITY : (double)bnum / (double)bden;
-    if (tk != 0x7fffffff && (tn < bt || (tn == bt && tk < bk))) {
-        bt = tn;
-        bk = tk;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ot = __shfl_xor_sync(0xffffffffu, bt, o);
-        const int ok = __shfl_xor_sync(0xffffffffu, bk, o);
-        if (ot < bt || (ot == bt && ok < bk)) {
-            bt = ot;
-            bk = ok;
-        }
-    }
-    bt_out = bt;
-    bk_out = bk;
+    Cand64 c{0.0, false};
+    const double a = dot3<double>(r.x, l.d0, r.y, l.d1, r.z, l.d2);
+    if (!(a > l.thr())) return c;
+    double num = -(dot3<double>(r.x, l.c0, r.y, l.c1, r.z, l.c2) + (double)r.w);
+    num = num > 0.0 ? num : 0.0;
+    c.t = num / a;
+    c.ok = true;
+    return c;
 }
-
-// One face walk: from the start plane s, ray shooting along each edge line,
-// the scan in TA (TC, or TS for the mixed form's FP64 predicates), vertices
-// solved in TS.  Lane i ends with vertex i (vx, vy, vz) and the plane of the
-// edge leaving it (ve); lane j records step j's hit plane (sbk) and merge
-// decision (sdec, 0 append, 1 merge with the previous vertex, 2 merge with
-// the first), nsteps the steps taken.  kNear: `near` (this warp) is set when
-// some step's scan met a row within 1e-6 of the current point.
-template <typename TC, typename TS, bool kGroup, typename TA = TC, bool kNear = false>
-__device__ void walk(const vec4_t<TC> *rows, int ALL, const uint16_t *list, int nlist, const vec4_t<TC> &eqc,
-                     const TS *eqv, const TS *p, int s, TC par_eps, TS same_eps, int lane, TS &vx, TS &vy, TS &vz,
-                     int &ve, int &n, bool &closed, int8_t &status, int &sbk, int &sdec, int &nsteps, const Grp<TC> &g,
-                     bool *near = nullptr)
+__device__ __forceinline__ int scan_wide(const ListRows<float> &rows, const Line<float> &ln, const Line64 &l64, int ways,
+                                         int lane, int &bk, float &bt)
 {
-    constexpr bool kWide = sizeof(TA) > sizeof(TC); // FP64 scan over FP32 rows
-    TC cx = 0, cy = 0, cz = 0; // the vertex rounded to the scan precision
-    vx = vy = vz = TS(0);
-    ve = -1;
-    n = 0;
-    closed = false;
-    sbk = -1;
-    sdec = 0;
-    nsteps = 0;
-    int e = s, prev = -1;
-    bool any_near = false;
-    TC curc[3] = {(TC)p[0], (TC)p[1], (TC)p[2]}; // current point, scan precision
-    TA cur[3] = {(TA)p[0], (TA)p[1], (TA)p[2]};  // and in FP64 for the wide scan
-    for (int step = 0; step < kWalkSteps; ++step) {
-        nsteps = step + 1;
-        // direction of the edge line: w_eq x w_e (counter-clockwise about w_eq)
-        const vec4_t<TC> ref_ = rows[e];
-        const TC d0 = eqc.y * ref_.z - eqc.z * ref_.y;
-        const TC d1 = eqc.z * ref_.x - eqc.x * ref_.z;
-        const TC d2 = eqc.x * ref_.y - eqc.y * ref_.x;
-        const TC thr = par_eps * sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-        // first hit along the edge line, the scan split over the group
-        TA bt;
-        int bk;
-        if constexpr (kWide) {
-            const TA q0 = (TA)eqv[0], q1 = (TA)eqv[1], q2 = (TA)eqv[2];
-            const TA rx = (TA)ref_.x, ry = (TA)ref_.y, rz = (TA)ref_.z;
-            const TA D0 = q1 * rz - q2 * ry, D1 = q2 * rx - q0 * rz, D2 = q0 * ry - q1 * rx;
-            const TA thr64 = (TA)par_eps * sqrt(D0 * D0 + D1 * D1 + D2 * D2);
-            hit_scan_wide(rows, ALL, list, nlist, kGroup ? 32 * g.gw + lane : lane, kGroup ? 32 * g.G : 32, d0, d1, d2,
-                          thr, curc[0], curc[1], curc[2], D0, D1, D2, thr64, cur[0], cur[1], cur[2], e, prev, bt, bk);
-        } else {
-            bool nr = false;
-            hit_scan<TC, TC, kNear>(rows, ALL, list, nlist, kGroup ? 32 * g.gw + lane : lane, kGroup ? 32 * g.G : 32, d0,
-                                    d1, d2, thr, curc[0], curc[1], curc[2], e, prev, bt, bk, nr);
-            any_near = any_near || nr;
-        }
-        if (kGroup) {
-            const int par = step & 1;
-            TA *sbt = kWide ? (TA *)&g.sh->btd[par][0] : (TA *)&g.sh->bt[par][0];
-            if (lane == 0) {
-                sbt[g.gw] = bt;
-                g.sh->bk[par][g.gw] = bk;
-            }
-            g.sync();
-            bt = sbt[0];
-            bk = g.sh->bk[par][0];
-            for (int w = 1; w < g.G; ++w) {
-                const TA ot = sbt[w];
-                const int ok = g.sh->bk[par][w];
-                if (ot < bt || (ot == bt && ok < bk)) {
-                    bt = ot;
-                    bk = ok;
+    float tf[kList / 32], num[kList / 32], den[kList / 32]; // den 0: the quotient itself is in q
+    double q[kList / 32];
+#pragma unroll
+    for (int j = 0; j < kList / 32; ++j) {
+        const int pos = lane + 32 * j;
+        tf[j] = INFINITY;
+        q[j] = 0.0;
+        num[j] = den[j] = 0.f;
+        if (32 * j < rows.n && pos < rows.n && pos != ln.e && pos != ln.prev) {
+            const float4 r = rows.get(pos);
+            const float g = dot3(r.x, ln.c0, r.y, ln.c1, r.z, ln.c2) + r.w;
+            if (fabsf(g) < 2e-6f) {
+                const Cand64 c = near_zero64(r, l64);
+                if (c.ok) {
+                    q[j] = c.t;
+                    tf[j] = (float)c.t <= 3.4e38f ? (float)c.t : 3.4e38f;
+                }
+            } else {
+                const float a = dot3(r.x, ln.d0, r.y, ln.d1, r.z, ln.d2);
+                if (a > ln.thr) {
+                    num[j] = -g > 0.f ? -g : 0.f;
+                    den[j] = a;
+                    const float t = __fdividef(num[j], a);
+                    tf[j] = t <= 3.4e38f ? t : 3.4e38f;
                 }
             }
         }
-        if (bk == 0x7fffffff) { // the edge line never leaves the region
-            status = kOpen;
+    }
+    return choose<float>(rows, tf, ways, lane, bk, bt,
+                         [&](int j) { return den[j] != 0.f ? (double)num[j] / (double)den[j] : q[j]; });
+}
+
+// The rule itself over every row: `ways` lanes, 32 at a time, two interleaved
+// chains each (rows of a chain come in increasing order, so a later row never
+// wins a tie against the chain's earlier choice).
+template <typename TC, bool kNear>
+__device__ int scan(const GlobalRows<TC> &rows, const Line<TC> &ln, int ways, int lane, int &bk_out, float &bt_out, bool &near)
+{
+    TC wt = TC(INFINITY);
+    int wk = kNoHit;
+    bool nr = false;
+    for (int l0 = 0; l0 < ways; l0 += 32) {
+        TC bnum = TC(1), bden = TC(0), bnum1 = TC(1), bden1 = TC(0);
+        int bk = kNoHit, bk1 = kNoHit;
+        auto consider = [&](int k, TC &bn, TC &bd, int &bi) {
+            const vec4_t<TC> r = rows.get(k);
+            const TC a = dot3(r.x, ln.d0, r.y, ln.d1, r.z, ln.d2);
+            TC num = -(dot3(r.x, ln.c0, r.y, ln.c1, r.z, ln.c2) + r.w);
+            if (k == ln.e || k == ln.prev) return;
+            if (kNear) nr = nr || fabs(num) < TC(1e-6);
+            if (!(a > ln.thr)) return;
+            num = num > TC(0) ? num : TC(0);
+            if (mul_t(num, bd) < mul_t(bn, a)) {
+                bn = num;
+                bd = a;
+                bi = k;
+            }
+        };
+        int k = l0 + lane;
+        for (; k + ways < rows.n; k += 2 * ways) {
+            consider(k, bnum, bden, bk);
+            consider(k + ways, bnum1, bden1, bk1);
+        }
+        if (k < rows.n) consider(k, bnum, bden, bk);
+        const TC lhs = mul_t(bnum1, bden), rhs = mul_t(bnum, bden1);
+        if (bk1 != kNoHit && (lhs < rhs || (lhs == rhs && bk1 < bk))) {
+            bnum = bnum1;
+            bden = bden1;
+            bk = bk1;
+        }
+        const TC bt = bk == kNoHit ? TC(INFINITY) : bnum / bden;
+        if (bt < wt || (bt == wt && bk < wk)) {
+            wt = bt;
+            wk = bk;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const TC ot = __shfl_xor_sync(kFull, wt, o);
+        const int ok = __shfl_xor_sync(kFull, wk, o);
+        if (ot < wt || (ot == wt && ok < wk)) {
+            wt = ot;
+            wk = ok;
+        }
+    }
+    if (kNear) near = near || __any_sync(kFull, nr);
+    bk_out = wk;
+    bt_out = (float)wt;
+    return wk == kNoHit ? kNone : kHit;
+}
+__device__ int scan_wide(const GlobalRows<float> &rows, const Line<float> &ln, const Line64 &l64, int ways, int lane,
+                         int &bk_out, float &bt_out)
+{
+    double wt = INFINITY;
+    int wk = kNoHit;
+    for (int l0 = 0; l0 < ways; l0 += 32) {
+        float bnum = 1.f, bden = 0.f;
+        int bk = kNoHit, tk = kNoHit;
+        double tn = INFINITY;
+        for (int k = l0 + lane; k < rows.n; k += ways) {
+            if (k == ln.e || k == ln.prev) continue;
+            const float4 r = rows.get(k);
+            const float g = dot3(r.x, ln.c0, r.y, ln.c1, r.z, ln.c2) + r.w;
+            if (fabsf(g) < 2e-6f) {
+                const Cand64 c = near_zero64(r, l64);
+                if (c.ok && (c.t < tn || (c.t == tn && k < tk))) {
+                    tn = c.t;
+                    tk = k;
+                }
+                continue;
+            }
+            const float a = dot3(r.x, ln.d0, r.y, ln.d1, r.z, ln.d2);
+            if (!(a > ln.thr)) continue;
+            const float num = -g > 0.f ? -g : 0.f;
+            const float lhs = mul_t(num, bden), rhs = mul_t(bnum, a);
+            if (lhs < rhs || (lhs == rhs && k < bk)) {
+                bnum = num;
+                bden = a;
+                bk = k;
+            }
+        }
+        double bt = bk == kNoHit ? INFINITY : (double)bnum / (double)bden;
+        if (tk != kNoHit && (tn < bt || (tn == bt && tk < bk))) {
+            bt = tn;
+            bk = tk;
+        }
+        if (bt < wt || (bt == wt && bk < wk)) {
+            wt = bt;
+            wk = bk;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double ot = __shfl_xor_sync(kFull, wt, o);
+        const int ok = __shfl_xor_sync(kFull, wk, o);
+        if (ot < wt || (ot == wt && ok < wk)) {
+            wt = ot;
+            wk = ok;
+        }
+    }
+    bk_out = wk;
+    bt_out = (float)wt;
+    return wk == kNoHit ? kNone : kHit;
+}
+
+// ---------------------------------------------------------------- walk
+// A face while it is walked.  Lane i ends with vertex i (vx, vy, vz) and the
+// plane of the edge leaving it (ve); lane j records step j's hit plane (sbk) and
+// merge decision (sdec, 0 append, 1 merge with the previous vertex, 2 merge with
+// the first), nsteps the steps taken.  Planes are the row source's positions.
+template <typename TS>
+struct Face {
+    TS vx, vy, vz;
+    int ve, n;
+    bool closed;
+    int8_t status;
+    int sbk, sdec, nsteps;
+};
+
+// One face walk from the start plane s: the scan in TC (kWide: FP64 predicates
+// near zero), vertices solved in TS.  kNear: `near` is set when some step's scan
+// met a row within 1e-6 of the current point.  False (list only): a point left
+// the ball, or the rule needs every row; the face is not valid.
+template <typename TC, typename TS, bool kWide, bool kNear, typename Rows>
+__device__ bool walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *eqv, const TS *p,
+                     int s, TC par_eps, TS same_eps, int lane, Face<TS> &f, bool &near)
+{
+    TS last[3] = {0, 0, 0}, first[3] = {0, 0, 0}; // vertices appended last and first (every lane)
+    f.vx = f.vy = f.vz = TS(0);
+    f.ve = -1;
+    f.n = 0;
+    f.closed = false;
+    f.status = kOk;
+    f.sbk = -1;
+    f.sdec = 0;
+    f.nsteps = 0;
+    near = false;
+    Line<TC> ln;
+    ln.e = s;
+    ln.prev = -1;
+    ln.c0 = (TC)p[0]; // current point, scan precision
+    ln.c1 = (TC)p[1];
+    ln.c2 = (TC)p[2];
+    Line64 l64; // and in FP64 for the wide scan
+    if (kWide) {
+        l64.c0 = p[0];
+        l64.c1 = p[1];
+        l64.c2 = p[2];
+    }
+    if (!ball.in((float)ln.c0, (float)ln.c1, (float)ln.c2)) return false;
+    for (int step = 0; step < kWalkSteps; ++step) {
+        f.nsteps = step + 1;
+        // direction of the edge line: w_eq x w_e (counter-clockwise about w_eq)
+        const vec4_t<TC> r = rows.get(ln.e);
+        ln.d0 = diff2(eqc.y, r.z, eqc.z, r.y);
+        ln.d1 = diff2(eqc.z, r.x, eqc.x, r.z);
+        ln.d2 = diff2(eqc.x, r.y, eqc.y, r.x);
+        ln.thr = par_eps * sqrt(dot3(ln.d0, ln.d0, ln.d1, ln.d1, ln.d2, ln.d2));
+        int bk;
+        float bt;
+        int what;
+        if constexpr (kWide) {
+            const double rx = r.x, ry = r.y, rz = r.z;
+            l64.d0 = diff2((double)eqv[1], rz, (double)eqv[2], ry);
+            l64.d1 = diff2((double)eqv[2], rx, (double)eqv[0], rz);
+            l64.d2 = diff2((double)eqv[0], ry, (double)eqv[1], rx);
+            l64.par_eps = (double)par_eps;
+            what = scan_wide(rows, ln, l64, ways, lane, bk, bt);
+        } else {
+            what = scan<TC, kNear>(rows, ln, ways, lane, bk, bt, near);
+        }
+        if (what == kGiveUp) return false;
+        if (what == kNone) { // the edge line never leaves the region (or its ball)
+            if (ball.d2 != INFINITY) return false;
+            f.status = kOpen;
             break;
         }
+        if (!ball.in((float)ln.c0 + bt * (float)ln.d0, (float)ln.c1 + bt * (float)ln.d1, (float)ln.c2 + bt * (float)ln.d2))
+            return false;
         // vertex = 3x3 solve of (edge plane, hit plane, face plane)
         TS V[3];
         TC Vc[3];
-        if (!warp_solve<TC, TS>(rows, e, bk, eqv, V, Vc, lane)) {
-            status = kSingular;
+        if (!warp_solve<TC, TS>(r, rows.get(bk), eqv, V, Vc, lane)) {
+            f.status = kSingular;
             break;
         }
         // 0 append, 1 zero-length edge on e (merge), 2 zero-length closing edge;
         // decided in the solve precision (on the scan-precision copies
         // where the rounding margin settles it)
         int decision = 0;
-        if (n > 0) {
+        if (f.n > 0) {
             int s1 = -1, s2 = 0;
             if (sizeof(TS) > sizeof(TC)) {
-                s1 = same_filter<TC, TS>(Vc, __shfl_sync(0xffffffffu, cx, n - 1),
-                                         __shfl_sync(0xffffffffu, cy, n - 1),
-                                         __shfl_sync(0xffffffffu, cz, n - 1), same_eps);
-                if (bk == s && s1 == 0)
-                    s2 = same_filter<TC, TS>(Vc, __shfl_sync(0xffffffffu, cx, 0),
-                                             __shfl_sync(0xffffffffu, cy, 0),
-                                             __shfl_sync(0xffffffffu, cz, 0), same_eps);
+                s1 = same_filter<TC, TS>(Vc, (TC)last[0], (TC)last[1], (TC)last[2], same_eps);
+                if (bk == s && s1 == 0) s2 = same_filter<TC, TS>(Vc, (TC)first[0], (TC)first[1], (TC)first[2], same_eps);
             }
             if (s1 == 1) {
                 decision = 1;
             } else if (s1 == 0 && s2 != -1) {
                 decision = s2 == 1 ? 2 : 0;
             } else {
-                const TS lx = __shfl_sync(0xffffffffu, vx, n - 1);
-                const TS ly = __shfl_sync(0xffffffffu, vy, n - 1);
-                const TS lz = __shfl_sync(0xffffffffu, vz, n - 1);
-                if (lane == 0) { // in the solve precision, on one lane
-                    if (fabs(V[0] - lx) + fabs(V[1] - ly) + fabs(V[2] - lz) < same_eps)
-                        decision = 1;
-                    else if (bk == s && fabs(V[0] - vx) + fabs(V[1] - vy) + fabs(V[2] - vz) < same_eps)
-                        decision = 2;
-                }
-                decision = __shfl_sync(0xffffffffu, decision, 0);
+                if (fabs(V[0] - last[0]) + fabs(V[1] - last[1]) + fabs(V[2] - last[2]) < same_eps)
+                    decision = 1;
+                else if (bk == s && fabs(V[0] - first[0]) + fabs(V[1] - first[1]) + fabs(V[2] - first[2]) < same_eps)
+                    decision = 2;
             }
         }
         if (lane == step) {
-            sbk = bk;
-            sdec = decision;
+            f.sbk = bk;
+            f.sdec = decision;
         }
-        if (decision == 1 && lane == n - 1) ve = bk; // the edge on e has zero length
-        const bool appended = (decision == 0);
-        if (appended) {
-            if (lane == n) {
-                vx = V[0];
-                vy = V[1];
-                vz = V[2];
-                cx = Vc[0];
-                cy = Vc[1];
-                cz = Vc[2];
-                ve = bk;
+        if (decision == 1 && lane == f.n - 1) f.ve = bk; // the edge on e has zero length
+        if (decision == 0) {
+            if (lane == f.n) {
+                f.vx = V[0];
+                f.vy = V[1];
+                f.vz = V[2];
+                f.ve = bk;
             }
-            n++;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                last[j] = V[j];
+                if (f.n == 0) first[j] = V[j];
+            }
+            f.n++;
         }
         if (bk == s) {
-            closed = true;
+            f.closed = true;
             break;
         }
-        if (n >= kVMax) {
-            status = kTruncated;
+        if (f.n >= kVMax) {
+            f.status = kTruncated;
             break;
         }
-        prev = e;
-        e = bk;
-        curc[0] = Vc[0];
-        curc[1] = Vc[1];
-        curc[2] = Vc[2];
+        ln.prev = ln.e;
+        ln.e = bk;
+        ln.c0 = Vc[0];
+        ln.c1 = Vc[1];
+        ln.c2 = Vc[2];
         if (kWide) {
-            cur[0] = (TA)V[0];
-            cur[1] = (TA)V[1];
-            cur[2] = (TA)V[2];
+            l64.c0 = V[0];
+            l64.c1 = V[1];
+            l64.c2 = V[2];
         }
+        if (!ball.in((float)ln.c0, (float)ln.c1, (float)ln.c2)) return false;
     }
-    if (!closed && status == kOk) status = kTruncated;
-    if (near) *near = any_near;
+    if (!f.closed && f.status == kOk) f.status = kTruncated;
+    return true;
 }
 
 // Mixed form: the walk runs in the scan precision TC (solves included, as the
@@ -585,35 +849,26 @@ __device__ void walk(const vec4_t<TC> *rows, int ALL, const uint16_t *list, int 
 // vertex (the four Cramer determinants), eight vertices per warp instruction
 // -- and every merge decision is taken again on the TS vertices.  When all
 // decisions agree, the face is the TS walk's face: the same hit planes, the
-// same TS vertices.  Returns false, and the caller walks again with every
+// same TS vertices.  Returns kAgain, and the caller walks again with every
 // predicate and every solve in TS, when a scan met a row within 1e-6 of the
 // current point other than the two it lies on (a sign or feasibility test
 // near zero), when the TC walk did not close normally, took more than 32
 // steps or met a vertex that is not finite in TS, or when a decision comes
-// out differently in TS.
-template <typename TC, typename TS, bool kGroup>
-__device__ bool walk_refined(const vec4_t<TC> *rows, int ALL, const uint16_t *list, int nlist, const vec4_t<TC> &eqc,
-                             const TS *eqv, const TS *p, int s, TC par_eps, TS same_eps, int lane, TS &vx, TS &vy,
-                             TS &vz, int &ve, int &n, bool &closed, int8_t &status, const Grp<TC> &g)
+// out differently in TS; kLeft when the walk left the list (see walk).
+enum : int { kRefined = 0, kAgain = 1, kLeft = 2 };
+template <typename TC, typename TS, typename Rows>
+__device__ int walk_refined(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *eqv,
+                            const TS *p, int s, TC par_eps, TS same_eps, int lane, Face<TS> &f)
 {
-    const unsigned full = 0xffffffffu;
+    const unsigned full = kFull;
     const TC eqf[4] = {eqc.x, eqc.y, eqc.z, eqc.w};
     const TC pf[3] = {(TC)p[0], (TC)p[1], (TC)p[2]};
-    TC fx, fy, fz;
-    int fve, fn, sbk, sdec, nsteps;
-    bool fclosed;
-    int8_t fst = kOk;
-    bool near = false;
-    walk<TC, TC, kGroup, TC, true>(rows, ALL, list, nlist, eqc, eqf, pf, s, par_eps, (TC)same_eps, lane, fx, fy, fz,
-                                   fve, fn, fclosed, fst, sbk, sdec, nsteps, g, &near);
-    if (kGroup) { // a row near a vertex in any warp's share of the scan
-        if (near && lane == 0) atomicOr(&g.sh->near, 1);
-        g.sync();
-        near = g.sh->near != 0;
-    }
+    Face<TC> w;
+    bool near;
+    if (!walk<TC, TC, false, true>(rows, ball, ways, eqc, eqf, pf, s, par_eps, (TC)same_eps, lane, w, near)) return kLeft;
+    const int sbk = w.sbk, sdec = w.sdec, nsteps = w.nsteps;
     // a predicate near zero: the caller walks again with FP64 predicates
-    if (near || fst != kOk || !fclosed || nsteps < 1 || nsteps > 32) return false;
-    if (kGroup && g.gw != 0) return true; // the leader refines; the caller shares its outcome
+    if (near || w.status != kOk || !w.closed || nsteps < 1 || nsteps > 32) return kAgain;
 
     // step j's vertex in TS, into lane j
     const int G = lane >> 2, L = lane & 3, gbase = lane & ~3;
@@ -624,13 +879,12 @@ __device__ bool walk_refined(const vec4_t<TC> *rows, int ALL, const uint16_t *li
         const int pb = __shfl_sync(full, sbk, j);          // its hit plane
         const int pj = __shfl_sync(full, sbk, max(j - 1, 0));
         const int pa = j == 0 ? s : pj;                    // and the edge plane it walked on
-        const bool in = (unsigned)pa < (unsigned)ALL && (unsigned)pb < (unsigned)ALL;
+        const bool in = (unsigned)pa < (unsigned)rows.n && (unsigned)pb < (unsigned)rows.n;
         planes_ok = planes_ok && in;
-        const TC *ra = reinterpret_cast<const TC *>(rows + (in ? pa : 0));
-        const TC *rb = reinterpret_cast<const TC *>(rows + (in ? pb : 0));
         // lane t of the group converts components 2t, 2t + 1 of [row a | row b]
-        const TS c0 = (TS)(L < 2 ? ra[2 * L] : rb[2 * L - 4]);
-        const TS c1 = (TS)(L < 2 ? ra[2 * L + 1] : rb[2 * L - 3]);
+        const vec4_t<TC> rr = rows.get(in ? (L < 2 ? pa : pb) : 0);
+        const TS c0 = (TS)(L & 1 ? rr.z : rr.x);
+        const TS c1 = (TS)(L & 1 ? rr.w : rr.y);
         TS m[8];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
@@ -651,7 +905,7 @@ __device__ bool walk_refined(const vec4_t<TC> *rows, int ALL, const uint16_t *li
         }
     }
     const bool mine = lane < nsteps;
-    if (!__all_sync(full, planes_ok && (!mine || (finite_bits(rx) && finite_bits(ry) && finite_bits(rz))))) return false;
+    if (!__all_sync(full, planes_ok && (!mine || (finite_bits(rx) && finite_bits(ry) && finite_bits(rz))))) return kAgain;
 
     // the decisions again, on the TS vertices: step j against the last
     // vertex appended before it and, on the closing step, the first vertex
@@ -671,583 +925,497 @@ __device__ bool walk_refined(const vec4_t<TC> *rows, int ALL, const uint16_t *li
         if (check && s2 < 0) s2 = (fabs(rx - Fx) + fabs(ry - Fy) + fabs(rz - Fz) < same_eps) ? 1 : 0;
     }
     const int dec = s1 == 1 ? 1 : (sbk == s && s2 == 1 ? 2 : 0);
-    if (!__all_sync(full, !check || dec == sdec)) return false;
+    if (!__all_sync(full, !check || dec == sdec)) return kAgain;
 
     // vertex o is the o-th appended step; its edge is the hit plane of the
     // last step before the next append, a closing merge excepted
-    n = __popc(amask);
-    const int so = lane < n ? (int)__fns(amask, 0, lane + 1) : 0;
-    const int snext = lane + 1 < n ? (int)__fns(amask, 0, lane + 2) : nsteps;
+    f.n = __popc(amask);
+    const int so = lane < f.n ? (int)__fns(amask, 0, lane + 1) : 0;
+    const int snext = lane + 1 < f.n ? (int)__fns(amask, 0, lane + 2) : nsteps;
     int kl = (snext - 1) & 31;
     if (__shfl_sync(full, sdec, kl) == 2) kl = (kl - 1) & 31;
     const int e_out = __shfl_sync(full, sbk, kl);
     const TS ox = __shfl_sync(full, rx, so), oy = __shfl_sync(full, ry, so), oz = __shfl_sync(full, rz, so);
-    if (lane < n) {
-        vx = ox;
-        vy = oy;
-        vz = oz;
-        ve = e_out;
+    if (lane < f.n) {
+        f.vx = ox;
+        f.vy = oy;
+        f.vz = oz;
+        f.ve = e_out;
     } else {
-        vx = vy = vz = TS(0);
-        ve = -1;
+        f.vx = f.vy = f.vz = TS(0);
+        f.ve = -1;
     }
-    closed = true;
-    status = kOk;
-    return true;
+    f.closed = true;
+    f.status = kOk;
+    return kRefined;
 }
 
-// Row pruning before the walk.  The face polygon is the intersection of the
-// half-planes the rows cut out of the face plane.  In coordinates u of that
-// plane centred on the start point p, row k reads m_k . u <= c_k, with
-// c_k = -(w_k . p + b_k) the distance from p to the row's plane (the rows are
-// normalised) and m_k the in-plane part of w_k.  For c_k > 0 the row's dual
-// point q_k = m_k / c_k lies strictly inside the convex hull of the other dual
-// points and the origin exactly when the row's line misses the polygon (the
-// polar of a polygon around p): such a row is never the first plane the walk
-// hits on an edge.  A sample of the rows (every eighth) gives, for eight
-// directions, the extreme dual points; their convex polygon lies inside that
-// hull, and so does the circle of radius r around the origin inscribed in it.
-// Every row whose dual point lies inside 0.98 r -- computed with c_k lowered
-// by a bound on its rounding -- is dropped, and the walk scans the kept rows
-// only, so its decisions (the first hit, ties to the lower row) are those of
-// the scan over every row.  Rows through or near p and rows that are not
-// finite are always kept; the sample uses only rows with c_k well above the
-// rounding bound, so that its dual points are accurate.  Returns the number
-// of kept rows (their indices in sh->list), or -1 -- the walk scans every
-// row -- when the sample gives no circle or more than kListCap rows are kept.
-template <typename TC, bool kGroup>
-__device__ int prune_rows(const vec4_t<TC> *rows, int ALL, const vec4_t<TC> &eqc, const TC *pc, int lane,
-                          const Grp<TC> &g)
+template <typename TC, typename TS, typename Rows>
+__device__ bool walk_fp64(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *p,
+                                       int s, TC par_eps, TS same_eps, int lane, Face<TS> &f)
 {
-    const unsigned full = 0xffffffffu;
-    GroupShared<TC> *sh = g.sh;
-    const int w = kGroup ? g.gw : 0, G = kGroup ? g.G : 1;
-    // orthonormal basis (e1, e2) of the face plane
-    TC nx = eqc.x, ny = eqc.y, nz = eqc.z;
-    const TC nn = nx * nx + ny * ny + nz * nz;
-    if (!(nn > TC(0)) || !finite_bits(nn)) return -1; // uniform: every lane reads the same plane
-    const TC inv = rsqrt(nn);
-    nx *= inv;
-    ny *= inv;
-    nz *= inv;
-    const TC ax = (fabs(nx) <= fabs(ny) && fabs(nx) <= fabs(nz)) ? TC(1) : TC(0);
-    const TC ay = (ax == TC(0) && fabs(ny) <= fabs(nz)) ? TC(1) : TC(0);
-    const TC az = (ax == TC(0) && ay == TC(0)) ? TC(1) : TC(0);
-    TC e1x = ay * nz - az * ny, e1y = az * nx - ax * nz, e1z = ax * ny - ay * nx;
-    const TC i1 = rsqrt(e1x * e1x + e1y * e1y + e1z * e1z);
-    e1x *= i1;
-    e1y *= i1;
-    e1z *= i1;
-    const TC e2x = ny * e1z - nz * e1y, e2y = nz * e1x - nx * e1z, e2z = nx * e1y - ny * e1x;
-    const TC p0 = pc[0], p1 = pc[1], p2 = pc[2];
-    // rounding of c_k in TC, and the sample's floor on c_k
-    const TC dc = (sizeof(TC) == 4 ? TC(1e-6) : TC(1e-14)) * (TC(1) + fabs(p0) + fabs(p1) + fabs(p2));
-    const TC cmin = TC(1000) * dc;
-    if (w == 0 && lane == 0) sh->nlist = 0;
+    const TS eqv[4] = {(TS)eqc.x, (TS)eqc.y, (TS)eqc.z, (TS)eqc.w};
+    bool near;
+    return walk<TC, TS, true, false>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f, near);
+}
 
-    // sample: the extreme dual point in directions 0, 45, ..., 315 degrees
-    TC bv[8];
-    int bi[8];
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-        bv[m] = TC(-INFINITY);
-        bi[m] = 0x7fffffff;
+// The whole walk of a form over one row source; false: the list does not do.
+template <typename TC, typename TS, typename Rows>
+__device__ bool face_walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *eqv, const TS *p,
+                          int s, TC par_eps, TS same_eps, int lane, Face<TS> &f, bool &again)
+{
+    again = false;
+    if constexpr (sizeof(TS) > sizeof(TC)) { // scan-precision walk, vertices refined in the solve precision
+        const int r = walk_refined<TC, TS>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f);
+        if (r == kRefined) return true;
+        if (r == kLeft) return false;
+        again = true; // FP64 predicates and FP64 solves
+        return walk_fp64<TC, TS>(rows, ball, ways, eqc, p, s, par_eps, same_eps, lane, f);
+    } else {
+        bool near;
+        return walk<TC, TS, false, false>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f, near);
     }
-    for (int k = 8 * (32 * w + lane); k < ALL; k += 8 * 32 * G) {
-        const vec4_t<TC> r = rows[k];
-        const TC c = -(r.x * p0 + r.y * p1 + r.z * p2 + r.w);
-        if (!(c >= cmin) || !finite_bits(c)) continue;
-        const TC ic = TC(1) / c;
-        const TC qx = (r.x * e1x + r.y * e1y + r.z * e1z) * ic;
-        const TC qy = (r.x * e2x + r.y * e2y + r.z * e2z) * ic;
-        const TC v[8] = {qx, qx + qy, qy, qy - qx, -qx, -qx - qy, -qy, qx - qy};
-#pragma unroll
-        for (int m = 0; m < 8; ++m)
-            if (v[m] > bv[m]) {
-                bv[m] = v[m];
-                bi[m] = k;
+}
+
+// ---------------------------------------------------------------- seeds
+// Start vertex of a seed region: the start plane's position and the vertex in
+// p, -1 when no pair is feasible, -2 when the list cannot decide (it does not
+// surely hold the nearest planes).  Every row outside the list holds at a point
+// of the ball; elsewhere the rows are tested one by one.
+template <typename TC, typename TS, typename Rows>
+__device__ int seed_start(const Rows &rows, const GlobalRows<TC> &all, const Ball &ball, float T, const TS *eqv, TS *p, TC eps,
+                          int lane)
+{
+    // pairs x <= 812 reach sorted positions up to 56: keep the 64 nearest,
+    // position q in lane q % 32, register q / 32
+    const int ksel = all.n < kTopK ? all.n : kTopK;
+    if (rows.n < ksel) return -2;
+    int top0 = -1, top1 = -1;
+    unsigned long long pk = ~0ull;
+    int pi = -1;
+    const TC pc[3] = {(TC)p[0], (TC)p[1], (TC)p[2]};
+    for (int sel = 0; sel < ksel; ++sel) {
+        unsigned long long bk = 0ull;
+        int bi = kNoHit;
+        for (int k = lane; k < rows.n; k += 32) {
+            const vec4_t<TC> v = rows.get(k);
+            const TC d = dot3(v.x, pc[0], v.y, pc[1], v.z, pc[2]) + v.w;
+            const unsigned long long key = order_key(d);
+            const bool below = key < pk || (key == pk && k > pi);
+            if (below && ahead(key, k, bk, bi)) {
+                bk = key;
+                bi = k;
             }
-    }
-#pragma unroll
-    for (int m = 0; m < 8; ++m)
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            const TC ov = __shfl_xor_sync(full, bv[m], o);
-            const int oi = __shfl_xor_sync(full, bi[m], o);
-            if (ov > bv[m] || (ov == bv[m] && oi < bi[m])) {
-                bv[m] = ov;
-                bi[m] = oi;
+            const unsigned long long ok = __shfl_xor_sync(kFull, bk, o);
+            const int oi = __shfl_xor_sync(kFull, bi, o);
+            if (ahead(ok, oi, bk, bi)) {
+                bk = ok;
+                bi = oi;
             }
         }
-    if (kGroup) {
-        if (lane < 8) {
-            TC v = bv[0];
-            int i = bi[0];
-#pragma unroll
-            for (int m = 1; m < 8; ++m)
-                if (lane == m) v = bv[m], i = bi[m];
-            sh->ext.v[w][lane] = v;
-            sh->ext.i[w][lane] = (int16_t)(i == 0x7fffffff ? -1 : i);
+        if (lane == (sel & 31)) {
+            if (sel < 32) top0 = bi;
+            else top1 = bi;
         }
-        g.sync();
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            bv[m] = TC(-INFINITY);
-            bi[m] = 0x7fffffff;
-            for (int u = 0; u < G; ++u) {
-                const TC ov = sh->ext.v[u][m];
-                const int oi = sh->ext.i[u][m] < 0 ? 0x7fffffff : (int)sh->ext.i[u][m];
-                if (ov > bv[m] || (ov == bv[m] && oi < bi[m])) {
-                    bv[m] = ov;
-                    bi[m] = oi;
-                }
+        pk = bk;
+        pi = bi;
+    }
+    if (ball.d2 != INFINITY) { // the farthest chosen plane well inside T: no plane left out is nearer
+        const vec4_t<TC> v = rows.get(pi);
+        const float c = -(float)(dot3(v.x, pc[0], v.y, pc[1], v.z, pc[2]) + v.w);
+        if (!(c < T * 0.999f - 1e-5f * coord_size(ball.x, ball.y, ball.z))) return -2;
+    }
+    int x_max = (all.n - 1) * (all.n - 2);
+    if (x_max > 812) x_max = 812;
+    if (x_max < 0) x_max = 0;
+    for (int x = 0; x <= x_max; ++x) {
+        int i, j;
+        get_i_j(x, all.n, i, j);
+        const int ri0 = __shfl_sync(kFull, top0, i & 31), ri1 = __shfl_sync(kFull, top1, i & 31);
+        const int rj0 = __shfl_sync(kFull, top0, j & 31), rj1 = __shfl_sync(kFull, top1, j & 31);
+        const int ri = i < 32 ? ri0 : ri1;
+        const int rj = j < 32 ? rj0 : rj1;
+        TS v[3];
+        TC vc[3];
+        warp_solve<TC, TS>(rows.get(ri), rows.get(rj), eqv, v, vc, lane);
+        bool bad = false;
+        for (int k = lane; k < rows.n; k += 32) {
+            if (k == ri || k == rj) continue;
+            const vec4_t<TC> r = rows.get(k);
+            if (dot3(r.x, vc[0], r.y, vc[1], r.z, vc[2]) + r.w > eps) bad = true;
+        }
+        if (__any_sync(kFull, bad)) continue;
+        if (ball.d2 != INFINITY && !ball.in((float)vc[0], (float)vc[1], (float)vc[2])) {
+            const int ki = rows.name(ri), kj = rows.name(rj);
+            for (int k = lane; k < all.n; k += 32) {
+                if (k == ki || k == kj) continue;
+                const vec4_t<TC> r = all.get(k);
+                if (dot3(r.x, vc[0], r.y, vc[1], r.z, vc[2]) + r.w > eps) bad = true;
             }
+            if (__any_sync(kFull, bad)) continue;
         }
-        g.sync(); // every warp has read the extremes: the list may overwrite them
+        p[0] = v[0];
+        p[1] = v[1];
+        p[2] = v[2];
+        return ri;
     }
-    // the extreme points in counter-clockwise order (lane m < 8: direction
-    // m), and the radius of the circle around the origin inscribed in their
-    // polygon: the smallest distance from the origin to an edge, which must
-    // have the origin strictly on its left
-    bool ok = true;
-#pragma unroll
-    for (int m = 0; m < 8; ++m) ok = ok && bi[m] != 0x7fffffff;
-    if (!ok) return -1; // a direction without a sampled row: the polygon may be open that way
-    int mine = bi[0];
-#pragma unroll
-    for (int m = 1; m < 8; ++m)
-        if ((lane & 7) == m) mine = bi[m];
-    const vec4_t<TC> er = rows[mine];
-    const TC eic = TC(1) / -(er.x * p0 + er.y * p1 + er.z * p2 + er.w);
-    const TC qx = (er.x * e1x + er.y * e1y + er.z * e1z) * eic;
-    const TC qy = (er.x * e2x + er.y * e2y + er.z * e2z) * eic;
-    const int nxt = (lane + 1) & 7;
-    const TC qx1 = __shfl_sync(full, qx, nxt), qy1 = __shfl_sync(full, qy, nxt);
-    const int bi1 = __shfl_sync(full, mine, nxt);
-    const bool edge = lane < 8 && bi1 != mine;
-    const TC dx = qx1 - qx, dy = qy1 - qy;
-    const TC cr = dy * qx - dx * qy; // (E1 - E0) x (O - E0)
-    const TC len = sqrt(dx * dx + dy * dy);
-    const bool bad = edge && !(cr > TC(0) && len > TC(0));
-    TC rad = edge && !bad ? cr / len : TC(INFINITY);
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) rad = fmin(rad, __shfl_xor_sync(full, rad, o));
-    rad = __shfl_sync(full, rad, 0);
-    const int edges = __popc(__ballot_sync(full, edge));
-    if (__any_sync(full, bad) || edges < 3 || !(rad > TC(0)) || !finite_bits(rad)) return -1;
-    const TC re = TC(0.98) * rad;
-    const TC re2 = re * re;
-
-    // every row: keep those whose dual point may lie outside the circle
-    for (int k0 = 32 * w; k0 < ALL; k0 += 32 * G) {
-        const int k = k0 + lane;
-        bool keep = false;
-        if (k < ALL) {
-            const vec4_t<TC> r = rows[k];
-            const TC c = -(r.x * p0 + r.y * p1 + r.z * p2 + r.w) - dc;
-            const TC m1 = r.x * e1x + r.y * e1y + r.z * e1z;
-            const TC m2 = r.x * e2x + r.y * e2y + r.z * e2z;
-            keep = !(c > TC(0)) || !(m1 * m1 + m2 * m2 < re2 * c * c);
-        }
-        const unsigned b = __ballot_sync(full, keep);
-        if (b) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(&sh->nlist, __popc(b));
-            base = __shfl_sync(full, base, 0);
-            const int pos = base + __popc(b & ((1u << lane) - 1u));
-            if (keep && pos < kListCap) sh->list[pos] = (uint16_t)k;
-        }
-    }
-    if (kGroup)
-        g.sync();
-    else
-        __syncwarp();
-    const int nl = sh->nlist;
-    return nl <= kListCap ? nl : -1;
+    return -1;
 }
 
-// Rows are staged normalised (|w| = 1, zero rows become 0.x + sign(b) inf):
-// signed geometric distances are then plain dot products, the same quantity
-// the reference's feasibility test computes as (w.x + b) * rsqrt(|w|^2)
-// (kernel.h:729-795).  TC is the scan precision, TS the solve precision.
-template <typename TC, typename TS, bool kGroup>
-__global__ void __launch_bounds__(256, 3) polygon_kernel(NetDev net, RegionsDev reg, ChunkDev ch, HashDev hs, Tolerances tol,
-                                                      int G_, int prune, unsigned long long *nfp64, int *err)
+// What the kernel needs of a face's walk.
+template <typename TS>
+struct Result {
+    TS vx, vy, vz; // lane i: vertex i
+    int ve;        // and the plane of the edge leaving it (-1: none)
+    int n, start;  // vertices; start plane
+    bool closed, again;
+    int8_t status;
+    float T;       // radius of the list used last, and the rows in it
+    int listed;
+};
+
+// Everything but the common face (a region with a parent whose FP32 walk stays in
+// its list and needs no FP64 predicate): seeds, repeats with another radius, FP64
+// predicates, every row.  Kept out of the kernel's registers.  `again`: only
+// the FP64 predicates are asked for, on the list as it is.
+template <typename TC, typename TS>
+__device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *list, int ways, const vec4_t<TC> &eqc,
+                                       const TS *mid, int start, TC eps, TC par_eps, TS same_eps, int lane, bool again,
+                                       int n, float T, Result<TS> &out)
 {
-    const int G = kGroup ? G_ : 1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int F = (blockDim.x >> 5) / G; // faces per block
-    const int gid = wib / G;
-    const int ALL = net.ALL;
-    const int N = net.N;
-    const int W = net.W;
-    vec4_t<TC> *rows = reinterpret_cast<vec4_t<TC> *>(smem_raw) + (size_t)gid * net.ALLP;
-    Grp<TC> g;
-    g.G = G;
-    g.gw = wib % G;
-    g.bar = 1 + gid;
-    g.sh = reinterpret_cast<GroupShared<TC> *>(smem_raw + (size_t)F * net.ALLP * sizeof(vec4_t<TC>) +
-                                               (size_t)gid * group_shared_bytes<TC>());
-    // (the group's shared block also holds the pruning list: one per face)
-    const TC eps = (TC)tol.eps, par_eps = (TC)tol.par_eps;
-    const TS same_eps = (TS)tol.same_eps;
-
-    long long head;
-    int count;
-    chunk_range(ch, head, count);
-    // a region per group: by launch position, or (fixed grid of the
-    // graph-driven loop) from the wave's work counter; the leader takes it
-    // and the group reads it from shared memory
-    long long rl_next = (long long)blockIdx.x * F + gid;
-    if (g.gw == 0 && lane == 0) {
-        umma::mbar_init(&g.sh->rbar, 1);
-        umma::fence_mbar_init();
+    const bool is_seed = start < 0;
+    const TS eqv[4] = {(TS)eqc.x, (TS)eqc.y, (TS)eqc.z, (TS)eqc.w};
+    TS p[3] = {mid[0], mid[1], mid[2]};
+    Ball ball{(float)p[0], (float)p[1], (float)p[2], -1.f};
+    const float size = coord_size(ball.x, ball.y, ball.z);
+    Face<TS> f;
+    bool done = false, wide = false;
+    int s = start, s_plane = start;
+    auto clear = [&] {
+        f.vx = f.vy = f.vz = TS(0);
+        f.n = 0;
+        f.ve = -1;
+        f.closed = false;
+        f.status = kNoStart;
+    };
+    clear();
+    if (is_seed) {
+        T = all.n > kList ? seed_radius<TC>(all, ball, lane) : INFINITY;
+        n = -1;
     }
-    uint32_t rphase = 0; // faces taken by this group: the row barrier's phase
-    for (;;) {
-        long long rl;
-        if (g.gw == 0) {
-            rl = ch.ctl ? next_work(ch.ctl, lane) : rl_next;
-            if (kGroup && lane == 0) {
-                g.sh->rl = rl;
-                g.sh->near = 0;
+    for (int tries = 0; tries < 5 && !done; ++tries) {
+        if (n < 0) n = collect<TC>(all, T, ball, list, lane);
+        if (n > kList) { // a smaller ball
+            T *= (float)kTarget / (float)n;
+            n = -1;
+            continue;
+        }
+        const ListRows<TC> rows{list, n};
+        ball.d2 = ball_radius2(T, size);
+        TS q[3] = {p[0], p[1], p[2]};
+        if (!is_seed) {
+            s = position<TC>(list, n, start, lane);
+        } else {
+            s = seed_start<TC, TS>(rows, all, ball, T, eqv, q, eps, lane);
+            if (s == -1) { // no feasible start
+                done = true;
+                s_plane = -1;
+                break;
             }
         }
-        rl_next += (long long)gridDim.x * F;
-        if (kGroup) {
-            g.sync();
-            rl = g.sh->rl;
-        }
-        if (rl >= count) break;
-        const long long rid = head + rl;
-        // the region's rows into shared memory by bulk copies (the leader
-        // issues them once every warp of the group is done with the previous
-        // face's rows), then normalised in place.  The first nsplit rows come
-        // from the parent's slot; they are the region's own but for the sign
-        // of the plane it was entered through, and are copied into its slot
-        // for its children.
-        vec4_t<TC> *grows = reinterpret_cast<vec4_t<TC> *>((TC *)ch.cons + (size_t)row_slot(ch, head, (int)rl) * net.ALLP * 4);
-        const int nsplit = ch.split ? ch.split[rl] : 0;
-        const int flip = nsplit ? reg.start[rid] : -1;
-        {
-            const uint32_t rbytes = (uint32_t)ALL * (uint32_t)sizeof(vec4_t<TC>);
-            if (!kGroup) __syncwarp(); // (a group has met at its barrier above)
-            if (g.gw == 0 && lane == 0) {
-                umma::fence_proxy_async(); // earlier generic reads of the rows before the copy's writes
-                umma::mbar_expect_tx(&g.sh->rbar, rbytes);
-                const uint32_t pbytes = (uint32_t)nsplit * (uint32_t)sizeof(vec4_t<TC>);
-                if (nsplit) {
-                    const TC *pr = (const TC *)ch.cons + (size_t)ring_slot(ch, reg.parent[rid]) * net.ALLP * 4;
-                    umma::bulk_g2s(rows, pr, pbytes, &g.sh->rbar);
-                }
-                if (rbytes > pbytes) umma::bulk_g2s(rows + nsplit, grows + nsplit, rbytes - pbytes, &g.sh->rbar);
-            }
-            if (!umma::mbar_wait(&g.sh->rbar, rphase & 1u, kRowWaitIters)) {
-                atomicOr(err, kErrWait);
-                umma::mbar_wait(&g.sh->rbar, rphase & 1u, kRowWaitIters); // nothing lands after the face is left
-            }
-            ++rphase;
-        }
-        for (int q = 32 * g.gw + lane; q < ALL; q += 32 * G) {
-            vec4_t<TC> v = rows[q];
-            if (q == flip) {
-                v.x = -v.x;
-                v.y = -v.y;
-                v.z = -v.z;
-                v.w = -v.w;
-            }
-            if (q < nsplit) grows[q] = v;
-            const TC n2 = norm2(v.x, v.y, v.z);
-            if (n2 > TC(0)) {
-                const TC inv = rsqrt(n2); // as the reference's distance normalisation
-                v.x *= inv;
-                v.y *= inv;
-                v.z *= inv;
-                v.w *= inv;
-            } else {
-                v.w = v.w > TC(0) ? TC(INFINITY) : (v.w < TC(0) ? TC(-INFINITY) : TC(NAN));
-            }
-            rows[q] = v;
-        }
-        if (kGroup)
-            g.sync();
-        else
-            __syncwarp();
-        TS eqv[4];
-        const vec4_t<TC> eqc = ld4<TC>((const TC *)ch.eq + (size_t)rl * 4); // scan precision copy
-        eqv[0] = (TS)eqc.x;
-        eqv[1] = (TS)eqc.y;
-        eqv[2] = (TS)eqc.z;
-        eqv[3] = (TS)eqc.w;
-        const TS *midp = (const TS *)reg.mid + (size_t)rid * 4;
-        TS p[3] = {midp[0], midp[1], midp[2]};
-        int s = reg.start[rid];
-        const bool is_seed = (s < 0);
-        int8_t status = kOk;
-
-        // ---------------------------------------------------- seed start search
-        if (is_seed) {
-            // pairs x <= 812 reach sorted positions up to 56: keep the 64 nearest,
-            // position q in lane q % 32, register q / 32.  In a group, every
-            // selection pass splits the rows over the warps (the partial
-            // choices meet in shared memory), and the warps test G pairs at a
-            // time, the smallest feasible x winning (measured on GB300: with
-            // every warp repeating the whole search, the seeds of a 4,096-row
-            // network took a whole wave's time)
-            const int ksel = ALL < kTopK ? ALL : kTopK;
-            const int k0 = kGroup ? 32 * g.gw + lane : lane, ks = kGroup ? 32 * G : 32;
-            int top0 = -1, top1 = -1;
-            unsigned long long pk = ~0ull;
-            int pi = -1;
-            const TC pc[3] = {(TC)p[0], (TC)p[1], (TC)p[2]};
-            for (int sel = 0; sel < ksel; ++sel) {
-                unsigned long long bk = 0ull;
-                int bi = 0x7fffffff;
-                for (int k = k0; k < ALL; k += ks) {
-                    const vec4_t<TC> v = rows[k];
-                    const TC d = v.x * pc[0] + v.y * pc[1] + v.z * pc[2] + v.w;
-                    const unsigned long long key = order_key<TC>(d);
-                    const bool below = key < pk || (key == pk && k > pi);
-                    if (below && ahead(key, k, bk, bi)) {
-                        bk = key;
-                        bi = k;
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const unsigned long long ok = __shfl_xor_sync(0xffffffffu, bk, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    if (ahead(ok, oi, bk, bi)) {
-                        bk = ok;
-                        bi = oi;
-                    }
-                }
-                if (kGroup) {
-                    const int par = sel & 1;
-                    if (lane == 0) {
-                        g.sh->seed.sk[par][g.gw] = bk;
-                        g.sh->bk[par][g.gw] = bi;
-                    }
-                    g.sync();
-                    bk = g.sh->seed.sk[par][0];
-                    bi = g.sh->bk[par][0];
-                    for (int w = 1; w < G; ++w)
-                        if (ahead(g.sh->seed.sk[par][w], g.sh->bk[par][w], bk, bi)) {
-                            bk = g.sh->seed.sk[par][w];
-                            bi = g.sh->bk[par][w];
-                        }
-                }
-                if (lane == (sel & 31)) {
-                    if (sel < 32) top0 = bi;
-                    else top1 = bi;
-                }
-                pk = bk;
-                pi = bi;
-            }
-            int x_max = (ALL - 1) * (ALL - 2);
-            if (x_max > 812) x_max = 812;
-            if (x_max < 0) x_max = 0;
-            s = -1;
-            for (int xb = 0, round = 0; xb <= x_max; xb += G, ++round) {
-                const int x = xb + (kGroup ? g.gw : 0);
-                bool good = false;
-                TS v[3];
-                int ri = -1;
-                if (x <= x_max) {
-                    int i, j;
-                    get_i_j(x, ALL, i, j);
-                    const int ri0 = __shfl_sync(0xffffffffu, top0, i & 31), ri1 = __shfl_sync(0xffffffffu, top1, i & 31);
-                    const int rj0 = __shfl_sync(0xffffffffu, top0, j & 31), rj1 = __shfl_sync(0xffffffffu, top1, j & 31);
-                    ri = i < 32 ? ri0 : ri1;
-                    const int rj = j < 32 ? rj0 : rj1;
-                    TC vc[3];
-                    warp_solve<TC, TS>(rows, ri, rj, eqv, v, vc, lane);
-                    bool bad = false;
-                    for (int k = lane; k < ALL; k += 32) {
-                        if (k == ri || k == rj) continue;
-                        const vec4_t<TC> r = rows[k];
-                        if (r.x * vc[0] + r.y * vc[1] + r.z * vc[2] + r.w > eps) bad = true;
-                    }
-                    good = !__any_sync(0xffffffffu, bad);
-                }
-                if (kGroup) { // the smallest feasible pair of the round, from its warp
-                    const int par = (round + ksel) & 1; // not the last selection pass's slots
-                    // (a warp still reading those may lag one barrier behind)
-                    if (lane == 0) g.sh->bk[par][g.gw] = good ? x : 0x7fffffff;
-                    g.sync();
-                    int xw = 0x7fffffff;
-                    for (int w = 0; w < G; ++w) xw = min(xw, g.sh->bk[par][w]);
-                    if (xw == 0x7fffffff) continue;
-                    if (good && x == xw && lane == 0) {
-                        g.sh->seed.sri = ri;
-                        g.sh->seed.sv[0] = (double)v[0];
-                        g.sh->seed.sv[1] = (double)v[1];
-                        g.sh->seed.sv[2] = (double)v[2];
-                    }
-                    g.sync();
-                    s = g.sh->seed.sri;
-                    p[0] = (TS)g.sh->seed.sv[0];
-                    p[1] = (TS)g.sh->seed.sv[1];
-                    p[2] = (TS)g.sh->seed.sv[2];
-                    g.sync(); // read by every warp before the pruning may overwrite it
-                    break;
-                }
-                if (good) {
-                    s = ri;
-                    p[0] = v[0];
-                    p[1] = v[1];
-                    p[2] = v[2];
-                    break;
-                }
-            }
-            if (s < 0) status = kNoStart;
-        }
-
-        // ---------------------------------------------------- row pruning
-        int nlist = -1;
-        const uint16_t *list = nullptr;
-        if (s >= 0 && prune && ALL >= kPruneMin) {
-            const TC pc3[3] = {(TC)p[0], (TC)p[1], (TC)p[2]};
-            nlist = prune_rows<TC, kGroup>(rows, ALL, eqc, pc3, lane, g);
-            if (nlist >= 0) list = g.sh->list;
-        }
-
-        // ---------------------------------------------------- walk
-        // lane i holds vertex i and the plane of the edge leaving it
-        TS vx = 0, vy = 0, vz = 0;
-        int ve = -1;
-        int n = 0;
-        bool closed = false;
         if (s >= 0) {
-            bool done = false;
-            if (sizeof(TS) > sizeof(TC)) // scan-precision walk, vertices refined in the solve precision
-            {
-                done = walk_refined<TC, TS, kGroup>(rows, ALL, list, nlist, eqc, eqv, p, s, par_eps, same_eps, lane, vx,
-                                                    vy, vz, ve, n, closed, status, g);
-                if (kGroup) { // the leader's outcome for the group
-                    if (g.gw == 0 && lane == 0) g.sh->done = done ? 1 : 0;
-                    g.sync();
-                    done = g.sh->done != 0;
-                }
-            }
-            if (!done) {
-                int sbk, sdec, nsteps;
-                if (sizeof(TS) > sizeof(TC)) { // mixed form: FP64 predicates and FP64 solves
-                    if (g.gw == 0 && lane == 0) atomicAdd(nfp64, 1ull);
-                    walk<TC, TS, kGroup, TS, false>(rows, ALL, list, nlist, eqc, eqv, p, s, par_eps, same_eps, lane, vx,
-                                                    vy, vz, ve, n, closed, status, sbk, sdec, nsteps, g);
+            if constexpr (sizeof(TS) > sizeof(TC)) {
+                if (again) {
+                    wide = true;
+                    done = walk_fp64<TC, TS>(rows, ball, ways, eqc, q, s, par_eps, same_eps, lane, f);
                 } else {
-                    walk<TC, TS, kGroup>(rows, ALL, list, nlist, eqc, eqv, p, s, par_eps, same_eps, lane, vx, vy, vz, ve,
-                                         n, closed, status, sbk, sdec, nsteps, g);
+                    done = face_walk<TC, TS>(rows, ball, ways, eqc, eqv, q, s, par_eps, same_eps, lane, f, wide);
                 }
+            } else {
+                done = face_walk<TC, TS>(rows, ball, ways, eqc, eqv, q, s, par_eps, same_eps, lane, f, wide);
             }
         }
-        const bool leader = !kGroup || g.gw == 0;
+        again = false;
+        if (done) {
+            s_plane = list->idx[s];
+            if (f.ve >= 0) f.ve = list->idx[f.ve];
+        } else {
+            if (n > 3 * kList / 4 || T == INFINITY) break;
+            T *= fminf((float)kList * 0.85f / (float)max(n, 1), 3.f); // a larger ball
+            n = -1;
+        }
+    }
+    if (!done) { // every row
+        const Ball whole{0.f, 0.f, 0.f, INFINITY};
+        clear();
+        wide = false;
+        s = start;
+        if (is_seed) s = seed_start<TC, TS>(all, all, whole, INFINITY, eqv, p, eps, lane);
+        if (s >= 0) face_walk<TC, TS>(all, whole, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f, wide);
+        s_plane = s;
+    }
+    out.vx = f.vx;
+    out.vy = f.vy;
+    out.vz = f.vz;
+    out.ve = f.ve;
+    out.n = f.n;
+    out.start = s_plane;
+    out.closed = f.closed;
+    out.again = wide;
+    out.status = f.status;
+    out.T = T;
+    out.listed = n;
+}
 
-        // ---------------------------------------------------- outputs
-        if (leader && lane == 0) { // the leader writes the face
-            reg.nv[rid] = n;
-            reg.status[rid] = status;
-        }
-        if (leader && lane < n) {
-            TS *vo = (TS *)reg.verts + ((size_t)rid * kVMax + lane) * 3;
-            vo[0] = vx;
-            vo[1] = vy;
-            vo[2] = vz;
-            reg.edges[(size_t)rid * kVMax + lane] = ve;
-        }
+// ---------------------------------------------------------------- neighbours
+__device__ __forceinline__ long long next_work(WaveCtl *ctl, int lane)
+{
+    unsigned int v = 0;
+    if (lane == 0) v = atomicAdd(&ctl->work, 1u);
+    return (long long)__shfl_sync(0xffffffffu, v, 0);
+}
 
-        // ---------------------------------------------------- neighbours
-        // the plane crossed by edge `lane` where a neighbour is to be
-        // inserted (else -1), published by the leader; warp gw of the group
-        // inserts the neighbours of the edges lane = gw (mod G), one after
-        // the other, each by the whole warp (measured on GB300: with the
-        // leader inserting all of them the other warps waited at the next
-        // face's barrier)
-        int kv = -1;
-        if (leader && lane < n && ve >= 0 && ve < N && (closed || lane < n - 1) && !(!is_seed && ve == s)) kv = ve;
-        if (kGroup) {
-            if (list) g.sync(); // every warp's walk has done with the pruning list
-            if (g.gw == 0) g.sh->ve[lane] = kv;
-            g.sync();
-            kv = g.sh->ve[lane];
+__device__ __forceinline__ unsigned long long load_slot(const unsigned long long *p)
+{
+    cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> a(*const_cast<unsigned long long *>(p));
+    return a.load(cuda::memory_order_relaxed);
+}
+
+// Insert the neighbours across the planes kv >= 0 (one per lane; the parent's
+// key with that bit flipped) into the region hash set.  Every lane probes for its
+// own key, so that the slots of all edges are read at once; where fingerprints
+// match, the whole warp compares the keys (lane l takes words l, l + 32, ...).
+// Returns the slot claimed for a new candidate (or the candidate slot this one
+// now shares), -1 when the key is a committed region already.  Among equal
+// candidate keys the smallest (parent, plane) id stays in the slot, so the
+// result does not depend on timing.  Region entries (tag 0) point at the region
+// store; candidate entries (tag 1) carry (wave position, plane) and point at
+// the parent's key.
+__device__ int insert_edges(const RegionsDev &reg, const HashDev &hs, long long head, int ALL, int W, const uint32_t *pkey,
+                            uint64_t phash, long long rl, int kv, int lane, int *err)
+{
+    int got = -1;
+    bool open = kv >= 0;
+    uint32_t fp = 0;
+    unsigned long long mine = 0, slot = 0;
+    if (open) {
+        const uint64_t h = flip_hash(phash, pkey[kv >> 5], kv);
+        fp = fp_of(h);
+        mine = slot_value(fp, 1, (uint32_t)(rl * ALL + kv));
+        slot = h & hs.mask;
+    }
+    for (int probe = 0; probe < kMaxProbes; ++probe) {
+        unsigned long long cur = 0ull;
+        bool match = false;
+        if (open) {
+            cur = load_slot(hs.slots + slot);
+            if (cur == kEmpty) {
+                const unsigned long long old = atomicCAS(hs.slots + slot, kEmpty, mine);
+                if (old == kEmpty) {
+                    got = (int)slot;
+                    open = false;
+                }
+                cur = old;
+            }
+            match = open && (uint32_t)(cur >> 32) == fp;
         }
-        const bool mine = !kGroup || lane % G == g.gw;
-        int rec = -1;
-        const uint32_t *pkey = reg.keys + (size_t)rid * W;
-        unsigned todo = __ballot_sync(0xffffffffu, mine && kv >= 0);
-        const uint64_t phash = reg.hash[rid];
+        unsigned todo = __ballot_sync(kFull, match);
         while (todo) {
             const int src = __ffs(todo) - 1;
             todo &= todo - 1u;
-            const int k = __shfl_sync(0xffffffffu, kv, src);
-            const int got = warp_insert(reg, hs, head, ALL, W, pkey, phash, rl, k, lane, err);
-            if (lane == src) rec = got;
+            const uint32_t id = (uint32_t)__shfl_sync(kFull, (uint32_t)cur & 0x7fffffffu, src);
+            const bool cand = __shfl_sync(kFull, (uint32_t)cur >> 31, src) != 0u;
+            const int k = __shfl_sync(kFull, kv, src);
+            const uint32_t *other = reg.keys + (size_t)(cand ? head + id / ALL : (long long)id) * W;
+            const int ok2 = cand ? (int)(id % ALL) : -1;
+            const int kw = k >> 5, ow = ok2 >= 0 ? ok2 >> 5 : -1;
+            const uint32_t kb = 1u << (k & 31), ob = ok2 >= 0 ? 1u << (ok2 & 31) : 0u;
+            bool differ = false;
+            for (int w = lane; w < W; w += 32) {
+                const uint32_t a = pkey[w] ^ (w == kw ? kb : 0u);
+                const uint32_t b = other[w] ^ (w == ow ? ob : 0u);
+                differ = differ || a != b;
+            }
+            if (!__any_sync(kFull, differ) && lane == src) {
+                open = false;
+                if (cand) {
+                    atomicMin(hs.slots + slot, mine);
+                    got = (int)slot;
+                }
+            }
         }
-        if (mine && lane < kVMax) ch.rec[(size_t)rl * kVMax + lane] = rec;
+        if (!__any_sync(kFull, open)) return got;
+        slot = (slot + (unsigned long long)probe + 1ull) & hs.mask;
+    }
+    if (open) atomicOr(err, kErrTableFull);
+    return got;
+}
+
+// ---------------------------------------------------------------- kernel
+// TC is the scan precision, TS the solve precision.
+//
+// What bounds it: the rows from HBM on wide networks (65.7 KB read and on average
+// 32 KB written per face of 4,104 rows), latency and issue slots on narrow ones,
+// the FP64 pipe where TS or TC is double.  A warp per face, rather than a group
+// that scans every row at every step from shared memory, because with the list a
+// step is four rows per lane and the rest of it (solve, decisions) is the same for
+// every warp of a group.  Measured on GB300, polygon phase of a whole marching:
+//   3-[512]x8-1 mixed (6.8 M faces)      378 ms -> 145 ms
+//   3-[256]x6-1 mixed (1.28 M)            29.4  -> 16.0
+//   3-[128]x4-1 mixed / fp32 / fp64 (265 K) 3.2 / 2.4 / 28.8 -> 2.7 / 1.75 / 8.6
+template <typename TC, typename TS>
+__global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDev net, RegionsDev reg, ChunkDev ch, HashDev hs,
+                                                                     Tolerances tol, int ways, unsigned long long *nfp64,
+                                                                     int *err)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    const int wib = threadIdx.x >> 5;
+    NearList<TC> *list = reinterpret_cast<NearList<TC> *>(smem_raw) + wib;
+    const int ALL = net.ALL, N = net.N, W = net.W;
+    const TC eps = (TC)tol.eps, par_eps = (TC)tol.par_eps;
+    const TS same_eps = (TS)tol.same_eps;
+    long long head;
+    int count;
+    chunk_range(ch, head, count);
+    // a region per warp: by launch position, or (fixed grid of the
+    // graph-driven loop) from the wave's work counter
+    long long rl_next = (long long)blockIdx.x * kFaceWarps + wib;
+    for (;;) {
+        const long long rl = ch.ctl ? next_work(ch.ctl, lane) : rl_next;
+        rl_next += (long long)gridDim.x * kFaceWarps;
+        if (rl >= count) break;
+        const long long rid = head + rl;
+        vec4_t<TC> *own = reinterpret_cast<vec4_t<TC> *>((TC *)ch.cons + (size_t)row_slot(ch, head, (int)rl) * net.ALLP * 4);
+        const int start = reg.start[rid], parent = reg.parent[rid];
+        GlobalRows<TC> all;
+        all.n = ALL;
+        all.own = own;
+        all.nsplit = ch.split ? ch.split[rl] : 0;
+        all.flip = all.nsplit ? start : -1;
+        all.par = all.nsplit ? reinterpret_cast<const vec4_t<TC> *>((const TC *)ch.cons + (size_t)ring_slot(ch, parent) * net.ALLP * 4)
+                             : own;
+        const TS *midp = (const TS *)reg.mid + (size_t)rid * 4;
+
+        // ------------------------------------------------ near list, walk
+        Result<TS> r;
+        r.T = INFINITY; // few rows: all of them
+        int what = kLeft;
+        if (start >= 0) {
+            if (ALL > kList) r.T = reg.reach[parent];
+            const Ball centre{(float)midp[0], (float)midp[1], (float)midp[2], -1.f};
+            Sieve<TC> sv(centre, r.T, list, lane);
+            stream_part<TC, true>(all.par, own, 0, all.nsplit, all.flip, sv);
+            stream_part<TC, false>(own, nullptr, all.nsplit, ALL, -1, sv);
+            sv.finish();
+            r.listed = sv.n;
+            if (sv.n <= kList) {
+                const vec4_t<TC> eqc = ld4<TC>((const TC *)ch.eq + (size_t)rl * 4); // scan precision copy
+                const TS eqv[4] = {(TS)eqc.x, (TS)eqc.y, (TS)eqc.z, (TS)eqc.w};
+                const TS p[3] = {midp[0], midp[1], midp[2]};
+                Ball ball{(float)p[0], (float)p[1], (float)p[2], -1.f};
+                ball.d2 = ball_radius2(r.T, coord_size(ball.x, ball.y, ball.z));
+                const ListRows<TC> rows{list, sv.n};
+                const int s = position<TC>(list, sv.n, start, lane);
+                Face<TS> f;
+                if (s >= 0) {
+                    if constexpr (sizeof(TS) > sizeof(TC)) {
+                        what = walk_refined<TC, TS>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f);
+                    } else {
+                        bool near;
+                        what = walk<TC, TS, false, false>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f, near)
+                                   ? kRefined
+                                   : kLeft;
+                    }
+                }
+                r.vx = f.vx;
+                r.vy = f.vy;
+                r.vz = f.vz;
+                r.n = f.n;
+                r.closed = f.closed;
+                r.status = f.status;
+                r.ve = what == kRefined && f.ve >= 0 ? (int)list->idx[f.ve] : -1;
+                r.start = start;
+            }
+        }
+        if (what != kRefined) {
+            Result<TS> o;
+            const vec4_t<TC> eqc = ld4<TC>((const TC *)ch.eq + (size_t)rl * 4);
+            face_slow<TC, TS>(all, list, ways, eqc, midp, start, eps, par_eps, same_eps, lane, what == kAgain, r.listed, r.T, o);
+            r = o;
+            if (r.again && lane == 0) atomicAdd(nfp64, 1ull);
+        }
+
+        // ------------------------------------------------ outputs
+        const int nv = r.n, ve = r.ve;
+        if (lane == 0) {
+            reg.nv[rid] = nv;
+            reg.status[rid] = r.status;
+            // the children's radius: their ball holds about as many planes per radius
+            reg.reach[rid] = r.T * ((float)kTarget / (float)max(r.listed, kTarget / 4));
+        }
+        if (lane < nv) {
+            TS *vo = (TS *)reg.verts + ((size_t)rid * kVMax + lane) * 3;
+            vo[0] = r.vx;
+            vo[1] = r.vy;
+            vo[2] = r.vz;
+            reg.edges[(size_t)rid * kVMax + lane] = ve;
+        }
+
+        // ------------------------------------------------ neighbours
+        // the plane crossed by edge `lane` where a neighbour is to be inserted
+        int kv = -1;
+        if (lane < nv && ve >= 0 && ve < N && (r.closed || lane < nv - 1) && !(start >= 0 && ve == r.start)) kv = ve;
+        ch.rec[(size_t)rl * kVMax + lane] =
+            insert_edges(reg, hs, head, ALL, W, reg.keys + (size_t)rid * W, reg.hash[rid], rl, kv, lane, err);
         __syncwarp();
     }
 }
 
 } // namespace
 
-// Faces per block for G warps per face: as many as keep a block's rows
-// (and each face's shared block) within 73 KB (three blocks per SM), at most
-// 8 / G, a power of two.
-int polygon_faces_per_block(size_t face_bytes, int G)
+// The lanes of the rule between near-equal hits (see the top of the file): 32
+// per warp of the face group that scanned every row from shared memory, eight
+// warps per block split between faces and the warps of a face as 73 KB of rows
+// allowed.  `face_warps` overrides the warps.
+static int rule_ways(int prec, int ALLP, int face_warps)
 {
+    if (face_warps > 0) return 32 * face_warps;
+    const size_t face_bytes = prec == kFloat64 ? sizeof(double) * 4 * (size_t)ALLP + 1120 : sizeof(float) * 4 * (size_t)ALLP + 1056;
     int F = 1;
-    while (2 * F * G <= 8 && (size_t)(2 * F) * face_bytes <= 73u * 1024u) F *= 2;
-    return F;
+    while (2 * F <= 8 && (size_t)(2 * F) * face_bytes <= 73u * 1024u) F *= 2;
+    return 32 * (8 / F);
 }
 
-// Automatic warps per face: eight warps per block, split between faces
-// and the warps of a face as the rows allow.
-int polygon_face_warps(int prec, int ALLP)
-{
-    const size_t face_bytes = prec == kFloat64 ? sizeof(double4) * (size_t)ALLP + group_shared_bytes<double>()
-                                               : sizeof(float4) * (size_t)ALLP + group_shared_bytes<float>();
-    const int F = polygon_faces_per_block(face_bytes, 1);
-    return 8 / F;
-}
+int polygon_face_warps(int prec, int ALLP) { return rule_ways(prec, ALLP, 0) / 32; }
 
 template <typename TC, typename TS>
-void launch_one(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs, const Tolerances &tol,
-                int *d_err, int G, int prune, unsigned long long *nfp64, cudaStream_t st)
+static void launch_one(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
+                       const Tolerances &tol, int *d_err, int ways, unsigned long long *nfp64, cudaStream_t st)
 {
-    const size_t row_bytes = sizeof(vec4_t<TC>) * (size_t)net.ALLP;
-    const int F = polygon_faces_per_block(row_bytes + group_shared_bytes<TC>(), G);
-    const size_t smem = (row_bytes + group_shared_bytes<TC>()) * F;
-    auto k = G > 1 ? polygon_kernel<TC, TS, true> : polygon_kernel<TC, TS, false>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int sms = device_sms();
-    const int threads = 32 * F * G;
-    int grid;
-    if (ch.ctl) { // wave size on the device: as many blocks as stay resident
-        int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
-        grid = sms * std::max(per_sm, 1);
-    } else {
-        const long long need = (ch.count + F - 1) / F;
-        grid = (int)std::min<long long>(need, (long long)sms * 16);
-    }
-    k<<<grid, threads, smem, st>>>(net, reg, ch, hs, tol, G, prune, nfp64, d_err);
+    auto k = polygon_kernel<TC, TS>;
+    const size_t smem = sizeof(NearList<TC>) * kFaceWarps;
+    int per_sm = 1; // as many blocks as stay resident
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kFaceWarps, smem);
+    long long grid = (long long)device_sms() * std::max(per_sm, 1);
+    if (!ch.ctl) grid = std::min<long long>(grid, (ch.count + kFaceWarps - 1) / kFaceWarps);
+    k<<<(unsigned)grid, 32 * kFaceWarps, smem, st>>>(net, reg, ch, hs, tol, ways, nfp64, d_err);
 }
 
 void launch_polygon(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
-                    const Tolerances &tol, int face_warps, int prune, unsigned long long *nfp64, int *d_err,
-                    cudaStream_t st)
+                    const Tolerances &tol, int face_warps, unsigned long long *nfp64, int *d_err, cudaStream_t st)
 {
     if (!ch.ctl && ch.count <= 0) return;
-    const int G = face_warps > 0 ? face_warps : polygon_face_warps(prec, net.ALLP);
+    const int ways = rule_ways(prec, net.ALLP, face_warps);
     if (prec == kFloat64)
-        launch_one<double, double>(net, reg, ch, hs, tol, d_err, G, prune, nfp64, st);
+        launch_one<double, double>(net, reg, ch, hs, tol, d_err, ways, nfp64, st);
     else if (prec == kMixed)
-        launch_one<float, double>(net, reg, ch, hs, tol, d_err, G, prune, nfp64, st);
+        launch_one<float, double>(net, reg, ch, hs, tol, d_err, ways, nfp64, st);
     else
-        launch_one<float, float>(net, reg, ch, hs, tol, d_err, G, prune, nfp64, st);
+        launch_one<float, float>(net, reg, ch, hs, tol, d_err, ways, nfp64, st);
 }
 
 } // namespace am

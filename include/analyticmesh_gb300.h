@@ -192,9 +192,9 @@ typedef enum {
                                  256 units and more), 3 as 2 with a layer's 128-row tiles multiplied in two
                                  passes, so that TMEM holds accumulators for twice as many regions (layers
                                  of 512 units).  All give the same bits. */
-    AM_OPT_FACE_WARPS = 7,    /* warps per face polygon: 0 (default) automatic (one for narrow networks,
-                                 up to eight for wide ones, whose rows leave room for few faces per SM),
-                                 or 1, 2, 4, 8.  The warps of a face split the walk's scan over the rows. */
+    AM_OPT_FACE_WARPS = 7,    /* 0 (default) automatic, or 1, 2, 4, 8.  A face is one warp's; the value only
+                                 names the rule that decides between two planes hit at nearly the same
+                                 place (see am_polygon.cu). */
     AM_OPT_TABLE_SLOTS = 8,   /* region hash table: 0 (default) sized by the engine (load factor <= 1/2,
                                  grown as regions are found); n > 0: fixed at n slots rounded up to a
                                  power of two, never grown.  A run that outgrows a fixed table returns
@@ -206,20 +206,16 @@ typedef enum {
                                  block after the seed phase, as a kernel would leave them, so that the
                                  wave loop's error decoding can be tested without a device fault.
                                  0 (default) off; stays set until set to 0. */
-    AM_OPT_PRUNE_ROWS = 10    /* 1: before walking a face, drop the constraint rows whose line provably
-                                 misses the polygon (a dual-space test against a sample of the rows), so
-                                 that the walk scans a few dozen rows per step instead of all; 0 (default):
-                                 every row.  Both give the same faces.  Measured on GB300 the two pruning
-                                 passes cost about what they save (+5 % on 3-[128]x4-1 in the mixed form,
-                                 -10 to -25 % on the 1536- and 4096-row networks), hence off. */
+    AM_OPT_PRUNE_ROWS = 10    /* 0 or 1: accepted, without effect.  The walk always works on the rows whose
+                                 planes are near the face, with the faces of every row. */
 } am_option;
 int am_set_option(am_engine *engine, int option, int64_t value);
 
 /* ---- autotuner (no counterpart in the reference): chooses AM_OPT_COMPOSE_TILE
- * (mixed form) and AM_OPT_FACE_WARPS for this engine's network architecture by
- * marching the first sample_regions regions of args once per candidate with
- * per-phase device timing (after an untimed pass), and sets them on the
- * engine.  The choice is remembered per architecture (widths, connections,
+ * (mixed form) for this engine's network architecture by marching the first
+ * sample_regions regions of args once per candidate with per-phase device
+ * timing (after an untimed pass), and sets it on the engine, with
+ * AM_OPT_FACE_WARPS at its automatic value.  The choice is remembered per architecture (widths, connections,
  * precision, sample size) for the life of the process; a later call for the
  * same architecture sets it without marching.  chosen (optional) receives
  * {compose tile, warps per face}.  The engine holds no marching result
