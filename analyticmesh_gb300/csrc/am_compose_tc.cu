@@ -300,6 +300,31 @@ __device__ void wp_produce(WPipe &p, const NetDev &net, const TcNet &tc, const W
         if (last[s] >= 0) umma::mbar_wait(p.full + s, (uint32_t)(last[s] / p.nstage) & 1u, kWaitIters);
 }
 
+// The six products of one K step (terms t of the weights, u of the operand, of
+// weight 2^-8(t+u), t + u <= 2), the same A consecutively: hh into the main
+// accumulator, the others into the correction's.
+__device__ __forceinline__ void issue_step(uint32_t d_main, uint32_t d_corr, uint64_t ad, uint64_t xd, uint64_t xu,
+                                           uint32_t idesc, bool fresh)
+{
+#ifdef NOCOLL
+#define MMA0 mma_bf16_a<0>
+#define MMA1 mma_bf16_a<0>
+#define MMA2 mma_bf16_a<0>
+#define MMA3 mma_bf16_a<0>
+#else
+#define MMA0 mma_bf16_a<0>
+#define MMA1 mma_bf16_a<1>
+#define MMA2 mma_bf16_a<2>
+#define MMA3 mma_bf16_a<3>
+#endif
+    umma::MMA1(d_main, ad, xd, idesc, fresh ? 0u : 1u);
+    umma::MMA2(d_corr, ad, xd + xu, idesc, fresh ? 0u : 1u);
+    umma::MMA3(d_corr, ad, xd + 2 * xu, idesc, 1u);
+    umma::MMA1(d_corr, ad + 1024u, xd, idesc, 1u);
+    umma::MMA3(d_corr, ad + 1024u, xd + xu, idesc, 1u);
+    umma::MMA0(d_corr, ad + 2048u, xd, idesc, 1u);
+}
+
 // (thread 0) D[mt] (+)= M . X over all K blocks of the operand in shared
 // memory: six products per K step (terms t, u of weight 2^-8(t+u), t + u <= 2)
 __device__ void gemm_issue(WPipe &p, const TcMat &m, int mtiles, const XOp &X, uint32_t tmem, bool first, int &g)
@@ -321,19 +346,7 @@ __device__ void gemm_issue(WPipe &p, const TcMat &m, int mtiles, const XOp &X, u
             // A: term t at +16 KB (1024 units), K step j at +32 B (2 units)
             const uint64_t ad = umma::desc_sw128(a0), xd = X.desc(0, kb, 0);
             #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                umma::mma_bf16(d_main, ad + 2u * j, xd + xj * j, idesc, (fresh && j == 0) ? 0u : 1u);
-                int q = 0;
-                #pragma unroll
-                for (int t = 0; t < 3; ++t)
-                    #pragma unroll
-                    for (int u = 0; u + t < 3; ++u) {
-                        if (t == 0 && u == 0) continue;
-                        umma::mma_bf16(d_corr, ad + 1024u * t + 2u * j, xd + xu * u + xj * j, idesc,
-                                       (fresh && j == 0 && q == 0) ? 0u : 1u);
-                        ++q;
-                    }
-            }
+            for (int j = 0; j < 4; ++j) issue_step(d_main, d_corr, ad + 2u * j, xd + xj * j, xu, idesc, fresh && j == 0);
             umma::commit(umma::smem_addr(p.done + s)); // frees the stage for the copy warp
             p.consumed = g + 1;
             ++g;
@@ -376,9 +389,9 @@ __host__ __device__ __forceinline__ int key_stride(int W) { return W | 1; }
 // (one thread) tile width of the wave: one tile per resident slot while the
 // wave is small, the widest tile otherwise; the plan's tiles.  Returns the
 // tile's columns.
-__device__ int plan_wave(WavePlan &plan, const ChunkDev &ch, int layers, int count, int slots, int ncols_max)
+__device__ int plan_wave(WavePlan &plan, const ChunkDev &ch, int layers, int count, int slots, int ncols_max, int group)
 {
-    plan_counts(plan, ch, layers, count);
+    plan_counts(plan, ch, layers, count, group);
     const int per = (count + slots - 1) / slots;
     int ncols = (4 * per + 15) / 16 * 16;
     ncols = ncols < 16 ? 16 : (ncols > ncols_max ? ncols_max : ncols);
@@ -404,7 +417,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
     int count;
     chunk_range(ch, head, count);
     if (count <= 0) return;
-    if (tid == 0) s_ncols = plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max);
+    if (tid == 0) s_ncols = plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max, 1);
     __syncthreads();
     const int ncols = s_ncols;
     const int R = ncols / 4;
@@ -701,6 +714,11 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
 constexpr int kSBuild = 512;            // builder threads (16 warps)
 constexpr int kSThreads = kSBuild + 64; // + the issuing warp and the weight-copy warp
 constexpr int kSFaceSumBytes = kSBuild * 16;
+// CTAs of a cluster work on tiles of the same class in step and share the weight
+// stream: each copies its part of a block into the shared memory of all of them
+// (multicast), so that a block leaves the L2 once per cluster.
+constexpr int kCluster = 2;
+constexpr uint16_t kClusterMask = (1u << kCluster) - 1u;
 
 __device__ __forceinline__ int jobs_of(const NetDev &net, int i)
 {
@@ -757,6 +775,7 @@ __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws
                                  const WavePlan &plan, int rounds, int *err, volatile int *abort)
 {
     const int nst = tc.nstage;
+    const size_t part = (size_t)umma::cluster_rank() * (kWBlockBytes / kCluster); // this CTA's part of a block
     int h = 0;
     int ps = 0;        // stage of block h (h % nst) ...
     uint32_t pph = 0u; // ... and (h / nst) & 1, kept incrementally
@@ -783,9 +802,9 @@ __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws
                         if (h >= nst && !swait(wdone + s, ph ^ 1u, err, abort)) continue;
                         if (*abort) continue;
                         umma::mbar_expect_tx(wfull + s, (uint32_t)kWBlockBytes);
-                        umma::bulk_g2s(ws + (size_t)s * kWBlockBytes,
-                                       m.blocks + (size_t)(mt * kblocks + kb) * kWBlockBytes, (uint32_t)kWBlockBytes,
-                                       wfull + s);
+                        umma::bulk_g2s_mc(ws + (size_t)s * kWBlockBytes + part,
+                                          m.blocks + (size_t)(mt * kblocks + kb) * kWBlockBytes + part,
+                                          (uint32_t)kWBlockBytes / kCluster, wfull + s, kClusterMask);
                         last[s] = h;
                     }
             }
@@ -848,20 +867,9 @@ __device__ void issue_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, 
                         const uint32_t d_corr = tmem + (uint32_t)((mper + mt - mt0) * ncols);
                         const uint64_t ad = wd0 + wstep * (uint64_t)s; // term t at +16 KB, K step j at +32 B
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            umma::mma_bf16(d_main, ad + 2u * j, xd + xj * j, idesc, (fresh && j == 0) ? 0u : 1u);
-                            int q = 0;
-#pragma unroll
-                            for (int tt = 0; tt < 3; ++tt)
-#pragma unroll
-                                for (int u = 0; u + tt < 3; ++u) {
-                                    if (tt == 0 && u == 0) continue;
-                                    umma::mma_bf16(d_corr, ad + 1024u * tt + 2u * j, xd + xu * u + xj * j, idesc,
-                                                   (fresh && j == 0 && q == 0) ? 0u : 1u);
-                                    ++q;
-                                }
-                        }
-                        umma::commit(umma::smem_addr(wdone + s)); // the producer may refill the stage
+                        for (int j = 0; j < 4; ++j)
+                            issue_step(d_main, d_corr, ad + 2u * j, xd + xj * j, xu, idesc, fresh && j == 0);
+                        umma::commit_mc(umma::smem_addr(wdone + s), kClusterMask); // the producers may refill the stage
                         consumed = h + 1;
                     }
                     umma::commit(umma::smem_addr(xdone + xs)); // the operand stage is free once these complete
@@ -878,7 +886,7 @@ __device__ void issue_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, 
         atomicOr(err, kErrWait);
 }
 
-__global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, TcNet tc, RegionsDev reg, ChunkDev ch,
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, TcNet tc, RegionsDev reg, ChunkDev ch,
                                                                     float iso, int slots, int *err)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -894,7 +902,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
     int count;
     chunk_range(ch, head, count);
     if (count <= 0) return;
-    if (tid == 0) s_ncols = plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max);
+    if (tid == 0) s_ncols = plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max, kCluster);
     __syncthreads();
     const int ncols = s_ncols;
     const int R = ncols / 4;
@@ -929,9 +937,12 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
     volatile int *abort = &s_abort;
     if (tid == 0) {
         s_abort = 0;
-        for (int b = 0; b < 6; ++b) umma::mbar_init(bars + b, 1);
-        umma::mbar_init(xfull, kSBuild);
-        umma::mbar_init(xfull + 1, kSBuild);
+        for (int b = 0; b < 3; ++b) {
+            umma::mbar_init(wfull + b, 1);
+            umma::mbar_init(wdone + b, kCluster); // every CTA's products are done with the stage
+        }
+        umma::mbar_init(xfull, kSBuild / 32); // (one arrival per warp)
+        umma::mbar_init(xfull + 1, kSBuild / 32);
         umma::mbar_init(xdone, 1);
         umma::mbar_init(xdone + 1, 1);
         umma::mbar_init(accdone, 1);
@@ -949,6 +960,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
     }
     umma::fence_before();
     __syncthreads();
+    umma::cluster_sync(); // the other CTAs' barriers are initialised
     umma::fence_after();
     const uint32_t tmem = tslot;
 
@@ -997,21 +1009,42 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
             }
             bar_builders(); // layer-1 rows written by every builder
 
-            // X[4r + c][k] = s_k(r) ? -C[r][k][c] : 0 (layer 1: +W0 rows from
-            // shared memory), one 64-deep K block at a time; every pass of a
-            // layer streams the same blocks.  Warp w owns the items w, w + 16,
-            // ... of a block (Items).  The first four items of the next block
-            // are loaded one step ahead, so that their latency hides behind
-            // the stage wait; raw values are kept and signed when stored (no
-            // use of a loaded value between the loads: they overlap).  The
-            // returned mask marks the items whose sign is the other one.
+            // X[4r + c][k] = s_k(r) ? -C[r][k][c] : 0, one 64-deep K block at a
+            // time; every pass of a layer streams the same blocks.  Warp w owns
+            // the items w, w + 16, ... of a block (Items).  The first four items
+            // of a block are loaded two steps ahead of their use, and nothing
+            // in the load depends on shared memory but the key words of its 64
+            // rows: the products keep the shared memory's bandwidth busy, and a
+            // dependent shared load costs hundreds of cycles then (measured: an
+            // LDS of the region's slots and of the key word per item made a
+            // block's loads take 2,200 cycles, against 1,536 of a weight
+            // block's products).  Raw values are kept and signed when stored.
+            // The returned mask marks the items whose sign is the other one
+            // (the plane the region was entered through).
             const Items items(R);
+            const bool one = items.half == 16; // an item's region is the warp's own pair: the tile of 32 regions
+            const int myr = 2 * warp + (lane & 1);
+            const int4 mine = one && myr < nreg ? ri[myr] : make_int4(0, 0, -1, 0);
             auto load_items = [&](int li, int job, int kb, int c, float4 *v) {
                 int src;
                 job_mat(net, tc, li, job, src);
                 const int K = net.nodes[src], rows0 = net.hoff[src];
                 const bool par = rows0 < jend;
                 unsigned other = 0u;
+                if (one) {
+                    const int k0 = kb * 64 + (lane >> 1), b0 = rows0 + k0;
+                    const uint32_t *kw = keys + (size_t)myr * KW + (b0 >> 5);
+                    const uint32_t w0 = kw[0], w1 = kw[1], w2 = kw[2]; // (words beyond the key: masked by K)
+                    const uint32_t lo = __funnelshift_r(w0, w1, b0), hi = __funnelshift_r(w1, w2, b0);
+                    const float4 *p = reinterpret_cast<const float4 *>(cons + (size_t)(uint32_t)(par ? mine.y : mine.x) * rstride) + b0;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const bool on = ((u < 2 ? lo : hi) >> (16 * (u & 1)) & 1u) && k0 + 16 * u < K && myr < nreg;
+                        v[u] = on ? p[16 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (b0 + 16 * u == mine.z) other |= 1u << u;
+                    }
+                    return other;
+                }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     int r, kk;
@@ -1021,19 +1054,18 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                     if (in && r < nreg && k < K && key_bit(keys + (size_t)r * KW, rows0 + k)) {
                         const int4 g = ri[r];
                         if (rows0 + k == g.z) other |= 1u << u;
-                        x = src == 1 ? w0s[k]
-                                     : ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)(rows0 + k) * 4);
+                        x = ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)(rows0 + k) * 4);
                     }
                     v[u] = x;
                 }
-                return src == 1 ? 0u : other;
+                return other;
             };
-            auto put_items = [&](const XOp &X, int c, const float4 *v, float sg, unsigned other) {
+            auto put_items = [&](const XOp &X, int c, const float4 *v, unsigned other) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     int r, kk;
                     if (items.at(warp + 16 * (4 * c + u), lane, r, kk)) {
-                        const float s1 = (other >> u) & 1u ? -sg : sg;
+                        const float s1 = (other >> u) & 1u ? 1.f : -1.f;
                         const float x[4] = {s1 * v[u].x, s1 * v[u].y, s1 * v[u].z, s1 * v[u].w};
                         X.put<2>(4 * r, kk, x);
                     }
@@ -1042,38 +1074,11 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
             const int nchunks = (2 * R + 63) / 64;
             // The epilogue of a pass reads its accumulators (warp w: TMEM
             // lanes 32 (w % 4).., column blocks cgrp, cgrp + ngrp, ... of each
-            // M tile) and stores their rows,
-            // except the last block, which stays in registers and is stored
-            // during the next pass's first step, while the tensor core works
-            // (a pass's 128 KB of rows take ~4 K cycles of the SM's store
-            // bandwidth alone, measured on GB300; registers allow one block).
-            // A barrier follows the deferred store, so that later loads see
-            // the rows.
+            // M tile) and stores their rows.
             const int ncb = ncols / 16;
             const int ncbw = cgrp < ncb ? (ncb - cgrp + ngrp - 1) / ngrp : 0; // this warp's column blocks
-            const int ncbu = (ncb + ngrp - 1) / ngrp;                          // the most any warp has
             const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
-            // o[0..kKeep-1][16]: the (at most kKeep) deferred column blocks in
-            // store order -- the first blocks of a pass are stored at once,
-            // before the TMEM is given up; a stored block leaves o[0] and the
-            // others move up (constant indices only, so that the blocks stay
-            // in registers; more than one block spilled at 96 registers)
-            constexpr int kKeep = 1;
-            float o[kKeep][16];
-            int nd = 0, def_i = 1, def_mt0 = 0; // deferred column blocks (uniform count), their pass
-            int def_first = 0, def_nit = 0;     // this warp's first deferred block, its blocks in that pass
-            bool def_ok = false;
-            auto shift_o = [&]() {
-#pragma unroll
-                for (int b = 0; b + 1 < kKeep; ++b)
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) o[b][k] = o[b + 1][k];
-            };
-            auto store_block = [&](int it) { // block it of the pass def_i / def_mt0, from o[0]
-                if (!def_ok || it >= def_nit) return; // (this warp's share)
-                const int li = def_i;
-                const int mt = def_mt0 + it / ncbw, cb = cgrp + (it % ncbw) * ngrp;
-                const int m = mt * 128 + q4 * 32 + lane;
+            auto store_block = [&](int li, int m, int cb, const float *o) { // 16 columns of unit m
                 if (m >= net.nodes[li + 1]) return;
                 const int row = net.hoff[li + 1] + m;
 #pragma unroll
@@ -1082,7 +1087,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                     if (r >= nreg) continue;
                     const uint32_t *key = keys + (size_t)r * KW;
                     float *cr = cons + (size_t)(uint32_t)ri[r].x * rstride;
-                    float v4[4] = {o[0][4 * qq], o[0][4 * qq + 1], o[0][4 * qq + 2], o[0][4 * qq + 3]};
+                    float v4[4] = {o[4 * qq], o[4 * qq + 1], o[4 * qq + 2], o[4 * qq + 3]};
                     for (int s = 0; s < net.nskip[li]; ++s) {
                         const SkipDev &sk = net.skip[li][s];
                         if (sk.kind == 0) {
@@ -1109,138 +1114,91 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
                     st4<float>(cr + (size_t)row * 4, make_float4(sg * v4[0], sg * v4[1], sg * v4[2], sg * v4[3]));
                 }
             };
-            float4 pre[4];
-            unsigned pre_other = 0u;
             for (int i = cls; i <= net.n_lin - 2; ++i) {
                 const int M = net.nodes[i + 1];
                 const int mtiles = (M + 127) / 128;
                 const int mper = (mtiles + tc.mgroups - 1) / tc.mgroups;
                 const int njobs = jobs_of(net, i);
-                pre_other = load_items(i, 0, 0, 0, pre);
-                for (int mt0 = 0; mt0 < mtiles; mt0 += mper) { // the products of this group of M tiles
-                const int mt1 = min(mtiles, mt0 + mper);
-                int t = 0; // step of the pass
-                for (int job = 0; job < njobs; ++job) {
+                // the operand blocks of the layer, once per pass: (job, kb) in
+                // order; `a` holds the block built next, `b` the one after it
+                float4 a[4], b[4];
+                unsigned ao, bo = 0u;
+                int lj = 0, lkb = 0, lp = 0; // the block loaded next, and its pass (by its first M tile)
+                auto load_next = [&](float4 *v) {
+                    if (lp >= mtiles) return 0u;
+                    const unsigned o = load_items(i, lj, lkb, 0, v);
                     int src;
-                    const TcMat &mat = job_mat(net, tc, i, job, src);
-                    const float sg = src == 1 ? 1.f : -1.f;
-                    const int nkb = mat.Kp / 64;
-                    for (int kb = 0; kb < nkb; ++kb, ++t) {
-                        // the next block: of this pass, else the next pass's
-                        // first (the next layer's first is loaded when the
-                        // layer begins: registers)
-                        int njob = job, nkb2 = kb + 1;
-                        bool more = true;
-                        if (nkb2 == nkb) {
-                            nkb2 = 0;
-                            if (++njob == njobs) {
-                                njob = 0;
-                                more = mt1 < mtiles;
-                            }
+                    if (++lkb == job_mat(net, tc, i, lj, src).Kp / 64) {
+                        lkb = 0;
+                        if (++lj == njobs) {
+                            lj = 0;
+                            lp += mper;
                         }
-                        const int xs = xb & 1, fill = xb >> 1;
-                        // stage free (an aborting CTA builds nothing but still arrives)
-                        const bool ok = fill < 1 ? !*abort : swait(xdone + xs, (uint32_t)((fill - 1) & 1), err, abort);
-                        const XOp &X = XS[xs];
-                        if (ok) {
-                            put_items(X, 0, pre, sg, pre_other);
-                            for (int c = 1; c < nchunks; ++c) {
-                                float4 t4[4];
-                                const unsigned other = load_items(i, job, kb, c, t4);
-                                put_items(X, c, t4, sg, other);
-                            }
-                        }
-                        umma::fence_proxy_async(); // generic-proxy stores -> the tensor cores
-                        umma::mbar_arrive(xfull + xs);
-                        ++xb;
-                        if (t < nd) {
-                            store_block(def_first + t);
-                            shift_o();
-                            if (t == nd - 1) bar_builders();
-                        }
-                        if (more) pre_other = load_items(i, njob, nkb2, 0, pre);
                     }
-                }
-                if (t < nd) { // a pass shorter than the deferred blocks
-                    for (; t < nd; ++t) {
-                        store_block(def_first + t);
-                        shift_o();
-                    }
-                    bar_builders();
-                }
-                nd = 0;
-                const float *bias = (const float *)net.bias[i];
-                const int mA = mt0 * 128 + q4 * 32 + lane, mB = mA + 128;
-                const float bA = mA < M ? bias[mA] : 0.f;                   // loaded while the products run
-                const float bB = mt0 + 1 < mt1 && mB < M ? bias[mB] : 0.f;
-                // the layer's products are in TMEM; the TMEM loads below are
-                // warp-collective, so the warp decides as one
-                bool acc_ok = swait(accdone, (uint32_t)(accph & 1), err, abort);
-                acc_ok = __all_sync(0xffffffffu, acc_ok) && !__any_sync(0xffffffffu, *abort != 0);
-                ++accph;
-                umma::fence_after();
-                // accumulators -> registers: main + correction (+ bias); the
-                // first blocks are stored at once, the last two (at most)
-                // kept in o for the next pass's first steps
-                const int nit = (mt1 - mt0) * ncbw;
-                const int nkeep = min(kKeep, nit);
-                def_i = i;
-                def_mt0 = mt0;
-                def_ok = acc_ok;
-                def_nit = nit;
-                def_first = nit - nkeep;
-                // (every block of the pass: three M tiles of 80 columns give a
-                // warp six, so no fixed bound)
-                for (int it0 = 0; it0 < nit; it0 += 4)
+                    return o;
+                };
+                ao = load_next(a);
+                bo = load_next(b);
+                for (int mt0 = 0; mt0 < mtiles; mt0 += mper) { // the products of this group of M tiles
+                    const int mt1 = min(mtiles, mt0 + mper);
+                    for (int job = 0; job < njobs; ++job) {
+                        int src;
+                        const int nkb = job_mat(net, tc, i, job, src).Kp / 64;
+                        for (int kb = 0; kb < nkb; ++kb) {
+                            const int xs = xb & 1, fill = xb >> 1;
+                            // stage free (an aborting CTA builds nothing but still arrives)
+                            const bool ok = fill < 1 ? !*abort : swait(xdone + xs, (uint32_t)((fill - 1) & 1), err, abort);
+                            const XOp &X = XS[xs];
+                            if (ok) {
+                                put_items(X, 0, a, ao);
+                                for (int c = 1; c < nchunks; ++c) {
+                                    float4 t4[4];
+                                    const unsigned other = load_items(i, job, kb, c, t4);
+                                    put_items(X, c, t4, other);
+                                }
+                            }
+                            umma::fence_proxy_async(); // generic-proxy stores -> the tensor cores
+                            __syncwarp();
+                            if (lane == 0) umma::mbar_arrive(xfull + xs);
+                            ++xb;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int it = it0 + u;
-                    if (!acc_ok || it >= nit) break;
-                    const int mt = mt0 + it / ncbw, cb = cgrp + (it % ncbw) * ngrp;
-                    const int mm = mt * 128 + q4 * 32 + lane;
-                    const float bm = mt == mt0 ? bA : (mt == mt0 + 1 ? bB : (mm < M ? bias[mm] : 0.f));
-                    // (eight columns at a time: fewer live registers; the
-                    // destination block by constant index: registers)
-                    const uint32_t ta = lane_base + (uint32_t)((mt - mt0) * ncols + cb * 16);
-                    const uint32_t tb = lane_base + (uint32_t)((mper + mt - mt0) * ncols + cb * 16);
-                    if (it < def_first) { // stored now
+                            for (int u = 0; u < 4; ++u) a[u] = b[u];
+                            ao = bo;
+                            bo = load_next(b);
+                        }
+                    }
+                    const float *bias = (const float *)net.bias[i];
+                    const int mA = mt0 * 128 + q4 * 32 + lane, mB = mA + 128;
+                    const float bA = mA < M ? bias[mA] : 0.f;                   // loaded while the products run
+                    const float bB = mt0 + 1 < mt1 && mB < M ? bias[mB] : 0.f;
+                    // the layer's products are in TMEM; the TMEM loads below are
+                    // warp-collective, so the warp decides as one
+                    bool acc_ok = swait(accdone, (uint32_t)(accph & 1), err, abort);
+                    acc_ok = __all_sync(0xffffffffu, acc_ok) && !__any_sync(0xffffffffu, *abort != 0);
+                    ++accph;
+                    umma::fence_after();
+                    // accumulators -> registers: main + correction (+ bias),
+                    // eight columns at a time (registers) -> rows
+                    const int nit = (mt1 - mt0) * ncbw;
+                    for (int it = 0; acc_ok && it < nit; ++it) {
+                        const int mt = mt0 + it / ncbw, cb = cgrp + (it % ncbw) * ngrp;
+                        const int mm = mt * 128 + q4 * 32 + lane;
+                        const float bm = mt == mt0 ? bA : (mt == mt0 + 1 ? bB : (mm < M ? bias[mm] : 0.f));
+                        const uint32_t ta = lane_base + (uint32_t)((mt - mt0) * ncols + cb * 16);
+                        const uint32_t tb = lane_base + (uint32_t)((mper + mt - mt0) * ncols + cb * 16);
+                        float o[16];
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             float v[8], vc[8];
                             umma::tmem_ld8x2(ta + 8 * h, tb + 8 * h, v, vc);
 #pragma unroll
-                            for (int k = 0; k < 8; ++k) o[0][8 * h + k] = (k & 3) == 3 ? v[k] + vc[k] + bm : v[k] + vc[k];
+                            for (int k = 0; k < 8; ++k) o[8 * h + k] = (k & 3) == 3 ? v[k] + vc[k] + bm : v[k] + vc[k];
                         }
-                        store_block(it);
-                    } else { // kept: into o[kKeep - 1] after the earlier kept ones moved up
-                        if (kKeep > 1) shift_o();
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float v[8], vc[8];
-                            umma::tmem_ld8x2(ta + 8 * h, tb + 8 * h, v, vc);
-#pragma unroll
-                            for (int k = 0; k < 8; ++k)
-                                o[kKeep - 1][8 * h + k] = (k & 3) == 3 ? v[k] + vc[k] + bm : v[k] + vc[k];
-                        }
+                        store_block(i, mm, cb, o);
                     }
+                    umma::fence_before(); // TMEM read out before the next products overwrite it
                 }
-                for (int b = nkeep; b < kKeep; ++b) shift_o(); // the kept blocks from o[0] on
-                umma::fence_before(); // TMEM read out before the next products overwrite it
-                nd = min(kKeep, (mt1 - mt0) * ncbu);
-                // the kept rows: stored during the next pass of this layer,
-                // or the next layer's first (whose early blocks read only rows
-                // of this layer's earlier passes and of this pass's first
-                // blocks ...), else now
-                const bool defer = mt1 < mtiles || (i < net.n_lin - 2 && nd <= 2 * mt0);
-                if (!defer) {
-                    for (int t2 = 0; t2 < nd; ++t2) {
-                        store_block(def_first + t2);
-                        shift_o();
-                    }
-                    nd = 0;
-                    bar_builders(); // rows of hidden layer i + 1 written by every builder
-                }
-                }
+                bar_builders(); // rows of hidden layer i + 1 written by every builder
             }
 
             // face plane: w_eq = W_L . X_L, X_L = -C of the last hidden layer
@@ -1310,6 +1268,7 @@ __global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, T
     }
     umma::fence_before();
     __syncthreads();
+    umma::cluster_sync(); // no copy or arrival reaches a CTA that has left
     if (warp == 0) umma::tmem_dealloc(tslot, (uint32_t)tmem_cols);
 }
 
@@ -1372,7 +1331,8 @@ void launch_compose_tc(const NetDev &net, const TcNet &tc, const RegionsDev &reg
     const int slots = sms; // one resident tile per SM, the wave's tiles strided over them
     if (tc.streamed) {
         cudaFuncSetAttribute(compose_tcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        compose_tcs_kernel<<<slots, kSThreads, smem, st>>>(net, tc, reg, ch, (float)iso, slots, d_err);
+        const int grid = slots / kCluster * kCluster;
+        compose_tcs_kernel<<<grid, kSThreads, smem, st>>>(net, tc, reg, ch, (float)iso, grid, d_err);
         return;
     }
     cudaFuncSetAttribute(compose_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

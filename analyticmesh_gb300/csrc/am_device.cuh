@@ -75,17 +75,24 @@ struct WavePlan {
     int cnt[kMaxLayers];        // regions per class
     int tile0[kMaxLayers + 1];  // first tile of each class
     int R, layers;
-};
+    int group;                  // a class's tiles are a multiple of this (the CTAs of a cluster
+};                              // take tiles of one class; a tile may then hold no region)
 
+__device__ __forceinline__ int plan_class_tiles(const WavePlan &w, int c, int R)
+{
+    const int n = (w.cnt[c] + R - 1) / R;
+    return (n + w.group - 1) / w.group * w.group;
+}
 __device__ __forceinline__ int plan_tiles(const WavePlan &w, int R)
 {
     int n = 0;
-    for (int c = 0; c < w.layers; ++c) n += (w.cnt[c] + R - 1) / R;
+    for (int c = 0; c < w.layers; ++c) n += plan_class_tiles(w, c, R);
     return n;
 }
 // (one thread) the class counts; then, R chosen, the tiles
-__device__ __forceinline__ void plan_counts(WavePlan &w, const ChunkDev &ch, int layers, int count)
+__device__ __forceinline__ void plan_counts(WavePlan &w, const ChunkDev &ch, int layers, int count, int group = 1)
 {
+    w.group = group;
     w.layers = ch.order ? layers : 1;
     for (int c = 0; c < w.layers; ++c) w.cnt[c] = ch.order ? ch.ccount[c] : count;
 }
@@ -95,7 +102,7 @@ __device__ __forceinline__ void plan_finish(WavePlan &w, int R)
     int n = 0;
     for (int c = 0; c < w.layers; ++c) {
         w.tile0[c] = n;
-        n += (w.cnt[c] + R - 1) / R;
+        n += plan_class_tiles(w, c, R);
     }
     w.tile0[w.layers] = n;
 }
@@ -134,7 +141,7 @@ __device__ __forceinline__ int4 tile_region(const WavePlan &w, const RegionsDev 
 }
 __device__ __forceinline__ int tile_nreg(const WavePlan &w, int t, int c)
 {
-    return min(w.R, w.cnt[c - 1] - (t - w.tile0[c - 1]) * w.R);
+    return max(0, min(w.R, w.cnt[c - 1] - (t - w.tile0[c - 1]) * w.R));
 }
 // a region's constraint row: the rows before jend from its parent's slot
 // (rewritten by no region of this wave), the plane it was entered through with
