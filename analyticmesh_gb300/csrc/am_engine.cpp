@@ -213,6 +213,7 @@ struct am_engine {
     // chunk
     DevBuf cons, eq, rec, blocksum, order, split;
     int chunk_cap = 0;
+    int append_cap = 0;       // blocks of blocksum (AppendScratch)
     int ring = 0;             // slots of cons (ChunkDev)
     long long ring_target = 0; // what ensure_ring last asked for
     bool ring_min = false;    // memory is short: no slots beyond a wave's
@@ -317,6 +318,7 @@ struct am_engine {
         cap = 0;
         hcap = 0;
         chunk_cap = 0;
+        append_cap = 0;
         num_regions = 0;
     }
 
@@ -371,8 +373,20 @@ struct am_engine {
         }
         AM_CUDA(eq.alloc(tc * 4 * (size_t)count, st));
         AM_CUDA(rec.alloc(sizeof(int32_t) * (size_t)kVMax * count, st));
-        AM_CUDA(blocksum.alloc(sizeof(int) * ((size_t)count * kVMax / 1024 + 6), st));
+        ensure_append(count);
         chunk_cap = count;
+    }
+
+    // the append's scratch for up to `rows` rows of candidates (zeroed: its
+    // counters start at zero)
+    void ensure_append(int rows)
+    {
+        const int blocks = append_blocks(rows);
+        if (blocks <= append_cap) return;
+        append_cap = 0;
+        AM_CUDA(blocksum.alloc(append_scratch_bytes(blocks), st));
+        AM_CUDA(cudaMemsetAsync(blocksum.p, 0, append_scratch_bytes(blocks), st));
+        append_cap = blocks;
     }
 
     // a network with no layer product has nothing to take from a parent
@@ -552,10 +566,8 @@ struct am_engine {
                 else
                     launch_compose(prec, net, reg, ch, iso, d_err.as<int>(), st);
                 launch_polygon(prec, net, reg, ch, hs, tol, face_warps, fp64_counter(), d_err.as<int>(), st);
-                launch_append(0, prec, net, reg, ch, hs, nullptr, nullptr, nullptr, chunk * kVMax,
-                              d_tail.as<long long>(), blocksum.as<int>(), (int)(blocksum.bytes / sizeof(int)),
-                              d_err.as<int>(), st);
-                launch_wave_step(ctl(), cond, st);
+                launch_append(0, prec, net, reg, ch, hs, nullptr, nullptr, nullptr, 0, d_tail.as<long long>(),
+                              blocksum.as<AppendScratch>(), append_cap, d_err.as<int>(), st, &cond);
                 cudaGraph_t captured = nullptr;
                 AM_CUDA(cudaStreamEndCapture(st, &captured));
                 AM_CUDA(cudaGraphInstantiate(&wexec, wgraph, 0));
@@ -869,7 +881,7 @@ void run_begin(am_engine *e, const RunArgs &a)
     const long long first_wave = std::min<long long>(chunk, e->lean ? 4ll * S + 1024 : std::max(4ll * S + 1024, 65536ll));
     e->ensure_regions(std::max<long long>(S, 1) + first_wave * kVMax);
     e->ensure_table((long long)S + first_wave * kVMax, false);
-    AM_CUDA(e->blocksum.grow(sizeof(int) * ((size_t)S / 1024 + 6), 0, st));
+    e->ensure_append((S + 31) / 32);
     AM_CUDA(cudaStreamSynchronize(st));
 
     e->run.launches = 0;
@@ -881,10 +893,10 @@ void run_begin(am_engine *e, const RunArgs &a)
         ChunkDev sc{};
         sc.rec = e->s_rec.as<int32_t>();
         launch_append(1, prec, net, e->regions(), sc, e->hashdev(), e->s_keys.as<uint32_t>(),
-                      e->s_hash.as<uint64_t>(), e->s_pts.p, S, e->d_tail.as<long long>(), e->blocksum.as<int>(),
-                      (int)(e->blocksum.bytes / sizeof(int)), e->d_err.as<int>(), st);
+                      e->s_hash.as<uint64_t>(), e->s_pts.p, S, e->d_tail.as<long long>(),
+                      e->blocksum.as<AppendScratch>(), e->append_cap, e->d_err.as<int>(), st);
     }
-    e->run.launches += 5; // + the parameter check
+    e->run.launches += 4; // + the parameter check
     AM_CUDA(cudaGetLastError());
     const long long tail = e->poll();
     e->num_regions = tail;
@@ -959,7 +971,7 @@ bool run_graph_done(am_engine *e)
     AM_CHECK(h->waves < kMaxWaves, "wave bound reached");
     r.tail = h->tail;
     r.chunks += h->waves;
-    r.launches += (e->classes() ? 6ll : 5ll) * h->waves;
+    r.launches += (e->classes() ? 4ll : 3ll) * h->waves;
     r.head = h->head;
     e->num_regions = r.tail;
     if (e->over_limit(r.tail)) return false; // stop: the regions so far stay
@@ -1012,15 +1024,15 @@ void run_host_loop(am_engine *e)
             t_poly += ms;
             AM_CUDA(cudaEventRecord(pa, st));
         }
-        launch_append(0, prec, net, reg, ch, hs, nullptr, nullptr, nullptr, count * kVMax, e->d_tail.as<long long>(),
-                      e->blocksum.as<int>(), (int)(e->blocksum.bytes / sizeof(int)), e->d_err.as<int>(), st);
+        launch_append(0, prec, net, reg, ch, hs, nullptr, nullptr, nullptr, 0, e->d_tail.as<long long>(),
+                      e->blocksum.as<AppendScratch>(), e->append_cap, e->d_err.as<int>(), st);
         if (e->phase_timing) {
             AM_CUDA(cudaEventRecord(pb, st));
             AM_CUDA(cudaEventSynchronize(pb));
             AM_CUDA(cudaEventElapsedTime(&ms, pa, pb));
             t_front += ms;
         }
-        launches += 4;
+        launches += 3;
         AM_CUDA(cudaGetLastError());
         head += count;
         tail = e->poll();

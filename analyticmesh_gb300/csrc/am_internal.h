@@ -165,17 +165,27 @@ void launch_seed_pack(const uint8_t *states, int S, int N, int W, uint32_t *keys
                       int *zeroed = nullptr);
 void launch_seed_insert(const uint32_t *keys, const uint64_t *hash, int S, int W, const HashDev &hs, int32_t *rec,
                         int *d_err, cudaStream_t st);
-// flags + scan + append.  mode 0: children of a chunk, mode 1: seeds.
+// append of the winners.  mode 0: children of a wave, mode 1: seeds.  cond: the
+// graph-driven loop's condition, which the append's last block sets after it has
+// advanced ctl to the next wave.
+struct AppendScratch {
+    unsigned int ticket, done; // zero between appends
+    unsigned int epoch;        // appends made
+    unsigned int pad;
+    long long new_tail;
+    unsigned long long entry[1]; // [blocks] winners per block, tagged with the append's number
+};
+inline size_t append_scratch_bytes(int blocks) { return sizeof(AppendScratch) + sizeof(unsigned long long) * (size_t)blocks; }
+int append_blocks(int rows_max);
 void launch_append(int mode, int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch,
                    const HashDev &hs, const uint32_t *seed_keys, const uint64_t *seed_hash, const void *seed_points,
-                   int n_items, long long *d_tail, int *d_blocksum, int nblocks_cap, int *d_err, cudaStream_t st);
+                   int n_items, long long *d_tail, AppendScratch *sc, int blocks_cap, int *d_err, cudaStream_t st,
+                   const cudaGraphConditionalHandle *cond = nullptr);
 void launch_rehash(const RegionsDev &reg, long long n, const HashDev &hs, int *d_err, cudaStream_t st);
-// graph-driven loop: advance ctl to the next wave and set the loop condition
 void launch_region_stats(const int32_t *nv, const int8_t *status, long long n, unsigned long long *out,
                          cudaStream_t st);
 // class lists and splits of a wave (ChunkDev); ccount must be zero
 void launch_wave_classes(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, cudaStream_t st);
-void launch_wave_step(WaveCtl *ctl, cudaGraphConditionalHandle cond, cudaStream_t st);
 int device_sms();
 // the network's parameter buffers, checked for NaN / infinity in one launch
 struct FiniteList {

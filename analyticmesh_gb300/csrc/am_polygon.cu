@@ -1031,36 +1031,57 @@ __device__ int seed_start(const Rows &rows, const GlobalRows<TC> &all, const Bal
     int x_max = (all.n - 1) * (all.n - 2);
     if (x_max > 812) x_max = 812;
     if (x_max < 0) x_max = 0;
-    for (int x = 0; x <= x_max; ++x) {
+    // eight pairs at a time, four lanes per pair (its Cramer determinants, the
+    // arithmetic of warp_solve); their vertices are tested one after the other,
+    // the first that every other row admits wins
+    const int G = lane >> 2, L = lane & 3, gbase = lane & ~3;
+    for (int x0 = 0; x0 <= x_max; x0 += 8) {
         int i, j;
-        get_i_j(x, all.n, i, j);
+        get_i_j(min(x0 + G, x_max), all.n, i, j);
         const int ri0 = __shfl_sync(kFull, top0, i & 31), ri1 = __shfl_sync(kFull, top1, i & 31);
         const int rj0 = __shfl_sync(kFull, top0, j & 31), rj1 = __shfl_sync(kFull, top1, j & 31);
         const int ri = i < 32 ? ri0 : ri1;
         const int rj = j < 32 ? rj0 : rj1;
-        TS v[3];
-        TC vc[3];
-        warp_solve<TC, TS>(rows.get(ri), rows.get(rj), eqv, v, vc, lane);
-        bool bad = false;
-        for (int k = lane; k < rows.n; k += 32) {
-            if (k == ri || k == rj) continue;
-            const vec4_t<TC> r = rows.get(k);
-            if (dot3(r.x, vc[0], r.y, vc[1], r.z, vc[2]) + r.w > eps) bad = true;
+        // lane t of the group converts components 2t, 2t + 1 of [row i | row j]
+        const vec4_t<TC> rr = rows.get(L < 2 ? ri : rj);
+        const TS c0 = (TS)(L & 1 ? rr.z : rr.x), c1 = (TS)(L & 1 ? rr.w : rr.y);
+        TS m[8];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            m[2 * t] = __shfl_sync(kFull, c0, gbase | t);
+            m[2 * t + 1] = __shfl_sync(kFull, c1, gbase | t);
         }
-        if (__any_sync(kFull, bad)) continue;
-        if (ball.d2 != INFINITY && !ball.in((float)vc[0], (float)vc[1], (float)vc[2])) {
-            const int ki = rows.name(ri), kj = rows.name(rj);
-            for (int k = lane; k < all.n; k += 32) {
-                if (k == ki || k == kj) continue;
-                const vec4_t<TC> r = all.get(k);
+        const TS a00 = L == 1 ? -m[3] : m[0], a01 = L == 2 ? -m[3] : m[1], a02 = L == 3 ? -m[3] : m[2];
+        const TS a10 = L == 1 ? -m[7] : m[4], a11 = L == 2 ? -m[7] : m[5], a12 = L == 3 ? -m[7] : m[6];
+        const TS a20 = L == 1 ? -eqv[3] : eqv[0], a21 = L == 2 ? -eqv[3] : eqv[1], a22 = L == 3 ? -eqv[3] : eqv[2];
+        const TS d = det3<TS>(a00, a01, a02, a10, a11, a12, a20, a21, a22);
+        const TS xv = d / __shfl_sync(kFull, d, gbase);
+        for (int g = 0; g < 8 && x0 + g <= x_max; ++g) {
+            const TS v[3] = {__shfl_sync(kFull, xv, 4 * g + 1), __shfl_sync(kFull, xv, 4 * g + 2),
+                             __shfl_sync(kFull, xv, 4 * g + 3)};
+            const TC vc[3] = {(TC)v[0], (TC)v[1], (TC)v[2]};
+            const int pi_ = __shfl_sync(kFull, ri, 4 * g), pj_ = __shfl_sync(kFull, rj, 4 * g);
+            bool bad = false;
+            for (int k = lane; k < rows.n; k += 32) {
+                if (k == pi_ || k == pj_) continue;
+                const vec4_t<TC> r = rows.get(k);
                 if (dot3(r.x, vc[0], r.y, vc[1], r.z, vc[2]) + r.w > eps) bad = true;
             }
             if (__any_sync(kFull, bad)) continue;
+            if (!ball.in((float)vc[0], (float)vc[1], (float)vc[2])) {
+                const int ki = rows.name(pi_), kj = rows.name(pj_);
+                for (int k = lane; k < all.n; k += 32) {
+                    if (k == ki || k == kj) continue;
+                    const vec4_t<TC> r = all.get(k);
+                    if (dot3(r.x, vc[0], r.y, vc[1], r.z, vc[2]) + r.w > eps) bad = true;
+                }
+                if (__any_sync(kFull, bad)) continue;
+            }
+            p[0] = v[0];
+            p[1] = v[1];
+            p[2] = v[2];
+            return pi_;
         }
-        p[0] = v[0];
-        p[1] = v[1];
-        p[2] = v[2];
-        return ri;
     }
     return -1;
 }
