@@ -404,17 +404,28 @@ __global__ void __launch_bounds__(kThreads, 1) compose_kernel(NetDev net, Region
 }
 
 template <typename T>
-__global__ void prepare_weights_kernel(const T *src, int M, int K, int Mp, T *dst)
+__global__ void load_kernel(LoadList list, int *err)
 {
-    // dst[k][m] = src[m][k], zero padding for m >= M
-    const long long n = (long long)K * Mp;
+    const LoadList::Item &it = list.item[blockIdx.y];
+    const T *src = (const T *)it.src;
+    T *dst = (T *)it.dst;
+    const long long n = it.Mp ? (long long)it.K * it.Mp : it.K;
+    bool bad = false;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(q / Mp), m = (int)(q % Mp);
-        dst[q] = m < M ? src[(size_t)m * K + k] : T(0);
+        T v;
+        if (it.Mp) {
+            const int k = (int)(q / it.Mp), m = (int)(q % it.Mp);
+            v = m < it.M ? src[(size_t)m * it.K + k] : T(0);
+        } else {
+            v = src[q];
+        }
+        bad |= !isfinite(v);
+        dst[q] = v;
     }
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(err, kErrNonFinite);
 }
 
-// the same for every listed linear in one launch (blockIdx.y); *nonfinite set
+// FP32 linears transposed and padded in one launch (blockIdx.y); *nonfinite set
 // where a value is not finite
 __global__ void prepare_list_kernel(PrepareList list, int *nonfinite)
 {
@@ -430,30 +441,19 @@ __global__ void prepare_list_kernel(PrepareList list, int *nonfinite)
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(nonfinite, 1);
 }
 
-// every value of the listed buffers finite; kErrNonFinite otherwise
-template <typename T>
-__global__ void check_finite_kernel(FiniteList list, int *err)
-{
-    const int b = blockIdx.y;
-    const T *p = (const T *)list.p[b];
-    bool bad = false;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < list.n[b]; q += (long long)gridDim.x * blockDim.x)
-        bad |= !isfinite(p[q]);
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(err, kErrNonFinite);
-}
-
 } // namespace
 
-void launch_check_finite(int prec, const FiniteList &list, int *d_err, cudaStream_t st)
+void launch_load(int prec, const LoadList &list, int *d_err, cudaStream_t st)
 {
     if (list.count <= 0) return;
     long long most = 1;
-    for (int b = 0; b < list.count; ++b) most = std::max(most, list.n[b]);
-    const dim3 grid((unsigned)std::min<long long>((most + 255) / 256, 64), (unsigned)list.count);
+    for (int b = 0; b < list.count; ++b)
+        most = std::max(most, (long long)list.item[b].K * std::max(list.item[b].Mp, 1));
+    const dim3 grid((unsigned)std::min<long long>((most + 255) / 256, 256), (unsigned)list.count);
     if (prec == kFloat64)
-        check_finite_kernel<double><<<grid, 256, 0, st>>>(list, d_err);
+        load_kernel<double><<<grid, 256, 0, st>>>(list, d_err);
     else
-        check_finite_kernel<float><<<grid, 256, 0, st>>>(list, d_err);
+        load_kernel<float><<<grid, 256, 0, st>>>(list, d_err);
 }
 
 template <typename T>
@@ -478,17 +478,6 @@ void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const Ch
 void launch_prepare_list(const PrepareList &list, int *nonfinite, cudaStream_t st)
 {
     if (list.count > 0) prepare_list_kernel<<<dim3(64, (unsigned)list.count), 256, 0, st>>>(list, nonfinite);
-}
-
-void launch_prepare_weights(int prec, const void *src, int M, int K, int Mp, void *dst, cudaStream_t st)
-{
-    const long long n = (long long)K * Mp;
-    if (n <= 0) return;
-    const int grid = (int)std::min<long long>((n + 255) / 256, 4096);
-    if (prec == kFloat64)
-        prepare_weights_kernel<double><<<grid, 256, 0, st>>>((const double *)src, M, K, Mp, (double *)dst);
-    else
-        prepare_weights_kernel<float><<<grid, 256, 0, st>>>((const float *)src, M, K, Mp, (float *)dst);
 }
 
 } // namespace am

@@ -219,7 +219,7 @@ struct am_engine {
     bool ring_min = false;    // memory is short: no slots beyond a wave's
     long long rows_from = 0;  // regions before this have no rows in the ring
     // seeds
-    DevBuf s_states, s_keys, s_hash, s_pts, s_rec;
+    DevBuf s_states, s_keys, s_hash, s_raw, s_pts, s_rec;
     // counters
     // wave control block (region tail, error bits, the graph-driven loop's
     // queue state), read back with one copy into pinned host memory
@@ -267,11 +267,12 @@ struct am_engine {
     // results
     bool has_am = false, has_mesh = false;
     long long num_regions = 0;
+    long long poly_verts = 0; // polygon corners of the result (the weld's vertex slots)
     am_stats stats{};
     int flip = 0;
     double iso = 0.0;
     // mesh
-    DevBuf w_table, w_rep, w_flag, w_vidx, w_bsum, w_fflag, w_fsize, w_fid, w_foff, w_verts, w_fs, w_fi, w_counts;
+    DevBuf w_table, w_rep, w_flag, w_vidx, w_bsum, w_fflag, w_fsize, w_fid, w_foff, w_verts, w_fs, w_fi;
     DevBuf w_voff, w_vsid, w_wslot; // compacted polygon vertex slots, their keys' table slots
     std::vector<double> mesh_verts;
     std::vector<int32_t> mesh_fs, mesh_fi;
@@ -675,25 +676,58 @@ void run_begin(am_engine *e, const RunArgs &a)
     for (int i = 0; i <= e->n_lin; ++i) net.nodes[i] = e->nodes[i];
     net.hoff[1] = 0;
     for (int h = 1; h < e->n_lin; ++h) net.hoff[h + 1] = net.hoff[h] + e->nodes[h];
+    // The parameters go straight from the caller's device memory into the
+    // engine's layouts; those in host memory by way of one staging buffer.
+    AM_CUDA(cudaMemsetAsync(e->d_err.p, 0, sizeof(int), st));
+    size_t stage_bytes = 0, stage_used = 0;
+    auto staged = [](size_t n) { return (n + 255) / 256 * 256; };
+    for (int i = 0; i < e->n_lin; ++i) {
+        AM_CHECK(weights[i] && biases[i], "a weight / bias pointer is NULL");
+        stage_bytes += staged(tc * (size_t)e->nodes[i + 1] * e->nodes[i]) + staged(tc * (size_t)e->nodes[i + 1]);
+    }
+    for (int t = 0; t < num_arc_tm && arc_tm_shapes; ++t)
+        stage_bytes += staged(tc * (size_t)std::max(arc_tm_shapes[2 * t], 0) * (size_t)std::max(arc_tm_shapes[2 * t + 1], 0));
+    stage_bytes += staged(tc * 3 * (size_t)e->E) + staged(tc * (size_t)e->E);
+    auto on_device = [&](const void *src, size_t n) -> const void * {
+        if (is_device_ptr(src)) return src;
+        AM_CUDA(e->scratch.reserve(stage_bytes));
+        char *d = e->scratch.as<char>() + stage_used;
+        stage_used += staged(n);
+        AM_CUDA(cudaMemcpyAsync(d, src, n, cudaMemcpyHostToDevice, st));
+        return d;
+    };
+    LoadList load;
+    load.count = 0;
+    auto flush = [&] {
+        launch_load(prec == kFloat64 ? kFloat64 : kFloat32, load, e->d_err.as<int>(), st);
+        load.count = 0;
+    };
+    auto add = [&](const void *src, void *dst, int M, int K, int Mp) {
+        if (load.count == 64) flush();
+        load.item[load.count++] = {src, dst, M, K, Mp};
+    };
+    const void *wsrc[kMaxLayers] = {};
     for (int i = 0; i < e->n_lin; ++i) {
         const int M = e->nodes[i + 1], K = e->nodes[i];
-        AM_CHECK(weights[i] && biases[i], "a weight / bias pointer is NULL");
-        upload(e->bias[i], biases[i], tc * M, st);
+        AM_CUDA(e->bias[i].reserve(tc * (size_t)M));
+        add(on_device(biases[i], tc * (size_t)M), e->bias[i].p, 0, M, 0);
         net.bias[i] = e->bias[i].p;
+        wsrc[i] = on_device(weights[i], tc * (size_t)M * K);
         if (i == 0) {
-            upload(e->w0, weights[0], tc * (size_t)M * 3, st);
+            AM_CUDA(e->w0.reserve(tc * (size_t)M * 3));
+            add(wsrc[0], e->w0.p, 0, 3 * M, 0);
             net.W0 = e->w0.p;
         } else {
             const int Mp = (M + 3) / 4 * 4;
-            upload(e->scratch, weights[i], tc * (size_t)M * K, st);
             AM_CUDA(e->wt[i].reserve(tc * (size_t)K * Mp));
-            launch_prepare_weights(prec == kFloat64 ? kFloat64 : kFloat32, e->scratch.p, M, K, Mp, e->wt[i].p, st);
+            add(wsrc[i], e->wt[i].p, M, K, Mp);
             net.Wt[i] = e->wt[i].p;
             net.Mp[i] = Mp;
         }
     }
     int ntm = 0;
     long long *tm_count = e->tm_count;
+    std::vector<const void *> tsrc((size_t)std::max(num_arc_tm, 0), nullptr);
     for (int i = 1; i < e->n_lin; ++i) {
         const int *row = e->arc.data() + (size_t)(i - 1) * e->arc_cols;
         net.nskip[i] = row[0];
@@ -709,10 +743,9 @@ void run_begin(am_engine *e, const RunArgs &a)
             } else {
                 AM_CHECK(ntm < 64, "too many transform matrices");
                 const int Mp = (h + 3) / 4 * 4;
-                upload(e->scratch, arc_tm[t], tc * (size_t)h * w, st);
+                if (!tsrc[(size_t)t]) tsrc[(size_t)t] = on_device(arc_tm[t], tc * (size_t)h * w);
                 AM_CUDA(e->tmt[ntm].reserve(tc * (size_t)w * Mp));
-                launch_prepare_weights(prec == kFloat64 ? kFloat64 : kFloat32, e->scratch.p, h, w, Mp,
-                                       e->tmt[ntm].p, st);
+                add(tsrc[(size_t)t], e->tmt[ntm].p, h, w, Mp);
                 sk.kind = 1;
                 sk.tmt = e->tmt[ntm].p;
                 sk.Mp = Mp;
@@ -723,32 +756,14 @@ void run_begin(am_engine *e, const RunArgs &a)
     }
     e->ntm = ntm;
     if (e->E) {
-        upload(e->wext, w_extra, tc * 3 * (size_t)e->E, st);
-        upload(e->bext, b_extra, tc * (size_t)e->E, st);
+        AM_CUDA(e->wext.reserve(tc * 3 * (size_t)e->E));
+        AM_CUDA(e->bext.reserve(tc * (size_t)e->E));
+        add(on_device(w_extra, tc * 3 * (size_t)e->E), e->wext.p, 0, 3 * e->E, 0);
+        add(on_device(b_extra, tc * (size_t)e->E), e->bext.p, 0, e->E, 0);
     }
     net.w_extra = e->wext.p;
     net.b_extra = e->bext.p;
-    {
-        // every parameter finite (checked on the device copies, one launch;
-        // decoded as AM_ERR_INVALID_ARGUMENT by the first poll)
-        FiniteList fl{};
-        auto add = [&](const void *p, long long n) {
-            if (p && n > 0 && fl.count < 64) {
-                fl.p[fl.count] = p;
-                fl.n[fl.count++] = n;
-            }
-        };
-        AM_CUDA(cudaMemsetAsync(e->d_err.p, 0, sizeof(int), st));
-        for (int i = 0; i < e->n_lin; ++i) add(e->bias[i].p, e->nodes[i + 1]);
-        add(e->w0.p, 3ll * e->nodes[1]);
-        for (int i = 1; i < e->n_lin; ++i) add(e->wt[i].p, (long long)e->nodes[i] * net.Mp[i]);
-        for (int t = 0; t < ntm; ++t) add(e->tmt[t].p, tm_count[t]);
-        if (e->E) {
-            add(e->wext.p, 3ll * e->E);
-            add(e->bext.p, e->E);
-        }
-        launch_check_finite(prec == kFloat64 ? kFloat64 : kFloat32, fl, e->d_err.as<int>(), st);
-    }
+    flush();
     if (prec == kMixed) {
         // three bf16 terms per weight, stored as 128 x 64 shared-memory block images
         TcNet &tc = e->tcnet;
@@ -757,9 +772,8 @@ void run_begin(am_engine *e, const RunArgs &a)
         tc.mgroups = 1;
         auto split = [&](DevBuf &buf, const void *src_fp32, int M, int K, TcMat &m) {
             const int Mp = (M + 127) / 128 * 128, Kp = (K + 63) / 64 * 64;
-            upload(e->scratch, src_fp32, sizeof(float) * (size_t)M * K, st);
             AM_CUDA(buf.reserve((size_t)(Mp / 128) * (Kp / 64) * kWBlockBytes));
-            launch_pack_weights(e->scratch.as<float>(), M, K, Mp, Kp, buf.p, st);
+            launch_pack_weights((const float *)src_fp32, M, K, Mp, Kp, buf.p, st);
             m.blocks = (const uint8_t *)buf.p;
             m.Mp = Mp;
             m.Kp = Kp;
@@ -767,12 +781,12 @@ void run_begin(am_engine *e, const RunArgs &a)
             tc.mtiles_max = std::max(tc.mtiles_max, Mp / 128);
         };
         for (int i = 1; i <= e->n_lin - 2; ++i) {
-            split(e->tc_lin[i], weights[i], e->nodes[i + 1], e->nodes[i], tc.lin[i]);
+            split(e->tc_lin[i], wsrc[i], e->nodes[i + 1], e->nodes[i], tc.lin[i]);
             const int *row = e->arc.data() + (size_t)(i - 1) * e->arc_cols;
             for (int c = 0; c < row[0]; ++c) {
                 const int from = row[1 + 2 * c], t = row[2 + 2 * c];
                 const int h = arc_tm_shapes[2 * t], w = arc_tm_shapes[2 * t + 1];
-                if ((h || w) && from >= 1) split(e->tc_skip[i][c], arc_tm[t], h, w, tc.skip[i][c]);
+                if ((h || w) && from >= 1) split(e->tc_skip[i][c], tsrc[(size_t)t], h, w, tc.skip[i][c]);
             }
         }
         // the operand also holds hidden layer 1 and the last hidden layer
@@ -846,23 +860,22 @@ void run_begin(am_engine *e, const RunArgs &a)
 
     // ---------------------------------------------------------- seeds
     const int S = num_points;
-    upload(e->s_states, states, (size_t)S * e->N, st);
-    {
-        // seed points in the solve precision
-        std::vector<double> pd(3 * (size_t)S);
-        std::vector<unsigned char> raw(tc * 3 * (size_t)S);
-        to_host(raw.data(), points, raw.size(), st);
-        AM_CUDA(cudaStreamSynchronize(st));
-        for (size_t q = 0; q < 3 * (size_t)S; ++q)
-            pd[q] = tc == 8 ? ((const double *)raw.data())[q] : (double)((const float *)raw.data())[q];
-        if (ts == 8) {
-            upload(e->s_pts, pd.data(), sizeof(double) * pd.size(), st);
-        } else {
-            std::vector<float> pf(pd.begin(), pd.end());
-            upload(e->s_pts, pf.data(), sizeof(float) * pf.size(), st);
-        }
-        AM_CUDA(cudaStreamSynchronize(st));
+    // (states and points in device memory are read where they are)
+    const void *dstates = states, *dpoints = points;
+    if (!is_device_ptr(states)) {
+        upload(e->s_states, states, (size_t)S * e->N, st);
+        dstates = e->s_states.p;
     }
+    if (!is_device_ptr(points)) {
+        upload(e->s_raw, points, tc * 3 * (size_t)S, st);
+        dpoints = e->s_raw.p;
+    }
+    AM_CUDA(e->s_pts.reserve(ts * 3 * (size_t)S));
+    SeedPoints sp;
+    sp.src = dpoints;
+    sp.dst = e->s_pts.p;
+    sp.pbytes = (int)tc;
+    sp.tbytes = (int)ts;
     AM_CUDA(e->s_keys.reserve(sizeof(uint32_t) * (size_t)S * e->W));
     AM_CUDA(e->s_hash.reserve(sizeof(uint64_t) * (size_t)S));
     AM_CUDA(e->s_rec.reserve(sizeof(int32_t) * (size_t)S));
@@ -882,11 +895,11 @@ void run_begin(am_engine *e, const RunArgs &a)
     e->ensure_regions(std::max<long long>(S, 1) + first_wave * kVMax);
     e->ensure_table((long long)S + first_wave * kVMax, false);
     e->ensure_append((S + 31) / 32);
-    AM_CUDA(cudaStreamSynchronize(st));
 
     e->run.launches = 0;
     AM_CUDA(cudaEventRecord(e->ev0, st));
-    launch_seed_pack(e->s_states.as<uint8_t>(), S, e->N, e->W, e->s_keys.as<uint32_t>(), e->s_hash.as<uint64_t>(), st);
+    launch_seed_pack((const uint8_t *)dstates, S, e->N, e->W, e->s_keys.as<uint32_t>(), e->s_hash.as<uint64_t>(), st,
+                     nullptr, sp);
     launch_seed_insert(e->s_keys.as<uint32_t>(), e->s_hash.as<uint64_t>(), S, e->W, e->hashdev(),
                        e->s_rec.as<int32_t>(), e->d_err.as<int>(), st);
     {
@@ -1061,10 +1074,15 @@ void run_end(am_engine *e)
     const double iso = run.iso;
     cudaEvent_t ev0 = e->ev0, ev1 = e->ev1;
     AM_CUDA(cudaEventRecord(ev1, st));
-    AM_CUDA(cudaEventSynchronize(ev1));
+    // face and status counts, reduced on the device; they and the control block
+    // come back in one copy
+    unsigned long long *d = (unsigned long long *)((char *)e->d_tail.p + kStatsOff);
+    const unsigned long long *h = (const unsigned long long *)((const char *)e->h_ctl + kStatsOff);
+    AM_CUDA(cudaMemsetAsync(d, 0, kStatsCount * sizeof(unsigned long long), st));
+    launch_region_stats(e->nv.as<int32_t>(), e->status.as<int8_t>(), tail, d, st);
+    e->poll(kCtlBytes);
     float total = 0;
     AM_CUDA(cudaEventElapsedTime(&total, ev0, ev1));
-    e->check_err();
 
     // statistics
     am_stats &sx = e->stats;
@@ -1076,14 +1094,6 @@ void run_end(am_engine *e)
     sx.frontier_ms = t_front;
     sx.kernel_launches = launches;
     {
-        // face and status counts, reduced on the device (48 bytes come back)
-        unsigned long long *d = (unsigned long long *)((char *)e->d_tail.p + kStatsOff);
-        const unsigned long long *h = (const unsigned long long *)((const char *)e->h_ctl + kStatsOff);
-        AM_CUDA(cudaMemsetAsync(d, 0, kStatsCount * sizeof(unsigned long long), st));
-        launch_region_stats(e->nv.as<int32_t>(), e->status.as<int8_t>(), tail, d, st);
-        AM_CUDA(cudaMemcpyAsync((char *)e->h_ctl + kStatsOff, d, (kStatsCount + 1) * sizeof(unsigned long long),
-                                cudaMemcpyDeviceToHost, st));
-        AM_CUDA(cudaStreamSynchronize(st));
         sx.num_faces = (int64_t)h[0];
         sx.max_polygon_verts = (int32_t)h[1];
         sx.num_nostart = (int64_t)h[2 + kNoStart - 1];
@@ -1091,6 +1101,7 @@ void run_end(am_engine *e)
         sx.num_truncated = (int64_t)h[2 + kTruncated - 1];
         sx.num_singular = (int64_t)h[2 + kSingular - 1];
         sx.num_fp64_walks = (int64_t)h[kFp64Slot];
+        e->poly_verts = (long long)h[2 + kSingular];
     }
     e->flip = flip_insideout ? 1 : 0;
     e->iso = iso;
@@ -1558,18 +1569,7 @@ int am_combine_mesh(am_engine *e, double scale, const double *center3)
         // the vertex slots in use, compacted (a face has ~4 of its 32)
         AM_CUDA(e->w_voff.reserve(sizeof(int) * (nr + 1)));
         AM_CUDA(e->w_fflag.reserve(sizeof(int) * (nr + 1)));
-        AM_CUDA(e->w_bsum.reserve(sizeof(int) * (nr / 1024 + 2)));
-        AM_CUDA(e->w_counts.reserve(sizeof(long long) * 3));
-        WeldBuffers wb{};
-        wb.voff = e->w_voff.as<int>();
-        wb.fflag = e->w_fflag.as<int>();
-        wb.bsum = e->w_bsum.as<int>();
-        wb.counts = e->w_counts.as<long long>();
-        launch_weld_slots(e->regions(), R, wb, st);
-        AM_CUDA(cudaGetLastError());
-        long long V = 0;
-        AM_CUDA(cudaMemcpyAsync(&V, wb.counts, sizeof(long long), cudaMemcpyDeviceToHost, st));
-        AM_CUDA(cudaStreamSynchronize(st));
+        const long long V = e->poly_verts;
         AM_CHECK(V < (1ll << 30), "too many polygon vertices for one mesh (2^30)");
         const long long ns = std::max<long long>(V, 1);
         unsigned long long tcap = 1;
@@ -1587,6 +1587,10 @@ int am_combine_mesh(am_engine *e, double scale, const double *center3)
         AM_CUDA(e->w_verts.reserve(e->ts * 3 * ns));
         AM_CUDA(e->w_fs.reserve(sizeof(int) * (nr + 1)));
         AM_CUDA(e->w_fi.reserve(sizeof(int) * ns));
+        WeldBuffers wb{};
+        wb.voff = e->w_voff.as<int>();
+        wb.fflag = e->w_fflag.as<int>();
+        wb.counts = (long long *)((char *)e->d_tail.p + kStatsOff) + kWeldSlot;
         wb.vsid = e->w_vsid.as<long long>();
         wb.table = e->w_table.as<unsigned long long>();
         wb.mask = tcap - 1;
@@ -1603,13 +1607,12 @@ int am_combine_mesh(am_engine *e, double scale, const double *center3)
         wb.face_idx = e->w_fi.as<int>();
         const double c0[3] = {0, 0, 0};
         AM_CUDA(cudaMemsetAsync(e->d_err.p, 0, sizeof(int), st));
+        launch_weld_slots(e->regions(), R, wb, st);
         launch_weld(e->prec, e->weld_mode, e->N, e->W, e->regions(), R, V, wb, scale, center3 ? center3 : c0, e->flip,
                     e->d_err.as<int>(), st);
         AM_CUDA(cudaGetLastError());
-        long long cnt[3] = {0, 0, 0};
-        AM_CUDA(cudaMemcpyAsync(cnt, wb.counts, sizeof(cnt), cudaMemcpyDeviceToHost, st));
-        AM_CUDA(cudaStreamSynchronize(st));
-        e->check_err();
+        e->poll(kCtlBytes); // the counts with the error bits
+        const long long *cnt = (const long long *)((const char *)e->h_ctl + kStatsOff) + kWeldSlot;
         e->stats.mesh_num_verts = cnt[0];
         e->stats.mesh_num_faces = cnt[1];
         e->stats.mesh_num_indices = cnt[2];

@@ -28,12 +28,19 @@ __device__ __forceinline__ unsigned long long load_slot(const unsigned long long
 
 // a warp per state: a word is one coalesced 32-byte read and a ballot (a thread
 // per state read bytes N apart from its neighbours')
-__global__ void seed_pack_kernel(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, int *zeroed)
+__global__ void seed_pack_kernel(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, int *zeroed,
+                                 SeedPoints pt)
 {
     if (zeroed && blockIdx.x == 0 && threadIdx.x == 0) *zeroed = 0;
     const int lane = threadIdx.x & 31;
     const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (s >= S) return;
+    if (pt.dst && lane < 3) { // (FP32 to FP64 is exact)
+        const size_t q = (size_t)s * 3 + lane;
+        const double v = pt.pbytes == 8 ? ((const double *)pt.src)[q] : (double)((const float *)pt.src)[q];
+        if (pt.tbytes == 8) ((double *)pt.dst)[q] = v;
+        else ((float *)pt.dst)[q] = (float)v;
+    }
     const uint8_t *row = states + (size_t)s * N;
     uint64_t h = 0;
     for (int w0 = 0; w0 < W; w0 += 32) {
@@ -343,11 +350,12 @@ __global__ void region_stats_kernel(const int32_t *nv, const int8_t *status, lon
     __shared__ unsigned int s[kStatsCount];
     if (threadIdx.x < kStatsCount) s[threadIdx.x] = 0u;
     __syncthreads();
-    unsigned int faces = 0, vmax = 0, bad[4] = {0u, 0u, 0u, 0u};
+    unsigned int faces = 0, vmax = 0, verts = 0, bad[4] = {0u, 0u, 0u, 0u};
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {
         const int v = nv[r];
         faces += v >= 3 ? 1u : 0u;
         vmax = max(vmax, (unsigned int)max(v, 0));
+        verts += (unsigned int)min(max(v, 0), kVMax);
         const int st = status[r];
         if (st >= kNoStart && st <= kSingular) bad[st - kNoStart]++;
     }
@@ -355,6 +363,7 @@ __global__ void region_stats_kernel(const int32_t *nv, const int8_t *status, lon
     for (int o = 16; o > 0; o >>= 1) {
         faces += __shfl_xor_sync(0xffffffffu, faces, o);
         vmax = max(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+        verts += __shfl_xor_sync(0xffffffffu, verts, o);
 #pragma unroll
         for (int b = 0; b < 4; ++b) bad[b] += __shfl_xor_sync(0xffffffffu, bad[b], o);
     }
@@ -362,12 +371,13 @@ __global__ void region_stats_kernel(const int32_t *nv, const int8_t *status, lon
         atomicAdd(&s[0], faces);
         atomicMax(&s[1], vmax);
         for (int b = 0; b < 4; ++b) atomicAdd(&s[2 + b], bad[b]);
+        atomicAdd(&s[6], verts);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         atomicAdd(out, (unsigned long long)s[0]);
         atomicMax(out + 1, (unsigned long long)s[1]);
-        for (int b = 0; b < 4; ++b) atomicAdd(out + 2 + b, (unsigned long long)s[2 + b]);
+        for (int b = 0; b < 5; ++b) atomicAdd(out + 2 + b, (unsigned long long)s[2 + b]);
     }
 }
 
@@ -388,10 +398,10 @@ __global__ void rehash_kernel(RegionsDev reg, long long n, HashDev hs, int *err)
 } // namespace
 
 void launch_seed_pack(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, cudaStream_t st,
-                      int *zeroed)
+                      int *zeroed, const SeedPoints &points)
 {
     if (S <= 0) return;
-    seed_pack_kernel<<<(S + 7) / 8, 256, 0, st>>>(states, S, N, W, keys, hash, zeroed);
+    seed_pack_kernel<<<(S + 7) / 8, 256, 0, st>>>(states, S, N, W, keys, hash, zeroed, points);
 }
 
 void launch_seed_insert(const uint32_t *keys, const uint64_t *hash, int S, int W, const HashDev &hs, int32_t *rec,

@@ -93,12 +93,14 @@ struct WaveCtl {
 
 // the control block's device / pinned allocation: WaveCtl, then the run's
 // statistics counters (faces, largest polygon, then one count per status
-// kNoStart .. kSingular, reduced at the end of a run), then the count of
-// faces walked again with FP64 predicates (accumulated during the run)
-constexpr int kStatsCount = 6;
+// kNoStart .. kSingular, then the polygon vertices, reduced at the end of a run),
+// then the count of faces walked again with FP64 predicates (accumulated during
+// the run), then the weld's counts
+constexpr int kStatsCount = 7;
 constexpr int kFp64Slot = kStatsCount;
+constexpr int kWeldSlot = kFp64Slot + 1; // vertices, faces, face indices
 constexpr size_t kStatsOff = (sizeof(WaveCtl) + 15) / 16 * 16;
-constexpr size_t kCtlBytes = kStatsOff + (kStatsCount + 1) * sizeof(unsigned long long);
+constexpr size_t kCtlBytes = kStatsOff + (kStatsCount + 4) * sizeof(unsigned long long);
 
 // A wave of regions.  The constraint rows live in a ring: region id r's rows
 // are at slot r % ring until a later wave takes the slot, so that a region
@@ -160,9 +162,15 @@ void launch_polygon(int prec, const NetDev &net, const RegionsDev &reg, const Ch
                     const Tolerances &tol, int face_warps, unsigned long long *nfp64, int *d_err,
                     cudaStream_t st);
 int polygon_face_warps(int prec, int ALLP);
-// zeroed: an int set to zero as well (optional)
+// zeroed: an int set to zero as well (optional); points: S x 3 seed points of
+// pbytes-byte floats, converted to tbytes-byte ones in dst (optional)
+struct SeedPoints {
+    const void *src = nullptr;
+    void *dst = nullptr;
+    int pbytes = 0, tbytes = 0;
+};
 void launch_seed_pack(const uint8_t *states, int S, int N, int W, uint32_t *keys, uint64_t *hash, cudaStream_t st,
-                      int *zeroed = nullptr);
+                      int *zeroed = nullptr, const SeedPoints &points = SeedPoints());
 void launch_seed_insert(const uint32_t *keys, const uint64_t *hash, int S, int W, const HashDev &hs, int32_t *rec,
                         int *d_err, cudaStream_t st);
 // append of the winners.  mode 0: children of a wave, mode 1: seeds.  cond: the
@@ -187,13 +195,17 @@ void launch_region_stats(const int32_t *nv, const int8_t *status, long long n, u
 // class lists and splits of a wave (ChunkDev); ccount must be zero
 void launch_wave_classes(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, cudaStream_t st);
 int device_sms();
-// the network's parameter buffers, checked for NaN / infinity in one launch
-struct FiniteList {
-    const void *p[64];
-    long long n[64];
+// the network's parameters into the engine's layouts, every value checked for NaN
+// and infinity (kErrNonFinite), in one launch
+struct LoadList {
+    struct Item {
+        const void *src; // device memory
+        void *dst;
+        int M, K, Mp;    // M x K to [K][Mp] (zero padding); Mp = 0: K values as they are
+    } item[64];
     int count;
 };
-void launch_check_finite(int prec, const FiniteList &list, int *d_err, cudaStream_t st);
+void launch_load(int prec, const LoadList &list, int *d_err, cudaStream_t st);
 struct PrepareList { // FP32 linears to transpose and pad
     struct Item {
         const float *src;
@@ -203,7 +215,6 @@ struct PrepareList { // FP32 linears to transpose and pad
     int count;
 };
 void launch_prepare_list(const PrepareList &list, int *nonfinite, cudaStream_t st);
-void launch_prepare_weights(int prec, const void *src, int M, int K, int Mp, void *dst, cudaStream_t st);
 
 // error report (am_verify.cu): out[0] max |f(v)| bits, out[1] max vertex
 // error bits, out[2] vertices, out[3] vertices left out (singular), out[4] faces
