@@ -13,9 +13,9 @@
 // unit's column of W meets an all-zero row of X: skipping it changes no bit of
 // the sums, about half the units are inactive, and each region has its own).
 // The weights stream through shared memory once per tile of up to 16 regions: a
-// copy warp brings [32 units x up to 256 rows] blocks into a four-stage ring
+// copy warp brings [32 units x up to 256 rows] blocks into a ring of stages
 // with bulk copies, and the regions' warps pass through the ring on their own,
-// up to four blocks apart, because their active counts differ (a block barrier
+// up to a ring apart, because their active counts differ (a block barrier
 // per 32 units would cost the slowest of 16 each time).  A warp reads only rows
 // it has written itself (or its parent's), so nothing else is shared.
 //
@@ -33,25 +33,30 @@ namespace am {
 
 namespace {
 
-constexpr int kWarps = 16;              // regions per tile at most
-constexpr int kThreads = 32 * kWarps + 32; // + the copy warp
 constexpr int kKC = 32;                 // operand units per block
-constexpr int kStages = 4;
 constexpr int kWait = 1 << 22;
-constexpr int kStageBytes = 32 * 1024;  // kKC units x pass rows
 constexpr int kPadBytes = 2048;         // lanes beyond a pass's last row read past the block's end
+constexpr int kStagesMax = 4;
 
+// FP32: one CTA of sixteen regions per SM.  FP64: four of four, so that a wave's
+// regions spread more evenly over the SMs and every round of tiles ends sooner
+// (the weights' extra traffic is nothing against the FP64 pipe's time: measured
+// 31.1 against 33.3 ms, and the same in FP32 3.1 against 3.1).
 template <typename T>
-constexpr int pass_rows() { return kStageBytes / (kKC * (int)sizeof(T)); } // 256 fp32, 128 fp64
-
-template <typename T>
-constexpr size_t compose_smem()
-{
-    return (size_t)kStages * kStageBytes + kPadBytes + (size_t)kWarps * kKC * sizeof(vec4_t<T>);
-}
+struct Cfg {
+    static constexpr bool f64 = sizeof(T) == 8;
+    static constexpr int warps = f64 ? 4 : 16;          // regions per tile at most
+    static constexpr int threads = 32 * warps + 32;     // + the copy warp
+    static constexpr int ctas = f64 ? 4 : 1;            // per SM
+    static constexpr int stages = f64 ? 3 : 4;
+    static constexpr int stage_bytes = (f64 ? 16 : 32) * 1024; // kKC units x pass rows
+    static constexpr int rows = stage_bytes / (kKC * (int)sizeof(T)); // per pass: 256 FP32, 64 FP64
+    static constexpr size_t smem =
+        (size_t)stages * stage_bytes + kPadBytes + (size_t)warps * kKC * (sizeof(vec4_t<T>) + sizeof(uint32_t));
+};
 
 struct Ring {
-    uint64_t full[kStages], empty[kStages];
+    uint64_t full[kStagesMax], empty[kStagesMax];
     int abort;
 };
 
@@ -96,26 +101,26 @@ __device__ void produce(const NetDev &net, const WavePlan &plan, int rounds, uns
     const int lane = threadIdx.x & 31;
     volatile int *abort = &ring.abort;
     int h = 0;
-    int last[kStages]; // (lane 0's view, the same in every lane) the last block copied into each stage
-    for (int s = 0; s < kStages; ++s) last[s] = -1;
+    int last[Cfg<T>::stages]; // (lane 0's view, the same in every lane) the last block copied into each stage
+    for (int s = 0; s < Cfg<T>::stages; ++s) last[s] = -1;
     for (int rd = 0; rd < rounds; ++rd) {
         const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
         if (t < 0) continue;
         for (int i = plan_class(plan, t); i < net.n_lin; ++i)
-            for (int mb = 0; mb < net.nodes[i + 1]; mb += pass_rows<T>())
+            for (int mb = 0; mb < net.nodes[i + 1]; mb += Cfg<T>::rows)
                 for (int job = 0, nj = jobs_of(net, i); job < nj; ++job) {
                     const Job jb = job_of(net, i, job);
-                    const int K = net.nodes[jb.src], ld = min(pass_rows<T>(), jb.Mp - mb);
+                    const int K = net.nodes[jb.src], ld = min(Cfg<T>::rows, jb.Mp - mb);
                     for (int k0 = 0; k0 < K; k0 += kKC, ++h) {
-                        const int s = h % kStages;
+                        const int s = h % Cfg<T>::stages;
                         int go = 1;
                         if (lane == 0)
-                            go = h < kStages || ring_wait(ring.empty + s, (uint32_t)(h / kStages - 1) & 1u, err, abort);
+                            go = h < Cfg<T>::stages || ring_wait(ring.empty + s, (uint32_t)(h / Cfg<T>::stages - 1) & 1u, err, abort);
                         if (!__shfl_sync(0xffffffffu, go, 0)) continue;
                         const int kc = min(kKC, K - k0);
                         const uint32_t row = (uint32_t)(ld * sizeof(T));
                         const T *src = (const T *)jb.wt + (size_t)k0 * jb.Mp + mb;
-                        unsigned char *dst = ws + (size_t)s * kStageBytes;
+                        unsigned char *dst = ws + (size_t)s * Cfg<T>::stage_bytes;
                         if (lane == 0) umma::mbar_expect_tx(ring.full + s, row * (uint32_t)kc);
                         __syncwarp();
                         if (ld == jb.Mp) { // whole rows of W^T: one contiguous run
@@ -124,7 +129,7 @@ __device__ void produce(const NetDev &net, const WavePlan &plan, int rounds, uns
                             umma::bulk_g2s(dst + (size_t)lane * row, src + (size_t)lane * jb.Mp, row, ring.full + s);
                         }
 #pragma unroll
-                        for (int q = 0; q < kStages; ++q)
+                        for (int q = 0; q < Cfg<T>::stages; ++q)
                             if (q == s) last[q] = h;
                     }
                 }
@@ -132,8 +137,8 @@ __device__ void produce(const NetDev &net, const WavePlan &plan, int rounds, uns
     // nothing lands in shared memory after the CTA has left (bounded)
     if (lane == 0)
 #pragma unroll
-        for (int s = 0; s < kStages; ++s)
-            if (last[s] >= 0) umma::mbar_wait(ring.full + s, (uint32_t)(last[s] / kStages) & 1u, kWait);
+        for (int s = 0; s < Cfg<T>::stages; ++s)
+            if (last[s] >= 0) umma::mbar_wait(ring.full + s, (uint32_t)(last[s] / Cfg<T>::stages) & 1u, kWait);
     __syncwarp();
 }
 
@@ -145,19 +150,55 @@ struct Region {
     int4 ri;
     int jend, lane;
     const uint32_t *key;
-    vec4_t<T> *xs; // the warp's operand block
+    vec4_t<T> *xs;  // the warp's packed operand block: rows ...
+    uint32_t *offs; // ... and where their units' weights are in the ring
     bool dense;
 };
 
-// one pass (32 RPL units of linear i from mb on) over every job's blocks
+// the products of the packed units i .. i + U - 1, in order
+template <typename T, int RPL, int U>
+__device__ __forceinline__ void units(const Region<T> &g, const unsigned char *w, int i, T acc[RPL][4])
+{
+    vec4_t<T> x[U];
+    T wu[U][RPL];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        x[u] = g.xs[i + u];
+        const T *p = reinterpret_cast<const T *>(w + g.offs[i + u]);
+#pragma unroll
+        for (int j = 0; j < RPL; ++j) wu[u][j] = p[32 * j];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < RPL; ++j) {
+            acc[j][0] = fma_t(wu[u][j], x[u].x, acc[j][0]);
+            acc[j][1] = fma_t(wu[u][j], x[u].y, acc[j][1]);
+            acc[j][2] = fma_t(wu[u][j], x[u].z, acc[j][2]);
+            acc[j][3] = fma_t(wu[u][j], x[u].w, acc[j][3]);
+        }
+}
+
+// the same for a linear of one unit (the output): lane c of four takes column c,
+// a quarter of the multiply-adds of a lane per unit (the FP64 pipe issues an
+// instruction at the same cost however few lanes are active)
+template <typename T>
+__device__ __forceinline__ void unit_face(const Region<T> &g, const unsigned char *w0, int i, T &acc)
+{
+    const T x = reinterpret_cast<const T *>(g.xs + i)[g.lane & 3];
+    acc = fma_t(*reinterpret_cast<const T *>(w0 + g.offs[i]), x, acc);
+}
+
+// one pass (32 RPL units of linear i from mb on; RPL 0: its only unit, in acc's
+// first element by column) over every job's blocks
 template <typename T, int RPL>
 __device__ void pass(const NetDev &net, int i, int mb, const Region<T> &g, const unsigned char *ws, Ring &ring, int &h,
-                     int *err, T acc[RPL][4])
+                     int *err, T (*acc)[4])
 {
     volatile int *abort = &ring.abort;
     for (int job = 0, nj = jobs_of(net, i); job < nj; ++job) {
         const Job jb = job_of(net, i, job);
-        const int K = net.nodes[jb.src], rows0 = net.hoff[jb.src], ld = min(pass_rows<T>(), jb.Mp - mb);
+        const int K = net.nodes[jb.src], rows0 = net.hoff[jb.src], ld = min(Cfg<T>::rows, jb.Mp - mb);
         const T *src = g.cons + (size_t)(uint32_t)(rows0 < g.jend ? g.ri.y : g.ri.x) * g.rstride + (size_t)rows0 * 4;
         auto load = [&](int k0, bool &on) {
             const int k = k0 + g.lane;
@@ -176,56 +217,33 @@ __device__ void pass(const NetDev &net, int i, int mb, const Region<T> &g, const
             x.y = sg * c.y;
             x.z = sg * c.z;
             x.w = sg * c.w;
-            unsigned mask = __ballot_sync(0xffffffffu, on);
-            if (g.dense) {
-                mask = K - k0 >= 32 ? 0xffffffffu : (1u << (K - k0)) - 1u;
-                if (!on) x.x = x.y = x.z = x.w = T(0);
+            // the block's active units, packed in order: the operand row and the
+            // offset of the unit's weights in the ring
+            const int s = h % Cfg<T>::stages;
+            const uint32_t off = (uint32_t)(s * Cfg<T>::stage_bytes + g.lane * ld * (int)sizeof(T));
+            const bool take = g.dense ? k0 + g.lane < K : on;
+            const unsigned mask = __ballot_sync(0xffffffffu, take);
+            const int n = __popc(mask), at = __popc(mask & ((1u << g.lane) - 1u));
+            if (!on) x.x = x.y = x.z = x.w = T(0);
+            if (take) {
+                g.xs[at] = x;
+                g.offs[at] = off;
             }
-            g.xs[g.lane] = x;
             __syncwarp();
             if (k0 + kKC < K) c = load(k0 + kKC, on);
-            const int s = h % kStages;
             // (the warp decides as one: after an abort nobody reads the ring)
-            const bool ok = __all_sync(0xffffffffu, ring_wait(ring.full + s, (uint32_t)(h / kStages) & 1u, err, abort));
+            const bool ok = __all_sync(0xffffffffu, ring_wait(ring.full + s, (uint32_t)(h / Cfg<T>::stages) & 1u, err, abort));
             if (ok) {
-                const T *w = reinterpret_cast<const T *>(ws + (size_t)s * kStageBytes) + g.lane;
-                while (mask) { // two active units at a time, in order
-                    const int ka = __ffs(mask) - 1;
-                    mask &= mask - 1u;
-                    const int kb = mask ? __ffs(mask) - 1 : -1;
-                    const vec4_t<T> xa = g.xs[ka];
-                    T wa[RPL];
-#pragma unroll
-                    for (int j = 0; j < RPL; ++j) wa[j] = w[ka * ld + 32 * j];
-                    if (kb >= 0) {
-                        mask &= mask - 1u;
-                        const vec4_t<T> xb = g.xs[kb];
-                        T wb[RPL];
-#pragma unroll
-                        for (int j = 0; j < RPL; ++j) wb[j] = w[kb * ld + 32 * j];
-#pragma unroll
-                        for (int j = 0; j < RPL; ++j) {
-                            acc[j][0] = fma_t(wa[j], xa.x, acc[j][0]);
-                            acc[j][1] = fma_t(wa[j], xa.y, acc[j][1]);
-                            acc[j][2] = fma_t(wa[j], xa.z, acc[j][2]);
-                            acc[j][3] = fma_t(wa[j], xa.w, acc[j][3]);
-                        }
-#pragma unroll
-                        for (int j = 0; j < RPL; ++j) {
-                            acc[j][0] = fma_t(wb[j], xb.x, acc[j][0]);
-                            acc[j][1] = fma_t(wb[j], xb.y, acc[j][1]);
-                            acc[j][2] = fma_t(wb[j], xb.z, acc[j][2]);
-                            acc[j][3] = fma_t(wb[j], xb.w, acc[j][3]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < RPL; ++j) {
-                            acc[j][0] = fma_t(wa[j], xa.x, acc[j][0]);
-                            acc[j][1] = fma_t(wa[j], xa.y, acc[j][1]);
-                            acc[j][2] = fma_t(wa[j], xa.z, acc[j][2]);
-                            acc[j][3] = fma_t(wa[j], xa.w, acc[j][3]);
-                        }
-                    }
+                const unsigned char *w = ws + g.lane * sizeof(T);
+                // U units' loads in flight (the FP64 pipe is slow enough for one)
+                constexpr int U = sizeof(T) == 8 ? 1 : (RPL > 4 ? 2 : 4);
+                int i = 0;
+                if constexpr (RPL == 0) {
+#pragma unroll 4
+                    for (; i < n; ++i) unit_face<T>(g, ws, i, acc[0][0]);
+                } else {
+                    for (; i + U <= n; i += U) units<T, RPL, U>(g, w, i, acc);
+                    for (; U > 1 && i < n; ++i) units<T, RPL, 1>(g, w, i, acc);
                 }
             }
             __syncwarp();
@@ -280,6 +298,19 @@ __device__ __forceinline__ void store_unit(const NetDev &net, int i, int m, cons
     }
 }
 
+template <typename T>
+__device__ void face_pass(const NetDev &net, int i, const Region<T> &g, const unsigned char *ws, Ring &ring, int &h, int *err,
+                          T iso, T *eq)
+{
+    T acc[1][4];
+    acc[0][0] = T(0);
+    pass<T, 0>(net, i, 0, g, ws, ring, h, err, acc);
+    T v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] = __shfl_sync(0xffffffffu, acc[0][0], c);
+    if (g.lane == 0) store_unit<T>(net, i, 0, g, v, iso, eq);
+}
+
 template <typename T, int RPL>
 __device__ void linear_pass(const NetDev &net, int i, int mb, const Region<T> &g, const unsigned char *ws, Ring &ring,
                             int &h, int *err, T iso, T *eq)
@@ -303,7 +334,7 @@ __device__ void linear_pass(const NetDev &net, int i, int mb, const Region<T> &g
 // barriers per 32 units, took 6.6 and 71 ms.  8,192 given states, every layer
 // (weights transposed and keys packed in the same call): 131 us against 238.
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 1) compose_kernel(NetDev net, RegionsDev reg, ChunkDev ch, T iso,
+__global__ void __launch_bounds__(Cfg<T>::threads, Cfg<T>::ctas) compose_kernel(NetDev net, RegionsDev reg, ChunkDev ch, T iso,
                                                               const int *nonfinite, int *err)
 {
     extern __shared__ __align__(128) unsigned char ws[]; // the weight ring, then the warps' operand blocks
@@ -317,19 +348,19 @@ __global__ void __launch_bounds__(kThreads, 1) compose_kernel(NetDev net, Region
     if (tid == 0) {
         // as few regions per tile as fill the grid: a small wave spreads over every SM
         plan_counts(plan, ch, net.n_lin - 1, count);
-        int R = min(kWarps, (count + (int)gridDim.x - 1) / (int)gridDim.x);
-        while (R < kWarps && plan_tiles(plan, R) > (int)gridDim.x) ++R;
+        int R = min(Cfg<T>::warps, (count + (int)gridDim.x - 1) / (int)gridDim.x);
+        while (R < Cfg<T>::warps && plan_tiles(plan, R) > (int)gridDim.x) ++R;
         plan_finish(plan, R);
         ring.abort = 0;
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < Cfg<T>::stages; ++s) {
             umma::mbar_init(ring.full + s, 1);
-            umma::mbar_init(ring.empty + s, kWarps);
+            umma::mbar_init(ring.empty + s, Cfg<T>::warps);
         }
         umma::fence_mbar_init();
     }
     __syncthreads();
     const int rounds = plan_rounds(plan, (int)gridDim.x);
-    if (warp == kWarps) {
+    if (warp == Cfg<T>::warps) {
         produce<T>(net, plan, rounds, ws, ring, err);
         return;
     }
@@ -337,7 +368,11 @@ __global__ void __launch_bounds__(kThreads, 1) compose_kernel(NetDev net, Region
     g.cons = (T *)ch.cons;
     g.rstride = (size_t)net.ALLP * 4;
     g.lane = lane;
-    g.xs = reinterpret_cast<vec4_t<T> *>(ws + (size_t)kStages * kStageBytes + kPadBytes) + warp * kKC;
+    {
+        unsigned char *pack = ws + (size_t)Cfg<T>::stages * Cfg<T>::stage_bytes + kPadBytes;
+        g.xs = reinterpret_cast<vec4_t<T> *>(pack) + warp * kKC;
+        g.offs = reinterpret_cast<uint32_t *>(pack + (size_t)Cfg<T>::warps * kKC * sizeof(vec4_t<T>)) + warp * kKC;
+    }
     // a weight that is not finite meets the zeros of inactive units too (NaN,
     // as in a dense product): then no unit is skipped
     g.dense = nonfinite && *nonfinite != 0;
@@ -349,11 +384,11 @@ __global__ void __launch_bounds__(kThreads, 1) compose_kernel(NetDev net, Region
         const bool live = warp < tile_nreg(plan, t, cls);
         if (!live) { // no region for this warp: it gives its share of every block back
             for (int i = cls; i < net.n_lin; ++i)
-                for (int mb = 0; mb < net.nodes[i + 1]; mb += pass_rows<T>())
+                for (int mb = 0; mb < net.nodes[i + 1]; mb += Cfg<T>::rows)
                     for (int job = 0, nj = jobs_of(net, i); job < nj; ++job)
                         for (int k0 = 0, K = net.nodes[job_of(net, i, job).src]; k0 < K; k0 += kKC, ++h) {
-                            const int s = h % kStages;
-                            __all_sync(0xffffffffu, ring_wait(ring.full + s, (uint32_t)(h / kStages) & 1u, err, &ring.abort));
+                            const int s = h % Cfg<T>::stages;
+                            __all_sync(0xffffffffu, ring_wait(ring.full + s, (uint32_t)(h / Cfg<T>::stages) & 1u, err, &ring.abort));
                             if (lane == 0) umma::mbar_arrive(ring.empty + s);
                         }
             continue;
@@ -389,14 +424,17 @@ __global__ void __launch_bounds__(kThreads, 1) compose_kernel(NetDev net, Region
         }
         __syncwarp(); // the rows written above are other lanes' operand
         for (int i = cls; i < net.n_lin; ++i) {
-            for (int mb = 0; mb < net.nodes[i + 1]; mb += pass_rows<T>()) {
-                const int n = (min(pass_rows<T>(), net.nodes[i + 1] - mb) + 31) / 32;
-                if (n <= 1) linear_pass<T, 1>(net, i, mb, g, ws, ring, h, err, iso, eq);
-                else if (n <= 2) linear_pass<T, 2>(net, i, mb, g, ws, ring, h, err, iso, eq);
-                else if (n <= 3) linear_pass<T, 3>(net, i, mb, g, ws, ring, h, err, iso, eq);
-                else if (n <= 4 || sizeof(T) == 8) linear_pass<T, 4>(net, i, mb, g, ws, ring, h, err, iso, eq);
-                else if (n <= 6) linear_pass<T, sizeof(T) == 4 ? 6 : 4>(net, i, mb, g, ws, ring, h, err, iso, eq);
-                else linear_pass<T, sizeof(T) == 4 ? 8 : 4>(net, i, mb, g, ws, ring, h, err, iso, eq);
+            for (int mb = 0; mb < net.nodes[i + 1]; mb += Cfg<T>::rows) {
+                const int n = (min(Cfg<T>::rows, net.nodes[i + 1] - mb) + 31) / 32;
+                if (i == net.n_lin - 1) face_pass<T>(net, i, g, ws, ring, h, err, iso, eq); // (one unit)
+                else if (n <= 1) linear_pass<T, 1>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                else if (n <= 2 || Cfg<T>::f64) linear_pass<T, 2>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                else if constexpr (!Cfg<T>::f64) {
+                    if (n <= 3) linear_pass<T, 3>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                    else if (n <= 4) linear_pass<T, 4>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                    else if (n <= 6) linear_pass<T, 6>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                    else linear_pass<T, 8>(net, i, mb, g, ws, ring, h, err, iso, eq);
+                }
             }
             __syncwarp(); // layer i + 1's rows become the next operand
         }
@@ -460,9 +498,10 @@ template <typename T>
 static void launch_one(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, T iso, const int *nonfinite,
                        int *d_err, cudaStream_t st)
 {
-    cudaFuncSetAttribute(compose_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)compose_smem<T>());
-    const int grid = ch.ctl ? device_sms() : std::min(device_sms(), ch.count);
-    compose_kernel<T><<<grid, kThreads, compose_smem<T>(), st>>>(net, reg, ch, iso, nonfinite, d_err);
+    cudaFuncSetAttribute(compose_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<T>::smem);
+    const int slots = device_sms() * Cfg<T>::ctas;
+    const int grid = ch.ctl ? slots : std::min(slots, ch.count);
+    compose_kernel<T><<<grid, Cfg<T>::threads, Cfg<T>::smem, st>>>(net, reg, ch, iso, nonfinite, d_err);
 }
 
 void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso, int *d_err,
