@@ -180,6 +180,37 @@ struct Items {
     }
 };
 
+// the connections of linear i that are no product (identities, the input) added
+// to unit m of a region
+__device__ __forceinline__ void add_skips(const NetDev &net, int i, int m, const float *cons, size_t rstride, const int4 &ri,
+                                          int jend, const uint32_t *key, float (&o)[4])
+{
+    for (int s = 0; s < net.nskip[i]; ++s) {
+        const SkipDev &sk = net.skip[i][s];
+        if (sk.kind == 0) {
+            if (sk.from == 0) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    if (m == c) o[c] += 1.f;
+            } else {
+                const int srow = net.hoff[sk.from] + m;
+                if (key_bit(key, srow)) {
+                    const float4 c = tile_row<float>(cons, rstride, ri, srow, jend);
+                    o[0] -= c.x;
+                    o[1] -= c.y;
+                    o[2] -= c.z;
+                    o[3] -= c.w;
+                }
+            }
+        } else if (sk.from == 0) {
+            const float *tt = (const float *)sk.tmt;
+            o[0] += tt[m];
+            o[1] += tt[(size_t)sk.Mp + m];
+            o[2] += tt[2 * (size_t)sk.Mp + m];
+        }
+    }
+}
+
 // X[n = 4r + c][k] = s_k(r) ? -C[r][src + k][c] : 0 for k < K, 0 up to Kp
 __device__ void stage_x_from_rows(const XOp &X, const float *cons, size_t rstride, const int4 *ri, int jend,
                                   const uint32_t *keys, int W, int nreg, int src, int K, int Kp)
@@ -188,22 +219,36 @@ __device__ void stage_x_from_rows(const XOp &X, const float *cons, size_t rstrid
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool par = src < jend;
     const int per = X.ncols / 2; // items per block
-    for (int q = warp; q < per * (Kp / 64); q += kThreads / 32) {
-        int r, k;
-        items.at(q % per, lane, r, k);
-        k += q / per * 64;
-        float x[4] = {0.f, 0.f, 0.f, 0.f};
-        const int row = src + k;
-        if (r < nreg && k < K && key_bit(keys + (size_t)r * W, row)) {
+    const int n = per * (Kp / 64);
+    constexpr int kU = 4, kWarpsM = kThreads / 32;
+    // four items' loads before the first is used (measured on GB300: one by one
+    // the rows of 32 regions x 128 units took 15 K cycles, most of a tile's time)
+    for (int q0 = warp; q0 < n; q0 += kU * kWarpsM) {
+        float4 v[kU];
+        float sg[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int q = q0 + u * kWarpsM;
+            int r, k;
+            items.at(q % per, lane, r, k);
+            k += q / per * 64;
+            const int row = src + k;
             const int4 g = ri[r];
-            const float4 c = ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)row * 4);
-            const float sg = row == g.z ? 1.f : -1.f;
-            x[0] = sg * c.x;
-            x[1] = sg * c.y;
-            x[2] = sg * c.z;
-            x[3] = sg * c.w;
+            const bool on = q < n && r < nreg && k < K && key_bit(keys + (size_t)r * W, row);
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (on) v[u] = ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)row * 4);
+            sg[u] = row == g.z ? 1.f : -1.f;
         }
-        X.put<2>(4 * r, k, x);
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int q = q0 + u * kWarpsM;
+            if (q >= n) break;
+            int r, k;
+            items.at(q % per, lane, r, k);
+            k += q / per * 64;
+            const float x[4] = {sg[u] * v[u].x, sg[u] * v[u].y, sg[u] * v[u].z, sg[u] * v[u].w};
+            X.put<2>(4 * r, k, x);
+        }
     }
 }
 
@@ -579,6 +624,13 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                 if (mt + 1 < mtiles) bnext = m + 128 < M ? bias[m + 128] : 0.f;
                 const int row = net.hoff[i + 1] + m;
                 for (int cb = cgrp; cb < ncols / 16; cb += ngrp) {
+                    // the four regions' slots and key words, read ahead of the accumulators
+                    uint32_t slot[4], kw[4];
+                    #pragma unroll
+                    for (int qq = 0; qq < 4; ++qq) {
+                        slot[qq] = (uint32_t)ri[cb * 4 + qq].x;
+                        kw[qq] = m < M ? keys[(cb * 4 + qq) * KW + (row >> 5)] : 0u;
+                    }
                     float v[16], vc[16];
                     umma::tmem_ld16x2(lane_base + (uint32_t)(mt * ncols + cb * 16),
                                       lane_base + (uint32_t)((mtiles + mt) * ncols + cb * 16), v, vc);
@@ -587,44 +639,16 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                     #pragma unroll
                     for (int qq = 0; qq < 4; ++qq) {
                         const int r = cb * 4 + qq;
-                        x[4 * qq] = x[4 * qq + 1] = x[4 * qq + 2] = x[4 * qq + 3] = 0.f;
-                        if (r < nreg) {
-                            const uint32_t *key = keys + (size_t)r * KW;
-                            float *cr = cons + (size_t)(uint32_t)ri[r].x * rstride;
-                            float o[4] = {v[4 * qq] + vc[4 * qq], v[4 * qq + 1] + vc[4 * qq + 1],
-                                          v[4 * qq + 2] + vc[4 * qq + 2], v[4 * qq + 3] + vc[4 * qq + 3] + bm};
-                            for (int s = 0; s < net.nskip[i]; ++s) {
-                                const SkipDev &sk = net.skip[i][s];
-                                if (sk.kind == 0) {
-                                    if (sk.from == 0) {
-                                        if (m < 3) o[m] += 1.f;
-                                    } else {
-                                        const int srow = net.hoff[sk.from] + m;
-                                        if (key_bit(key, srow)) {
-                                            const float4 c = tile_row<float>(cons, rstride, ri[r], srow, jend);
-                                            o[0] -= c.x;
-                                            o[1] -= c.y;
-                                            o[2] -= c.z;
-                                            o[3] -= c.w;
-                                        }
-                                    }
-                                } else if (sk.from == 0) {
-                                    const float *tt = (const float *)sk.tmt;
-                                    o[0] += tt[m];
-                                    o[1] += tt[(size_t)sk.Mp + m];
-                                    o[2] += tt[2 * (size_t)sk.Mp + m];
-                                }
-                            }
-                            const bool act = key_bit(key, row);
-                            const float sg = act ? -1.f : 1.f;
-                            st4<float>(cr + (size_t)row * 4, make_float4(sg * o[0], sg * o[1], sg * o[2], sg * o[3]));
-                            if (act) {
-                                x[4 * qq] = o[0];
-                                x[4 * qq + 1] = o[1];
-                                x[4 * qq + 2] = o[2];
-                                x[4 * qq + 3] = o[3];
-                            }
-                        }
+                        float o[4] = {v[4 * qq] + vc[4 * qq], v[4 * qq + 1] + vc[4 * qq + 1],
+                                      v[4 * qq + 2] + vc[4 * qq + 2], v[4 * qq + 3] + vc[4 * qq + 3] + bm};
+                        if (net.nskip[i] && r < nreg) add_skips(net, i, m, cons, rstride, ri[r], jend, keys + (size_t)r * KW, o);
+                        const bool act = r < nreg && ((kw[qq] >> (row & 31)) & 1u);
+                        const float sg = act ? -1.f : 1.f;
+                        if (r < nreg)
+                            st4<float>(cons + (size_t)slot[qq] * rstride + (size_t)row * 4,
+                                       make_float4(sg * o[0], sg * o[1], sg * o[2], sg * o[3]));
+                        #pragma unroll
+                        for (int c = 0; c < 4; ++c) x[4 * qq + c] = act ? o[c] : 0.f;
                     }
                     X.put<4>(cb * 16, m, x);
                     X.put<4>(cb * 16 + 8, m, x + 8);
@@ -1076,44 +1100,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
             // lanes 32 (w % 4).., column blocks cgrp, cgrp + ngrp, ... of each
             // M tile) and stores their rows.
             const int ncb = ncols / 16;
-            const int ncbw = cgrp < ncb ? (ncb - cgrp + ngrp - 1) / ngrp : 0; // this warp's column blocks
             const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
-            auto store_block = [&](int li, int m, int cb, const float *o) { // 16 columns of unit m
-                if (m >= net.nodes[li + 1]) return;
-                const int row = net.hoff[li + 1] + m;
-#pragma unroll
-                for (int qq = 0; qq < 4; ++qq) {
-                    const int r = cb * 4 + qq;
-                    if (r >= nreg) continue;
-                    const uint32_t *key = keys + (size_t)r * KW;
-                    float *cr = cons + (size_t)(uint32_t)ri[r].x * rstride;
-                    float v4[4] = {o[4 * qq], o[4 * qq + 1], o[4 * qq + 2], o[4 * qq + 3]};
-                    for (int s = 0; s < net.nskip[li]; ++s) {
-                        const SkipDev &sk = net.skip[li][s];
-                        if (sk.kind == 0) {
-                            if (sk.from == 0) {
-                                if (m < 3) v4[m] += 1.f;
-                            } else {
-                                const int srow = net.hoff[sk.from] + m;
-                                if (key_bit(key, srow)) {
-                                    const float4 c = tile_row<float>(cons, rstride, ri[r], srow, jend);
-                                    v4[0] -= c.x;
-                                    v4[1] -= c.y;
-                                    v4[2] -= c.z;
-                                    v4[3] -= c.w;
-                                }
-                            }
-                        } else if (sk.from == 0) {
-                            const float *tt = (const float *)sk.tmt;
-                            v4[0] += tt[m];
-                            v4[1] += tt[(size_t)sk.Mp + m];
-                            v4[2] += tt[2 * (size_t)sk.Mp + m];
-                        }
-                    }
-                    const float sg = key_bit(key, row) ? -1.f : 1.f;
-                    st4<float>(cr + (size_t)row * 4, make_float4(sg * v4[0], sg * v4[1], sg * v4[2], sg * v4[3]));
-                }
-            };
             for (int i = cls; i <= net.n_lin - 2; ++i) {
                 const int M = net.nodes[i + 1];
                 const int mtiles = (M + 127) / 128;
@@ -1178,23 +1165,39 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
                     ++accph;
                     umma::fence_after();
                     // accumulators -> registers: main + correction (+ bias),
-                    // eight columns at a time (registers) -> rows
-                    const int nit = (mt1 - mt0) * ncbw;
-                    for (int it = 0; acc_ok && it < nit; ++it) {
-                        const int mt = mt0 + it / ncbw, cb = cgrp + (it % ncbw) * ngrp;
-                        const int mm = mt * 128 + q4 * 32 + lane;
-                        const float bm = mt == mt0 ? bA : (mt == mt0 + 1 ? bB : (mm < M ? bias[mm] : 0.f));
-                        const uint32_t ta = lane_base + (uint32_t)((mt - mt0) * ncols + cb * 16);
-                        const uint32_t tb = lane_base + (uint32_t)((mper + mt - mt0) * ncols + cb * 16);
-                        float o[16];
+                    // eight columns at a time (registers) -> rows; the four
+                    // regions' slots and key words read ahead of them
+                    for (int mt = mt0; acc_ok && mt < mt1; ++mt) {
+                        const int m = mt * 128 + q4 * 32 + lane, row = net.hoff[i + 1] + m;
+                        const float bm = mt == mt0 ? bA : (mt == mt0 + 1 ? bB : (m < M ? bias[m] : 0.f));
+                        for (int cb = cgrp; cb < ncb; cb += ngrp) {
+                            uint32_t slot[4], kw[4];
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float v[8], vc[8];
-                            umma::tmem_ld8x2(ta + 8 * h, tb + 8 * h, v, vc);
+                            for (int qq = 0; qq < 4; ++qq) {
+                                slot[qq] = (uint32_t)ri[cb * 4 + qq].x;
+                                kw[qq] = m < M ? keys[(cb * 4 + qq) * KW + (row >> 5)] : 0u;
+                            }
+                            const uint32_t ta = lane_base + (uint32_t)((mt - mt0) * ncols + cb * 16);
+                            const uint32_t tb = lane_base + (uint32_t)((mper + mt - mt0) * ncols + cb * 16);
 #pragma unroll
-                            for (int k = 0; k < 8; ++k) o[8 * h + k] = (k & 3) == 3 ? v[k] + vc[k] + bm : v[k] + vc[k];
+                            for (int h = 0; h < 2; ++h) {
+                                float v[8], vc[8];
+                                umma::tmem_ld8x2(ta + 8 * h, tb + 8 * h, v, vc);
+                                if (m >= M) continue;
+#pragma unroll
+                                for (int q2 = 0; q2 < 2; ++q2) {
+                                    const int qq = 2 * h + q2, r = cb * 4 + qq;
+                                    if (r >= nreg) continue;
+                                    float o[4] = {v[4 * q2] + vc[4 * q2], v[4 * q2 + 1] + vc[4 * q2 + 1],
+                                                  v[4 * q2 + 2] + vc[4 * q2 + 2], v[4 * q2 + 3] + vc[4 * q2 + 3] + bm};
+                                    if (net.nskip[i])
+                                        add_skips(net, i, m, cons, rstride, ri[r], jend, keys + (size_t)r * KW, o);
+                                    const float sg = (kw[qq] >> (row & 31)) & 1u ? -1.f : 1.f;
+                                    st4<float>(cons + (size_t)slot[qq] * rstride + (size_t)row * 4,
+                                               make_float4(sg * o[0], sg * o[1], sg * o[2], sg * o[3]));
+                                }
+                            }
                         }
-                        store_block(i, mm, cb, o);
                     }
                     umma::fence_before(); // TMEM read out before the next products overwrite it
                 }
