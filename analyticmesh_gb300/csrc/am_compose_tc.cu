@@ -725,18 +725,30 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
 // ---------------------------------------------------------------- streamed operand
 // Wide layers: three bf16 terms of a resident K x ncols operand leave room for
 // only a few regions per tile, and every tile streams all weight blocks again.
-// Here the operand is not resident.  The epilogue writes the constraint rows
-// only; the next layer's masked operand is rebuilt one 64-deep K block at a
-// time from those rows (just written, still in L2) into a two-stage ring by
-// sixteen builder warps while one issuing thread runs the products on the
-// other stage.  K blocks are the outer loop of the products, so one block of
-// the operand serves every M tile of the layer and the tile is as wide as
-// TMEM allows (two accumulators per M tile in 512 columns).  The operand
-// values, the order of the products into each accumulator and the epilogue
-// and face-plane arithmetic are those of compose_tc_kernel, so both kernels
-// give the same bits.
-constexpr int kSBuild = 512;            // builder threads (16 warps)
-constexpr int kSThreads = kSBuild + 64; // + the issuing warp and the weight-copy warp
+// Here the operand lives in a scratch area of device memory per CTA (in L2 while
+// it is used), as the shared-memory image of its 64-deep K blocks, and is copied
+// one block at a time into a two-stage ring by a copy warp of its own, as the
+// weights are by another.  Sixteen row warps write it: the blocks of the layer
+// the tile starts from out of the parents' rows, once per tile, and every
+// later layer's in the epilogue that computes its rows.  K blocks are the outer
+// loop of the products, so one block of the operand serves every M tile of a
+// pass, and the tile is as wide as TMEM allows (two accumulators per M tile in
+// 512 columns).  A pass's accumulators are in two halves, so that the row warps
+// read out one half while the products go into the other (pass_group).
+// What bounds it (measured on GB300, 3-[512]x8-1 with connections, 32 regions a
+// tile): a pass of eight operand blocks takes 47 K cycles, its products 25 K.  The
+// row warps' stores -- 31 bytes a cycle and SM, whoever issues them -- need 10 K
+// per pass for rows and operand, mostly beside the products; the products wait
+// for the first half's operand (8 K) and accumulators (4 K) around the passes'
+// ends, and lose about 400 cycles per weight block to barriers between blocks.
+// With the row warps rebuilding every block of every pass in shared memory from
+// the rows the composition took 308 ms of a marching, this way 275 ms; with six
+// layers of 256 units 16.5 and 15.4 ms.
+// The operand values, the order of the products into each accumulator and the
+// epilogue and face-plane arithmetic are those of compose_tc_kernel, so both
+// kernels give the same bits.
+constexpr int kSBuild = 512;            // threads of the row warps (16)
+constexpr int kSThreads = kSBuild + 96; // + the issuing warp and the weight- and operand-copy warps
 constexpr int kSFaceSumBytes = kSBuild * 16;
 // CTAs of a cluster work on tiles of the same class in step and share the weight
 // stream: each copies its part of a block into the shared memory of all of them
@@ -767,6 +779,68 @@ __device__ const TcMat &job_mat(const NetDev &net, const TcNet &tc, int i, int j
     return tc.lin[i];
 }
 
+// 64-deep operand blocks of a pass over linear i: those of its product jobs
+__device__ __forceinline__ int pass_blocks(const NetDev &net, const TcNet &tc, int i)
+{
+    int n = 0, src;
+    const int njobs = jobs_of(net, i);
+    for (int job = 0; job < njobs; ++job) n += job_mat(net, tc, i, job, src).Kp / 64;
+    return n;
+}
+
+// The operand image: a term of a 64-deep block is ncols / 8 chunks of eight
+// columns, a chunk 64 rows of 16 bytes.  That is the canonical MN-major layout
+// without swizzle (eight rows of a chunk: 128 contiguous bytes), so a warp whose
+// lanes hold consecutive rows stores 512 contiguous bytes, in the scratch as in
+// shared memory, and any multiple of 16 columns will do.  (Measured on GB300: the
+// products run at the same rate as from a 128-byte swizzle, 64 cycles at 128
+// columns.)
+__host__ __device__ __forceinline__ uint32_t op_term_bytes(int ncols) { return (uint32_t)ncols * 128u; }
+__device__ __forceinline__ void op_put8(uint8_t *blk, uint32_t term, int chunk, int k, const float *x)
+{
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split2(x[2 * i], x[2 * i + 1], h[i], m[i], l[i]);
+    uint8_t *p = blk + chunk * 1024 + k * 16;
+    *reinterpret_cast<uint4 *>(p) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4 *>(p + term) = make_uint4(m[0], m[1], m[2], m[3]);
+    *reinterpret_cast<uint4 *>(p + 2 * term) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// Hidden layers whose operand a tile of class c needs and does not compute: c
+// itself, written first, and then in ascending order the earlier ones that feed a
+// tensor-core connection.
+__device__ __forceinline__ uint32_t parent_operands(const NetDev &net, int cls)
+{
+    uint32_t mask = cls <= net.n_lin - 2 ? 1u << cls : 0u;
+    for (int i = cls; i <= net.n_lin - 2; ++i)
+        for (int s = 0; s < net.nskip[i]; ++s)
+            if (tc_skip(net.skip[i][s]) && net.skip[i][s].from <= cls) mask |= 1u << net.skip[i][s].from;
+    return mask;
+}
+__device__ __forceinline__ int op_blocks(const NetDev &net, int layer) { return (net.nodes[layer] + 63) / 64; }
+// blocks written before layer `layer`'s, of the layers in `mask`
+__device__ __forceinline__ int parent_blocks_before(const NetDev &net, uint32_t mask, int cls, int layer)
+{
+    if (layer == cls) return 0;
+    int n = op_blocks(net, cls);
+    for (int l = 1; l < layer; ++l)
+        if (l != cls && ((mask >> l) & 1u)) n += op_blocks(net, l);
+    return n;
+}
+
+// Operand blocks taken together, from block b of a pass of n blocks: the first
+// two and the last two when the pass has tiles in both halves.  Within such a
+// pair the first half's products come before the second half's, so that the
+// first half's accumulators are complete two products early: their epilogue and
+// the next pass's first operand blocks run under the second half's products, and
+// the second half's epilogue under the next pass's first ones.  Each accumulator
+// receives its products in the order of the blocks either way.
+__device__ __forceinline__ int pass_group(int b, int n, bool two)
+{
+    return two && ((b == 0 && n >= 2) || (b == n - 2 && n >= 4)) ? 2 : 1;
+}
+
 __device__ __forceinline__ void bar_builders() { asm volatile("bar.sync 1, %0;" ::"r"(kSBuild) : "memory"); }
 
 // Bounded wait of the streamed kernel: false at once when the CTA is
@@ -787,8 +861,15 @@ __device__ __forceinline__ bool swait(uint64_t *bar, uint32_t parity, int *err, 
     return false;
 }
 
+// the same decided as one warp
+__device__ __forceinline__ bool wwait(uint64_t *bar, uint32_t parity, int *err, volatile int *abort)
+{
+    return __all_sync(0xffffffffu, swait(bar, parity, err, abort));
+}
+
 // (one thread of its own warp) the weight blocks through the nstage ring, in
-// the order the products consume them -- tile, layer, job, K block, M tile --
+// the order the products consume them -- tile, layer, group of M tiles, operand
+// blocks (pass_group), half of the group, M tile --
 // running ahead of the products by up to nstage blocks: block h goes into
 // stage h % nstage once the products of block h - nstage have completed.
 // Measured on GB300: with the copies issued from the same thread as the
@@ -796,10 +877,10 @@ __device__ __forceinline__ bool swait(uint64_t *bar, uint32_t parity, int *err, 
 // products before its refill (about as long as the 24 products themselves),
 // so the tensor pipe was idle most of the time.
 __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, uint64_t *wfull, uint64_t *wdone,
-                                 const WavePlan &plan, int rounds, int *err, volatile int *abort)
+                                 int half, const WavePlan &plan, int rounds, int *err, volatile int *abort)
 {
     const int nst = tc.nstage;
-    const size_t part = (size_t)umma::cluster_rank() * (kWBlockBytes / kCluster); // this CTA's part of a block
+    const size_t part_off = (size_t)umma::cluster_rank() * (kWBlockBytes / kCluster); // this CTA's part of a block
     int h = 0;
     int ps = 0;        // stage of block h (h % nst) ...
     uint32_t pph = 0u; // ... and (h / nst) & 1, kept incrementally
@@ -809,29 +890,44 @@ __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws
         if (t < 0) continue;
         for (int i = plan_class(plan, t); i <= net.n_lin - 2; ++i) {
             const int mtl = (net.nodes[i + 1] + 127) / 128, mper = (mtl + tc.mgroups - 1) / tc.mgroups;
+            const int nblk = pass_blocks(net, tc, i);
             for (int mt0 = 0; mt0 < mtl; mt0 += mper) {
-            const int njobs = jobs_of(net, i);
-            for (int job = 0; job < njobs; ++job) {
-                int src;
-                const TcMat &m = job_mat(net, tc, i, job, src);
-                const int mtiles = m.Mp / 128, kblocks = m.Kp / 64;
-                for (int kb = 0; kb < kblocks; ++kb)
-                    for (int mt = mt0; mt < min(mtiles, mt0 + mper); ++mt, ++h) {
-                        const int s = ps;
-                        const uint32_t ph = pph; // phase of block h - nst's products
-                        if (++ps == nst) {
-                            ps = 0;
-                            pph ^= 1u;
+                const int mt1 = min(mtl, mt0 + mper), mh = min(mt1, mt0 + half);
+                int job0 = 0, kb0 = 0; // block b
+                for (int b = 0, gs; b < nblk; b += gs) {
+                    gs = pass_group(b, nblk, mh < mt1);
+                    int job = 0, kb = 0;
+                    for (int part = 0; part < 2; ++part) {
+                        job = job0;
+                        kb = kb0;
+                        for (int u = 0; u < gs; ++u) {
+                            int src;
+                            const TcMat &m = job_mat(net, tc, i, job, src);
+                            const int kblocks = m.Kp / 64;
+                            for (int mt = part ? mh : mt0; mt < (part ? mt1 : mh); ++mt, ++h) {
+                                const int s = ps;
+                                const uint32_t ph = pph; // phase of block h - nst's products
+                                if (++ps == nst) {
+                                    ps = 0;
+                                    pph ^= 1u;
+                                }
+                                if (h >= nst && !swait(wdone + s, ph ^ 1u, err, abort)) continue;
+                                if (*abort) continue;
+                                umma::mbar_expect_tx(wfull + s, (uint32_t)kWBlockBytes);
+                                umma::bulk_g2s_mc(ws + (size_t)s * kWBlockBytes + part_off,
+                                                  m.blocks + (size_t)(mt * kblocks + kb) * kWBlockBytes + part_off,
+                                                  (uint32_t)kWBlockBytes / kCluster, wfull + s, kClusterMask);
+                                last[s] = h;
+                            }
+                            if (++kb == kblocks) {
+                                kb = 0;
+                                ++job;
+                            }
                         }
-                        if (h >= nst && !swait(wdone + s, ph ^ 1u, err, abort)) continue;
-                        if (*abort) continue;
-                        umma::mbar_expect_tx(wfull + s, (uint32_t)kWBlockBytes);
-                        umma::bulk_g2s_mc(ws + (size_t)s * kWBlockBytes + part,
-                                          m.blocks + (size_t)(mt * kblocks + kb) * kWBlockBytes + part,
-                                          (uint32_t)kWBlockBytes / kCluster, wfull + s, kClusterMask);
-                        last[s] = h;
                     }
-            }
+                    job0 = job;
+                    kb0 = kb;
+                }
             }
         }
     }
@@ -841,81 +937,282 @@ __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws
         if (last[s] >= 0) umma::mbar_wait(wfull + s, (uint32_t)(last[s] / nst) & 1u, kWaitIters);
 }
 
-// (one thread) the products: operand blocks through the two-stage ring,
-// weight blocks from the producer's ring, six products per K step into the
-// main (hi.hi) and the correction accumulator of each M tile.  The commits
-// that free the operand stages and publish the layer's accumulators are
-// made whatever happens, so that the builders never wait on a partner that
-// gave up.
+// A walk over the CTA's weight blocks in the order the products take them (that
+// of produce_streamed), and what each block needs and completes.
+struct ProductWalk {
+    int rd, i, mt0, mt1, mh, b, gs, part, u, mt; // round, linear, M tiles of the pass [mt0, mh, mt1), group, half, block of it, M tile
+    int mper, mtl, nblk;
+    int pass[2], xb; // passes with a first / second half, and operand blocks, before this one's
+    __device__ __forceinline__ bool first_of_pass() const { return b + u == 0; }
+    __device__ __forceinline__ bool new_operand() const { return part == 0 && mt == mt0; }
+    __device__ __forceinline__ bool new_half() const { return b + u == 0 && mt == (part ? mh : mt0); }
+    __device__ __forceinline__ bool last_of_operand() const { return mt == mt1 - 1; }
+    __device__ __forceinline__ bool last_of_half() const { return b + gs == nblk && u == gs - 1 && (mt == mh - 1 || mt == mt1 - 1); }
+    __device__ __forceinline__ int operand() const { return xb + u; }
+    __device__ __forceinline__ int half_pass() const { return part ? pass[1] : pass[0]; }
+
+    __device__ __forceinline__ void enter_group()
+    {
+        gs = pass_group(b, nblk, mh < mt1);
+        part = u = 0;
+        mt = mt0;
+    }
+    __device__ __forceinline__ void enter_pass()
+    {
+        mt1 = min(mtl, mt0 + mper);
+        mh = min(mt1, mt0 + half_);
+        b = 0;
+        enter_group();
+    }
+    __device__ __forceinline__ void enter_layer(const NetDev &net, const TcNet &tc)
+    {
+        mtl = (net.nodes[i + 1] + 127) / 128;
+        mper = (mtl + tc.mgroups - 1) / tc.mgroups;
+        nblk = pass_blocks(net, tc, i);
+        mt0 = 0;
+        enter_pass();
+    }
+    // the first tile from round rd on that has products
+    __device__ __forceinline__ bool enter_tile(const NetDev &net, const TcNet &tc, const WavePlan &plan, int rounds)
+    {
+        for (; rd < rounds; ++rd) {
+            const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+            if (t < 0) continue;
+            i = plan_class(plan, t);
+            if (i > net.n_lin - 2) continue;
+            enter_layer(net, tc);
+            return true;
+        }
+        return false;
+    }
+    __device__ __forceinline__ bool start(const NetDev &net, const TcNet &tc, const WavePlan &plan, int rounds, int half)
+    {
+        half_ = half;
+        rd = pass[0] = pass[1] = xb = 0;
+        return enter_tile(net, tc, plan, rounds);
+    }
+    __device__ __forceinline__ bool next(const NetDev &net, const TcNet &tc, const WavePlan &plan, int rounds)
+    {
+        if (++mt < (part ? mt1 : mh)) return true;
+        if (++u < gs) {
+            mt = part ? mh : mt0;
+            return true;
+        }
+        if (part == 0 && mh < mt1) {
+            part = 1;
+            u = 0;
+            mt = mh;
+            return true;
+        }
+        xb += gs;
+        b += gs;
+        if (b < nblk) {
+            enter_group();
+            return true;
+        }
+        ++pass[0];
+        pass[1] += mh < mt1;
+        mt0 += mper;
+        if (mt0 < mtl) {
+            enter_pass();
+            return true;
+        }
+        if (++i <= net.n_lin - 2) {
+            enter_layer(net, tc);
+            return true;
+        }
+        ++rd;
+        return enter_tile(net, tc, plan, rounds);
+    }
+
+private:
+    int half_;
+};
+
+// (one warp, one elected lane issuing: the walk's values are the same in every
+// lane, so the descriptors stay in uniform registers) the products: operand and
+// weight blocks from the copy warps' rings, six products per K step into the main
+// (hi.hi) and the correction accumulator of each M tile.  The tensor pipe takes
+// two or three products ahead (measured on GB300: 24 products are issued in 1,495
+// of the 1,766 cycles they take), so a gap of more than about 150 cycles in the
+// issuing stream leaves it idle: the walk's next step and the look at the next
+// block's barriers are made between the K steps, and a block's end costs a commit
+// and a branch (with the bookkeeping and waits between the blocks, the pipe stood
+// for 800 to 900 cycles per block of 1,536).  The commits that free the operand
+// stages and publish the accumulators are made whatever happens, so that the
+// row warps never wait on a partner that gave up.
 __device__ void issue_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, uint64_t *wfull, uint64_t *wdone,
-                               const XOp *XS, uint64_t *xfull, uint64_t *xdone, uint64_t *accdone, uint32_t tmem,
-                               int ncols, const WavePlan &plan, int rounds, int *err, volatile int *abort)
+                               uint8_t *xs0, uint64_t *xfull, uint64_t *xdone, uint64_t *accdone, uint64_t *accfree,
+                               uint32_t tmem, int ncols, int half, const WavePlan &plan, int rounds, int *err,
+                               volatile int *abort)
 {
     const int nst = tc.nstage;
-    int h = 0, xb = 0, consumed = 0;
-    int ws_ = 0;       // stage of weight block h (h % nst) ...
-    uint32_t wph = 0u; // ... and its phase parity ((h / nst) & 1), kept incrementally
+    int consumed = 0;
+    int s = 0;        // stage of weight block h (h % nst) ...
+    uint32_t ph = 0u; // ... and its phase parity ((h / nst) & 1), kept incrementally
     // weight stage q's descriptor = wd0 + q * wstep (start address field)
     const uint64_t wd0 = umma::desc_sw128(umma::smem_addr(ws));
     const uint64_t wstep = (uint64_t)(kWBlockBytes >> 4);
-    // operand descriptors of the two stages; term and K step add constant offsets
-    const uint64_t xd0 = XS[0].desc(0, 0, 0), xd1 = XS[1].desc(0, 0, 0);
-    const uint64_t xu = XS[0].ustep(), xj = XS[0].jstep();
-    const uint32_t idesc = XS[0].idesc();
-    for (int rd = 0; rd < rounds; ++rd) {
-        const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
-        if (t < 0) continue;
-        for (int i = plan_class(plan, t); i <= net.n_lin - 2; ++i) {
-            const int mtl = (net.nodes[i + 1] + 127) / 128, mper = (mtl + tc.mgroups - 1) / tc.mgroups;
-            for (int mt0 = 0; mt0 < mtl; mt0 += mper) { // a group of M tiles, its own accumulators
-            const int njobs = jobs_of(net, i);
-            for (int job = 0; job < njobs; ++job) {
-                int src;
-                const TcMat &m = job_mat(net, tc, i, job, src);
-                const int mtiles = m.Mp / 128, kblocks = m.Kp / 64;
-                for (int kb = 0; kb < kblocks; ++kb) {
-                    const int xs = xb & 1;
-                    const uint64_t xd = xs ? xd1 : xd0;
-                    const bool xok = swait(xfull + xs, (uint32_t)(xb >> 1) & 1u, err, abort); // operand block built
-                    const bool fresh = job == 0 && kb == 0;
-                    for (int mt = mt0; mt < min(mtiles, mt0 + mper); ++mt, ++h) {
-                        const int s = ws_;
-                        const uint32_t ph = wph;
-                        if (++ws_ == nst) {
-                            ws_ = 0;
-                            wph ^= 1u;
-                        }
-                        if (!xok || !swait(wfull + s, ph, err, abort)) continue;
-                        umma::fence_after();
-                        const uint32_t d_main = tmem + (uint32_t)((mt - mt0) * ncols);
-                        const uint32_t d_corr = tmem + (uint32_t)((mper + mt - mt0) * ncols);
-                        const uint64_t ad = wd0 + wstep * (uint64_t)s; // term t at +16 KB, K step j at +32 B
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            issue_step(d_main, d_corr, ad + 2u * j, xd + xj * j, xu, idesc, fresh && j == 0);
-                        umma::commit_mc(umma::smem_addr(wdone + s), kClusterMask); // the producers may refill the stage
-                        consumed = h + 1;
-                    }
-                    umma::commit(umma::smem_addr(xdone + xs)); // the operand stage is free once these complete
-                    ++xb;
-                }
+    // operand descriptors of the two stages; term and K step (16 rows of every chunk) add constant offsets
+    const uint32_t term = op_term_bytes(ncols);
+    const uint64_t xd0 = umma::desc_mn(umma::smem_addr(xs0), 128u, 1024u);
+    const uint64_t xu = term >> 4, xj = 16u;
+    const uint32_t idesc = umma::idesc_bf16_bmn(128, ncols);
+    ProductWalk w;
+    bool more = w.start(net, tc, plan, rounds, half);
+    bool ready = false, ok = true;
+    int last_s = 0;
+    uint32_t last_ph = 0u;
+    while (more) {
+        const int xs = w.operand() & 1;
+        if (w.new_operand()) ok = true;
+        if (!ready) { // in order: the block's waits that apply (seen before, when ready)
+            if (w.new_half() && w.half_pass() > 0) ok = wwait(accfree + w.part, (uint32_t)(w.half_pass() - 1) & 1u, err, abort) && ok;
+            if (w.new_operand()) ok = wwait(xfull + xs, (uint32_t)(w.operand() >> 1) & 1u, err, abort) && ok;
+            ok = wwait(wfull + s, ph, err, abort) && ok;
+        }
+        umma::fence_after();
+        const uint32_t d_main = tmem + (uint32_t)(2 * (w.mt - w.mt0) * ncols), d_corr = d_main + (uint32_t)ncols;
+        const uint64_t ad = wd0 + wstep * (uint64_t)s; // term t at +16 KB, K step j at +32 B
+        const uint64_t xd = xd0 + (uint64_t)xs * (3u * xu);
+        const bool fresh = w.first_of_pass();
+        const bool xlast = w.last_of_operand(), hlast = w.last_of_half();
+        const uint32_t abar = umma::smem_addr(accdone + w.part);
+        const uint32_t xbar = umma::smem_addr(xdone + xs), wbar = umma::smem_addr(wdone + s);
+        const bool go = ok;
+        if (go && umma::elect()) issue_step(d_main, d_corr, ad, xd, xu, idesc, fresh);
+        __syncwarp();
+        if (go) ++consumed;
+        const int s_last = s;
+        const uint32_t ph_last = ph;
+        if (++s == nst) {
+            s = 0;
+            ph ^= 1u;
+        }
+        more = w.next(net, tc, plan, rounds);
+        if (go && umma::elect()) issue_step(d_main, d_corr, ad + 2u, xd + xj, xu, idesc, false);
+        __syncwarp();
+        ready = go && more && umma::mbar_test(wfull + s, ph);
+        if (ready && w.new_operand()) ready = umma::mbar_test(xfull + (w.operand() & 1), (uint32_t)(w.operand() >> 1) & 1u);
+        if (ready && w.new_half() && w.half_pass() > 0) ready = umma::mbar_test(accfree + w.part, (uint32_t)(w.half_pass() - 1) & 1u);
+        ready = __all_sync(0xffffffffu, ready);
+        if (go && umma::elect()) issue_step(d_main, d_corr, ad + 4u, xd + 2u * xj, xu, idesc, false);
+        __syncwarp();
+        if (umma::elect()) {
+            if (go) {
+                issue_step(d_main, d_corr, ad + 6u, xd + 3u * xj, xu, idesc, false);
+                umma::commit_mc(wbar, kClusterMask); // the producers may refill the stage
             }
-            umma::commit(umma::smem_addr(accdone)); // the group's accumulators are complete
-            }
+            if (xlast) umma::commit(xbar); // the operand stage is free once these complete
+            if (hlast) umma::commit(abar); // the half's accumulators are complete
+        }
+        __syncwarp();
+        if (go) {
+            last_s = s_last;
+            last_ph = ph_last;
         }
     }
     // the last products have completed before TMEM is released
-    if (consumed > 0 &&
-        !umma::mbar_wait(wdone + (consumed - 1) % nst, (uint32_t)((consumed - 1) / nst) & 1u, kWaitIters))
-        atomicOr(err, kErrWait);
+    if (consumed > 0 && !umma::mbar_wait(wdone + last_s, last_ph, kWaitIters)) atomicOr(err, kErrWait);
+}
+
+// Progress of the row warps, for the operand copy, a count per warp: [0] operand
+// blocks written from the parents' rows, [1], [2] passes whose first / second half
+// has been read out and written.  (Counts and not barrier phases: the copy may
+// look at one long after the next has been raised.)
+struct Progress {
+    uint32_t n[3][kSBuild / 32];
+};
+__device__ __forceinline__ void progress_set(uint32_t *c, uint32_t v)
+{
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(umma::smem_addr(c)), "r"(v) : "memory");
+}
+// (one warp) every row warp has reached `target`
+__device__ __forceinline__ bool progress_wait(const uint32_t *c, uint32_t target, int *err, volatile int *abort)
+{
+    const uint32_t mine = umma::smem_addr(c + (threadIdx.x & (kSBuild / 32 - 1)));
+    for (int it = 0; it < kWaitIters; ++it) {
+        uint32_t v;
+        asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(mine) : "memory");
+        if (__all_sync(0xffffffffu, (int32_t)(v - target) >= 0)) return true;
+        if (__any_sync(0xffffffffu, *abort != 0)) return false;
+        __nanosleep(32);
+    }
+    if ((threadIdx.x & 31) == 0) atomicOr(err, kErrWait);
+    *abort = 1;
+    return false;
+}
+
+// (a warp of its own, one lane copying) the operand blocks through the two-stage ring, in
+// the order the products consume them, each once the row warps have written it
+// and the stage is free.  Rows written by other threads are read here by the
+// copy engine: every writer fences (generic to async proxy) before its warp counts.
+__device__ void copy_operand(const NetDev &net, const TcNet &tc, uint8_t *xs0, uint64_t *xfull, uint64_t *xdone,
+                             const Progress &prog, const uint8_t *xg, int ncols, int half, const WavePlan &plan,
+                             int rounds, int *err, volatile int *abort)
+{
+    const uint32_t bytes = 3u * op_term_bytes(ncols);
+    const bool lead = (threadIdx.x & 31) == 0;
+    int xb = 0;
+    uint32_t pass = 0, conv = 0;
+    int last0 = -1, last1 = -1; // the last block copied into each stage
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int t = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
+        if (t < 0) continue;
+        const int cls = plan_class(plan, t);
+        const uint32_t mask = parent_operands(net, cls);
+        uint32_t prev_pass = 0;
+        int prev_mper = 1;
+        for (int i = cls; i <= net.n_lin - 2; ++i) {
+            const int mtl = (net.nodes[i + 1] + 127) / 128, mper = (mtl + tc.mgroups - 1) / tc.mgroups;
+            const uint32_t layer_pass = pass;
+            const int njobs = jobs_of(net, i);
+            for (int mt0 = 0; mt0 < mtl; mt0 += mper, ++pass)
+                for (int job = 0; job < njobs; ++job) {
+                    int src;
+                    const int nkb = job_mat(net, tc, i, job, src).Kp / 64;
+                    const uint32_t before = src <= cls ? conv + (uint32_t)parent_blocks_before(net, mask, cls, src) : 0u;
+                    for (int kb = 0; kb < nkb; ++kb, ++xb) {
+                        const int xs = xb & 1, fl = xb >> 1;
+                        bool ok = fl < 1 || wwait(xdone + xs, (uint32_t)(fl - 1) & 1u, err, abort);
+                        if (ok && mt0 == 0) {
+                            if (src <= cls) {
+                                ok = progress_wait(prog.n[0], before + (uint32_t)kb + 1u, err, abort);
+                            } else if (job == 0) { // the M tile of linear i - 1 that computes these rows
+                                const int mt = kb / 2, g = mt / prev_mper, part = mt - g * prev_mper >= half ? 1 : 0;
+                                ok = progress_wait(prog.n[1 + part], prev_pass + (uint32_t)g + 1u, err, abort);
+                            } // (a connection's source was complete before the job before it)
+                        }
+                        if (!ok) continue;
+                        if (lead) {
+                            umma::mbar_expect_tx(xfull + xs, bytes);
+                            uint8_t *dst = xs0 + (size_t)xs * bytes;
+                            const uint8_t *from = xg + tc.xoff[src] + (size_t)kb * bytes;
+                            for (uint32_t q = 0; q < bytes; q += bytes / 3) umma::bulk_g2s(dst + q, from + q, bytes / 3, xfull + xs);
+                        }
+                        __syncwarp();
+                        if (xs) last1 = xb;
+                        else last0 = xb;
+                    }
+                }
+            prev_pass = layer_pass;
+            prev_mper = mper;
+        }
+        for (int l = 1; l <= cls; ++l)
+            if ((mask >> l) & 1u) conv += (uint32_t)op_blocks(net, l);
+    }
+    // nothing lands in shared memory after the CTA has left (bounded)
+    if (last0 >= 0) umma::mbar_wait(xfull, (uint32_t)(last0 >> 1) & 1u, kWaitIters);
+    if (last1 >= 0) umma::mbar_wait(xfull + 1, (uint32_t)(last1 >> 1) & 1u, kWaitIters);
 }
 
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, TcNet tc, RegionsDev reg, ChunkDev ch,
                                                                     float iso, int slots, int *err)
 {
     extern __shared__ uint8_t smem_raw[];
-    // wfull[3], wdone[3] (weight ring), xfull[2], xdone[2] (operand ring), accdone
-    __shared__ uint64_t bars[11];
+    // wfull[3], wdone[3] (weight ring), xfull[2], xdone[2] (operand ring), accdone[2], accfree[2] (per half)
+    __shared__ uint64_t bars[14];
+    __shared__ Progress prog;
     __shared__ uint32_t tslot;
     __shared__ int s_abort; // a wait ran out: nothing more is issued, epilogues are skipped
     __shared__ WavePlan plan;
@@ -935,28 +1232,22 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
     int tmem_cols = 32;
     const int mper_max = (tc.mtiles_max + tc.mgroups - 1) / tc.mgroups;
     while (tmem_cols < 2 * mper_max * ncols) tmem_cols <<= 1;
+    const int half = (mper_max + 1) / 2; // M tiles of a group's first half
     const size_t rstride = (size_t)net.ALLP * 4;
     const int KW = key_stride(net.W); // odd: lanes on consecutive regions read distinct banks
 
     uint8_t *base = smem_raw + ((1024u - (umma::smem_addr(smem_raw) & 1023u)) & 1023u);
-    XOp XS[2];
-    const int natoms = (ncols + 63) / 64;
-    const size_t plane = (size_t)(tc.mn ? natoms * 64 : ncols) * 64 * 2; // one term of one K block
-    for (int x = 0; x < 2; ++x) {
-        XS[x].mn = tc.mn != 0;
-        XS[x].ncols = ncols;
-        XS[x].natoms = natoms;
-        XS[x].xbytes = plane;
-        XS[x].xs = base + (size_t)x * 3 * plane; // hi, mid, lo
-    }
-    uint8_t *ws = base + 6 * plane;
+    const uint32_t term = op_term_bytes(ncols); // one term of one K block of the operand
+    uint8_t *xs0 = base;                        // two stages of hi, mid, lo
+    uint8_t *xg = tc.xbuf + (size_t)blockIdx.x * tc.xcta;
+    uint8_t *ws = base + 6 * (size_t)term;
     uint32_t *keys = reinterpret_cast<uint32_t *>(ws + (size_t)tc.nstage * kWBlockBytes);
     float4 *w0s = reinterpret_cast<float4 *>(keys + (size_t)(tc.ncols_max / 4) * key_stride(net.W));
     float *wls = reinterpret_cast<float *>(w0s + net.nodes[1]);
     // the face plane's partial sums use the operand ring: it is idle then
     // (the tile's products are complete, the next tile's operand not begun)
     float *fsum = reinterpret_cast<float *>(base);
-    uint64_t *wfull = bars, *wdone = bars + 3, *xfull = bars + 6, *xdone = bars + 8, *accdone = bars + 10;
+    uint64_t *wfull = bars, *wdone = bars + 3, *xfull = bars + 6, *xdone = bars + 8, *accdone = bars + 10, *accfree = bars + 12;
 
     volatile int *abort = &s_abort;
     if (tid == 0) {
@@ -965,11 +1256,15 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
             umma::mbar_init(wfull + b, 1);
             umma::mbar_init(wdone + b, kCluster); // every CTA's products are done with the stage
         }
-        umma::mbar_init(xfull, kSBuild / 32); // (one arrival per warp)
-        umma::mbar_init(xfull + 1, kSBuild / 32);
+        umma::mbar_init(xfull, 1);
+        umma::mbar_init(xfull + 1, 1);
         umma::mbar_init(xdone, 1);
         umma::mbar_init(xdone + 1, 1);
         umma::mbar_init(accdone, 1);
+        umma::mbar_init(accdone + 1, 1);
+        umma::mbar_init(accfree, kSBuild / 32); // (one arrival per row warp)
+        umma::mbar_init(accfree + 1, kSBuild / 32);
+        for (int w = 0; w < kSBuild / 32; ++w) prog.n[0][w] = prog.n[1][w] = prog.n[2][w] = 0u;
         umma::fence_mbar_init();
     }
     if (warp == 0) umma::tmem_alloc(&tslot, (uint32_t)tmem_cols);
@@ -989,17 +1284,19 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
     const uint32_t tmem = tslot;
 
     if (warp == kSBuild / 32) {
-        if (lane == 0)
-            issue_streamed(net, tc, ws, wfull, wdone, XS, xfull, xdone, accdone, tmem, ncols, plan, rounds, err,
-                           abort);
+        issue_streamed(net, tc, ws, wfull, wdone, xs0, xfull, xdone, accdone, accfree, tmem, ncols, half, plan,
+                       rounds, err, abort);
         __syncwarp(); // the warp reaches the block barrier below converged
     } else if (warp == kSBuild / 32 + 1) {
-        if (lane == 0) produce_streamed(net, tc, ws, wfull, wdone, plan, rounds, err, abort);
+        if (lane == 0) produce_streamed(net, tc, ws, wfull, wdone, half, plan, rounds, err, abort);
+        __syncwarp();
+    } else if (warp == kSBuild / 32 + 2) {
+        copy_operand(net, tc, xs0, xfull, xdone, prog, xg, ncols, half, plan, rounds, err, abort);
         __syncwarp();
     } else {
-        // epilogue: warp w reads TMEM lanes 32 (w % 4).. and every fourth column block
+        // the row warps: operand blocks from the parents' rows, epilogues, the face plane
         const int q4 = warp & 3, cgrp = warp >> 2, ngrp = kSBuild / 128;
-        int xb = 0, accph = 0;
+        uint32_t pass = 0, pass1 = 0, nconv = 0; // passes read out, those of two halves, operand blocks written from parents' rows
         float *cons = (float *)ch.cons;
         for (int rd = 0; rd < rounds; ++rd) {
             const int tile = plan_tile(plan, rd, (int)blockIdx.x, (int)gridDim.x);
@@ -1010,20 +1307,21 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
             bar_builders(); // the previous tile is done with the keys
             if (tid < nreg) ri[tid] = tile_region(plan, reg, ch, head, tile, cls, tid);
             bar_builders();
-            for (int q = tid; q < R * net.W; q += kSBuild) {
-                const int rr = q / net.W, w = q % net.W;
-                keys[rr * KW + w] = rr < nreg ? reg.keys[(size_t)(head + ri[rr].w) * net.W + w] : 0u;
+            for (int rr = warp; rr < R; rr += kSBuild / 32) { // a region's words together in flight
+                const uint32_t *key = reg.keys + (size_t)(rr < nreg ? head + ri[rr].w : 0) * net.W;
+#pragma unroll 4
+                for (int w = lane; w < net.W; w += 32) keys[rr * KW + w] = rr < nreg ? key[w] : 0u;
             }
             bar_builders();
             // class 1: hidden layer 1 = linear 0 rows (sign-flipped); the extra constraints
             const int n1 = net.nodes[1];
-            for (int q = tid; cls == 1 && q < nreg * n1; q += kSBuild) {
-                const int rr = q / n1, m = q % n1;
-                const float sg = key_bit(keys + (size_t)rr * KW, m) ? -1.f : 1.f;
-                const float4 w = w0s[m];
-                st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)m * 4,
-                           make_float4(sg * w.x, sg * w.y, sg * w.z, sg * w.w));
-            }
+            for (int rr = warp; cls == 1 && rr < nreg; rr += kSBuild / 32)
+                for (int m = lane; m < n1; m += 32) {
+                    const float sg = key_bit(keys + (size_t)rr * KW, m) ? -1.f : 1.f;
+                    const float4 w = w0s[m];
+                    st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)m * 4,
+                               make_float4(sg * w.x, sg * w.y, sg * w.z, sg * w.w));
+                }
             const float *we = (const float *)net.w_extra;
             const float *be = (const float *)net.b_extra;
             for (int q = tid; q < nreg * net.E; q += kSBuild) {
@@ -1033,175 +1331,169 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
             }
             bar_builders(); // layer-1 rows written by every builder
 
-            // X[4r + c][k] = s_k(r) ? -C[r][k][c] : 0, one 64-deep K block at a
-            // time; every pass of a layer streams the same blocks.  Warp w owns
-            // the items w, w + 16, ... of a block (Items).  The first four items
-            // of a block are loaded two steps ahead of their use, and nothing
-            // in the load depends on shared memory but the key words of its 64
-            // rows: the products keep the shared memory's bandwidth busy, and a
-            // dependent shared load costs hundreds of cycles then (measured: an
-            // LDS of the region's slots and of the key word per item made a
-            // block's loads take 2,200 cycles, against 1,536 of a weight
-            // block's products).  Raw values are kept and signed when stored.
-            // The returned mask marks the items whose sign is the other one
-            // (the plane the region was entered through).
-            const Items items(R);
-            const bool one = items.half == 16; // an item's region is the warp's own pair: the tile of 32 regions
-            const int myr = 2 * warp + (lane & 1);
-            const int4 mine = one && myr < nreg ? ri[myr] : make_int4(0, 0, -1, 0);
-            auto load_items = [&](int li, int job, int kb, int c, float4 *v) {
-                int src;
-                job_mat(net, tc, li, job, src);
-                const int K = net.nodes[src], rows0 = net.hoff[src];
+            // The operand of the layers the parents computed:
+            // X[4r + c][k] = s_k(r) ? -C[r][k][c] : 0, block by block.  A warp
+            // item is two regions x 32 rows, a row per lane: loads and stores of
+            // 512 contiguous bytes.  Two items' rows are loaded before the two
+            // before them are stored.  Raw values are kept and signed when
+            // stored; `other` marks the rows whose sign is the other one (the
+            // plane the region was entered through).
+            const int cpb = ((R + 15) / 16 + 1) / 2; // chunks of two items per warp and block
+            const uint32_t xblk = 3u * term;
+            const uint32_t pmask = parent_operands(net, cls);
+            for (uint32_t left = pmask; left;) {
+                const int layer = (left >> cls) & 1u ? cls : __ffs(left) - 1;
+                left &= ~(1u << layer);
+                const int K = net.nodes[layer], rows0 = net.hoff[layer];
                 const bool par = rows0 < jend;
-                unsigned other = 0u;
-                if (one) {
-                    const int k0 = kb * 64 + (lane >> 1), b0 = rows0 + k0;
-                    const uint32_t *kw = keys + (size_t)myr * KW + (b0 >> 5);
-                    const uint32_t w0 = kw[0], w1 = kw[1], w2 = kw[2]; // (words beyond the key: masked by K)
-                    const uint32_t lo = __funnelshift_r(w0, w1, b0), hi = __funnelshift_r(w1, w2, b0);
-                    const float4 *p = reinterpret_cast<const float4 *>(cons + (size_t)(uint32_t)(par ? mine.y : mine.x) * rstride) + b0;
+                auto load = [&](int kb, int j, float4 *v) {
+                    unsigned other = 0u;
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        const bool on = ((u < 2 ? lo : hi) >> (16 * (u & 1)) & 1u) && k0 + 16 * u < K && myr < nreg;
-                        v[u] = on ? p[16 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (b0 + 16 * u == mine.z) other |= 1u << u;
+                        const int q = warp + 16 * (2 * j + (u >> 1)), r = (q >> 1) * 2 + (u & 1);
+                        const int k = kb * 64 + (q & 1) * 32 + lane;
+                        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (r < nreg && k < K && key_bit(keys + (size_t)r * KW, rows0 + k)) {
+                            const int4 g = ri[r];
+                            if (rows0 + k == g.z) other |= 1u << u;
+                            v[u] = ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)(rows0 + k) * 4);
+                        }
                     }
                     return other;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    int r, kk;
-                    const bool in = items.at(warp + 16 * (4 * c + u), lane, r, kk);
-                    const int k = kb * 64 + kk;
-                    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (in && r < nreg && k < K && key_bit(keys + (size_t)r * KW, rows0 + k)) {
-                        const int4 g = ri[r];
-                        if (rows0 + k == g.z) other |= 1u << u;
-                        x = ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)(rows0 + k) * 4);
+                };
+                const int n = op_blocks(net, layer) * cpb;
+                float4 a[4], b[4];
+                unsigned ao = load(0, 0, a), bo = 0u;
+                int kb = 0, j = 0;
+                for (int c = 0; c < n; ++c) {
+                    const int k0 = kb, j0 = j;
+                    if (++j == cpb) {
+                        j = 0;
+                        ++kb;
                     }
-                    v[u] = x;
-                }
-                return other;
-            };
-            auto put_items = [&](const XOp &X, int c, const float4 *v, unsigned other) {
+                    if (c + 1 < n) bo = load(kb, j, b);
+                    uint8_t *blk = xg + tc.xoff[layer] + (size_t)k0 * xblk;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    int r, kk;
-                    if (items.at(warp + 16 * (4 * c + u), lane, r, kk)) {
-                        const float s1 = (other >> u) & 1u ? 1.f : -1.f;
-                        const float x[4] = {s1 * v[u].x, s1 * v[u].y, s1 * v[u].z, s1 * v[u].w};
-                        X.put<2>(4 * r, kk, x);
+                    for (int u = 0; u < 2; ++u) {
+                        const int q = warp + 16 * (2 * j0 + u);
+                        if (q >= R) continue;
+                        const float s0 = (ao >> (2 * u)) & 1u ? 1.f : -1.f, s1 = (ao >> (2 * u + 1)) & 1u ? 1.f : -1.f;
+                        const float x[8] = {s0 * a[2 * u].x,     s0 * a[2 * u].y,     s0 * a[2 * u].z,     s0 * a[2 * u].w,
+                                            s1 * a[2 * u + 1].x, s1 * a[2 * u + 1].y, s1 * a[2 * u + 1].z, s1 * a[2 * u + 1].w};
+                        op_put8(blk, term, q >> 1, (q & 1) * 32 + lane, x);
                     }
+                    if (j == 0) { // the block's last chunk
+                        ++nconv;
+                        // (the fence waits for the stores: later blocks two together)
+                        if (k0 < 4 || (k0 & 1) == 1 || c + 1 == n) {
+                            umma::fence_proxy_async_all();
+                            __syncwarp();
+                            if (lane == 0) progress_set(&prog.n[0][warp], nconv);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) a[u] = b[u];
+                    ao = bo;
                 }
-            };
-            const int nchunks = (2 * R + 63) / 64;
-            // The epilogue of a pass reads its accumulators (warp w: TMEM
-            // lanes 32 (w % 4).., column blocks cgrp, cgrp + ngrp, ... of each
-            // M tile) and stores their rows.
+            }
+            // The epilogue of a half pass reads its accumulators (warp w: TMEM
+            // lanes 32 (w % 4).., column blocks cgrp, cgrp + ngrp, ... of each M
+            // tile), and stores their rows and the next layer's operand.
             const int ncb = ncols / 16;
             const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
             for (int i = cls; i <= net.n_lin - 2; ++i) {
-                const int M = net.nodes[i + 1];
-                const int mtiles = (M + 127) / 128;
+                const int M = net.nodes[i + 1], mtiles = (M + 127) / 128;
                 const int mper = (mtiles + tc.mgroups - 1) / tc.mgroups;
-                const int njobs = jobs_of(net, i);
-                // the operand blocks of the layer, once per pass: (job, kb) in
-                // order; `a` holds the block built next, `b` the one after it
-                float4 a[4], b[4];
-                unsigned ao, bo = 0u;
-                int lj = 0, lkb = 0, lp = 0; // the block loaded next, and its pass (by its first M tile)
-                auto load_next = [&](float4 *v) {
-                    if (lp >= mtiles) return 0u;
-                    const unsigned o = load_items(i, lj, lkb, 0, v);
-                    int src;
-                    if (++lkb == job_mat(net, tc, i, lj, src).Kp / 64) {
-                        lkb = 0;
-                        if (++lj == njobs) {
-                            lj = 0;
-                            lp += mper;
-                        }
-                    }
-                    return o;
-                };
-                ao = load_next(a);
-                bo = load_next(b);
-                for (int mt0 = 0; mt0 < mtiles; mt0 += mper) { // the products of this group of M tiles
-                    const int mt1 = min(mtiles, mt0 + mper);
-                    for (int job = 0; job < njobs; ++job) {
-                        int src;
-                        const int nkb = job_mat(net, tc, i, job, src).Kp / 64;
-                        for (int kb = 0; kb < nkb; ++kb) {
-                            const int xs = xb & 1, fill = xb >> 1;
-                            // stage free (an aborting CTA builds nothing but still arrives)
-                            const bool ok = fill < 1 ? !*abort : swait(xdone + xs, (uint32_t)((fill - 1) & 1), err, abort);
-                            const XOp &X = XS[xs];
-                            if (ok) {
-                                put_items(X, 0, a, ao);
-                                for (int c = 1; c < nchunks; ++c) {
-                                    float4 t4[4];
-                                    const unsigned other = load_items(i, job, kb, c, t4);
-                                    put_items(X, c, t4, other);
-                                }
-                            }
-                            umma::fence_proxy_async(); // generic-proxy stores -> the tensor cores
-                            __syncwarp();
-                            if (lane == 0) umma::mbar_arrive(xfull + xs);
-                            ++xb;
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) a[u] = b[u];
-                            ao = bo;
-                            bo = load_next(b);
-                        }
-                    }
-                    const float *bias = (const float *)net.bias[i];
-                    const int mA = mt0 * 128 + q4 * 32 + lane, mB = mA + 128;
-                    const float bA = mA < M ? bias[mA] : 0.f;                   // loaded while the products run
-                    const float bB = mt0 + 1 < mt1 && mB < M ? bias[mB] : 0.f;
-                    // the layer's products are in TMEM; the TMEM loads below are
+                const float *bias = (const float *)net.bias[i];
+                uint8_t *xl = i < net.n_lin - 2 ? xg + tc.xoff[i + 1] : nullptr;
+                const int Kx = (M + 63) / 64 * 64; // operand rows, zero beyond M
+                for (int part = 0, mt0 = 0; mt0 < mtiles;) {
+                    const int e1 = min(mtiles, mt0 + mper), eh = min(e1, mt0 + half);
+                    const int ma = part ? eh : mt0, mb = part ? e1 : eh;
+                    const int mA = ma * 128 + q4 * 32 + lane;
+                    const float bA = ma < mb && mA < M ? bias[mA] : 0.f; // loaded while the products run
+                    // the half's products are in TMEM; the TMEM loads below are
                     // warp-collective, so the warp decides as one
-                    bool acc_ok = swait(accdone, (uint32_t)(accph & 1), err, abort);
+                    bool acc_ok = swait(accdone + part, (part ? pass1 : pass) & 1u, err, abort);
                     acc_ok = __all_sync(0xffffffffu, acc_ok) && !__any_sync(0xffffffffu, *abort != 0);
-                    ++accph;
                     umma::fence_after();
-                    // accumulators -> registers: main + correction (+ bias),
-                    // eight columns at a time (registers) -> rows; the four
-                    // regions' slots and key words read ahead of them
-                    for (int mt = mt0; acc_ok && mt < mt1; ++mt) {
-                        const int m = mt * 128 + q4 * 32 + lane, row = net.hoff[i + 1] + m;
-                        const float bm = mt == mt0 ? bA : (mt == mt0 + 1 ? bB : (m < M ? bias[m] : 0.f));
-                        for (int cb = cgrp; cb < ncb; cb += ngrp) {
-                            uint32_t slot[4], kw[4];
+                    // accumulators -> registers: main + correction, sixteen columns
+                    // at a time; once the half's last ones are out, the products
+                    // may overwrite it.  Then + bias and connections -> rows and
+                    // the next operand.
+                    int c = cgrp, mt = ma;
+                    bool have = acc_ok && ma < mb && c < ncb;
+                    if (!have) {
+                        umma::fence_before();
+                        __syncwarp();
+                        if (lane == 0) umma::mbar_arrive(accfree + part);
+                    }
+                    while (have) {
+                        const int c0 = c, m = mt * 128 + q4 * 32 + lane, row = net.hoff[i + 1] + m;
+                        const float bm = mt == ma ? bA : (m < M ? bias[m] : 0.f);
+                        uint8_t *xrow = xl && m < Kx ? xl + (size_t)(m >> 6) * xblk : nullptr;
+                        float *rowp = cons + (size_t)row * 4;
+                        const int lim = m < M ? nreg : 0; // regions with a row here
+                        // the four regions' slots and key bits, read ahead of the accumulators
+                        uint32_t slot[4];
+                        unsigned acts = 0u;
 #pragma unroll
-                            for (int qq = 0; qq < 4; ++qq) {
-                                slot[qq] = (uint32_t)ri[cb * 4 + qq].x;
-                                kw[qq] = m < M ? keys[(cb * 4 + qq) * KW + (row >> 5)] : 0u;
-                            }
-                            const uint32_t ta = lane_base + (uint32_t)((mt - mt0) * ncols + cb * 16);
-                            const uint32_t tb = lane_base + (uint32_t)((mper + mt - mt0) * ncols + cb * 16);
+                        for (int qq = 0; qq < 4; ++qq) {
+                            slot[qq] = (uint32_t)ri[c0 * 4 + qq].x;
+                            if (c0 * 4 + qq < lim && key_bit(keys + (size_t)(c0 * 4 + qq) * KW, row)) acts |= 1u << qq;
+                        }
+                        float sum[4][4];
+                        {
+                            const uint32_t ta = lane_base + (uint32_t)(2 * (mt - mt0) * ncols + c0 * 16);
+                            float vc[16];
+                            umma::tmem_ld16x2(ta, ta + (uint32_t)ncols, &sum[0][0], vc);
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                float v[8], vc[8];
-                                umma::tmem_ld8x2(ta + 8 * h, tb + 8 * h, v, vc);
-                                if (m >= M) continue;
+                            for (int e = 0; e < 16; ++e) sum[e >> 2][e & 3] += vc[e];
+                        }
+                        c += ngrp;
+                        if (c >= ncb) {
+                            c = cgrp;
+                            have = ++mt < mb;
+                        }
+                        if (!have) {
+                            umma::fence_before(); // TMEM read out before the next products overwrite it
+                            __syncwarp();
+                            if (lane == 0) umma::mbar_arrive(accfree + part);
+                        }
 #pragma unroll
-                                for (int q2 = 0; q2 < 2; ++q2) {
-                                    const int qq = 2 * h + q2, r = cb * 4 + qq;
-                                    if (r >= nreg) continue;
-                                    float o[4] = {v[4 * q2] + vc[4 * q2], v[4 * q2 + 1] + vc[4 * q2 + 1],
-                                                  v[4 * q2 + 2] + vc[4 * q2 + 2], v[4 * q2 + 3] + vc[4 * q2 + 3] + bm};
+                        for (int h = 0; h < 2; ++h) {
+                            float x[8];
+#pragma unroll
+                            for (int q2 = 0; q2 < 2; ++q2) {
+                                const int qq = 2 * h + q2, r = c0 * 4 + qq;
+                                float(&o)[4] = sum[qq];
+                                o[3] += bm;
+                                const bool act = (acts >> qq) & 1u;
+                                if (r < lim) {
                                     if (net.nskip[i])
                                         add_skips(net, i, m, cons, rstride, ri[r], jend, keys + (size_t)r * KW, o);
-                                    const float sg = (kw[qq] >> (row & 31)) & 1u ? -1.f : 1.f;
-                                    st4<float>(cons + (size_t)slot[qq] * rstride + (size_t)row * 4,
-                                               make_float4(sg * o[0], sg * o[1], sg * o[2], sg * o[3]));
+                                    const float sg = act ? -1.f : 1.f;
+                                    st4<float>(rowp + (size_t)slot[qq] * rstride, make_float4(sg * o[0], sg * o[1], sg * o[2], sg * o[3]));
                                 }
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) x[4 * q2 + e] = act ? o[e] : 0.f;
                             }
+                            if (xrow) op_put8(xrow, term, c0 * 2 + h, m & 63, x);
                         }
                     }
-                    umma::fence_before(); // TMEM read out before the next products overwrite it
+                    umma::fence_proxy_async_all(); // the operand's rows, for the copy
+                    __syncwarp();
+                    if (lane == 0) progress_set(&prog.n[1 + part][warp], pass + 1u);
+                    if (part == 0 && eh < e1) {
+                        part = 1;
+                    } else {
+                        pass1 += part;
+                        ++pass;
+                        part = 0;
+                        mt0 += mper;
+                    }
                 }
-                bar_builders(); // rows of hidden layer i + 1 written by every builder
+                bar_builders(); // rows of hidden layer i + 1 written by every row warp
             }
 
             // face plane: w_eq = W_L . X_L, X_L = -C of the last hidden layer
@@ -1316,8 +1608,7 @@ int device_sms()
 size_t tc_smem_bytes(const TcNet &tc, int ncols, int W)
 {
     if (tc.streamed) { // two operand stages of one K block each (the face-plane sums reuse them)
-        const size_t cols = tc.mn ? (size_t)(ncols + 63) / 64 * 64 : (size_t)ncols;
-        return 1024 + std::max<size_t>(6 * cols * 64 * 2, (size_t)kSFaceSumBytes) + (size_t)tc.nstage * kWBlockBytes +
+        return 1024 + std::max<size_t>(6 * (size_t)op_term_bytes(ncols), (size_t)kSFaceSumBytes) + (size_t)tc.nstage * kWBlockBytes +
                (size_t)(tc.ncols_max / 4) * key_stride(W) * 4 + 16 * (size_t)tc.n1 + 4 * (size_t)tc.k_last + 16;
     }
     const size_t cols = tc.mn ? (size_t)(ncols + 63) / 64 * 64 : (size_t)ncols;
@@ -1334,7 +1625,7 @@ void launch_compose_tc(const NetDev &net, const TcNet &tc, const RegionsDev &reg
     const int slots = sms; // one resident tile per SM, the wave's tiles strided over them
     if (tc.streamed) {
         cudaFuncSetAttribute(compose_tcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        const int grid = slots / kCluster * kCluster;
+        const int grid = std::min(slots, tc.xctas) / kCluster * kCluster;
         compose_tcs_kernel<<<grid, kSThreads, smem, st>>>(net, tc, reg, ch, (float)iso, grid, d_err);
         return;
     }

@@ -204,6 +204,7 @@ struct am_engine {
     DevBuf v_ids, v_keys, v_rows, v_eq, v_out;
     // tensor-core composition (mixed form): bf16 hi/lo weights
     DevBuf tc_lin[kMaxLayers], tc_skip[kMaxLayers][kMaxSkips];
+    DevBuf tc_x; // the streamed composition's operand (TcNet::xbuf)
     TcNet tcnet{};
     // regions
     DevBuf keys, hash, mid, start, parent, reach, nv, status, verts, edges;
@@ -819,28 +820,25 @@ void run_begin(am_engine *e, const RunArgs &a)
         // With mgroups > 1 a layer's M tiles are multiplied in that many
         // passes, each with its own accumulators, so that the tile can be
         // wider than two accumulators per M tile of the widest layer allow
-        // (the operand is rebuilt once per pass).
+        // (the operand is copied once per pass).
         auto streamed_tile = [&](int mgroups) {
             TcNet ts = tc;
             ts.streamed = 1;
             ts.mgroups = mgroups;
             ts.ncols_max = 0;
             const int mper = (ts.mtiles_max + mgroups - 1) / mgroups;
-            for (int mn = 1; mn >= 0 && ts.ncols_max < 16; --mn) {
-                ts.mn = mn;
-                for (int ncols = std::min(256, 256 / mper) / 16 * 16; ncols >= 16 && ts.ncols_max < 16; ncols -= 16)
-                    for (int ns = 3; ns >= 1; --ns) {
-                        ts.ncols_max = ncols;
-                        ts.nstage = ns;
-                        if (tc_smem_bytes(ts, ncols, e->W) <= smem_cap) break;
-                        ts.ncols_max = 0;
-                    }
-            }
+            for (int ncols = std::min(256, 256 / mper) / 16 * 16; ncols >= 16 && ts.ncols_max < 16; ncols -= 16)
+                for (int ns = 3; ns >= 1; --ns) {
+                    ts.ncols_max = ncols;
+                    ts.nstage = ns;
+                    if (tc_smem_bytes(ts, ncols, e->W) <= smem_cap) break;
+                    ts.ncols_max = 0;
+                }
             return ts;
         };
         TcNet ts = streamed_tile(1);
         if (tc.mtiles_max >= 2 && e->compose_tile != 2) {
-            // two passes pay for rebuilding the operand and a second epilogue
+            // two passes pay for copying the operand twice and a second epilogue
             // per layer: automatically only for twice the tile width with two
             // weight stages or more (measured on GB300: 3-[512]x8-1 faster
             // with 128 columns in two passes than 64 in one, 3-[256]x6-1
@@ -852,6 +850,31 @@ void run_begin(am_engine *e, const RunArgs &a)
                                    (e->compose_tile == 0 && tc.kp_max >= 256 && ts.ncols_max > tc.ncols_max);
         if (ts.ncols_max >= 16 && (want_streamed || tc.ncols_max < 16)) tc = ts;
         AM_CHECK(e->compose_tile != 1 || !tc.streamed, "resident operand tile does not fit");
+        if (tc.streamed) {
+            // the operand's scratch: a layer that feeds a tensor-core connection keeps its own
+            // area, the others alternate between two; fewer CTAs where memory is short
+            uint32_t kept = 0;
+            for (int i = 1; i <= e->n_lin - 2; ++i)
+                for (int s = 0; s < net.nskip[i]; ++s)
+                    if (net.skip[i][s].kind == 1 && net.skip[i][s].from >= 1) kept |= 1u << net.skip[i][s].from;
+            auto bytes = [&](int l) { return (size_t)((e->nodes[l] + 63) / 64) * 384 * (size_t)tc.ncols_max; };
+            size_t two[2] = {0, 0}, off = 0;
+            for (int l = 1; l <= e->n_lin - 2; ++l)
+                if (!((kept >> l) & 1u)) two[l & 1] = std::max(two[l & 1], bytes(l));
+            for (int l = 1; l <= e->n_lin - 2; ++l) {
+                const bool own = (kept >> l) & 1u;
+                tc.xoff[l] = (uint32_t)(own ? two[0] + two[1] + off : (l & 1 ? two[0] : 0));
+                if (own) off += bytes(l);
+            }
+            tc.xcta = (two[0] + two[1] + off + 1023) / 1024 * 1024;
+            tc.xctas = device_sms();
+            for (cudaError_t rc; (rc = e->tc_x.reserve(tc.xcta * (size_t)tc.xctas)) != cudaSuccess;
+                 tc.xctas = std::max(2, tc.xctas / 4 * 2)) {
+                cudaGetLastError();
+                if (tc.xctas <= 2) AM_CUDA(rc);
+            }
+            tc.xbuf = e->tc_x.as<uint8_t>();
+        }
         AM_CHECK(tc.nstage >= 1 && tc.ncols_max >= 16, "layer widths too large for the tensor-core composition tile");
         AM_CHECK(tc_smem_bytes(tc, tc.ncols_max, e->W) <= smem_cap,
                  "tensor-core composition tile exceeds shared memory");

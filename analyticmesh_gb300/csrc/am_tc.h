@@ -30,9 +30,14 @@ struct TcNet {
     int nstage;                         // weight blocks in flight (1 or 2; up to 3 with the streamed operand)
     int mn;                             // operand layout: 1 MN-major (64-column atoms), 0 K-major
     int n1, k_last;                     // widths of hidden layer 1 and of the last hidden layer
-    int streamed;                       // operand rebuilt per 64-wide K block from the rows (wide layers)
+    int streamed;                       // operand in scratch, copied one 64-deep K block at a time (wide layers)
     int mgroups;                        // streamed: a layer's M tiles in this many passes, each with its own
                                         // accumulators (TMEM holds 2 x ceil(mtiles / mgroups) x ncols columns)
+    // streamed: scratch for the operand, xcta bytes for each of xctas CTAs, hidden layer l's at xoff[l]
+    uint8_t *xbuf;
+    size_t xcta;
+    int xctas;
+    uint32_t xoff[kMaxLayers];
 };
 
 size_t tc_smem_bytes(const TcNet &tc, int ncols, int W);

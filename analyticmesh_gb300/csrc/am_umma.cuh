@@ -63,6 +63,19 @@ __device__ __forceinline__ uint64_t desc_sw128_mn(uint32_t saddr, uint32_t lbo, 
     return d;
 }
 
+// descriptor of an MN-major operand without swizzle: 8 x 8 core matrices (eight K
+// rows of sixteen bytes); leading byte offset = stride between 8-row K groups,
+// stride byte offset = stride between chunks of eight MN elements
+__device__ __forceinline__ uint64_t desc_mn(uint32_t saddr, uint32_t lbo, uint32_t sbo)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)1 << 46;
+    return d;
+}
+
 // instruction descriptor, kind::f16: D fp32, A and B bf16, both K-major
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N)
 {
@@ -106,6 +119,14 @@ __device__ __forceinline__ void mma_bf16_a(uint32_t tmem_d, uint64_t adesc, uint
     }
 }
 
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect()
+{
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void commit(uint32_t mbar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
@@ -133,6 +154,9 @@ __device__ __forceinline__ void cluster_sync()
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// ... and of device memory too
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
 // one warp allocates `ncols` TMEM columns; the base address lands in *slot
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols)

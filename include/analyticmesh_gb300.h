@@ -187,9 +187,9 @@ typedef enum {
                                  queried (am_get_stats, am_get_regions, am_region_rows).  0 (default):
                                  no limit */
     AM_OPT_COMPOSE_TILE = 6,  /* "mixed" composition on the tensor cores: 0 (default) automatic, 1 the
-                                 operand of a tile stays in shared memory for all layers, 2 it is rebuilt
-                                 per 64-deep block from the rows just written (wider tiles for layers of
-                                 256 units and more), 3 as 2 with a layer's 128-row tiles multiplied in two
+                                 operand of a tile stays in shared memory for all layers, 2 it is kept in
+                                 device memory and copied one 64-deep block at a time (wider tiles for
+                                 layers of 256 units and more), 3 as 2 with a layer's 128-row tiles multiplied in two
                                  passes, so that TMEM holds accumulators for twice as many regions (layers
                                  of 512 units).  All give the same bits. */
     AM_OPT_FACE_WARPS = 7,    /* 0 (default) automatic, or 1, 2, 4, 8.  A face is one warp's; the value only

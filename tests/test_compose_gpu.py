@@ -151,3 +151,31 @@ def test_layers_of_three_and_five_m_tiles(widths):
         ref_rows, ref_eq = compose_fp64(net, eng.regions().bits[:n])
         assert rel_err(rows, ref_rows) <= 1e-5 and rel_err(eq, ref_eq) <= 1e-5, tile
         eng.close()
+
+
+@pytest.mark.parametrize("chunk", [0, 700])
+def test_operand_of_parents_and_connections(chunk):
+    """Tiles that start after the layer a region was entered through, with
+    tensor-core connections from layers before and after it and widths that
+    leave every kind of remainder: the streamed operand (one and two passes)
+    against the resident one over a whole march, bit for bit."""
+    m = wl.geometric([72, 130, 72, 200, 48], 5, perturb=0.02, skips=[[0], [1, 1, 0], [2, 1, 1, 2, 2], [1, 1, 3], [0]],
+                     tm_shapes=[[0, 0], [200, 72], [200, 130], [48, 72]])
+    net = wl.net_arrays(m)
+    st, pt = wl.seeds_for(m, init_num=64, seed=3)
+    out = []
+    for tile in (1, 2, 3):
+        opt = {_lib.AM_OPT_COMPOSE_TILE: tile}
+        if chunk:
+            opt[_lib.AM_OPT_CHUNK] = chunk
+        eng = engine.march(net, st, pt, "mixed", options=opt)
+        out.append(eng.regions())
+        eng.close()
+    a = out[0]
+    assert a.num > 2000
+    used = np.arange(a.edges.shape[1])[None, :] < a.nverts[:, None]  # (slots behind the polygon are not written)
+    for b in out[1:]:
+        for x, y in ((a.bits, b.bits), (a.nverts, b.nverts), (a.status, b.status)):
+            assert np.array_equal(x, y)
+        assert np.array_equal(a.edges[used], b.edges[used])
+        assert np.array_equal(a.verts[used].view(np.int64), b.verts[used].view(np.int64))
