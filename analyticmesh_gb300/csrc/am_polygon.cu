@@ -994,6 +994,40 @@ __device__ int seed_start(const Rows &rows, const GlobalRows<TC> &all, const Bal
     unsigned long long pk = ~0ull;
     int pi = -1;
     const TC pc[3] = {(TC)p[0], (TC)p[1], (TC)p[2]};
+    if (rows.n <= kList) { // each row's rank among all, its key computed once
+        constexpr int kPer = kList / 32;
+        unsigned long long key[kPer];
+        int rank[kPer];
+#pragma unroll
+        for (int t = 0; t < kPer; ++t) {
+            const int k = lane + 32 * t;
+            key[t] = 0ull;
+            rank[t] = k < rows.n ? 0 : kNoHit;
+            if (k < rows.n) {
+                const vec4_t<TC> v = rows.get(k);
+                key[t] = order_key(dot3(v.x, pc[0], v.y, pc[1], v.z, pc[2]) + v.w);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kPer; ++t)
+            for (int l = 0; l < 32 && 32 * t + l < rows.n; ++l) {
+                const unsigned long long ok = __shfl_sync(kFull, key[t], l);
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) rank[u] += ahead(ok, 32 * t + l, key[u], lane + 32 * u);
+            }
+        for (int sel = 0; sel < ksel; ++sel) {
+            int mine = -1;
+#pragma unroll
+            for (int t = 0; t < kPer; ++t)
+                if (rank[t] == sel) mine = lane + 32 * t;
+            const int at = __shfl_sync(kFull, mine, __ffs(__ballot_sync(kFull, mine >= 0)) - 1);
+            if (lane == (sel & 31)) {
+                if (sel < 32) top0 = at;
+                else top1 = at;
+            }
+            pi = at;
+        }
+    } else
     for (int sel = 0; sel < ksel; ++sel) {
         unsigned long long bk = 0ull;
         int bi = kNoHit;
@@ -1035,6 +1069,25 @@ __device__ int seed_start(const Rows &rows, const GlobalRows<TC> &all, const Bal
     // arithmetic of warp_solve); their vertices are tested one after the other,
     // the first that every other row admits wins
     const int G = lane >> 2, L = lane & 3, gbase = lane & ~3;
+    // the rows in FP32, held by the lanes: a vertex that one of them shuts out by
+    // more than the FP32 error (a row's and a determinant's rounding, a quotient's,
+    // a product's, three sums': 9 x 2^-24 of the products' sizes; 2^-20 asked for)
+    // needs neither the divisions nor a test in TC.  (FP64 is what a seed's search
+    // costs: 813 pairs.  Measured on GB300, eight boxes around 64 x 3 networks in
+    // FP64, a batch of marchings: 8.0 ms with every pair divided and tested row
+    // after row and the nearest planes picked one by one, 7.4 ms this way.)
+    constexpr int kPer = kList / 32;
+    const bool held = rows.n <= kList;
+    float4 fr[kPer];
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+        fr[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (held && lane + 32 * t < rows.n) {
+            const vec4_t<TC> r = rows.get(lane + 32 * t);
+            fr[t] = make_float4((float)r.x, (float)r.y, (float)r.z, (float)r.w);
+        }
+    }
+    const float feps = (float)eps + 1e-30f;
     for (int x0 = 0; x0 <= x_max; x0 += 8) {
         int i, j;
         get_i_j(min(x0 + G, x_max), all.n, i, j);
@@ -1055,8 +1108,31 @@ __device__ int seed_start(const Rows &rows, const GlobalRows<TC> &all, const Bal
         const TS a10 = L == 1 ? -m[7] : m[4], a11 = L == 2 ? -m[7] : m[5], a12 = L == 3 ? -m[7] : m[6];
         const TS a20 = L == 1 ? -eqv[3] : eqv[0], a21 = L == 2 ? -eqv[3] : eqv[1], a22 = L == 3 ? -eqv[3] : eqv[2];
         const TS d = det3<TS>(a00, a01, a02, a10, a11, a12, a20, a21, a22);
-        const TS xv = d / __shfl_sync(kFull, d, gbase);
+        const TS d0 = __shfl_sync(kFull, d, gbase);
+        unsigned shut = 0u; // pairs of the eight that some row shuts out for certain
+        if (held) {
+            // (a quotient of determinants that FP32 does not hold to its precision shuts nothing out)
+            const float fd = (float)d, f0 = (float)d0;
+            const float fx = d == TS(0) ? 0.f : (fminf(fabsf(fd), fabsf(f0)) < 1e-30f ? NAN : fd / f0);
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+                const float a = __shfl_sync(kFull, fx, 4 * g + 1), b = __shfl_sync(kFull, fx, 4 * g + 2),
+                            c = __shfl_sync(kFull, fx, 4 * g + 3);
+                const int gi = __shfl_sync(kFull, ri, 4 * g), gj = __shfl_sync(kFull, rj, 4 * g);
+#pragma unroll
+                for (int t = 0; t < kPer; ++t) {
+                    const int k = lane + 32 * t;
+                    const float d = fr[t].x * a + fr[t].y * b + fr[t].z * c + fr[t].w;
+                    const float z = fabsf(fr[t].x * a) + fabsf(fr[t].y * b) + fabsf(fr[t].z * c) + fabsf(fr[t].w);
+                    if (d > feps + z * 9.5367431640625e-7f && k != gi && k != gj) shut |= 1u << g;
+                }
+            }
+            shut = __reduce_or_sync(kFull, shut);
+        }
+        if (shut == 0xffu) continue;
+        const TS xv = d / d0;
         for (int g = 0; g < 8 && x0 + g <= x_max; ++g) {
+            if ((shut >> g) & 1u) continue;
             const TS v[3] = {__shfl_sync(kFull, xv, 4 * g + 1), __shfl_sync(kFull, xv, 4 * g + 2),
                              __shfl_sync(kFull, xv, 4 * g + 3)};
             const TC vc[3] = {(TC)v[0], (TC)v[1], (TC)v[2]};

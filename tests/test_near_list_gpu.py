@@ -63,3 +63,20 @@ def test_faces_from_the_near_list_are_the_oracles(name):
             assert e.error_report(0)["max_abs_f"] <= 1e-5
         e.close()
     eng.close()
+
+
+@pytest.mark.parametrize("widths", [[29], [30], [61], [62], [31, 62], [62, 63]], ids=lambda w: "rows%d" % (sum(w) + 3))
+def test_seeds_whose_nearest_pairs_are_shut_out(widths):
+    """A box corner inside the surface: at its seeds most pairs of near planes meet
+    outside it, so the start search goes on for many pairs.  Row counts around
+    those of a lane's rows (32, 64, 128), against the oracle's search."""
+    m = wl.geometric(widths, 11, perturb=0.05)
+    corner = ([[1, 0, 0], [0, 1, 0], [0, 0, 1]], [-0.05, 0.02, -0.1])
+    net = wl.net_arrays(m, *corner)
+    st, pt = wl.seeds_for(m, init_num=200, seed=5, w_extra=corner[0], b_extra=corner[1])
+    ref = oracle.run_oracle(net, st, pt, dtype="float64")
+    eng = engine.march(net, st, pt, "float64")
+    c = compare.canonical(eng.regions(), ref, tol=1e-9)
+    assert c["only_a"] == 0 and c["only_b"] == 0, c
+    assert c["faces_mismatch"] == 0 and c["faces_only_a"] == 0 and c["faces_only_b"] == 0, c
+    eng.close()
