@@ -308,7 +308,7 @@ struct WPipe {
     uint8_t *ws;
     int nstage;
     int *err;
-    int consumed;          // (thread 0) blocks whose products were issued
+    int consumed;          // (warp 0) blocks whose products were issued
     volatile int *abort;   // the CTA's abort flag (shared memory)
 };
 
@@ -370,8 +370,9 @@ __device__ __forceinline__ void issue_step(uint32_t d_main, uint32_t d_corr, uin
     umma::MMA0(d_corr, ad + 2048u, xd, idesc, 1u);
 }
 
-// (thread 0) D[mt] (+)= M . X over all K blocks of the operand in shared
-// memory: six products per K step (terms t, u of weight 2^-8(t+u), t + u <= 2)
+// (warp 0, one elected lane issuing: see issue_streamed) D[mt] (+)= M . X over all
+// K blocks of the operand in shared memory: six products per K step (terms t, u of
+// weight 2^-8(t+u), t + u <= 2)
 __device__ void gemm_issue(WPipe &p, const TcMat &m, int mtiles, const XOp &X, uint32_t tmem, bool first, int &g)
 {
     const int ncols = X.ncols;
@@ -380,9 +381,9 @@ __device__ void gemm_issue(WPipe &p, const TcMat &m, int mtiles, const XOp &X, u
     const int kblocks = m.Kp / 64;
     for (int mt = 0; mt < mtiles; ++mt) {
         for (int kb = 0; kb < kblocks; ++kb) {
-            if (*p.abort) return;
             const int s = g % p.nstage;
-            if (!wp_wait(p, p.full + s, (uint32_t)(g / p.nstage) & 1u)) return;
+            const bool ok = *p.abort == 0 && wp_wait(p, p.full + s, (uint32_t)(g / p.nstage) & 1u);
+            if (!__all_sync(0xffffffffu, ok)) return;
             umma::fence_after();
             const uint32_t a0 = umma::smem_addr(p.ws + (size_t)s * kWBlockBytes);
             const uint32_t d_main = tmem + (uint32_t)(mt * ncols);            // hh
@@ -390,9 +391,12 @@ __device__ void gemm_issue(WPipe &p, const TcMat &m, int mtiles, const XOp &X, u
             const bool fresh = first && kb == 0;
             // A: term t at +16 KB (1024 units), K step j at +32 B (2 units)
             const uint64_t ad = umma::desc_sw128(a0), xd = X.desc(0, kb, 0);
-            #pragma unroll
-            for (int j = 0; j < 4; ++j) issue_step(d_main, d_corr, ad + 2u * j, xd + xj * j, xu, idesc, fresh && j == 0);
-            umma::commit(umma::smem_addr(p.done + s)); // frees the stage for the copy warp
+            if (umma::elect()) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) issue_step(d_main, d_corr, ad + 2u * j, xd + xj * j, xu, idesc, fresh && j == 0);
+                umma::commit(umma::smem_addr(p.done + s)); // frees the stage for the copy warp
+            }
+            __syncwarp();
             p.consumed = g + 1;
             ++g;
         }
@@ -580,7 +584,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
         for (int i = cls; i <= net.n_lin - 2; ++i) {
             const int M = net.nodes[i + 1];
             const int mtiles = (M + 127) / 128;
-            if (tid == 0) gemm_issue(pp, tc.lin[i], mtiles, X, tmem, true, g);
+            if (warp == 0) gemm_issue(pp, tc.lin[i], mtiles, X, tmem, true, g);
             for (int s = 0; s < net.nskip[i]; ++s) {
                 const SkipDev &sk = net.skip[i][s];
                 if (tc_skip(sk)) {
@@ -595,7 +599,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                                       net.nodes[sk.from], tc.skip[i][s].Kp);
                     umma::fence_proxy_async();
                     bar_main();
-                    if (tid == 0) gemm_issue(pp, tc.skip[i][s], mtiles, X, tmem, false, g);
+                    if (warp == 0) gemm_issue(pp, tc.skip[i][s], mtiles, X, tmem, false, g);
                 }
             }
             // the first M tile's bias, loaded while the products run
