@@ -7,8 +7,8 @@
 // columns each, UMMA N = 4 x regions, chosen per launch from the chunk size so
 // that small frontier waves still spread over every SM) and keeps the masked
 // operand X_l = diag(s_l) A_l on chip the whole way through the network, as
-// bf16 terms in 128B-swizzled shared memory (MN-major, or K-major for layers
-// too wide for 64-column atoms): the B operand of tcgen05.mma.  The layer
+// bf16 terms in shared memory (MN-major core matrices without swizzle): the B
+// operand of tcgen05.mma.  The layer
 // weights are the A operand (K-major); they are pre-split and
 // stored in global memory as the exact shared-memory image of their 128 x 64
 // blocks, so one bulk copy (cp.async.bulk, completing on an mbarrier) stages a
@@ -29,7 +29,7 @@
 // sign-flipped constraint rows to HBM for the polygon kernel, and writes the
 // next layer's masked operand straight back into shared memory.  The face
 // plane (output layer, one row) is a 4 x K dot product per region in fp32,
-// one warp per region, from the operand in shared memory.
+// from the operand in shared memory.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -60,71 +60,42 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t &h, uint32_t &
     l = *reinterpret_cast<const uint32_t *>(&lb);
 }
 
-// The masked operand X (ncols x Kp, three bf16 terms `xbytes` apart) in
-// shared memory, in one of two layouts.  MN-major (64-column atoms): the
-// thread that owns one K row writes 8 consecutive columns with one 16-byte
-// store per term.  K-major (any multiple of 16 columns, 2-byte stores): used
-// when a 64-column atom of the widest K does not fit beside the weights.
+// The masked operand X (ncols x Kp) is kept as three bf16 terms in 64-deep blocks.
+// The operand image: a term of a 64-deep block is ncols / 8 chunks of eight
+// columns, a chunk 64 rows of 16 bytes.  That is the canonical MN-major layout
+// without swizzle (eight rows of a chunk: 128 contiguous bytes), so a warp whose
+// lanes hold consecutive rows stores 512 contiguous bytes, in scratch (the streamed
+// operand) as in shared memory, and any multiple of 16 columns will do.  (Measured on GB300: the
+// products run at the same rate as from a 128-byte swizzle, 64 cycles at 128
+// columns; with the swizzled layout, two regions x 16 rows per warp item, the
+// composition of ragged widths with connections took 1.95 ms against 1.72, of
+// 128 x 4 1.80 against 1.74.)
+__host__ __device__ __forceinline__ uint32_t op_term_bytes(int ncols) { return (uint32_t)ncols * 128u; }
+__device__ __forceinline__ void op_put8(uint8_t *blk, uint32_t term, int chunk, int k, const float *x)
+{
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split2(x[2 * i], x[2 * i + 1], h[i], m[i], l[i]);
+    uint8_t *p = blk + chunk * 1024 + k * 16;
+    *reinterpret_cast<uint4 *>(p) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4 *>(p + term) = make_uint4(m[0], m[1], m[2], m[3]);
+    *reinterpret_cast<uint4 *>(p + 2 * term) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// the whole operand in shared memory
 struct XOp {
     uint8_t *xs;
-    size_t xbytes;
-    int ncols, natoms;
-    bool mn;
-
-    __device__ __forceinline__ uint32_t off(int n, int k) const
+    uint32_t term; // bytes of a term of a block
+    __device__ __forceinline__ uint8_t *block(int kb) const { return xs + (size_t)kb * 3 * term; }
+    // columns 8 chunk .. 8 chunk + 7 of row k
+    __device__ __forceinline__ void put8(int chunk, int k, const float *x) const { op_put8(block(k >> 6), term, chunk, k & 63, x); }
+    // hi + mid + lo of region r's columns of row k
+    __device__ __forceinline__ void get4(int r, int k, float *v) const
     {
-        return mn ? umma::mn_sw128_offset(n, k, natoms) : umma::sw128_offset(n, k, ncols);
-    }
-    // columns n0 .. n0 + 2w - 1 of row k (n0 a multiple of 2w, w = 2 or 4)
-    template <int w>
-    __device__ __forceinline__ void put(int n0, int k, const float *v) const
-    {
-        uint32_t h[w], m[w], l[w];
-#pragma unroll
-        for (int i = 0; i < w; ++i) split2(v[2 * i], v[2 * i + 1], h[i], m[i], l[i]);
-        if (mn) {
-            const uint32_t o = off(n0, k);
-            if (w == 4) {
-                *reinterpret_cast<uint4 *>(xs + o) = make_uint4(h[0], h[1], h[2 % w], h[3 % w]);
-                *reinterpret_cast<uint4 *>(xs + xbytes + o) = make_uint4(m[0], m[1], m[2 % w], m[3 % w]);
-                *reinterpret_cast<uint4 *>(xs + 2 * xbytes + o) = make_uint4(l[0], l[1], l[2 % w], l[3 % w]);
-            } else {
-                *reinterpret_cast<uint2 *>(xs + o) = make_uint2(h[0], h[1]);
-                *reinterpret_cast<uint2 *>(xs + xbytes + o) = make_uint2(m[0], m[1]);
-                *reinterpret_cast<uint2 *>(xs + 2 * xbytes + o) = make_uint2(l[0], l[1]);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 2 * w; ++i) {
-                const uint32_t o = off(n0 + i, k);
-                const int sh = (i & 1) * 16;
-                *reinterpret_cast<uint16_t *>(xs + o) = (uint16_t)(h[i >> 1] >> sh);
-                *reinterpret_cast<uint16_t *>(xs + xbytes + o) = (uint16_t)(m[i >> 1] >> sh);
-                *reinterpret_cast<uint16_t *>(xs + 2 * xbytes + o) = (uint16_t)(l[i >> 1] >> sh);
-            }
-        }
-    }
-    // hi + mid + lo of columns n0 .. n0 + 3 (n0 a multiple of 4) of row k
-    __device__ __forceinline__ void get4(int n0, int k, float *v) const
-    {
-        uint32_t hw[2], mw[2], lw[2];
-        if (mn) {
-            const uint32_t o = off(n0, k);
-            const uint2 h = *reinterpret_cast<const uint2 *>(xs + o);
-            const uint2 m = *reinterpret_cast<const uint2 *>(xs + xbytes + o);
-            const uint2 l = *reinterpret_cast<const uint2 *>(xs + 2 * xbytes + o);
-            hw[0] = h.x, hw[1] = h.y, mw[0] = m.x, mw[1] = m.y, lw[0] = l.x, lw[1] = l.y;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const uint32_t o0 = off(n0 + 2 * i, k), o1 = off(n0 + 2 * i + 1, k);
-                auto pair = [&](size_t t) {
-                    return (uint32_t)*reinterpret_cast<const uint16_t *>(xs + t + o0) |
-                           ((uint32_t)*reinterpret_cast<const uint16_t *>(xs + t + o1) << 16);
-                };
-                hw[i] = pair(0), mw[i] = pair(xbytes), lw[i] = pair(2 * xbytes);
-            }
-        }
+        const uint8_t *p = block(k >> 6) + (r >> 1) * 1024 + (k & 63) * 16 + (r & 1) * 8;
+        const uint2 h = *reinterpret_cast<const uint2 *>(p), m = *reinterpret_cast<const uint2 *>(p + term),
+                    l = *reinterpret_cast<const uint2 *>(p + 2 * term);
+        const uint32_t hw[2] = {h.x, h.y}, mw[2] = {m.x, m.y}, lw[2] = {l.x, l.y};
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&hw[i]));
@@ -133,50 +104,6 @@ struct XOp {
             v[2 * i] = a.x + b.x + c.x;
             v[2 * i + 1] = a.y + b.y + c.y;
         }
-    }
-    // descriptor of term u for K block kb, K step j (16 deep) of the block
-    __device__ __forceinline__ uint64_t desc(int u, int kb, int j) const
-    {
-        const uint32_t base = umma::smem_addr(xs) + (uint32_t)(u * xbytes);
-        if (mn) {
-            const uint32_t kgroup = (uint32_t)natoms * 1024u;
-            return umma::desc_sw128_mn(base + (uint32_t)(kb * 8 + 2 * j) * kgroup, 1024u, kgroup);
-        }
-        return umma::desc_sw128(base + (uint32_t)(kb * ncols * 128 + j * 32));
-    }
-    __device__ __forceinline__ uint32_t idesc() const
-    {
-        return mn ? umma::idesc_bf16_bmn(128, ncols) : umma::idesc_bf16(128, ncols);
-    }
-    // descriptor steps (16-byte units of the start address field) from term
-    // u to u + 1 and from K step j to j + 1: desc(u, kb, j) = desc(0, kb, 0)
-    // + u * ustep() + j * jstep()
-    __device__ __forceinline__ uint32_t ustep() const { return (uint32_t)(xbytes >> 4); }
-    __device__ __forceinline__ uint32_t jstep() const { return mn ? (uint32_t)natoms * 128u : 2u; }
-};
-
-// Operand items (region r, row k of a 64-deep block) in the order the warps take
-// them: a warp item is two regions x sixteen rows, so that its loads are two runs
-// of 256 bytes and its stores fill whole 128-byte rows of the swizzled operand
-// (measured on GB300 with a lane per region instead: 32 lines per load, and the
-// block's loads took longer than its 48 products).
-struct Items {
-    int half, shift; // region pairs; their log2, or -1
-    __device__ __forceinline__ explicit Items(int R)
-    {
-        half = R / 2;
-        shift = -1;
-        for (int b = 0; b < 8; ++b)
-            if (half == 1 << b) shift = b;
-    }
-    // item `idx` of 2 R per block: false beyond the last
-    __device__ __forceinline__ bool at(int idx, int lane, int &r, int &k) const
-    {
-        const int kg = shift >= 0 ? idx >> shift : idx / half;
-        const int pair = idx - kg * half;
-        r = 2 * pair + (lane & 1);
-        k = kg * 16 + (lane >> 1);
-        return kg < 4;
     }
 };
 
@@ -211,43 +138,44 @@ __device__ __forceinline__ void add_skips(const NetDev &net, int i, int m, const
     }
 }
 
-// X[n = 4r + c][k] = s_k(r) ? -C[r][src + k][c] : 0 for k < K, 0 up to Kp
-__device__ void stage_x_from_rows(const XOp &X, const float *cons, size_t rstride, const int4 *ri, int jend,
-                                  const uint32_t *keys, int W, int nreg, int src, int K, int Kp)
+// X[n = 4r + c][k] = s_k(r) ? -C[r][src + k][c] : 0 for k < K, 0 to the end of the
+// last block.  A warp item is two regions x 32 rows, a row per lane: loads and
+// stores of 512 contiguous bytes.
+__device__ void stage_x_from_rows(const XOp &X, int R, const float *cons, size_t rstride, const int4 *ri, int jend,
+                                  const uint32_t *keys, int W, int nreg, int src, int K)
 {
-    const Items items(X.ncols / 4);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool par = src < jend;
-    const int per = X.ncols / 2; // items per block
-    const int n = per * (Kp / 64);
-    constexpr int kU = 4, kWarpsM = kThreads / 32;
-    // four items' loads before the first is used (measured on GB300: one by one
-    // the rows of 32 regions x 128 units took 15 K cycles, most of a tile's time)
+    constexpr int kU = 2, kWarpsM = kThreads / 32;
+    const int n = R * ((K + 63) / 64);
+    // the items' loads before the first is used (measured on GB300: one by one the
+    // rows of 32 regions x 128 units took 15 K cycles, most of a tile's time)
     for (int q0 = warp; q0 < n; q0 += kU * kWarpsM) {
-        float4 v[kU];
-        float sg[kU];
+        float4 v[kU][2];
+        unsigned other = 0u; // rows with the other sign
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
-            const int q = q0 + u * kWarpsM;
-            int r, k;
-            items.at(q % per, lane, r, k);
-            k += q / per * 64;
-            const int row = src + k;
-            const int4 g = ri[r];
-            const bool on = q < n && r < nreg && k < K && key_bit(keys + (size_t)r * W, row);
-            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (on) v[u] = ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)row * 4);
-            sg[u] = row == g.z ? 1.f : -1.f;
+            const int q = q0 + u * kWarpsM, kb = q / R, in = q - kb * R;
+            const int k = kb * 64 + (in & 1) * 32 + lane;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = (in >> 1) * 2 + e;
+                v[u][e] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (q < n && r < nreg && k < K && key_bit(keys + (size_t)r * W, src + k)) {
+                    const int4 g = ri[r];
+                    v[u][e] = ld4<float>(cons + (size_t)(uint32_t)(par ? g.y : g.x) * rstride + (size_t)(src + k) * 4);
+                    if (src + k == g.z) other |= 1u << (2 * u + e);
+                }
+            }
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
-            const int q = q0 + u * kWarpsM;
+            const int q = q0 + u * kWarpsM, kb = q / R, in = q - kb * R;
             if (q >= n) break;
-            int r, k;
-            items.at(q % per, lane, r, k);
-            k += q / per * 64;
-            const float x[4] = {sg[u] * v[u].x, sg[u] * v[u].y, sg[u] * v[u].z, sg[u] * v[u].w};
-            X.put<2>(4 * r, k, x);
+            const float s0 = (other >> (2 * u)) & 1u ? 1.f : -1.f, s1 = (other >> (2 * u + 1)) & 1u ? 1.f : -1.f;
+            const float4 a = v[u][0], b = v[u][1];
+            const float x[8] = {s0 * a.x, s0 * a.y, s0 * a.z, s0 * a.w, s1 * b.x, s1 * b.y, s1 * b.z, s1 * b.w};
+            X.put8(in >> 1, kb * 64 + (in & 1) * 32 + lane, x);
         }
     }
 }
@@ -373,11 +301,11 @@ __device__ __forceinline__ void issue_step(uint32_t d_main, uint32_t d_corr, uin
 // (warp 0, one elected lane issuing: see issue_streamed) D[mt] (+)= M . X over all
 // K blocks of the operand in shared memory: six products per K step (terms t, u of
 // weight 2^-8(t+u), t + u <= 2)
-__device__ void gemm_issue(WPipe &p, const TcMat &m, int mtiles, const XOp &X, uint32_t tmem, bool first, int &g)
+__device__ void gemm_issue(WPipe &p, const TcMat &m, int mtiles, const XOp &X, int ncols, uint32_t tmem, bool first, int &g)
 {
-    const int ncols = X.ncols;
-    const uint32_t idesc = X.idesc();
-    const uint64_t xu = X.ustep(), xj = X.jstep();
+    const uint32_t idesc = umma::idesc_bf16_bmn(128, ncols);
+    const uint64_t xd0 = umma::desc_mn(umma::smem_addr(X.xs), 128u, 1024u);
+    const uint64_t xu = X.term >> 4, xj = 16u; // to the next term and K step (16 rows of every chunk)
     const int kblocks = m.Kp / 64;
     for (int mt = 0; mt < mtiles; ++mt) {
         for (int kb = 0; kb < kblocks; ++kb) {
@@ -390,7 +318,7 @@ __device__ void gemm_issue(WPipe &p, const TcMat &m, int mtiles, const XOp &X, u
             const uint32_t d_corr = tmem + (uint32_t)((mtiles + mt) * ncols); // the rest
             const bool fresh = first && kb == 0;
             // A: term t at +16 KB (1024 units), K step j at +32 B (2 units)
-            const uint64_t ad = umma::desc_sw128(a0), xd = X.desc(0, kb, 0);
+            const uint64_t ad = umma::desc_sw128(a0), xd = xd0 + 3u * xu * (uint64_t)kb;
             if (umma::elect()) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) issue_step(d_main, d_corr, ad + 2u * j, xd + xj * j, xu, idesc, fresh && j == 0);
@@ -479,12 +407,9 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
 
     uint8_t *base = smem_raw + ((1024u - (umma::smem_addr(smem_raw) & 1023u)) & 1023u);
     XOp X;
-    X.mn = tc.mn != 0;
-    X.ncols = ncols;
-    X.natoms = (ncols + 63) / 64;
-    X.xbytes = (size_t)(X.mn ? X.natoms * 64 : ncols) * tc.kp_max * 2; // one bf16 term of the operand
-    X.xs = base;                                                     // hi, mid, lo
-    uint8_t *ws = base + 3 * X.xbytes;                               // nstage weight blocks
+    X.term = op_term_bytes(ncols);
+    X.xs = base;
+    uint8_t *ws = base + (size_t)(tc.kp_max / 64) * 3 * X.term;      // nstage weight blocks
     uint32_t *keys = reinterpret_cast<uint32_t *>(ws + (size_t)tc.nstage * kWBlockBytes); // the tile's bits
     // per CTA, for every tile: linear 0 as (w0, w1, w2, b) per unit and the
     // face-plane weights (the output linear's only row)
@@ -530,22 +455,23 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
         bar_main(); // the previous tile is done with the keys and the operand
         if (tid < nreg) ri[tid] = tile_region(plan, reg, ch, head, t, cls, tid);
         bar_main();
-        for (int q = tid; q < R * net.W; q += kThreads) {
-            const int rr = q / net.W, w = q % net.W;
-            keys[rr * KW + w] = rr < nreg ? reg.keys[(size_t)(head + ri[rr].w) * net.W + w] : 0u;
+        for (int rr = warp; rr < R; rr += kThreads / 32) { // a region's words together in flight
+            const uint32_t *key = reg.keys + (size_t)(rr < nreg ? head + ri[rr].w : 0) * net.W;
+#pragma unroll 2
+            for (int w = lane; w < net.W; w += 32) keys[rr * KW + w] = rr < nreg ? key[w] : 0u;
         }
         bar_main(); // every thread reads every region's bits below
 
         // class 1: hidden layer 1 = linear 0 rows (sign-flipped); the extra constraints
         {
             const int n1 = net.nodes[1];
-            for (int q = tid; cls == 1 && q < nreg * n1; q += kThreads) {
-                const int rr = q / n1, m = q % n1;
-                const float sg = key_bit(keys + (size_t)rr * KW, m) ? -1.f : 1.f;
-                const float4 w = w0s[m];
-                st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)m * 4,
-                           make_float4(sg * w.x, sg * w.y, sg * w.z, sg * w.w));
-            }
+            for (int rr = warp; cls == 1 && rr < nreg; rr += kThreads / 32)
+                for (int m = lane; m < n1; m += 32) {
+                    const float sg = key_bit(keys + (size_t)rr * KW, m) ? -1.f : 1.f;
+                    const float4 w = w0s[m];
+                    st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)m * 4,
+                               make_float4(sg * w.x, sg * w.y, sg * w.z, sg * w.w));
+                }
             const float *we = (const float *)net.w_extra;
             const float *be = (const float *)net.b_extra;
             for (int q = tid; q < nreg * net.E; q += kThreads) {
@@ -555,24 +481,24 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
             }
         }
         if (cls > 1) { // the operand of linear cls, from the parent's rows
-            stage_x_from_rows(X, cons, rstride, ri, jend, keys, KW, nreg, net.hoff[cls], net.nodes[cls],
-                              (net.nodes[cls] + 63) / 64 * 64);
+            stage_x_from_rows(X, R, cons, rstride, ri, jend, keys, KW, nreg, net.hoff[cls], net.nodes[cls]);
         } else {
             const int n1 = net.nodes[1];
-            // X_1 = diag(s_1) [W0 | b0]; regions fastest across the lanes:
-            // consecutive regions' columns share a 128-byte operand row
-            const int Kp = (n1 + 63) / 64 * 64;
-            for (int q = tid; q < R * Kp; q += kThreads) {
-                const int r = q % R, k = q / R;
-                float x[4] = {0.f, 0.f, 0.f, 0.f};
-                if (r < nreg && k < n1 && key_bit(keys + (size_t)r * KW, k)) {
-                    const float4 w = w0s[k];
-                    x[0] = w.x;
-                    x[1] = w.y;
-                    x[2] = w.z;
-                    x[3] = w.w;
+            // X_1 = diag(s_1) [W0 | b0], two regions x 32 units at a time
+            for (int q = warp; q < R * ((n1 + 63) / 64); q += kThreads / 32) {
+                const int kb = q / R, in = q - kb * R, k = kb * 64 + (in & 1) * 32 + lane;
+                const float4 w = k < n1 ? w0s[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+                float x[8];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int r = (in >> 1) * 2 + e;
+                    const bool on = r < nreg && k < n1 && key_bit(keys + (size_t)r * KW, k);
+                    x[4 * e] = on ? w.x : 0.f;
+                    x[4 * e + 1] = on ? w.y : 0.f;
+                    x[4 * e + 2] = on ? w.z : 0.f;
+                    x[4 * e + 3] = on ? w.w : 0.f;
                 }
-                X.put<2>(4 * r, k, x);
+                X.put8(in >> 1, k, x);
             }
         }
         umma::fence_proxy_async();
@@ -584,7 +510,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
         for (int i = cls; i <= net.n_lin - 2; ++i) {
             const int M = net.nodes[i + 1];
             const int mtiles = (M + 127) / 128;
-            if (warp == 0) gemm_issue(pp, tc.lin[i], mtiles, X, tmem, true, g);
+            if (warp == 0) gemm_issue(pp, tc.lin[i], mtiles, X, ncols, tmem, true, g);
             for (int s = 0; s < net.nskip[i]; ++s) {
                 const SkipDev &sk = net.skip[i][s];
                 if (tc_skip(sk)) {
@@ -595,11 +521,10 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                     }
                     bar_main();
                     if (s_stop) break; // written by thread 0 before the barrier: uniform
-                    stage_x_from_rows(X, cons, rstride, ri, jend, keys, KW, nreg, net.hoff[sk.from],
-                                      net.nodes[sk.from], tc.skip[i][s].Kp);
+                    stage_x_from_rows(X, R, cons, rstride, ri, jend, keys, KW, nreg, net.hoff[sk.from], net.nodes[sk.from]);
                     umma::fence_proxy_async();
                     bar_main();
-                    if (warp == 0) gemm_issue(pp, tc.skip[i][s], mtiles, X, tmem, false, g);
+                    if (warp == 0) gemm_issue(pp, tc.skip[i][s], mtiles, X, ncols, tmem, false, g);
                 }
             }
             // the first M tile's bias, loaded while the products run
@@ -616,11 +541,11 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
             gemm_observe(pp, s_last);
             // epilogue: accumulators -> constraint rows (HBM) and the next operand (smem)
             const int Kn = (M + 63) / 64 * 64; // next operand's padded K (the face plane reads it too)
-            for (int q = tid; q < R * (Kn - M); q += kThreads) {
-                const int r = q % R, k = M + q / R;
-                const float z[4] = {0.f, 0.f, 0.f, 0.f};
-                X.put<2>(4 * r, k, z);
-            }
+            for (int c = warp; c < R / 2; c += kThreads / 32)
+                for (int k = M + lane; k < Kn; k += 32) {
+                    const float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                    X.put8(c, k, z);
+                }
             for (int mt = 0; mt < mtiles; ++mt) {
                 const int m = mt * 128 + q4 * 32 + lane;
                 const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
@@ -654,8 +579,8 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
                         #pragma unroll
                         for (int c = 0; c < 4; ++c) x[4 * qq + c] = act ? o[c] : 0.f;
                     }
-                    X.put<4>(cb * 16, m, x);
-                    X.put<4>(cb * 16 + 8, m, x + 8);
+                    X.put8(cb * 2, m, x);
+                    X.put8(cb * 2 + 1, m, x + 8);
                 }
             }
             umma::fence_proxy_async();
@@ -675,18 +600,21 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
             const float bl = ((const float *)net.bias[i])[0];
             constexpr int kWarps = kThreads / 32;
             for (int r0 = 0; r0 < R; r0 += 32) {
-                const int r = r0 + lane;
+                // thread (region fr of these 32, K residue fw): sixteen
+                // consecutive rows of two regions per warp and step
+                const int fr = 2 * warp + (lane & 1), fw = lane >> 1, r = r0 + fr;
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
                 if (r < R)
-                    for (int k = warp; k < K; k += kWarps) {
+#pragma unroll 4
+                    for (int k = fw; k < K; k += kWarps) {
                         const float w = wls[k];
                         float x[4];
-                        X.get4(4 * r, k, x);
+                        X.get4(r, k, x);
 #pragma unroll
                         for (int c = 0; c < 4; ++c) acc[c] = fmaf(w, x[c], acc[c]);
                     }
-                // partial sums: [warp][lane][4]
-                reinterpret_cast<float4 *>(fsum)[warp * 32 + lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                // partial sums: [residue][region][4]
+                reinterpret_cast<float4 *>(fsum)[fw * 32 + fr] = make_float4(acc[0], acc[1], acc[2], acc[3]);
                 bar_main();
                 if (tid < 128) {
                     const int rr = tid >> 2, c = tid & 3, rg = r0 + rr;
@@ -790,25 +718,6 @@ __device__ __forceinline__ int pass_blocks(const NetDev &net, const TcNet &tc, i
     const int njobs = jobs_of(net, i);
     for (int job = 0; job < njobs; ++job) n += job_mat(net, tc, i, job, src).Kp / 64;
     return n;
-}
-
-// The operand image: a term of a 64-deep block is ncols / 8 chunks of eight
-// columns, a chunk 64 rows of 16 bytes.  That is the canonical MN-major layout
-// without swizzle (eight rows of a chunk: 128 contiguous bytes), so a warp whose
-// lanes hold consecutive rows stores 512 contiguous bytes, in the scratch as in
-// shared memory, and any multiple of 16 columns will do.  (Measured on GB300: the
-// products run at the same rate as from a 128-byte swizzle, 64 cycles at 128
-// columns.)
-__host__ __device__ __forceinline__ uint32_t op_term_bytes(int ncols) { return (uint32_t)ncols * 128u; }
-__device__ __forceinline__ void op_put8(uint8_t *blk, uint32_t term, int chunk, int k, const float *x)
-{
-    uint32_t h[4], m[4], l[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) split2(x[2 * i], x[2 * i + 1], h[i], m[i], l[i]);
-    uint8_t *p = blk + chunk * 1024 + k * 16;
-    *reinterpret_cast<uint4 *>(p) = make_uint4(h[0], h[1], h[2], h[3]);
-    *reinterpret_cast<uint4 *>(p + term) = make_uint4(m[0], m[1], m[2], m[3]);
-    *reinterpret_cast<uint4 *>(p + 2 * term) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
 // Hidden layers whose operand a tile of class c needs and does not compute: c
@@ -1615,8 +1524,7 @@ size_t tc_smem_bytes(const TcNet &tc, int ncols, int W)
         return 1024 + std::max<size_t>(6 * (size_t)op_term_bytes(ncols), (size_t)kSFaceSumBytes) + (size_t)tc.nstage * kWBlockBytes +
                (size_t)(tc.ncols_max / 4) * key_stride(W) * 4 + 16 * (size_t)tc.n1 + 4 * (size_t)tc.k_last + 16;
     }
-    const size_t cols = tc.mn ? (size_t)(ncols + 63) / 64 * 64 : (size_t)ncols;
-    return 1024 + 3 * cols * tc.kp_max * 2 + (size_t)tc.nstage * kWBlockBytes + (size_t)(tc.ncols_max / 4) * key_stride(W) * 4 +
+    return 1024 + (size_t)(tc.kp_max / 64) * 3 * op_term_bytes(ncols) + (size_t)tc.nstage * kWBlockBytes + (size_t)(tc.ncols_max / 4) * key_stride(W) * 4 +
            16 * (size_t)tc.n1 + 4 * (size_t)tc.k_last + 16 + (size_t)kFaceSumBytes;
 }
 

@@ -797,23 +797,20 @@ void run_begin(am_engine *e, const RunArgs &a)
         // beside two weight blocks in flight (one if that leaves no room),
         // two accumulators (main + correction) per M tile in 512 TMEM columns
         const size_t smem_cap = 227u * 1024u - 2048u; // less the kernels' static shared memory
-        // preference: MN-major operand (whole 64-column atoms), two weight
-        // stages, then one; then the K-major operand (any 16 columns)
+        // with two weight stages, else with one; above 128 columns whole
+        // multiples of them (the face plane takes 32 regions at a time)
         tc.ncols_max = 0;
         tc.n1 = e->nodes[1];
         tc.k_last = e->nodes[e->n_lin - 1];
-        for (int mn = 1; mn >= 0 && tc.ncols_max < 16; --mn)
-            for (tc.nstage = 2; tc.nstage >= 1; --tc.nstage) {
-                const long long room = (long long)smem_cap - 1024 - (long long)tc.nstage * kWBlockBytes -
-                                       64ll * (e->W | 1) * 4 - 16ll * tc.n1 - 4ll * tc.k_last - 16 - 512 * 16;
-                long long c = std::max<long long>(0, room) / (6ll * tc.kp_max);
-                if (mn) c = c / 64 * 64;
-                int ncols = (int)std::min<long long>(c, 256);
-                ncols = std::min(ncols, 256 / tc.mtiles_max) / 16 * 16;
-                tc.ncols_max = ncols;
-                tc.mn = mn;
-                if (ncols >= 16) break;
-            }
+        for (tc.nstage = 2; tc.nstage >= 1; --tc.nstage) {
+            const long long room = (long long)smem_cap - 1024 - (long long)tc.nstage * kWBlockBytes - 64ll * (e->W | 1) * 4 -
+                                   16ll * tc.n1 - 4ll * tc.k_last - 16 - 512 * 16;
+            const long long c = std::max<long long>(0, room) / (6ll * tc.kp_max);
+            int ncols = (int)std::min<long long>(c, 256 / tc.mtiles_max) / 16 * 16;
+            if (ncols > 128) ncols = ncols / 128 * 128;
+            tc.ncols_max = ncols;
+            if (ncols >= 16) break;
+        }
         // streamed operand (wide layers): two 64-deep operand blocks, so the
         // tile is as wide as TMEM allows; taken when that is wider
         // (the widest tile first, then the most weight stages in flight)

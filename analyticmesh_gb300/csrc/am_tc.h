@@ -28,7 +28,6 @@ struct TcNet {
     int kp_max;                         // largest padded K of any operand
     int mtiles_max;                     // largest number of 128-row tiles of any layer
     int nstage;                         // weight blocks in flight (1 or 2; up to 3 with the streamed operand)
-    int mn;                             // operand layout: 1 MN-major (64-column atoms), 0 K-major
     int n1, k_last;                     // widths of hidden layer 1 and of the last hidden layer
     int streamed;                       // operand in scratch, copied one 64-deep K block at a time (wide layers)
     int mgroups;                        // streamed: a layer's M tiles in this many passes, each with its own
