@@ -345,12 +345,9 @@ __global__ void __launch_bounds__(Cfg<T>::threads, Cfg<T>::ctas) compose_kernel(
     int count;
     chunk_range(ch, head, count);
     if (count <= 0) return;
-    if (tid == 0) {
-        // as few regions per tile as fill the grid: a small wave spreads over every SM
-        plan_counts(plan, ch, net.n_lin - 1, count);
-        int R = min(Cfg<T>::warps, (count + (int)gridDim.x - 1) / (int)gridDim.x);
-        while (R < Cfg<T>::warps && plan_tiles(plan, R) > (int)gridDim.x) ++R;
-        plan_finish(plan, R);
+    // as few regions per tile as fill the grid: a small wave spreads over every SM
+    if (warp == 0) plan_wave(plan, ch, net.n_lin - 1, count, (int)gridDim.x, Cfg<T>::warps, 1);
+    if (tid == 32) {
         ring.abort = 0;
         for (int s = 0; s < Cfg<T>::stages; ++s) {
             umma::mbar_init(ring.full + s, 1);

@@ -363,20 +363,6 @@ __device__ __forceinline__ void bar_main() { asm volatile("bar.sync 2, %0;" ::"r
 // reading consecutive regions' bits hit distinct banks
 __host__ __device__ __forceinline__ int key_stride(int W) { return W | 1; }
 
-// (one thread) tile width of the wave: one tile per resident slot while the
-// wave is small, the widest tile otherwise; the plan's tiles.  Returns the
-// tile's columns.
-__device__ int plan_wave(WavePlan &plan, const ChunkDev &ch, int layers, int count, int slots, int ncols_max, int group)
-{
-    plan_counts(plan, ch, layers, count, group);
-    const int per = (count + slots - 1) / slots;
-    int ncols = (4 * per + 15) / 16 * 16;
-    ncols = ncols < 16 ? 16 : (ncols > ncols_max ? ncols_max : ncols);
-    while (ncols < ncols_max && plan_tiles(plan, ncols / 4) > slots) ncols += 16;
-    plan_finish(plan, ncols / 4);
-    return ncols;
-}
-
 __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net, TcNet tc, RegionsDev reg, ChunkDev ch,
                                                                   float iso, int slots, int *err)
 {
@@ -387,54 +373,51 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
     __shared__ int s_abort; // a pipeline wait ran out (thread 0 or the copy warp)
     __shared__ int s_stop;  // thread 0's view of it, published before a tile barrier: uniform
     __shared__ WavePlan plan;
-    __shared__ int s_ncols;
     __shared__ int4 ri[64]; // the tile's regions (at most 256 columns)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     long long head;
     int count;
     chunk_range(ch, head, count);
     if (count <= 0) return;
-    if (tid == 0) s_ncols = plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max, 1);
-    __syncthreads();
-    const int ncols = s_ncols;
-    const int R = ncols / 4;
-    if ((int)blockIdx.x >= plan.tile0[plan.layers]) return;
-    const int rounds = plan_rounds(plan, (int)gridDim.x);
-    int tmem_cols = 32;
-    while (tmem_cols < 2 * tc.mtiles_max * ncols) tmem_cols <<= 1;
-    const size_t rstride = (size_t)net.ALLP * 4;
     const int KW = key_stride(net.W); // odd: lanes on consecutive regions read distinct banks
-
     uint8_t *base = smem_raw + ((1024u - (umma::smem_addr(smem_raw) & 1023u)) & 1023u);
     XOp X;
-    X.term = op_term_bytes(ncols);
     X.xs = base;
-    uint8_t *ws = base + (size_t)(tc.kp_max / 64) * 3 * X.term;      // nstage weight blocks
+    // (the layout is the widest tile's)
+    uint8_t *ws = base + (size_t)(tc.kp_max / 64) * 3 * op_term_bytes(tc.ncols_max);      // nstage weight blocks
     uint32_t *keys = reinterpret_cast<uint32_t *>(ws + (size_t)tc.nstage * kWBlockBytes); // the tile's bits
     // per CTA, for every tile: linear 0 as (w0, w1, w2, b) per unit and the
     // face-plane weights (the output linear's only row)
     float4 *w0s = reinterpret_cast<float4 *>(keys + (size_t)(tc.ncols_max / 4) * key_stride(net.W));
     float *wls = reinterpret_cast<float *>(w0s + net.nodes[1]);
     float *fsum = reinterpret_cast<float *>(reinterpret_cast<uintptr_t>(wls + net.nodes[net.n_lin - 1] + 3) & ~(uintptr_t)15);
-
     WPipe pp{bars, bars + 2, ws, tc.nstage, err, 0, &s_abort};
-    if (tid == 0) {
-        s_abort = 0;
-        s_stop = 0;
-        for (int b = 0; b < 4; ++b) umma::mbar_init(bars + b, 1);
-        umma::fence_mbar_init();
-    }
-    if (warp == 0) umma::tmem_alloc(&tslot, (uint32_t)tmem_cols);
-    {
+    if (warp == 0) { // one tile per resident slot while the wave is small, the widest tile otherwise
+        plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max / 4, 4);
+        if (lane == 0) {
+            s_abort = 0;
+            s_stop = 0;
+            for (int b = 0; b < 4; ++b) umma::mbar_init(bars + b, 1);
+            umma::fence_mbar_init();
+        }
+    } else {
         const float *W0 = (const float *)net.W0;
         const float *b0 = (const float *)net.bias[0];
-        for (int m = tid; tid < kThreads && m < net.nodes[1]; m += kThreads)
+        for (int m = tid - 32; m < net.nodes[1]; m += kThreads)
             w0s[m] = make_float4(W0[3 * m], W0[3 * m + 1], W0[3 * m + 2], b0[m]);
         const int il = net.n_lin - 1;
         const float *wl = (const float *)net.Wt[il]; // [K][Mp], column 0
-        for (int k = tid; tid < kThreads && k < net.nodes[il]; k += kThreads) wls[k] = wl[(size_t)k * net.Mp[il]];
+        for (int k = tid - 32; k < net.nodes[il]; k += kThreads) wls[k] = wl[(size_t)k * net.Mp[il]];
     }
-    __syncthreads(); // barriers initialised, for the copy warp too
+    __syncthreads(); // the plan; barriers initialised, for the copy warp too
+    const int R = plan.R, ncols = 4 * R;
+    if ((int)blockIdx.x >= plan.tile0[plan.layers]) return;
+    const int rounds = plan_rounds(plan, (int)gridDim.x);
+    int tmem_cols = 32;
+    while (tmem_cols < 2 * tc.mtiles_max * ncols) tmem_cols <<= 1;
+    const size_t rstride = (size_t)net.ALLP * 4;
+    X.term = op_term_bytes(ncols);
+    if (warp == 0) umma::tmem_alloc(&tslot, (uint32_t)tmem_cols); // (read after a tile's barriers)
     if (warp == kThreads / 32) { // the copy warp: the weight blocks of every tile
         if (lane == 0) wp_produce(pp, net, tc, plan, rounds);
         __syncwarp();
@@ -1129,17 +1112,16 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
     __shared__ uint32_t tslot;
     __shared__ int s_abort; // a wait ran out: nothing more is issued, epilogues are skipped
     __shared__ WavePlan plan;
-    __shared__ int s_ncols;
     __shared__ int4 ri[64]; // the tile's regions (at most 256 columns)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     long long head;
     int count;
     chunk_range(ch, head, count);
     if (count <= 0) return;
-    if (tid == 0) s_ncols = plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max, kCluster);
+    // one tile per resident slot while the wave is small, the widest tile otherwise
+    if (warp == 0) plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max / 4, 4, kCluster);
     __syncthreads();
-    const int ncols = s_ncols;
-    const int R = ncols / 4;
+    const int R = plan.R, ncols = 4 * R;
     if ((int)blockIdx.x >= plan.tile0[plan.layers]) return;
     const int rounds = plan_rounds(plan, (int)gridDim.x);
     int tmem_cols = 32;

@@ -89,22 +89,37 @@ __device__ __forceinline__ int plan_tiles(const WavePlan &w, int R)
     for (int c = 0; c < w.layers; ++c) n += plan_class_tiles(w, c, R);
     return n;
 }
-// (one thread) the class counts; then, R chosen, the tiles
-__device__ __forceinline__ void plan_counts(WavePlan &w, const ChunkDev &ch, int layers, int count, int group = 1)
+// (one warp) The wave's plan, and its R: the first of R0, R0 + step, ... whose tiles
+// fit `slots`, at most rmax (at most 32 steps away); R0 is a slot's share of the
+// regions.  The classes' counts, the sizes and the tiles are a lane's each (one
+// thread's loops over them took 1 to 2 us of every wave on GB300).
+__device__ __forceinline__ int plan_wave(WavePlan &w, const ChunkDev &ch, int layers, int count, int slots, int rmax, int step,
+                                         int group = 1)
 {
-    w.group = group;
-    w.layers = ch.order ? layers : 1;
-    for (int c = 0; c < w.layers; ++c) w.cnt[c] = ch.order ? ch.ccount[c] : count;
-}
-__device__ __forceinline__ void plan_finish(WavePlan &w, int R)
-{
-    w.R = R;
-    int n = 0;
-    for (int c = 0; c < w.layers; ++c) {
-        w.tile0[c] = n;
-        n += plan_class_tiles(w, c, R);
+    const int lane = threadIdx.x & 31;
+    const int n = ch.order ? layers : 1;
+    if (lane == 0) {
+        w.group = group;
+        w.layers = n;
     }
-    w.tile0[w.layers] = n;
+    if (lane < n) w.cnt[lane] = ch.order ? ch.ccount[lane] : count;
+    __syncwarp();
+    const int per = (count + slots - 1) / slots, r0 = min(rmax, max((per + step - 1) / step, 1) * step);
+    const int mine = r0 + step * lane;
+    const bool fits = mine >= rmax || plan_tiles(w, mine) <= slots;
+    const int R = min(rmax, r0 + step * (__ffs(__ballot_sync(0xffffffffu, fits)) - 1));
+    int sum = lane < n ? plan_class_tiles(w, lane, R) : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += below;
+    }
+    if (lane == 0) {
+        w.R = R;
+        w.tile0[0] = 0;
+    }
+    if (lane < n) w.tile0[lane + 1] = sum;
+    return R;
 }
 // the tile of round j on CTA b of G, -1 when there is none
 __device__ __forceinline__ int plan_tile(const WavePlan &w, int j, int b, int G)
