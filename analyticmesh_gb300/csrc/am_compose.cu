@@ -329,10 +329,13 @@ __device__ void linear_pass(const NetDev &net, int i, int mb, const Region<T> &g
 }
 
 // Measured on GB300, composition of all 265 K regions of 3-[128]x4-1 in waves of
-// 7 K (parents' rows on both sides): fp32 3.1 ms, fp64 33 ms; a 16-region x
+// 7 K (parents' rows on both sides): fp32 2.7 ms, fp64 28.5 ms; a 16-region x
 // 64-row register tile per CTA over every unit, operand staged behind two block
 // barriers per 32 units, took 6.6 and 71 ms.  8,192 given states, every layer
-// (weights transposed and keys packed in the same call): 131 us against 238.
+// (weights transposed and keys packed in the same call): 112 us against 238.
+// (Two neighbouring units per fma.rn.f32x2 and the operand's columns doubled, 13
+// instructions per active unit instead of 22, measured the same in fp32: the
+// chain of a block -- rows, packing, ring, products -- bounds it.)
 template <typename T>
 __global__ void __launch_bounds__(Cfg<T>::threads, Cfg<T>::ctas) compose_kernel(NetDev net, RegionsDev reg, ChunkDev ch, T iso,
                                                               const int *nonfinite, int *err)
