@@ -131,55 +131,74 @@ __device__ __forceinline__ bool is_winner(const AppendArgs &a, int r, int lane, 
     return (uint32_t)load_slot(a.hs.slots + rec) == ((1u << 31) | (myid & 0x7fffffffu));
 }
 
-// (the whole warp) the winner in slot i of row r becomes region rid
+// (the whole warp) the winners `won` of row r become the regions from rid0 on.  A
+// lane each for their records, so that a row costs one chain of loads whatever
+// its winners; the keys' words by the warp.  (Measured on GB300, frontier phase:
+// with the winners one after the other 0.90 ms for 3-[128]x4-1 and 12.8 for
+// 3-[512]x8-1, this way 0.79 and 11.7.)
 template <typename TS>
-__device__ __forceinline__ void append_one(const AppendArgs &a, int r, int i, long long rid, long long head, int lane)
+__device__ __forceinline__ void append_row(const AppendArgs &a, int r, uint32_t won, long long rid0, long long head, int lane)
 {
-    if (rid >= a.reg.cap) {
-        if (lane == 0) atomicOr(a.err, kErrCapacity);
-        return;
-    }
     const int W = a.net.W;
-    uint32_t *key = a.reg.keys + (size_t)rid * W;
-    TS *mid = (TS *)a.reg.mid + (size_t)rid * 4;
-    uint64_t h;
+    const long long rid = rid0 + __popc(won & ((1u << lane) - 1u));
+    bool mine = (won >> lane) & 1u;
+    if (mine && rid >= a.reg.cap) {
+        atomicOr(a.err, kErrCapacity);
+        mine = false;
+    }
+    const uint32_t writes = __ballot_sync(0xffffffffu, mine);
+    const long long parent = head + r; // (children)
+    const int q = r * 32 + lane;       // the candidate: edge slot or seed
+    int k = -1;
+    TS m[3] = {TS(0), TS(0), TS(0)};
+    uint64_t h = 0;
     if (a.mode == 1) {
-        const int q = r * 32 + i;
-        const uint32_t *sk = a.seed_keys + (size_t)q * W;
-        for (int w = lane; w < W; w += 32) key[w] = sk[w];
-        h = a.seed_hash[q];
-        const TS *pt = (const TS *)a.seed_points + (size_t)q * 3;
-        if (lane < 4) mid[lane] = lane < 3 ? pt[lane] : TS(0);
-        if (lane == 0) {
-            a.reg.start[rid] = -1;
-            a.reg.parent[rid] = -1;
+        if (mine) {
+            h = a.seed_hash[q];
+            const TS *pt = (const TS *)a.seed_points + (size_t)q * 3;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) m[c] = pt[c];
         }
     } else {
-        const long long parent = head + r;
-        const int k = a.reg.edges[(size_t)parent * kVMax + i];
-        const uint32_t *pk = a.reg.keys + (size_t)parent * W;
-        for (int w = lane; w < W; w += 32) key[w] = pk[w] ^ (w == (k >> 5) ? 1u << (k & 31) : 0u);
-        h = flip_hash(a.reg.hash[parent], pk[k >> 5], k);
-        const int n = a.reg.nv[parent];
-        if (lane < 4) {
-            TS m = TS(0);
-            if (lane < 3) {
-                const TS v0 = ((const TS *)a.reg.verts)[((size_t)parent * kVMax + i) * 3 + lane];
-                const TS v1 = ((const TS *)a.reg.verts)[((size_t)parent * kVMax + (i + 1) % n) * 3 + lane];
-                m = (v0 + v1) / TS(2);
-            }
-            mid[lane] = m;
+        const int n = a.reg.nv[parent]; // (a winner is one of the polygon's edges)
+        const uint64_t ph = a.reg.hash[parent];
+        TS v[3] = {TS(0), TS(0), TS(0)};
+        if (lane < n) {
+            k = a.reg.edges[(size_t)parent * kVMax + lane];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] = ((const TS *)a.reg.verts)[((size_t)parent * kVMax + lane) * 3 + c];
         }
-        if (lane == 0) {
-            a.reg.start[rid] = k;
-            a.reg.parent[rid] = (int32_t)parent;
+        const int after = lane + 1 < n ? lane + 1 : 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const TS w = __shfl_sync(0xffffffffu, v[c], after);
+            m[c] = (v[c] + w) / TS(2);
         }
+        if (mine) h = flip_hash(ph, a.reg.keys[(size_t)parent * W + (k >> 5)], k);
     }
-    if (lane == 0) {
+    if (mine) {
+        TS *mid = (TS *)a.reg.mid + (size_t)rid * 4;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) mid[c] = m[c];
+        mid[3] = TS(0);
+        a.reg.start[rid] = k;
+        a.reg.parent[rid] = a.mode == 1 ? -1 : (int32_t)parent;
         a.reg.hash[rid] = h;
         a.reg.nv[rid] = 0;
         a.reg.status[rid] = 0;
-        a.hs.slots[a.ch.rec[r * 32 + i]] = slot_value(fp_of(h), 0, (uint32_t)rid);
+        a.hs.slots[a.ch.rec[q]] = slot_value(fp_of(h), 0, (uint32_t)rid);
+    }
+    for (int w0 = 0; w0 < W; w0 += 32) {
+        const int w = w0 + lane;
+        const uint32_t p = a.mode != 1 && w < W ? a.reg.keys[(size_t)parent * W + w] : 0u;
+        for (uint32_t b = writes; b; b &= b - 1u) {
+            const int i = __ffs(b) - 1;
+            const int ki = __shfl_sync(0xffffffffu, k, i);
+            const long long to = __shfl_sync(0xffffffffu, rid, i);
+            if (w >= W) continue;
+            const uint32_t word = a.mode == 1 ? a.seed_keys[(size_t)(r * 32 + i) * W + w] : p ^ (w == (ki >> 5) ? 1u << (ki & 31) : 0u);
+            a.reg.keys[(size_t)to * W + w] = word;
+        }
     }
 }
 
@@ -210,7 +229,7 @@ __device__ void wave_step(WaveCtl &c, cudaGraphConditionalHandle cond)
 // graph-driven loop, the queue.  The counts carry the append's number, so that
 // nothing has to be cleared between appends.  Measured on GB300 against a count
 // kernel, a write kernel (a thread per winner) and a step kernel, frontier phase:
-// 3-[512]x8-1 17.4 -> 12.6 ms, 3-[256]x6-1 2.5 -> 2.2 ms; with a quarter of the
+// 3-[512]x8-1 17.4 -> 11.7 ms, 3-[256]x6-1 2.5 -> 2.1 ms; with a quarter of the
 // blocks (a warp then walks several rows one after the other) 19.5 and 3.1 ms.
 template <typename TS>
 __global__ void __launch_bounds__(kAppendThreads) append_kernel(AppendArgs a, cudaGraphConditionalHandle cond, int step)
@@ -283,13 +302,8 @@ __global__ void __launch_bounds__(kAppendThreads) append_kernel(AppendArgs a, cu
 #pragma unroll
     for (int w = 0; w < kAppendWarps; ++w) base += s_part[w];
     for (int r = warp; r < n; r += kAppendWarps) {
-        uint32_t b = won[r];
-        long long rid = base + (long long)pre[r];
-        while (b) {
-            const int i = __ffs(b) - 1;
-            b &= b - 1u;
-            append_one<TS>(a, r0 + r, i, rid++, head, lane);
-        }
+        const uint32_t b = won[r];
+        if (b) append_row<TS>(a, r0 + r, b, base + (long long)pre[r], head, lane);
     }
     if (tid == 0) {
         if (ticket == blocks - 1) a.sc->new_tail = base + total;
