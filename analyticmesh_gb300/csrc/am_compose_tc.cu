@@ -437,9 +437,8 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
         const int nreg = tile_nreg(plan, t, cls);
         bar_main(); // the previous tile is done with the keys and the operand
         if (tid < nreg) ri[tid] = tile_region(plan, reg, ch, head, t, cls, tid);
-        bar_main();
-        for (int rr = warp; rr < R; rr += kThreads / 32) { // a region's words together in flight
-            const uint32_t *key = reg.keys + (size_t)(rr < nreg ? head + ri[rr].w : 0) * net.W;
+        for (int rr = warp; rr < R; rr += kThreads / 32) { // (beside it) a region's words together in flight
+            const uint32_t *key = reg.keys + (size_t)(rr < nreg ? head + tile_pos(plan, ch, t, cls, rr) : 0) * net.W;
 #pragma unroll 2
             for (int w = lane; w < net.W; w += 32) keys[rr * KW + w] = rr < nreg ? key[w] : 0u;
         }
@@ -1201,9 +1200,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
             const int nreg = tile_nreg(plan, tile, cls);
             bar_builders(); // the previous tile is done with the keys
             if (tid < nreg) ri[tid] = tile_region(plan, reg, ch, head, tile, cls, tid);
-            bar_builders();
-            for (int rr = warp; rr < R; rr += kSBuild / 32) { // a region's words together in flight
-                const uint32_t *key = reg.keys + (size_t)(rr < nreg ? head + ri[rr].w : 0) * net.W;
+            for (int rr = warp; rr < R; rr += kSBuild / 32) { // (beside it) a region's words together in flight
+                const uint32_t *key = reg.keys + (size_t)(rr < nreg ? head + tile_pos(plan, ch, tile, cls, rr) : 0) * net.W;
 #pragma unroll 4
                 for (int w = lane; w < net.W; w += 32) keys[rr * KW + w] = rr < nreg ? key[w] : 0u;
             }

@@ -135,14 +135,19 @@ __device__ __forceinline__ int plan_class(const WavePlan &w, int t)
     return c + 1;
 }
 
+// wave position of region r of tile t, class c
+__device__ __forceinline__ int tile_pos(const WavePlan &w, const ChunkDev &ch, int t, int c, int r)
+{
+    const int idx = (t - w.tile0[c - 1]) * w.R + r;
+    return ch.order ? ch.order[(size_t)(c - 1) * ch.order_cap + idx] : idx;
+}
 // One region of a tile: x its own rows' slot, y its parent's, z the plane it
 // was entered through (its row changes sign between the two; -1 for class 1),
 // w its wave position.
 __device__ __forceinline__ int4 tile_region(const WavePlan &w, const RegionsDev &reg, const ChunkDev &ch, long long head,
                                             int t, int c, int r)
 {
-    const int idx = (t - w.tile0[c - 1]) * w.R + r;
-    const int rl = ch.order ? ch.order[(size_t)(c - 1) * ch.order_cap + idx] : idx;
+    const int rl = tile_pos(w, ch, t, c, r);
     int4 o;
     o.x = (int)row_slot(ch, head, rl);
     o.y = o.x;
