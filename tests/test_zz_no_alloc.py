@@ -147,3 +147,33 @@ def test_noalloc_rejects_misaligned_outputs():
     # aligned: accepted
     assert L.am_compose_rows_noalloc(*args, C.c_void_p(buf.data_ptr()), C.c_void_p(eq.data_ptr()), None) == 0
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_noalloc_non_finite_weights_meet_inactive_units(bad):
+    """The composition walks active units only; with a weight that is not finite
+    every unit counts, as in a dense product: non-finite entries where a dense
+    FP64 composition has them, the same values elsewhere."""
+    model = wl.geometric([24, 40], 3, perturb=0.05)
+    net = wl.net_arrays(model)
+    W = [np.array(w, np.float64) for w in net.W]
+    W[1][5, 7] = bad  # unit 5 of the second layer sees unit 7 of the first
+    dev = torch.device("cuda")
+    Ws = [torch.tensor(w, dtype=torch.float32, device=dev).contiguous() for w in W]
+    Bs = [torch.tensor(b, dtype=torch.float32, device=dev).contiguous() for b in net.b]
+    states = torch.randint(0, 2, (70, 64), dtype=torch.uint8, generator=torch.Generator().manual_seed(1)).to(dev)
+    rows = torch.zeros((70, 64, 4), dtype=torch.float32, device=dev)
+    eq = torch.zeros((70, 4), dtype=torch.float32, device=dev)
+    assert _call(net.nodes, Ws, Bs, states, 0.0, rows, eq) == 0
+    torch.cuda.synchronize()
+    s = states.cpu().numpy().astype(np.float64)
+    A1 = np.broadcast_to(np.concatenate([W[0], np.asarray(net.b[0])[:, None]], 1), (70, 24, 4))
+    with np.errstate(invalid="ignore"):
+        A2 = np.einsum("mk,rkc->rmc", W[1], A1 * s[:, :24, None])
+        A2[:, :, 3] += net.b[1]
+        ref = np.concatenate([A1, A2], 1) * (1 - 2 * s)[:, :, None]
+    got = rows.double().cpu().numpy()
+    assert np.array_equal(np.isfinite(got), np.isfinite(ref))
+    ok = np.isfinite(ref)
+    np.testing.assert_allclose(got[ok], ref[ok], rtol=1e-5, atol=1e-5 * np.abs(ref[ok]).max())
