@@ -279,23 +279,12 @@ __device__ void wp_produce(WPipe &p, const NetDev &net, const TcNet &tc, const W
 __device__ __forceinline__ void issue_step(uint32_t d_main, uint32_t d_corr, uint64_t ad, uint64_t xd, uint64_t xu,
                                            uint32_t idesc, bool fresh)
 {
-#ifdef NOCOLL
-#define MMA0 mma_bf16_a<0>
-#define MMA1 mma_bf16_a<0>
-#define MMA2 mma_bf16_a<0>
-#define MMA3 mma_bf16_a<0>
-#else
-#define MMA0 mma_bf16_a<0>
-#define MMA1 mma_bf16_a<1>
-#define MMA2 mma_bf16_a<2>
-#define MMA3 mma_bf16_a<3>
-#endif
-    umma::MMA1(d_main, ad, xd, idesc, fresh ? 0u : 1u);
-    umma::MMA2(d_corr, ad, xd + xu, idesc, fresh ? 0u : 1u);
-    umma::MMA3(d_corr, ad, xd + 2 * xu, idesc, 1u);
-    umma::MMA1(d_corr, ad + 1024u, xd, idesc, 1u);
-    umma::MMA3(d_corr, ad + 1024u, xd + xu, idesc, 1u);
-    umma::MMA0(d_corr, ad + 2048u, xd, idesc, 1u);
+    umma::mma_bf16_a<1>(d_main, ad, xd, idesc, fresh ? 0u : 1u);
+    umma::mma_bf16_a<2>(d_corr, ad, xd + xu, idesc, fresh ? 0u : 1u);
+    umma::mma_bf16_a<3>(d_corr, ad, xd + 2 * xu, idesc, 1u);
+    umma::mma_bf16_a<1>(d_corr, ad + 1024u, xd, idesc, 1u);
+    umma::mma_bf16_a<3>(d_corr, ad + 1024u, xd + xu, idesc, 1u);
+    umma::mma_bf16_a<0>(d_corr, ad + 2048u, xd, idesc, 1u);
 }
 
 // (warp 0, one elected lane issuing: see issue_streamed) D[mt] (+)= M . X over all
@@ -736,7 +725,7 @@ __device__ __forceinline__ int pass_group(int b, int n, bool two)
     return two && ((b == 0 && n >= 2) || (b == n - 2 && n >= 4)) ? 2 : 1;
 }
 
-__device__ __forceinline__ void bar_builders() { asm volatile("bar.sync 1, %0;" ::"r"(kSBuild) : "memory"); }
+__device__ __forceinline__ void bar_rows() { asm volatile("bar.sync 1, %0;" ::"r"(kSBuild) : "memory"); }
 
 // Bounded wait of the streamed kernel: false at once when the CTA is
 // aborting, and false -- with the error bit kErrWait and the abort flag set --
@@ -1198,14 +1187,14 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
             const int cls = plan_class(plan, tile);
             const int jend = cls > 1 ? net.hoff[cls + 1] : 0; // rows before this are in the parent's slot
             const int nreg = tile_nreg(plan, tile, cls);
-            bar_builders(); // the previous tile is done with the keys
+            bar_rows(); // the previous tile is done with the keys
             if (tid < nreg) ri[tid] = tile_region(plan, reg, ch, head, tile, cls, tid);
             for (int rr = warp; rr < R; rr += kSBuild / 32) { // (beside it) a region's words together in flight
                 const uint32_t *key = reg.keys + (size_t)(rr < nreg ? head + tile_pos(plan, ch, tile, cls, rr) : 0) * net.W;
 #pragma unroll 4
                 for (int w = lane; w < net.W; w += 32) keys[rr * KW + w] = rr < nreg ? key[w] : 0u;
             }
-            bar_builders();
+            bar_rows();
             // class 1: hidden layer 1 = linear 0 rows (sign-flipped); the extra constraints
             const int n1 = net.nodes[1];
             for (int rr = warp; cls == 1 && rr < nreg; rr += kSBuild / 32)
@@ -1222,7 +1211,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
                 st4<float>(cons + (size_t)(uint32_t)ri[rr].x * rstride + (size_t)(net.N + e) * 4,
                            make_float4(we[3 * e], we[3 * e + 1], we[3 * e + 2], be[e]));
             }
-            bar_builders(); // layer-1 rows written by every builder
+            bar_rows(); // layer-1 rows written by every row warp
 
             // The operand of the layers the parents computed:
             // X[4r + c][k] = s_k(r) ? -C[r][k][c] : 0, block by block.  A warp
@@ -1386,7 +1375,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
                         mt0 += mper;
                     }
                 }
-                bar_builders(); // rows of hidden layer i + 1 written by every row warp
+                bar_rows(); // rows of hidden layer i + 1 written by every row warp
             }
 
             // face plane: w_eq = W_L . X_L, X_L = -C of the last hidden layer
@@ -1420,7 +1409,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
                         }
                     }
                     reinterpret_cast<float4 *>(fsum)[fw * 32 + fr] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                    bar_builders();
+                    bar_rows();
                     if (live && tid < 128) {
                         const int rr = tid >> 2, c = tid & 3, rg = r0 + rr;
                         float a = 0.f;
@@ -1449,7 +1438,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
                             ((float *)ch.eq)[(size_t)ri[rg].w * 4 + c] = a;
                         }
                     }
-                    bar_builders();
+                    bar_rows();
                 }
             }
         }
