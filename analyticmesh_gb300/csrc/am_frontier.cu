@@ -240,8 +240,15 @@ __global__ void __launch_bounds__(kAppendThreads) append_kernel(AppendArgs a, cu
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     long long head = 0;
     int rows;
-    if (a.mode == 1) rows = (a.n_items + 31) / 32;
-    else chunk_range(a.ch, head, rows);
+    if (a.mode == 1) {
+        rows = (a.n_items + 31) / 32;
+    } else if (a.ch.ctl) { // (not head and count: wave_step moves them while blocks are still to come)
+        head = a.ch.ctl->append_head;
+        rows = a.ch.ctl->append_count;
+    } else {
+        head = a.ch.head;
+        rows = a.ch.count;
+    }
     // (a row per warp at least; at least one block, for the step)
     const int blocks = max(1, min((int)gridDim.x, (rows + kAppendWarps - 1) / kAppendWarps));
     if ((int)blockIdx.x >= blocks) return;

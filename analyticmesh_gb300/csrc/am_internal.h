@@ -89,6 +89,13 @@ struct WaveCtl {
     long long stop_tail; // stop after the wave that takes tail past this (a region limit)
     long long rows_from; // regions before this have no rows in the ring (it was reallocated)
     int ccount[kMaxLayers]; // regions of the wave per class (see ChunkDev)
+    // the range of the wave whose children the append takes: a copy of head and
+    // count that the wave's polygon kernel makes.  The append's last block moves head
+    // and count on while other blocks of its grid may not have started yet; those
+    // read this copy, which nothing writes before the append has ended.
+    long long append_head;
+    int append_count;
+    int pad1;
 };
 
 // the control block's device / pinned allocation: WaveCtl, then the run's

@@ -1378,6 +1378,10 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
     long long head;
     int count;
     chunk_range(ch, head, count);
+    if (ch.ctl && blockIdx.x == 0 && threadIdx.x == 0) { // the wave's range for the append
+        ch.ctl->append_head = head;
+        ch.ctl->append_count = count;
+    }
     // a region per warp: by launch position, or (fixed grid of the
     // graph-driven loop) from the wave's work counter
     long long rl_next = (long long)blockIdx.x * kFaceWarps + wib;

@@ -1,0 +1,35 @@
+"""The append while other work holds the SMs: its blocks then start late, some
+after the block that finishes the wave has moved the queue on.  Every network of a
+batch of small ones beside wide ones gives the regions it gives alone, in the same
+order, on every repeat and on engines that are used again."""
+import numpy as np
+import pytest
+
+from analyticmesh_gb300 import engine, workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("form", ["mixed", "float32"])
+def test_small_networks_beside_wide_ones_repeat_their_own_regions(form):
+    models = [wl.geometric([24 + 8 * (i % 5)] * (2 + i % 3), 200 + i, perturb=0.01) for i in range(10)]
+    models[3:3] = [wl.sphere()]
+    models.append(wl.geometric([128] * 4, 222, perturb=0.01))
+    nets = [wl.net_arrays(m) for m in models]
+    seeds = [wl.seeds_for(m, init_num=64, seed=30 + i) for i, m in enumerate(models)]
+    alone = []
+    for net, (st, pt) in zip(nets, seeds):
+        e = engine.march(net, st, pt, form)
+        alone.append(e.regions())
+        e.close()
+    assert all(r.num > 50 for r in alone)
+    engines = [engine.Engine(form, n.nodes, n.arc_table, n.num_extra) for n in nets]
+    for repeat in range(4):
+        engine.run_batch(engines, nets, [s[0] for s in seeds], [s[1] for s in seeds])
+        for i, (e, want) in enumerate(zip(engines, alone)):
+            got = e.regions()
+            assert got.num == want.num, (repeat, i)
+            for x, y in ((got.bits, want.bits), (got.start, want.start), (got.nverts, want.nverts)):
+                assert np.array_equal(x, y), (repeat, i)
+    for e in engines:
+        e.close()
