@@ -15,6 +15,7 @@
 
 #include "am_device.cuh"
 #include "am_internal.h"
+#include "am_rules.h"
 
 namespace am {
 
@@ -99,8 +100,7 @@ __global__ void seed_insert_kernel(const uint32_t *keys, const uint64_t *hash, i
     rec[s] = r;
 }
 
-constexpr int kAppendThreads = 256;
-constexpr int kAppendWarps = kAppendThreads / 32;
+constexpr int kAppendThreads = 32 * kAppendWarps;
 constexpr int kSpinIters = 1 << 24; // bound of the wait for an earlier block's count
 
 struct AppendArgs {
@@ -249,10 +249,9 @@ __global__ void __launch_bounds__(kAppendThreads) append_kernel(AppendArgs a, cu
         head = a.ch.head;
         rows = a.ch.count;
     }
-    // (a row per warp at least; at least one block, for the step)
-    const int blocks = max(1, min((int)gridDim.x, (rows + kAppendWarps - 1) / kAppendWarps));
+    const int blocks = append_blocks_used(rows, (int)gridDim.x);
     if ((int)blockIdx.x >= blocks) return;
-    const int span = (rows + blocks - 1) / blocks;
+    const int span = append_span(rows, (int)gridDim.x);
     if (tid == 0) s_ticket = (int)atomicAdd(&a.sc->ticket, 1u);
     __syncthreads();
     const int ticket = s_ticket;
@@ -432,14 +431,7 @@ void launch_seed_insert(const uint32_t *keys, const uint64_t *hash, int S, int W
     seed_insert_kernel<<<(S + 127) / 128, 128, 0, st>>>(keys, hash, S, W, hs, rec, d_err);
 }
 
-// most rows per block: their winners and prefixes in shared memory
-constexpr int kSpanMax = 4096;
-
-int append_blocks(int rows_max)
-{
-    return std::max(std::min((rows_max + kAppendWarps - 1) / kAppendWarps, 8 * device_sms()),
-                    (rows_max + kSpanMax - 1) / kSpanMax);
-}
+int append_blocks(int rows_max) { return append_grid(rows_max, device_sms()); }
 
 void launch_append(int mode, int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch,
                    const HashDev &hs, const uint32_t *seed_keys, const uint64_t *seed_hash, const void *seed_points,
@@ -467,7 +459,7 @@ void launch_append(int mode, int prec, const NetDev &net, const RegionsDev &reg,
         cudaMemcpyAsync(d_err, &e, sizeof(int), cudaMemcpyHostToDevice, st);
         return;
     }
-    const size_t smem = sizeof(uint32_t) * 2 * (size_t)((rows + nb - 1) / nb);
+    const size_t smem = sizeof(uint32_t) * 2 * (size_t)append_span_room(rows, nb);
     const cudaGraphConditionalHandle h = cond ? *cond : cudaGraphConditionalHandle{};
     if (prec == kFloat32)
         append_kernel<float><<<nb, kAppendThreads, smem, st>>>(a, h, cond ? 1 : 0);

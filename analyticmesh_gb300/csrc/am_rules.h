@@ -1,0 +1,47 @@
+// am_rules.h -- rules of sizes and of the host path as plain functions, without CUDA,
+// so that they can be checked over their whole range on the CPU.
+#pragma once
+
+#ifdef __CUDACC__
+#define AM_RULE __host__ __device__ inline
+#else
+#define AM_RULE inline
+#endif
+
+namespace am {
+
+// ---------------------------------------------------------------- append
+constexpr int kAppendWarps = 8;    // per block; a row is a warp's
+constexpr int kAppendSpanMax = 4096; // most rows per block: their winners and prefixes in shared memory
+
+// blocks of the grid for at most rows_max rows
+AM_RULE int append_grid(int rows_max, int sms)
+{
+    const int fill = (rows_max + kAppendWarps - 1) / kAppendWarps, most = 8 * sms;
+    const int least = (rows_max + kAppendSpanMax - 1) / kAppendSpanMax;
+    const int n = fill < most ? fill : most;
+    return n > least ? n : least;
+}
+// what a wave of `rows` rows makes of it: a row per warp at least, one block at least
+// (for the step), `span` rows per block
+AM_RULE int append_blocks_used(int rows, int grid)
+{
+    const int fill = (rows + kAppendWarps - 1) / kAppendWarps;
+    const int n = fill < grid ? fill : grid;
+    return n > 1 ? n : 1;
+}
+AM_RULE int append_span(int rows, int grid)
+{
+    const int blocks = append_blocks_used(rows, grid);
+    return (rows + blocks - 1) / blocks;
+}
+// the largest span of any wave of at most rows_max rows: while the grid is not full a
+// span has up to kAppendWarps rows, whatever rows_max / grid is (rows_max 9: two
+// blocks, five rows each, but eight rows are one block's)
+AM_RULE int append_span_room(int rows_max, int grid)
+{
+    const int full = (rows_max + grid - 1) / grid;
+    return full > kAppendWarps ? full : kAppendWarps;
+}
+
+} // namespace am

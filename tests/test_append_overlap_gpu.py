@@ -33,3 +33,20 @@ def test_small_networks_beside_wide_ones_repeat_their_own_regions(form):
                 assert np.array_equal(x, y), (repeat, i)
     for e in engines:
         e.close()
+
+
+@pytest.mark.parametrize("chunk", [9, 17, 48])
+def test_waves_shorter_than_a_small_largest_wave(chunk):
+    """Graph-driven waves of every length up to a largest wave of a few rows."""
+    m = wl.geometric([40, 40], 7, perturb=0.02)
+    net = wl.net_arrays(m)
+    st, pt = wl.seeds_for(m, init_num=400, seed=3)
+    out = []
+    for c in (None, chunk):
+        e = engine.march(net, st[:8], pt[:8], "float64", chunk=c)
+        out.append(e.regions())
+        e.close()
+    a, b = out
+    assert a.num > 200
+    for x, y in ((a.bits, b.bits), (a.start, b.start), (a.nverts, b.nverts)):
+        assert np.array_equal(x, y)
