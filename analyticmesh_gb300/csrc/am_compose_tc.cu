@@ -653,11 +653,6 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
 constexpr int kSBuild = 512;            // threads of the row warps (16)
 constexpr int kSThreads = kSBuild + 96; // + the issuing warp and the weight- and operand-copy warps
 constexpr int kSFaceSumBytes = kSBuild * 16;
-// CTAs of a cluster work on tiles of the same class in step and share the weight
-// stream: each copies its part of a block into the shared memory of all of them
-// (multicast), so that a block leaves the L2 once per cluster.
-constexpr int kCluster = 2;
-constexpr uint16_t kClusterMask = (1u << kCluster) - 1u;
 
 __device__ __forceinline__ int jobs_of(const NetDev &net, int i)
 {
@@ -764,7 +759,6 @@ __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws
                                  int half, const WavePlan &plan, int rounds, int *err, volatile int *abort)
 {
     const int nst = tc.nstage;
-    const size_t part_off = (size_t)umma::cluster_rank() * (kWBlockBytes / kCluster); // this CTA's part of a block
     int h = 0;
     int ps = 0;        // stage of block h (h % nst) ...
     uint32_t pph = 0u; // ... and (h / nst) & 1, kept incrementally
@@ -798,9 +792,8 @@ __device__ void produce_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws
                                 if (h >= nst && !swait(wdone + s, ph ^ 1u, err, abort)) continue;
                                 if (*abort) continue;
                                 umma::mbar_expect_tx(wfull + s, (uint32_t)kWBlockBytes);
-                                umma::bulk_g2s_mc(ws + (size_t)s * kWBlockBytes + part_off,
-                                                  m.blocks + (size_t)(mt * kblocks + kb) * kWBlockBytes + part_off,
-                                                  (uint32_t)kWBlockBytes / kCluster, wfull + s, kClusterMask);
+                                umma::bulk_g2s(ws + (size_t)s * kWBlockBytes, m.blocks + (size_t)(mt * kblocks + kb) * kWBlockBytes,
+                                               (uint32_t)kWBlockBytes, wfull + s);
                                 last[s] = h;
                             }
                             if (++kb == kblocks) {
@@ -985,7 +978,7 @@ __device__ void issue_streamed(const NetDev &net, const TcNet &tc, uint8_t *ws, 
         if (umma::elect()) {
             if (go) {
                 issue_step(d_main, d_corr, ad + 6u, xd + 3u * xj, xu, idesc, false);
-                umma::commit_mc(wbar, kClusterMask); // the producers may refill the stage
+                umma::commit(wbar); // the copy warp may refill the stage
             }
             if (xlast) umma::commit(xbar); // the operand stage is free once these complete
             if (hlast) umma::commit(abar); // the half's accumulators are complete
@@ -1090,7 +1083,7 @@ __device__ void copy_operand(const NetDev &net, const TcNet &tc, uint8_t *xs0, u
     if (last1 >= 0) umma::mbar_wait(xfull + 1, (uint32_t)(last1 >> 1) & 1u, kWaitIters);
 }
 
-__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, TcNet tc, RegionsDev reg, ChunkDev ch,
+__global__ void __launch_bounds__(kSThreads, 1) compose_tcs_kernel(NetDev net, TcNet tc, RegionsDev reg, ChunkDev ch,
                                                                     float iso, int slots, int *err)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -1107,7 +1100,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
     chunk_range(ch, head, count);
     if (count <= 0) return;
     // one tile per resident slot while the wave is small, the widest tile otherwise
-    if (warp == 0) plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max / 4, 4, kCluster);
+    if (warp == 0) plan_wave(plan, ch, net.n_lin - 1, count, slots, tc.ncols_max / 4, 4);
     __syncthreads();
     const int R = plan.R, ncols = 4 * R;
     if ((int)blockIdx.x >= plan.tile0[plan.layers]) return;
@@ -1137,7 +1130,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
         s_abort = 0;
         for (int b = 0; b < 3; ++b) {
             umma::mbar_init(wfull + b, 1);
-            umma::mbar_init(wdone + b, kCluster); // every CTA's products are done with the stage
+            umma::mbar_init(wdone + b, 1);
         }
         umma::mbar_init(xfull, 1);
         umma::mbar_init(xfull + 1, 1);
@@ -1162,7 +1155,6 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
     }
     umma::fence_before();
     __syncthreads();
-    umma::cluster_sync(); // the other CTAs' barriers are initialised
     umma::fence_after();
     const uint32_t tmem = tslot;
 
@@ -1445,7 +1437,6 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSThreads, 1)
     }
     umma::fence_before();
     __syncthreads();
-    umma::cluster_sync(); // no copy or arrival reaches a CTA that has left
     if (warp == 0) umma::tmem_dealloc(tslot, (uint32_t)tmem_cols);
 }
 
@@ -1506,7 +1497,7 @@ void launch_compose_tc(const NetDev &net, const TcNet &tc, const RegionsDev &reg
     const int slots = sms; // one resident tile per SM, the wave's tiles strided over them
     if (tc.streamed) {
         cudaFuncSetAttribute(compose_tcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        const int grid = std::min(slots, tc.xctas) / kCluster * kCluster;
+        const int grid = std::min(slots, tc.xctas);
         compose_tcs_kernel<<<grid, kSThreads, smem, st>>>(net, tc, reg, ch, (float)iso, grid, d_err);
         return;
     }

@@ -75,14 +75,9 @@ struct WavePlan {
     int cnt[kMaxLayers];        // regions per class
     int tile0[kMaxLayers + 1];  // first tile of each class
     int R, layers;
-    int group;                  // a class's tiles are a multiple of this (the CTAs of a cluster
-};                              // take tiles of one class; a tile may then hold no region)
+};
 
-__device__ __forceinline__ int plan_class_tiles(const WavePlan &w, int c, int R)
-{
-    const int n = (w.cnt[c] + R - 1) / R;
-    return (n + w.group - 1) / w.group * w.group;
-}
+__device__ __forceinline__ int plan_class_tiles(const WavePlan &w, int c, int R) { return (w.cnt[c] + R - 1) / R; }
 __device__ __forceinline__ int plan_tiles(const WavePlan &w, int R)
 {
     int n = 0;
@@ -93,15 +88,11 @@ __device__ __forceinline__ int plan_tiles(const WavePlan &w, int R)
 // fit `slots`, at most rmax (at most 32 steps away); R0 is a slot's share of the
 // regions.  The classes' counts, the sizes and the tiles are a lane's each (one
 // thread's loops over them took 1 to 2 us of every wave on GB300).
-__device__ __forceinline__ int plan_wave(WavePlan &w, const ChunkDev &ch, int layers, int count, int slots, int rmax, int step,
-                                         int group = 1)
+__device__ __forceinline__ int plan_wave(WavePlan &w, const ChunkDev &ch, int layers, int count, int slots, int rmax, int step)
 {
     const int lane = threadIdx.x & 31;
     const int n = ch.order ? layers : 1;
-    if (lane == 0) {
-        w.group = group;
-        w.layers = n;
-    }
+    if (lane == 0) w.layers = n;
     if (lane < n) w.cnt[lane] = ch.order ? ch.ccount[lane] : count;
     __syncwarp();
     const int per = (count + slots - 1) / slots, r0 = min(rmax, max((per + step - 1) / step, 1) * step);
@@ -161,7 +152,7 @@ __device__ __forceinline__ int4 tile_region(const WavePlan &w, const RegionsDev 
 }
 __device__ __forceinline__ int tile_nreg(const WavePlan &w, int t, int c)
 {
-    return max(0, min(w.R, w.cnt[c - 1] - (t - w.tile0[c - 1]) * w.R));
+    return min(w.R, w.cnt[c - 1] - (t - w.tile0[c - 1]) * w.R);
 }
 // a region's constraint row: the rows before jend from its parent's slot
 // (rewritten by no region of this wave), the plane it was entered through with

@@ -865,10 +865,9 @@ void run_begin(am_engine *e, const RunArgs &a)
             }
             tc.xcta = (two[0] + two[1] + off + 1023) / 1024 * 1024;
             tc.xctas = device_sms();
-            for (cudaError_t rc; (rc = e->tc_x.reserve(tc.xcta * (size_t)tc.xctas)) != cudaSuccess;
-                 tc.xctas = std::max(2, tc.xctas / 4 * 2)) {
+            for (cudaError_t rc; (rc = e->tc_x.reserve(tc.xcta * (size_t)tc.xctas)) != cudaSuccess; tc.xctas /= 2) {
                 cudaGetLastError();
-                if (tc.xctas <= 2) AM_CUDA(rc);
+                if (tc.xctas <= 1) AM_CUDA(rc);
             }
             tc.xbuf = e->tc_x.as<uint8_t>();
         }
