@@ -23,6 +23,7 @@
 #include "../../include/analyticmesh_gb300.h"
 #include "am_internal.h"
 #include "am_mesh.h"
+#include "am_rules.h"
 #include "am_tc.h"
 
 using namespace am;
@@ -164,6 +165,19 @@ bool is_device_ptr(const void *p)
         return false;
     }
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+}
+
+// a caller's array of `element`-byte values that kernels on this device may read where it is
+bool in_place(const void *p, size_t element)
+{
+    cudaPointerAttributes a;
+    int dev = 0;
+    if (!p || cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const MemoryType type = a.type == cudaMemoryTypeDevice ? kMemDevice : (a.type == cudaMemoryTypeManaged ? kMemManaged : kMemHost);
+    return read_in_place(type, a.device, dev, (uint64_t)(uintptr_t)p, (int)element);
 }
 
 // copy n bytes from a host or device pointer to a device buffer
@@ -678,7 +692,8 @@ void run_begin(am_engine *e, const RunArgs &a)
     net.hoff[1] = 0;
     for (int h = 1; h < e->n_lin; ++h) net.hoff[h + 1] = net.hoff[h] + e->nodes[h];
     // The parameters go straight from the caller's device memory into the
-    // engine's layouts; those in host memory by way of one staging buffer.
+    // engine's layouts; those that kernels cannot read where they are (read_in_place)
+    // by way of one staging buffer.
     AM_CUDA(cudaMemsetAsync(e->d_err.p, 0, sizeof(int), st));
     size_t stage_bytes = 0, stage_used = 0;
     auto staged = [](size_t n) { return (n + 255) / 256 * 256; };
@@ -690,11 +705,11 @@ void run_begin(am_engine *e, const RunArgs &a)
         stage_bytes += staged(tc * (size_t)std::max(arc_tm_shapes[2 * t], 0) * (size_t)std::max(arc_tm_shapes[2 * t + 1], 0));
     stage_bytes += staged(tc * 3 * (size_t)e->E) + staged(tc * (size_t)e->E);
     auto on_device = [&](const void *src, size_t n) -> const void * {
-        if (is_device_ptr(src)) return src;
+        if (in_place(src, tc)) return src;
         AM_CUDA(e->scratch.reserve(stage_bytes));
         char *d = e->scratch.as<char>() + stage_used;
         stage_used += staged(n);
-        AM_CUDA(cudaMemcpyAsync(d, src, n, cudaMemcpyHostToDevice, st));
+        AM_CUDA(cudaMemcpyAsync(d, src, n, is_device_ptr(src) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
         return d;
     };
     LoadList load;
@@ -879,13 +894,13 @@ void run_begin(am_engine *e, const RunArgs &a)
 
     // ---------------------------------------------------------- seeds
     const int S = num_points;
-    // (states and points in device memory are read where they are)
+    // (states and points on this device are read where they are)
     const void *dstates = states, *dpoints = points;
-    if (!is_device_ptr(states)) {
+    if (!in_place(states, 1)) {
         upload(e->s_states, states, (size_t)S * e->N, st);
         dstates = e->s_states.p;
     }
-    if (!is_device_ptr(points)) {
+    if (!in_place(points, tc)) {
         upload(e->s_raw, points, tc * 3 * (size_t)S, st);
         dpoints = e->s_raw.p;
     }

@@ -2,6 +2,8 @@
 // so that they can be checked over their whole range on the CPU.
 #pragma once
 
+#include <cstdint>
+
 #ifdef __CUDACC__
 #define AM_RULE __host__ __device__ inline
 #else
@@ -9,6 +11,17 @@
 #endif
 
 namespace am {
+
+// ---------------------------------------------------------------- callers' memory
+// May kernels on device `current` read a caller's array of `element`-byte values where
+// it is?  Managed memory and memory of the same device, aligned to its elements; all
+// else -- host memory, another device's memory (there need be no peer mapping), an
+// odd address (a load that is not aligned faults) -- is copied to the device first.
+enum MemoryType : int { kMemHost = 0, kMemDevice = 1, kMemManaged = 2 };
+AM_RULE bool read_in_place(MemoryType type, int device, int current, uint64_t address, int element)
+{
+    return (type == kMemManaged || (type == kMemDevice && device == current)) && address % (uint64_t)element == 0;
+}
 
 // ---------------------------------------------------------------- append
 constexpr int kAppendWarps = 8;    // per block; a row is a warp's
