@@ -383,6 +383,7 @@ struct am_engine {
     void ensure_chunk(int count)
     {
         if (count <= chunk_cap) return;
+        chunk_cap = 0; // (should one of the allocations fail, none is taken for there)
         if (classes()) {
             AM_CUDA(order.alloc(sizeof(int32_t) * (size_t)(n_lin - 1) * count, st));
             AM_CUDA(split.alloc(sizeof(int32_t) * (size_t)count, st));
@@ -1795,6 +1796,8 @@ int am_region_rows(am_engine *e, int64_t first, int count, double *rows, double 
         if (count == 0) return;
         e->ensure_chunk(count);
         if (count > e->ring) {
+            e->ring = 0; // (should the allocation fail)
+            e->ring_target = 0;
             AM_CUDA(e->cons.alloc(e->tc * 4 * (size_t)e->ALLP * (size_t)count, st));
             e->ring = count;
         }
