@@ -327,7 +327,7 @@ struct am_engine {
     {
         drop_graph();
         for (DevBuf *b : {&keys, &hash, &mid, &start, &parent, &reach, &nv, &status, &verts, &edges, &table, &cons, &eq, &rec,
-                          &blocksum, &order, &split})
+                          &blocksum, &order, &split, &tc_x})
             b->reset();
         ring = 0;
         ring_target = 0;
@@ -409,18 +409,13 @@ struct am_engine {
     // a network with no layer product has nothing to take from a parent
     bool classes() const { return n_lin >= 3; }
 
-    // the ring of constraint rows: a wave's slots and the history in which
-    // its regions find their parents.  A parent is at most about one level of
-    // the breadth-first queue away, and a level held 28 to 39 regions per
-    // hidden unit on the benchmark networks (N = 512 .. 4,096): 48 N, at most
-    // an eighth of the free memory.  A batch member's ring grows with its
-    // waves: two waves, which always reach the parents while a wave holds a
-    // whole level.  Slots never hold less than a wave.
+    // the ring of constraint rows (ring_slots): what goes beyond a wave takes at most
+    // an eighth of the free memory.  Slots never hold less than a wave.
     void ensure_ring(int wave, long long head)
     {
         const size_t per = tc * 4 * (size_t)ALLP;
         long long target = wave;
-        if (classes() && !ring_min) target = run.lean ? 2ll * wave : std::max(run.chunk, wave) + 48ll * N;
+        if (classes() && !ring_min) target = ring_slots(wave, run.chunk, N, run.lean || chunk_opt > 0);
         if (wave <= ring && target <= ring_target) return;
         long long want = target;
         if (want > wave) {
@@ -460,12 +455,41 @@ struct am_engine {
         }
         return ch;
     }
+    // the rows' ring goes back to the device (at once, inside a batch too)
+    void give_back_rows()
+    {
+        cudaGetLastError();
+        const bool direct = cons.p && !cons.pooled;
+        void *p = cons.p;
+        if (direct) {
+            cons.p = nullptr;
+            cons.bytes = 0;
+        }
+        cons.reset();
+        if (st) cudaStreamSynchronize(st);
+        if (direct) cudaFree(p);
+        ring = 0;
+        ring_target = 0;
+    }
+    // allocations `f` (safe to repeat); where memory runs out, the ring, which is the
+    // largest buffer that nothing but a marching needs, is given back first
+    template <class F>
+    void with_rows_memory(F &&f)
+    {
+        try {
+            f();
+        } catch (const Failure &x) {
+            if (x.code != AM_ERR_OUT_OF_MEMORY || !cons.p) throw;
+            give_back_rows();
+            f();
+        }
+    }
     // room for a wave of `count` more regions' children; where memory runs
     // out, the ring gives its history back first
     void ensure_wave(int wave, long long head, long long tail, int count, bool fit_cap)
     {
-        ensure_chunk(wave);
         auto stores = [&] {
+            ensure_chunk(wave);
             ensure_regions(tail + (long long)count * kVMax);
             ensure_table(std::max<long long>(tail + (long long)count * kVMax, fit_cap ? cap : 0), true);
         };
@@ -473,10 +497,7 @@ struct am_engine {
             stores();
         } catch (const Failure &x) {
             if (x.code != AM_ERR_OUT_OF_MEMORY || ring <= wave) throw;
-            cudaGetLastError();
-            cons.reset();
-            ring = 0;
-            ring_target = 0;
+            give_back_rows();
             ring_min = true;
             stores();
         }
@@ -923,13 +944,16 @@ void run_begin(am_engine *e, const RunArgs &a)
     const int chunk = e->default_chunk();
     e->ring_min = false;
     e->rows_from = 0;
-    e->ensure_chunk(std::min(chunk, std::max(S, 1024)));
+    if (e->chunk_opt > 0 && e->ring > ring_slots(chunk, chunk, e->N, true)) e->give_back_rows(); // (of earlier runs)
     // the first stores hold the seeds' children of a first wave (a batch
     // member's, or a small network's, grow on demand from there)
     const long long first_wave = std::min<long long>(chunk, e->lean ? 4ll * S + 1024 : std::max(4ll * S + 1024, 65536ll));
-    e->ensure_regions(std::max<long long>(S, 1) + first_wave * kVMax);
-    e->ensure_table((long long)S + first_wave * kVMax, false);
-    e->ensure_append((S + 31) / 32);
+    e->with_rows_memory([&] {
+        e->ensure_chunk(std::min(chunk, std::max(S, 1024)));
+        e->ensure_regions(std::max<long long>(S, 1) + first_wave * kVMax);
+        e->ensure_table((long long)S + first_wave * kVMax, false);
+        e->ensure_append((S + 31) / 32);
+    });
 
     e->run.launches = 0;
     AM_CUDA(cudaEventRecord(e->ev0, st));
@@ -1515,16 +1539,19 @@ int am_error_report(am_engine *e, int64_t sample_regions, am_error_report_t *out
         for (long long j = 0; j < k; ++j) ids[(size_t)j] = (long long)((double)j * (double)R / (double)k);
         for (long long j = 1; j < k; ++j) ids[(size_t)j] = std::max(ids[(size_t)j], ids[(size_t)j - 1] + 1);
         for (long long j = k - 1; j >= 0 && ids[(size_t)j] >= R; --j) ids[(size_t)j] = R - 1 - (k - 1 - j);
-        AM_CUDA(e->v_ids.reserve(sizeof(long long) * (size_t)k));
-        AM_CUDA(cudaMemcpyAsync(e->v_ids.p, ids.data(), sizeof(long long) * (size_t)k, cudaMemcpyHostToDevice, st));
-        const NetDev n64 = network_fp64(e);
+        NetDev n64;
         // FP64 rows in slices of at most 1 GiB
         const long long per = (long long)e->ALLP * 4 * (long long)sizeof(double);
         const int slice = (int)std::max<long long>(1, std::min<long long>(k, ((long long)1 << 30) / per));
-        AM_CUDA(e->v_keys.reserve(sizeof(uint32_t) * (size_t)slice * e->W));
-        AM_CUDA(e->v_rows.reserve((size_t)per * slice));
-        AM_CUDA(e->v_eq.reserve(sizeof(double) * 4 * (size_t)slice));
-        AM_CUDA(e->v_out.reserve(sizeof(unsigned long long) * 5));
+        e->with_rows_memory([&] {
+            AM_CUDA(e->v_ids.reserve(sizeof(long long) * (size_t)k));
+            n64 = network_fp64(e);
+            AM_CUDA(e->v_keys.reserve(sizeof(uint32_t) * (size_t)slice * e->W));
+            AM_CUDA(e->v_rows.reserve((size_t)per * slice));
+            AM_CUDA(e->v_eq.reserve(sizeof(double) * 4 * (size_t)slice));
+            AM_CUDA(e->v_out.reserve(sizeof(unsigned long long) * 5));
+        });
+        AM_CUDA(cudaMemcpyAsync(e->v_ids.p, ids.data(), sizeof(long long) * (size_t)k, cudaMemcpyHostToDevice, st));
         AM_CUDA(cudaMemsetAsync(e->v_out.p, 0, sizeof(unsigned long long) * 5, st));
         const RegionsDev reg = e->regions();
         for (long long off = 0; off < k; off += slice) {
@@ -1602,26 +1629,28 @@ int am_combine_mesh(am_engine *e, double scale, const double *center3)
         const long long R = e->num_regions;
         const long long nr = std::max<long long>(R, 1);
         // the vertex slots in use, compacted (a face has ~4 of its 32)
-        AM_CUDA(e->w_voff.reserve(sizeof(int) * (nr + 1)));
-        AM_CUDA(e->w_fflag.reserve(sizeof(int) * (nr + 1)));
         const long long V = e->poly_verts;
         AM_CHECK(V < (1ll << 30), "too many polygon vertices for one mesh (2^30)");
         const long long ns = std::max<long long>(V, 1);
         unsigned long long tcap = 1;
         while (tcap < (unsigned long long)ns * 2ull) tcap <<= 1;
-        AM_CUDA(e->w_vsid.reserve(sizeof(long long) * ns));
-        AM_CUDA(e->w_table.reserve(sizeof(unsigned long long) * tcap));
-        AM_CUDA(e->w_rep.reserve(sizeof(int) * ns));
-        AM_CUDA(e->w_wslot.reserve(sizeof(unsigned) * ns));
-        AM_CUDA(e->w_flag.reserve(sizeof(int) * ns));
-        AM_CUDA(e->w_vidx.reserve(sizeof(int) * ns));
-        AM_CUDA(e->w_bsum.reserve(sizeof(int) * (std::max(ns, nr) / 1024 + 2)));
-        AM_CUDA(e->w_fsize.reserve(sizeof(int) * (nr + 1)));
-        AM_CUDA(e->w_fid.reserve(sizeof(int) * (nr + 1)));
-        AM_CUDA(e->w_foff.reserve(sizeof(int) * (nr + 1)));
-        AM_CUDA(e->w_verts.reserve(e->ts * 3 * ns));
-        AM_CUDA(e->w_fs.reserve(sizeof(int) * (nr + 1)));
-        AM_CUDA(e->w_fi.reserve(sizeof(int) * ns));
+        e->with_rows_memory([&] {
+            AM_CUDA(e->w_voff.reserve(sizeof(int) * (nr + 1)));
+            AM_CUDA(e->w_fflag.reserve(sizeof(int) * (nr + 1)));
+            AM_CUDA(e->w_vsid.reserve(sizeof(long long) * ns));
+            AM_CUDA(e->w_table.reserve(sizeof(unsigned long long) * tcap));
+            AM_CUDA(e->w_rep.reserve(sizeof(int) * ns));
+            AM_CUDA(e->w_wslot.reserve(sizeof(unsigned) * ns));
+            AM_CUDA(e->w_flag.reserve(sizeof(int) * ns));
+            AM_CUDA(e->w_vidx.reserve(sizeof(int) * ns));
+            AM_CUDA(e->w_bsum.reserve(sizeof(int) * (std::max(ns, nr) / 1024 + 2)));
+            AM_CUDA(e->w_fsize.reserve(sizeof(int) * (nr + 1)));
+            AM_CUDA(e->w_fid.reserve(sizeof(int) * (nr + 1)));
+            AM_CUDA(e->w_foff.reserve(sizeof(int) * (nr + 1)));
+            AM_CUDA(e->w_verts.reserve(e->ts * 3 * ns));
+            AM_CUDA(e->w_fs.reserve(sizeof(int) * (nr + 1)));
+            AM_CUDA(e->w_fi.reserve(sizeof(int) * ns));
+        });
         WeldBuffers wb{};
         wb.voff = e->w_voff.as<int>();
         wb.fflag = e->w_fflag.as<int>();
@@ -1794,7 +1823,7 @@ int am_region_rows(am_engine *e, int64_t first, int count, double *rows, double 
     return guarded(e, [&] {
         cudaStream_t st = e->st;
         if (count == 0) return;
-        e->ensure_chunk(count);
+        e->with_rows_memory([&] { e->ensure_chunk(count); });
         if (count > e->ring) {
             e->ring = 0; // (should the allocation fail)
             e->ring_target = 0;

@@ -23,6 +23,19 @@ AM_RULE bool read_in_place(MemoryType type, int device, int current, uint64_t ad
     return (type == kMemManaged || (type == kMemDevice && device == current)) && address % (uint64_t)element == 0;
 }
 
+// ---------------------------------------------------------------- ring of rows
+// Slots wanted for the constraint rows of waves of up to `wave` regions (the largest:
+// `chunk`) and the history in which their regions find their parents.  A parent is at
+// most about one level of the breadth-first queue away, and a level held 28 to 39
+// regions per hidden unit on the benchmark networks (512 .. 4,096 units): 48 a unit.
+// Where memory is bounded -- the caller gave the wave's size, or many networks march
+// side by side -- two waves, which reach the parents while a wave holds a whole level.
+AM_RULE long long ring_slots(int wave, int chunk, int units, bool bounded)
+{
+    if (bounded) return 2ll * wave;
+    return (long long)(chunk > wave ? chunk : wave) + 48ll * units;
+}
+
 // ---------------------------------------------------------------- append
 constexpr int kAppendWarps = 8;    // per block; a row is a warp's
 constexpr int kAppendSpanMax = 4096; // most rows per block: their winners and prefixes in shared memory

@@ -172,7 +172,12 @@ int am_run_batch(am_engine *const *engines, const am_run_args *args, int count, 
 int am_region_rows(am_engine *engine, int64_t first, int count, double *rows, double *eq);
 
 typedef enum {
-    AM_OPT_CHUNK = 1,         /* regions per wave (default: ~2 GiB of constraint rows, whole rounds of composition tiles) */
+    AM_OPT_CHUNK = 1,         /* regions per wave (default: ~2 GiB of constraint rows, whole rounds of
+                                 composition tiles, and beside them the rows of 48 earlier regions per
+                                 hidden unit, in which regions find their parents': 13 GB at 4,096 units
+                                 in FP32, at most an eighth of the free memory).  A given size bounds the
+                                 rows to those of two waves.  The rows stay with the engine between calls;
+                                 where memory runs out they are given back before a call fails. */
     AM_OPT_PHASE_TIMING = 2,  /* 1: time compose / polygon / frontier separately */
     AM_OPT_WELD = 3,          /* CombineMesh vertex weld: 0 = topological (default: a vertex is named by
                                  its two edge planes and the region key without those bits, which is
