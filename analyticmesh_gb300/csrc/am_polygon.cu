@@ -52,6 +52,7 @@
 
 #include "am_device.cuh"
 #include "am_internal.h"
+#include "am_rules.h"
 
 namespace am {
 
@@ -302,7 +303,9 @@ struct Sieve {
     }
 };
 
-// A pass over the rows by plain loads (a repeat with another T: rare)
+// A pass over the rows by plain loads (a repeat with another T: rare).  A row of zeros
+// (a dead unit) is no plane -- NaN once normalised, it is never hit, near or violated --
+// and is left out; the kernel's own pass keeps it, since looking for it costs every face.
 template <typename TC>
 __device__ int collect(const GlobalRows<TC> &g, float T, const Ball &ball, NearList<TC> *list, int lane)
 {
@@ -313,7 +316,7 @@ __device__ int collect(const GlobalRows<TC> &g, float T, const Ball &ball, NearL
         vec4_t<TC> v;
         v.x = v.y = v.z = v.w = TC(0);
         if (in) v = g.raw(k);
-        sv.take(v, k, in);
+        sv.take(v, k, in && !(v.x == TC(0) && v.y == TC(0) && v.z == TC(0) && v.w == TC(0)));
     }
     sv.finish();
     return sv.n;
@@ -375,7 +378,8 @@ __device__ __forceinline__ int position(const NearList<TC> *list, int n, int k, 
 
 // A radius that holds about kTarget rows: every lane's rows in four groups, the
 // smallest distance of each; T is the distance that 60 of the 128 groups reach
-// (rows spread evenly over the groups: ln(1 / (1 - 60 / 128)) rows per group).
+// (rows spread evenly over the groups: ln(1 / (1 - 60 / 128)) rows per group), or all
+// of them where fewer have a row with a normal (dead units).
 template <typename TC>
 __device__ float seed_radius(const GlobalRows<TC> &g, const Ball &ball, int lane)
 {
@@ -391,16 +395,21 @@ __device__ float seed_radius(const GlobalRows<TC> &g, const Ball &ball, int lane
         for (int j = 0; j < 4; ++j)
             if (j == q) m[j] = min(m[j], key);
     }
+    int finite = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) finite += m[j] < 0x7f800000u;
+    const int need = seed_groups(__reduce_add_sync(kFull, finite));
+    if (need == 0) return kReachMax;
     unsigned lo = 0u, hi = 0x7f800000u;
     for (int it = 0; it < 20; ++it) {
         const unsigned mid = (lo + hi) / 2u;
         int c = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) c += m[j] <= mid;
-        if (__reduce_add_sync(kFull, c) >= 60) hi = mid;
+        if (__reduce_add_sync(kFull, c) >= need) hi = mid;
         else lo = mid;
     }
-    return fmaxf(__uint_as_float(hi), 1e-30f);
+    return clamp_reach(__uint_as_float(hi));
 }
 
 // ---------------------------------------------------------------- scans
@@ -1203,10 +1212,15 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
         T = all.n > kList ? seed_radius<TC>(all, ball, lane) : INFINITY;
         n = -1;
     }
+    if (n > kList) { // (only if dead units are in it is the same ball worth another pass)
+        bool dead = false;
+        for (int j = lane; j < kList; j += 32) dead = dead || list->row[j].w != list->row[j].w;
+        if (__any_sync(kFull, dead)) n = -1;
+    }
     for (int tries = 0; tries < 5 && !done; ++tries) {
         if (n < 0) n = collect<TC>(all, T, ball, list, lane);
         if (n > kList) { // a smaller ball
-            T *= (float)kTarget / (float)n;
+            T = clamp_reach(T * ((float)kTarget / (float)n));
             n = -1;
             continue;
         }
@@ -1240,7 +1254,7 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
             s_plane = list->idx[s];
             if (f.ve >= 0) f.ve = list->idx[f.ve];
         } else {
-            if (n > 3 * kList / 4 || T == INFINITY) break;
+            if (n > 3 * kList / 4 || T >= kReachMax) break;
             T *= fminf((float)kList * 0.85f / (float)max(n, 1), 3.f); // a larger ball
             n = -1;
         }
@@ -1455,8 +1469,7 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
         if (lane == 0) {
             reg.nv[rid] = nv;
             reg.status[rid] = r.status;
-            // the children's radius: their ball holds about as many planes per radius
-            reg.reach[rid] = r.T * ((float)kTarget / (float)max(r.listed, kTarget / 4));
+            reg.reach[rid] = child_reach(r.T, r.listed, kTarget);
         }
         if (lane < nv) {
             TS *vo = (TS *)reg.verts + ((size_t)rid * kVMax + lane) * 3;

@@ -36,6 +36,27 @@ AM_RULE long long ring_slots(int wave, int chunk, int units, bool bounded)
     return (long long)(chunk > wave ? chunk : wave) + 48ll * units;
 }
 
+// ---------------------------------------------------------------- near list
+// A near list's radius stays a finite, positive number: a region's children scale
+// theirs from it, so that one that is infinite, zero or NaN would be every
+// descendant's.  (1e18: its square is still finite.)
+constexpr float kReachMin = 1e-30f, kReachMax = 1e18f;
+AM_RULE float clamp_reach(float T)
+{
+    const float t = T < kReachMax ? T : kReachMax; // (NaN: the largest)
+    return t > kReachMin ? t : kReachMin;
+}
+// the radius of a region's children, its own list having `listed` rows within T: a
+// ball holds about as many planes per radius (at most four times as large)
+AM_RULE float child_reach(float T, int listed, int target)
+{
+    const int least = target / 4;
+    return clamp_reach(T * ((float)target / (float)(listed > least ? listed : least)));
+}
+// groups of rows, of those with a plane at a finite distance, that a seed's radius
+// is to reach
+AM_RULE int seed_groups(int finite) { return finite < 60 ? finite : 60; }
+
 // ---------------------------------------------------------------- append
 constexpr int kAppendWarps = 8;    // per block; a row is a warp's
 constexpr int kAppendSpanMax = 4096; // most rows per block: their winners and prefixes in shared memory

@@ -36,3 +36,26 @@ int in_place(int type, int device, uint64_t address, int element) {
     return read_in_place((MemoryType)type, device, 0, address, element);
 }""")
     assert bool(L.in_place(kind, device, C.c_uint64(address), element)) is want
+
+
+def test_near_list_radius_recovers_from_any_value(tmp_path):
+    """The radius a region hands to its children is finite and positive whatever it came
+    from, and generations whose lists count the planes within it (a density of planes
+    per radius, up to a network's rows) come to lists of about the target."""
+    L = rules(tmp_path, "float child(float T, int listed) { return child_reach(T, listed, 64); }\n"
+                        "int groups(int finite) { return seed_groups(finite); }\n"
+                        "float clamped(float T) { return clamp_reach(T); }")
+    L.child.restype = L.clamped.restype = C.c_float
+    L.child.argtypes, L.clamped.argtypes = [C.c_float, C.c_int], [C.c_float]
+    inf = float("inf")
+    for T in (inf, float("nan"), -1.0, 0.0, 1e-45, 1e-30, 1e-3, 1.0, 1e18, 3.4e38):
+        for listed in (-1, 0, 1, 16, 64, 128, 12800):
+            assert 0 < L.child(T, listed) <= 1.0001e18, (T, listed)
+        assert 0 < L.clamped(T) < inf
+        for rows, density in ((200, 300.0), (4096, 2e4), (12800, 1e6)):
+            t = L.child(T, 64)
+            for _ in range(120):  # 48 decades by 64 / 200 or by 4 a generation: 97 or 80
+                t = L.child(t, min(rows, int(density * t)))
+            assert 32 <= min(rows, density * t) <= 128, (T, rows, t)
+    for finite in range(0, 129):
+        assert L.groups(finite) == min(finite, 60)
