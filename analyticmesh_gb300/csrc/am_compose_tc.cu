@@ -30,6 +30,7 @@
 // next layer's masked operand straight back into shared memory.  The face
 // plane (output layer, one row) is a 4 x K dot product per region in fp32,
 // from the operand in shared memory.
+#include <algorithm>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -1486,6 +1487,19 @@ size_t tc_smem_bytes(const TcNet &tc, int ncols, int W)
     }
     return 1024 + (size_t)(tc.kp_max / 64) * 3 * op_term_bytes(ncols) + (size_t)tc.nstage * kWBlockBytes + (size_t)(tc.ncols_max / 4) * key_stride(W) * 4 +
            16 * (size_t)tc.n1 + 4 * (size_t)tc.k_last + 16 + (size_t)kFaceSumBytes;
+}
+
+size_t tc_smem_cap()
+{
+    static const size_t own = [] { // (a rounded figure would refuse widths that fit: a layer of 8,192 units has 464 bytes to spare)
+        cudaFuncAttributes a = {}, b = {};
+        if (cudaFuncGetAttributes(&a, compose_tc_kernel) != cudaSuccess || cudaFuncGetAttributes(&b, compose_tcs_kernel) != cudaSuccess) {
+            cudaGetLastError();
+            return (size_t)2048;
+        }
+        return std::max(a.sharedSizeBytes, b.sharedSizeBytes);
+    }();
+    return 227u * 1024u - own;
 }
 
 void launch_compose_tc(const NetDev &net, const TcNet &tc, const RegionsDev &reg, const ChunkDev &ch, double iso,

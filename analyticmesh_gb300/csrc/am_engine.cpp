@@ -833,7 +833,7 @@ void run_begin(am_engine *e, const RunArgs &a)
         // widest tile: three operand terms (3 x ncols x kp_max x 2 bytes)
         // beside two weight blocks in flight (one if that leaves no room),
         // two accumulators (main + correction) per M tile in 512 TMEM columns
-        const size_t smem_cap = 227u * 1024u - 2048u; // less the kernels' static shared memory
+        const size_t smem_cap = tc_smem_cap();
         // with two weight stages, else with one; above 128 columns whole
         // multiples of them (the face plane takes 32 regions at a time)
         tc.ncols_max = 0;

@@ -40,6 +40,7 @@ struct TcNet {
 };
 
 size_t tc_smem_bytes(const TcNet &tc, int ncols, int W);
+size_t tc_smem_cap(); // most of it a launch may have: a CTA's, less the kernels' own static shared memory
 void launch_compose_tc(const NetDev &net, const TcNet &tc, const RegionsDev &reg, const ChunkDev &ch, double iso,
                        int *d_err, cudaStream_t st);
 void launch_pack_weights(const float *src, int M, int K, int Mp, int Kp, void *dst, cudaStream_t st);
