@@ -34,7 +34,7 @@ __global__ void seed_pack_kernel(const uint8_t *states, int S, int N, int W, uin
 {
     if (zeroed && blockIdx.x == 0 && threadIdx.x == 0) *zeroed = 0;
     const int lane = threadIdx.x & 31;
-    const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const long long s = warp_row(blockIdx.x, blockDim.x, threadIdx.x);
     if (s >= S) return;
     if (pt.dst && lane < 3) { // (FP32 to FP64 is exact)
         const size_t q = (size_t)s * 3 + lane;
@@ -421,7 +421,7 @@ void launch_seed_pack(const uint8_t *states, int S, int N, int W, uint32_t *keys
                       int *zeroed, const SeedPoints &points)
 {
     if (S <= 0) return;
-    seed_pack_kernel<<<(S + 7) / 8, 256, 0, st>>>(states, S, N, W, keys, hash, zeroed, points);
+    seed_pack_kernel<<<((unsigned)S + 7u) / 8u, 256, 0, st>>>(states, S, N, W, keys, hash, zeroed, points);
 }
 
 void launch_seed_insert(const uint32_t *keys, const uint64_t *hash, int S, int W, const HashDev &hs, int32_t *rec,

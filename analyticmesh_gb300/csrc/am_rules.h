@@ -23,6 +23,13 @@ AM_RULE bool read_in_place(MemoryType type, int device, int current, uint64_t ad
     return (type == kMemManaged || (type == kMemDevice && device == current)) && address % (uint64_t)element == 0;
 }
 
+// ---------------------------------------------------------------- seeds
+// the row of a warp per row, in 64 bits: 2^27 rows are 2^32 threads
+AM_RULE long long warp_row(unsigned block, unsigned block_threads, unsigned thread)
+{
+    return ((long long)block * block_threads + thread) >> 5;
+}
+
 // ---------------------------------------------------------------- ring of rows
 // Slots wanted for the constraint rows of waves of up to `wave` regions (the largest:
 // `chunk`) and the history in which their regions find their parents.  A parent is at

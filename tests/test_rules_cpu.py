@@ -59,3 +59,11 @@ def test_near_list_radius_recovers_from_any_value(tmp_path):
             assert 32 <= min(rows, density * t) <= 128, (T, rows, t)
     for finite in range(0, 129):
         assert L.groups(finite) == min(finite, 60)
+
+
+def test_a_seeds_warp_among_more_than_2_to_the_27(tmp_path):
+    L = rules(tmp_path, "long long row(unsigned b, unsigned n, unsigned t) { return warp_row(b, n, t); }")
+    L.row.restype = C.c_longlong
+    for row in (0, 1, 7, 8, 2**27 - 1, 2**27, 2**27 + 9, 2**31 - 2):
+        for lane in (0, 31):
+            assert L.row(row // 8, 256, row % 8 * 32 + lane) == row
