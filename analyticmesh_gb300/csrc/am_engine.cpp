@@ -262,6 +262,7 @@ struct am_engine {
     long long max_regions = 0; // AM_OPT_MAX_REGIONS (0: no limit)
     int compose_tile = 0;      // AM_OPT_COMPOSE_TILE: 0 automatic, 1 resident operand, 2 streamed operand
     int face_warps = 0;        // AM_OPT_FACE_WARPS: the rule between near-equal hits, 0 automatic
+    bool every_row = false;    // AM_OPT_EVERY_ROW: faces walked over every row
     long long table_slots = 0; // AM_OPT_TABLE_SLOTS: fixed region hash table size, 0 automatic
     int inject_err = 0;        // AM_OPT_INJECT_ERROR: error bits set in the control block after the seeds
     bool limit_hit = false;    // the last run stopped at the region limit
@@ -574,6 +575,7 @@ struct am_engine {
         add(&prec, sizeof(prec));
         add(&chunk, sizeof(chunk));
         add(&face_warps, sizeof(face_warps));
+        add(&every_row, sizeof(every_row));
         add(&iso, sizeof(iso));
         add(&tol, sizeof(tol));
         add(&net, sizeof(net));
@@ -603,7 +605,7 @@ struct am_engine {
                     launch_compose_tc(net, tcnet, reg, ch, iso, d_err.as<int>(), st);
                 else
                     launch_compose(prec, net, reg, ch, iso, d_err.as<int>(), st);
-                launch_polygon(prec, net, reg, ch, hs, tol, face_warps, fp64_counter(), d_err.as<int>(), st);
+                launch_polygon(prec, net, reg, ch, hs, tol, face_warps, every_row, fp64_counter(), d_err.as<int>(), st);
                 launch_append(0, prec, net, reg, ch, hs, nullptr, nullptr, nullptr, 0, d_tail.as<long long>(),
                               blocksum.as<AppendScratch>(), append_cap, d_err.as<int>(), st, &cond);
                 cudaGraph_t captured = nullptr;
@@ -1088,7 +1090,7 @@ void run_host_loop(am_engine *e)
             t_comp += ms;
             AM_CUDA(cudaEventRecord(pa, st));
         }
-        launch_polygon(prec, net, reg, ch, hs, tol, e->face_warps, e->fp64_counter(), e->d_err.as<int>(), st);
+        launch_polygon(prec, net, reg, ch, hs, tol, e->face_warps, e->every_row, e->fp64_counter(), e->d_err.as<int>(), st);
         if (e->phase_timing) {
             AM_CUDA(cudaEventRecord(pb, st));
             AM_CUDA(cudaEventSynchronize(pb));
@@ -1290,6 +1292,11 @@ int am_set_option(am_engine *e, int option, int64_t value)
     if (option == AM_OPT_PRUNE_ROWS) {
         if (value != 0 && value != 1) return AM_ERR_INVALID_ARGUMENT;
         return AM_OK; // the walk always leaves out the rows that cannot bound the face (am_polygon.cu)
+    }
+    if (option == AM_OPT_EVERY_ROW) {
+        if (value != 0 && value != 1) return AM_ERR_INVALID_ARGUMENT;
+        e->every_row = value != 0;
+        return AM_OK;
     }
     if (option == AM_OPT_INJECT_ERROR) {
         if (value < 0 || value > (kErrTableFull | kErrWait | kErrCapacity | kErrNonFinite)) return AM_ERR_INVALID_ARGUMENT;

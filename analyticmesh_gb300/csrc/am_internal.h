@@ -164,9 +164,10 @@ struct Tolerances {
 void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso, int *d_err,
                     cudaStream_t st, const int *nonfinite = nullptr);
 // face_warps: sets the rule between near-equal hits (0: by the rows' size)
+// every_row: no near list
 // nfp64: counts the faces the mixed form walks again with FP64 predicates
 void launch_polygon(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
-                    const Tolerances &tol, int face_warps, unsigned long long *nfp64, int *d_err,
+                    const Tolerances &tol, int face_warps, bool every_row, unsigned long long *nfp64, int *d_err,
                     cudaStream_t st);
 int polygon_face_warps(int prec, int ALLP);
 // zeroed: an int set to zero as well (optional); points: S x 3 seed points of

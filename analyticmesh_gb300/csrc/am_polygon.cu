@@ -1186,11 +1186,11 @@ struct Result {
 // Everything but the common face (a region with a parent whose FP32 walk stays in
 // its list and needs no FP64 predicate): seeds, repeats with another radius, FP64
 // predicates, every row.  Kept out of the kernel's registers.  `again`: only
-// the FP64 predicates are asked for, on the list as it is.
+// the FP64 predicates are asked for, on the list as it is.  `every_row`: no list.
 template <typename TC, typename TS>
 __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *list, int ways, const vec4_t<TC> &eqc,
                                        const TS *mid, int start, TC eps, TC par_eps, TS same_eps, int lane, bool again,
-                                       int n, float T, Result<TS> &out)
+                                       int n, float T, bool every_row, Result<TS> &out)
 {
     const bool is_seed = start < 0;
     const TS eqv[4] = {(TS)eqc.x, (TS)eqc.y, (TS)eqc.z, (TS)eqc.w};
@@ -1217,7 +1217,7 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
         for (int j = lane; j < kList; j += 32) dead = dead || list->row[j].w != list->row[j].w;
         if (__any_sync(kFull, dead)) n = -1;
     }
-    for (int tries = 0; tries < 5 && !done; ++tries) {
+    for (int tries = 0; tries < 5 && !done && !every_row; ++tries) {
         if (n < 0) n = collect<TC>(all, T, ball, list, lane);
         if (n > kList) { // a smaller ball
             T = clamp_reach(T * ((float)kTarget / (float)n));
@@ -1379,8 +1379,8 @@ __device__ int insert_edges(const RegionsDev &reg, const HashDev &hs, long long 
 //   3-[128]x4-1 mixed / fp32 / fp64 (265 K) 3.2 / 2.4 / 28.8 -> 2.7 / 1.7 / 8.5
 template <typename TC, typename TS>
 __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDev net, RegionsDev reg, ChunkDev ch, HashDev hs,
-                                                                     Tolerances tol, int ways, unsigned long long *nfp64,
-                                                                     int *err)
+                                                                     Tolerances tol, int ways, bool every_row,
+                                                                     unsigned long long *nfp64, int *err)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
@@ -1427,7 +1427,7 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
             stream_part<TC, false>(own, nullptr, all.nsplit, ALL, -1, sv);
             sv.finish();
             r.listed = sv.n;
-            if (sv.n <= kList) {
+            if (sv.n <= kList && !every_row) {
                 const vec4_t<TC> eqc = ld4<TC>((const TC *)ch.eq + (size_t)rl * 4); // scan precision copy
                 const TS eqv[4] = {(TS)eqc.x, (TS)eqc.y, (TS)eqc.z, (TS)eqc.w};
                 const TS p[3] = {midp[0], midp[1], midp[2]};
@@ -1459,7 +1459,7 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
         if (what != kRefined) {
             Result<TS> o;
             const vec4_t<TC> eqc = ld4<TC>((const TC *)ch.eq + (size_t)rl * 4);
-            face_slow<TC, TS>(all, list, ways, eqc, midp, start, eps, par_eps, same_eps, lane, what == kAgain, r.listed, r.T, o);
+            face_slow<TC, TS>(all, list, ways, eqc, midp, start, eps, par_eps, same_eps, lane, what == kAgain, r.listed, r.T, every_row, o);
             r = o;
             if (r.again && lane == 0) atomicAdd(nfp64, 1ull);
         }
@@ -1508,7 +1508,7 @@ int polygon_face_warps(int prec, int ALLP) { return rule_ways(prec, ALLP, 0) / 3
 
 template <typename TC, typename TS>
 static void launch_one(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
-                       const Tolerances &tol, int *d_err, int ways, unsigned long long *nfp64, cudaStream_t st)
+                       const Tolerances &tol, int *d_err, int ways, bool every_row, unsigned long long *nfp64, cudaStream_t st)
 {
     auto k = polygon_kernel<TC, TS>;
     const size_t smem = sizeof(NearList<TC>) * kFaceWarps;
@@ -1516,20 +1516,20 @@ static void launch_one(const NetDev &net, const RegionsDev &reg, const ChunkDev 
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kFaceWarps, smem);
     long long grid = (long long)device_sms() * std::max(per_sm, 1);
     if (!ch.ctl) grid = std::min<long long>(grid, (ch.count + kFaceWarps - 1) / kFaceWarps);
-    k<<<(unsigned)grid, 32 * kFaceWarps, smem, st>>>(net, reg, ch, hs, tol, ways, nfp64, d_err);
+    k<<<(unsigned)grid, 32 * kFaceWarps, smem, st>>>(net, reg, ch, hs, tol, ways, every_row, nfp64, d_err);
 }
 
 void launch_polygon(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
-                    const Tolerances &tol, int face_warps, unsigned long long *nfp64, int *d_err, cudaStream_t st)
+                    const Tolerances &tol, int face_warps, bool every_row, unsigned long long *nfp64, int *d_err, cudaStream_t st)
 {
     if (!ch.ctl && ch.count <= 0) return;
     const int ways = rule_ways(prec, net.ALLP, face_warps);
     if (prec == kFloat64)
-        launch_one<double, double>(net, reg, ch, hs, tol, d_err, ways, nfp64, st);
+        launch_one<double, double>(net, reg, ch, hs, tol, d_err, ways, every_row, nfp64, st);
     else if (prec == kMixed)
-        launch_one<float, double>(net, reg, ch, hs, tol, d_err, ways, nfp64, st);
+        launch_one<float, double>(net, reg, ch, hs, tol, d_err, ways, every_row, nfp64, st);
     else
-        launch_one<float, float>(net, reg, ch, hs, tol, d_err, ways, nfp64, st);
+        launch_one<float, float>(net, reg, ch, hs, tol, d_err, ways, every_row, nfp64, st);
 }
 
 } // namespace am

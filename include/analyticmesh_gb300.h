@@ -211,8 +211,11 @@ typedef enum {
                                  block after the seed phase, as a kernel would leave them, so that the
                                  wave loop's error decoding can be tested without a device fault.
                                  0 (default) off; stays set until set to 0. */
-    AM_OPT_PRUNE_ROWS = 10    /* 0 or 1: accepted, without effect.  The walk always works on the rows whose
+    AM_OPT_PRUNE_ROWS = 10,   /* 0 or 1: accepted, without effect.  The walk always works on the rows whose
                                  planes are near the face, with the faces of every row. */
+    AM_OPT_EVERY_ROW = 11     /* test hook, 1: every face is walked over all rows, as a face is where the
+                                 rows near it do not decide.  The same faces, several times slower.
+                                 0 (default) off. */
 } am_option;
 int am_set_option(am_engine *engine, int option, int64_t value);
 
