@@ -237,15 +237,20 @@ __device__ __forceinline__ int same_filter(const TC *Vc, TC px, TC py, TC pz, TS
 
 // ---------------------------------------------------------------- the ball
 // A row left out has its plane farther than T from p, up to the rounding of the
-// FP32 test (a few 1e-7 of the coordinates' size).  For a point x with
-// |x - p| <= D its value is below -(T - D), and the edge line reaches its plane
-// beyond |x - p| = T; with T - D >= D / 16 + 1e-4 of the coordinates' size the
-// computed quotient of such a row is larger than that of any hit within the
-// ball, whatever the line's angle to the plane: with m = T - D, t the hit's
-// distance (<= 2 D) and a the row's slope, the computed quotient is at least
-// (a (t + m) - 1e-6) / (a + 5e-7) and (m - 1e-6) / (a + 5e-7), and m^2 > 4e-6 D
-// puts one of the two above t for every a.  The same margin keeps its value
-// away from the 1e-6 and 2e-6 of the near-zero predicates.
+// FP32 test: a few 1e-7 of the coordinates' size s = |p|_1 + T, which bounds the
+// points of the ball and, beside their distance, the planes' offsets.  For a point x
+// with |x - p| <= D its value is below -(T - D), and the edge line reaches its plane
+// beyond |x - p| = T; with T - D >= D / 16 + 1e-4 s the computed quotient of such a
+// row is larger than that of any hit within the ball, whatever the line's angle to
+// the plane: with m = T - D, t the hit's distance (<= 2 D) and a the row's slope, the
+// computed quotient is at least (a (t + m) - 1e-6 s) / (a + 5e-7) and
+// (m - 1e-6 s) / (a + 5e-7), and m^2 > 5e-6 D s puts one of the two above t for every
+// a (m^2 >= 4 (D / 16) (1e-4 s) = 2.5e-5 D s).  The bound goes with the scale of the
+// coordinates.  The mixed form's near-zero predicates (1e-6 and 2e-6) do not: there m
+// is 4e-6 more, so that a row left out is never near zero.  (With s = 1 + |p|_1, which
+// does not shrink with the shape, every face of a shape of 1e-3 was walked over every
+// row: 3-[128]x4-1 scaled by 1e-3, polygon phase on GB300 in float64 / mixed / float32
+// 30.0 / 13.6 / 4.9 ms, with this size 9.2 / 7.7 / 1.9; at scale 1 9.2 / 3.1 / 1.9.)
 struct Ball {
     float x, y, z, d2; // centre, squared radius (< 0: nothing is inside, infinite: every row is in the list)
     __device__ __forceinline__ bool in(float px, float py, float pz) const
@@ -254,11 +259,12 @@ struct Ball {
         return d2 == INFINITY || dx * dx + dy * dy + dz * dz <= d2; // (NaN: outside)
     }
 };
-__device__ __forceinline__ float coord_size(float x, float y, float z) { return 1.f + fabsf(x) + fabsf(y) + fabsf(z); }
-__device__ __forceinline__ float ball_radius2(float T, float size)
+__device__ __forceinline__ float coord_size(const Ball &b, float T) { return fabsf(b.x) + fabsf(b.y) + fabsf(b.z) + T; }
+template <bool kPredicates> // (the mixed form)
+__device__ __forceinline__ float ball_radius2(const Ball &b, float T)
 {
     if (T == INFINITY) return INFINITY;
-    const float D = (T - 1e-4f * size) * (16.f / 17.f);
+    const float D = (T - 1e-4f * coord_size(b, T) - (kPredicates ? 4e-6f : 0.f)) * (16.f / 17.f);
     return D > 0.f ? D * D : -1.f;
 }
 
@@ -1069,7 +1075,7 @@ __device__ int seed_start(const Rows &rows, const GlobalRows<TC> &all, const Bal
     if (ball.d2 != INFINITY) { // the farthest chosen plane well inside T: no plane left out is nearer
         const vec4_t<TC> v = rows.get(pi);
         const float c = -(float)(dot3(v.x, pc[0], v.y, pc[1], v.z, pc[2]) + v.w);
-        if (!(c < T * 0.999f - 1e-5f * coord_size(ball.x, ball.y, ball.z))) return -2;
+        if (!(c < T * 0.999f - 1e-5f * coord_size(ball, T))) return -2;
     }
     int x_max = (all.n - 1) * (all.n - 2);
     if (x_max > 812) x_max = 812;
@@ -1196,7 +1202,6 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
     const TS eqv[4] = {(TS)eqc.x, (TS)eqc.y, (TS)eqc.z, (TS)eqc.w};
     TS p[3] = {mid[0], mid[1], mid[2]};
     Ball ball{(float)p[0], (float)p[1], (float)p[2], -1.f};
-    const float size = coord_size(ball.x, ball.y, ball.z);
     Face<TS> f;
     bool done = false, wide = false;
     int s = start, s_plane = start;
@@ -1225,7 +1230,7 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
             continue;
         }
         const ListRows<TC> rows{list, n};
-        ball.d2 = ball_radius2(T, size);
+        ball.d2 = ball_radius2<(sizeof(TS) > sizeof(TC))>(ball, T);
         TS q[3] = {p[0], p[1], p[2]};
         if (!is_seed) {
             s = position<TC>(list, n, start, lane);
@@ -1432,7 +1437,7 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
                 const TS eqv[4] = {(TS)eqc.x, (TS)eqc.y, (TS)eqc.z, (TS)eqc.w};
                 const TS p[3] = {midp[0], midp[1], midp[2]};
                 Ball ball{(float)p[0], (float)p[1], (float)p[2], -1.f};
-                ball.d2 = ball_radius2(r.T, coord_size(ball.x, ball.y, ball.z));
+                ball.d2 = ball_radius2<(sizeof(TS) > sizeof(TC))>(ball, r.T);
                 const ListRows<TC> rows{list, sv.n};
                 const int s = position<TC>(list, sv.n, start, lane);
                 Face<TS> f;

@@ -31,20 +31,7 @@ CASES = {
 }
 
 
-@pytest.mark.parametrize("form", ["float32", "mixed", "float64"])
-@pytest.mark.parametrize("name", list(CASES))
-def test_faces_of_the_list_and_of_every_row_are_equal(name, form):
-    factory, level, boxed, limit = CASES[name]
-    if form == "float64" and name in ("deep", "large_skip"):
-        limit //= 4
-    m = factory()
-    if level is None:
-        x = torch.nn.functional.normalize(torch.randn(2048, 3, generator=torch.Generator().manual_seed(1)), dim=1) * 0.5
-        with torch.no_grad():
-            level = float(m(x).double().mean())
-    box = BOX if boxed else (None, None)
-    net = wl.net_arrays(m, *box)
-    st, pt = wl.seeds_for(m, init_num=96, seed=3, iso=level, w_extra=box[0], b_extra=box[1])
+def compare_walks(net, st, pt, level, form, limit):
     out, walks = [], []
     for every in (0, 1):
         eng = engine.Engine(form, net.nodes, net.arc_table, net.num_extra)
@@ -65,3 +52,36 @@ def test_faces_of_the_list_and_of_every_row_are_equal(name, form):
     used = np.arange(a.edges.shape[1])[None, :] < a.nverts[:, None]
     assert np.array_equal(a.edges[used], b.edges[used])
     assert np.array_equal(a.verts[used].view(np.int64), b.verts[used].view(np.int64))
+
+
+@pytest.mark.parametrize("form", ["float32", "mixed", "float64"])
+@pytest.mark.parametrize("name", list(CASES))
+def test_faces_of_the_list_and_of_every_row_are_equal(name, form):
+    factory, level, boxed, limit = CASES[name]
+    if form == "float64" and name in ("deep", "large_skip"):
+        limit //= 4
+    m = factory()
+    if level is None:
+        x = torch.nn.functional.normalize(torch.randn(2048, 3, generator=torch.Generator().manual_seed(1)), dim=1) * 0.5
+        with torch.no_grad():
+            level = float(m(x).double().mean())
+    box = BOX if boxed else (None, None)
+    net = wl.net_arrays(m, *box)
+    st, pt = wl.seeds_for(m, init_num=96, seed=3, iso=level, w_extra=box[0], b_extra=box[1])
+    compare_walks(net, st, pt, level, form, limit)
+
+
+@pytest.mark.parametrize("form", ["float32", "mixed", "float64"])
+@pytest.mark.parametrize("scale,shift", [(1e-2, 0), (1e-3, 0), (1e-4, 0), (1e3, 0), (1.0, 20.0), (1e-2, 0.3)])
+@pytest.mark.parametrize("name", ["sphere128x4", "deep"])
+def test_faces_of_small_large_and_distant_shapes(name, scale, shift, form):
+    """The shape scaled, and moved by `shift` along a diagonal: the list's margin goes with
+    the coordinates' size."""
+    factory, level, _, _ = CASES[name]
+    m = factory()
+    net = wl.net_arrays(m)
+    st, pt = wl.seeds_for(m, init_num=96, seed=3, iso=level)
+    t = shift * np.array([0.6, -0.3, 0.7])
+    net.W[0] = net.W[0] / scale
+    net.b[0] = net.b[0] - net.W[0] @ t
+    compare_walks(net, st, pt * scale + t, level, form, 60000)
