@@ -170,14 +170,6 @@ __device__ __forceinline__ vec4_t<T> tile_row(const T *cons, size_t rstride, con
     return v;
 }
 
-// ---------------------------------------------------------------- warp
-__device__ __forceinline__ int warp_sum(int v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // ---------------------------------------------------------------- 3x3
 // Cramer's rule for A x + b = 0 with rows (r0, r1, r2) -- the reference's
 // solve_3x3 (backend/inc/kernel.h:553-571).  Returns the determinant.

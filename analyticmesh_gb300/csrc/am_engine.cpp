@@ -187,12 +187,6 @@ void upload(DevBuf &dst, const void *src, size_t n, cudaStream_t st)
     if (n) AM_CUDA(cudaMemcpyAsync(dst.p, src, n, is_device_ptr(src) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
 }
 
-void to_host(void *dst, const void *src, size_t n, cudaStream_t st)
-{
-    if (!n) return;
-    AM_CUDA(cudaMemcpyAsync(dst, src, n, is_device_ptr(src) ? cudaMemcpyDeviceToHost : cudaMemcpyHostToHost, st));
-}
-
 } // namespace
 
 struct am_engine {

@@ -231,11 +231,4 @@ void launch_to_double(const void *src, long long n, void *dst, cudaStream_t st);
 void launch_verify(int ts_bytes, const RegionsDev &reg, const long long *ids, int count, const double *rows,
                    const double *eq, int ALLP, int ALL, unsigned long long *out, cudaStream_t st);
 
-// mesh weld (CombineMesh)
-struct MeshDev {
-    unsigned long long *vslots; // weld table: packed (vertex slot id) per hash slot
-    unsigned long long vmask;
-    int64_t *vkey;              // [nslots_total][2] quantised key per vertex slot (x,y | z)
-};
-
 } // namespace am

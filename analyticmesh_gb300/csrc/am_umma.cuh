@@ -181,18 +181,6 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                  : "memory");
 }
 
-// contiguous shared -> global copy on the bulk-copy engine, in the thread's
-// bulk group (alignment as above)
-__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes)
-{
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_addr(src)), "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-// the thread's bulk groups have read their shared memory / have completed
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
 // has phase `parity` completed?  (non-blocking)
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity)
 {
@@ -267,25 +255,6 @@ __device__ __forceinline__ void tmem_ld16x2(uint32_t a, uint32_t b, float *v, fl
     for (int i = 0; i < 16; ++i) {
         v[i] = __uint_as_float(r[i]);
         w[i] = __uint_as_float(r[16 + i]);
-    }
-}
-
-// 32 lanes x 32 bit, 8 consecutive columns per thread from two addresses
-__device__ __forceinline__ void tmem_ld8x2(uint32_t a, uint32_t b, float *v, float *w)
-{
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n"
-        "tcgen05.wait::ld.sync.aligned;\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(a), "r"(b)
-        : "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        v[i] = __uint_as_float(r[i]);
-        w[i] = __uint_as_float(r[8 + i]);
     }
 }
 
