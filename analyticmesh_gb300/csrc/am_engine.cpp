@@ -255,7 +255,7 @@ struct am_engine {
     bool lean = false; // batch member: region store and table start small and grow on demand
     long long max_regions = 0; // AM_OPT_MAX_REGIONS (0: no limit)
     int compose_tile = 0;      // AM_OPT_COMPOSE_TILE: 0 automatic, 1 resident operand, 2 streamed operand
-    int face_warps = 0;        // AM_OPT_FACE_WARPS: the rule between near-equal hits, 0 automatic
+    int rule_warps = 0;        // AM_OPT_FACE_WARPS: the rule between near-equal hits, 0 automatic
     bool every_row = false;    // AM_OPT_EVERY_ROW: faces walked over every row
     long long table_slots = 0; // AM_OPT_TABLE_SLOTS: fixed region hash table size, 0 automatic
     int inject_err = 0;        // AM_OPT_INJECT_ERROR: error bits set in the control block after the seeds
@@ -568,7 +568,7 @@ struct am_engine {
                                order.p, split.p, (const void *)(size_t)ring};
         add(&prec, sizeof(prec));
         add(&chunk, sizeof(chunk));
-        add(&face_warps, sizeof(face_warps));
+        add(&rule_warps, sizeof(rule_warps));
         add(&every_row, sizeof(every_row));
         add(&iso, sizeof(iso));
         add(&tol, sizeof(tol));
@@ -599,7 +599,7 @@ struct am_engine {
                     launch_compose_tc(net, tcnet, reg, ch, iso, d_err.as<int>(), st);
                 else
                     launch_compose(prec, net, reg, ch, iso, d_err.as<int>(), st);
-                launch_polygon(prec, net, reg, ch, hs, tol, face_warps, every_row, fp64_counter(), d_err.as<int>(), st);
+                launch_polygon(prec, net, reg, ch, hs, tol, rule_warps, every_row, fp64_counter(), d_err.as<int>(), st);
                 launch_append(0, prec, net, reg, ch, hs, nullptr, nullptr, nullptr, 0, d_tail.as<long long>(),
                               blocksum.as<AppendScratch>(), append_cap, d_err.as<int>(), st, &cond);
                 cudaGraph_t captured = nullptr;
@@ -1084,7 +1084,7 @@ void run_host_loop(am_engine *e)
             t_comp += ms;
             AM_CUDA(cudaEventRecord(pa, st));
         }
-        launch_polygon(prec, net, reg, ch, hs, tol, e->face_warps, e->every_row, e->fp64_counter(), e->d_err.as<int>(), st);
+        launch_polygon(prec, net, reg, ch, hs, tol, e->rule_warps, e->every_row, e->fp64_counter(), e->d_err.as<int>(), st);
         if (e->phase_timing) {
             AM_CUDA(cudaEventRecord(pb, st));
             AM_CUDA(cudaEventSynchronize(pb));
@@ -1269,7 +1269,7 @@ int am_set_option(am_engine *e, int option, int64_t value)
     }
     if (option == AM_OPT_FACE_WARPS) {
         if (value != 0 && value != 1 && value != 2 && value != 4 && value != 8) return AM_ERR_INVALID_ARGUMENT;
-        e->face_warps = (int)value;
+        e->rule_warps = (int)value;
         return AM_OK;
     }
     if (option == AM_OPT_COMPOSE_TILE) {
@@ -1357,8 +1357,8 @@ int am_autotune(am_engine *e, const am_run_args *x, int64_t sample_regions, int3
         auto it = g_tune.find(key);
         if (it != g_tune.end()) {
             e->compose_tile = it->second.first;
-            e->face_warps = it->second.second;
-            if (chosen) chosen[0] = e->compose_tile, chosen[1] = e->face_warps;
+            e->rule_warps = it->second.second;
+            if (chosen) chosen[0] = e->compose_tile, chosen[1] = e->rule_warps;
             return AM_OK;
         }
     }
@@ -1366,11 +1366,11 @@ int am_autotune(am_engine *e, const am_run_args *x, int64_t sample_regions, int3
                     x->num_arc_tm, x->w_extra, x->b_extra, x->iso, x->flip_insideout, nullptr};
     const long long keep_max = e->max_regions;
     const bool keep_pt = e->phase_timing;
-    const int keep_ct = e->compose_tile, keep_fw = e->face_warps;
+    const int keep_ct = e->compose_tile, keep_fw = e->rule_warps;
     int last_rc = AM_OK;
     auto sample = [&](int ct, int fw, double &comp, double &poly) {
         e->compose_tile = ct;
-        e->face_warps = fw;
+        e->rule_warps = fw;
         e->max_regions = sample_regions;
         e->phase_timing = true;
         e->has_am = false;
@@ -1397,7 +1397,7 @@ int am_autotune(am_engine *e, const am_run_args *x, int64_t sample_regions, int3
     for (int ct : cts)
         if (sample(ct, 0, c, p) && c < best) best = c, best_ct = ct;
     // (a face is one warp's whatever the option says: its automatic value)
-    if (best_ct >= 0) best_fw = polygon_face_warps(e->prec, e->ALLP);
+    if (best_ct >= 0) best_fw = hit_rule_lanes(e->prec == kFloat64, e->ALLP, 0) / 32;
     e->max_regions = keep_max;
     e->phase_timing = keep_pt;
     e->has_am = false; // the samples are not a result
@@ -1410,11 +1410,11 @@ int am_autotune(am_engine *e, const am_run_args *x, int64_t sample_regions, int3
     });
     if (best_ct < 0 || best_fw < 0) {
         e->compose_tile = keep_ct;
-        e->face_warps = keep_fw;
+        e->rule_warps = keep_fw;
         return last_rc != AM_OK ? last_rc : AM_ERR_CUDA;
     }
     e->compose_tile = best_ct;
-    e->face_warps = best_fw;
+    e->rule_warps = best_fw;
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
         g_tune[key] = {best_ct, best_fw};

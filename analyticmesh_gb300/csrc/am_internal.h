@@ -163,13 +163,12 @@ struct Tolerances {
 // nonfinite: device flag, non-zero when a weight may not be finite (null: all are)
 void launch_compose(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, double iso, int *d_err,
                     cudaStream_t st, const int *nonfinite = nullptr);
-// face_warps: sets the rule between near-equal hits (0: by the rows' size)
+// rule_warps: sets the rule between near-equal hits (hit_rule_lanes)
 // every_row: no near list
 // nfp64: counts the faces the mixed form walks again with FP64 predicates
 void launch_polygon(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
-                    const Tolerances &tol, int face_warps, bool every_row, unsigned long long *nfp64, int *d_err,
+                    const Tolerances &tol, int rule_warps, bool every_row, unsigned long long *nfp64, int *d_err,
                     cudaStream_t st);
-int polygon_face_warps(int prec, int ALLP);
 // zeroed: an int set to zero as well (optional); points: S x 3 seed points of
 // pbytes-byte floats, converted to tbytes-byte ones in dst (optional)
 struct SeedPoints {

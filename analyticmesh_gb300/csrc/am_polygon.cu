@@ -1496,21 +1496,6 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
 
 } // namespace
 
-// The lanes of the rule between near-equal hits (see the top of the file): 32
-// per warp of the face group that scanned every row from shared memory, eight
-// warps per block split between faces and the warps of a face as 73 KB of rows
-// allowed.  `face_warps` overrides the warps.
-static int rule_ways(int prec, int ALLP, int face_warps)
-{
-    if (face_warps > 0) return 32 * face_warps;
-    const size_t face_bytes = prec == kFloat64 ? sizeof(double) * 4 * (size_t)ALLP + 1120 : sizeof(float) * 4 * (size_t)ALLP + 1056;
-    int F = 1;
-    while (2 * F <= 8 && (size_t)(2 * F) * face_bytes <= 73u * 1024u) F *= 2;
-    return 32 * (8 / F);
-}
-
-int polygon_face_warps(int prec, int ALLP) { return rule_ways(prec, ALLP, 0) / 32; }
-
 template <typename TC, typename TS>
 static void launch_one(const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
                        const Tolerances &tol, int *d_err, int ways, bool every_row, unsigned long long *nfp64, cudaStream_t st)
@@ -1525,10 +1510,10 @@ static void launch_one(const NetDev &net, const RegionsDev &reg, const ChunkDev 
 }
 
 void launch_polygon(int prec, const NetDev &net, const RegionsDev &reg, const ChunkDev &ch, const HashDev &hs,
-                    const Tolerances &tol, int face_warps, bool every_row, unsigned long long *nfp64, int *d_err, cudaStream_t st)
+                    const Tolerances &tol, int rule_warps, bool every_row, unsigned long long *nfp64, int *d_err, cudaStream_t st)
 {
     if (!ch.ctl && ch.count <= 0) return;
-    const int ways = rule_ways(prec, net.ALLP, face_warps);
+    const int ways = hit_rule_lanes(prec == kFloat64, net.ALLP, rule_warps);
     if (prec == kFloat64)
         launch_one<double, double>(net, reg, ch, hs, tol, d_err, ways, every_row, nfp64, st);
     else if (prec == kMixed)

@@ -64,6 +64,19 @@ AM_RULE float child_reach(float T, int listed, int target)
 // is to reach
 AM_RULE int seed_groups(int finite) { return finite < 60 ? finite : 60; }
 
+// ---------------------------------------------------------------- near-equal hits
+// Lanes of the rule that says which of two planes hit at nearly the same place comes
+// first (am_polygon.cu).  Rounding decides there, and a few regions of a marching depend
+// on it, so the rule stays what it was when eight warps a block scanned faces' rows from
+// 73 KB of shared memory: 32 lanes for each warp that a face of this many rows had.
+// `warps` (AM_OPT_FACE_WARPS) > 0: that many instead.
+AM_RULE int hit_rule_lanes(bool fp64_rows, int ALLP, int warps)
+{
+    if (warps > 0) return 32 * warps;
+    const int one = fp64_rows ? 256 : 512, two = fp64_rows ? 544 : 1096, four = fp64_rows ? 1128 : 2264;
+    return ALLP <= one ? 32 : (ALLP <= two ? 64 : (ALLP <= four ? 128 : 256));
+}
+
 // ---------------------------------------------------------------- append
 constexpr int kAppendWarps = 8;    // per block; a row is a warp's
 constexpr int kAppendSpanMax = 4096; // most rows per block: their winners and prefixes in shared memory

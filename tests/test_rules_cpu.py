@@ -67,3 +67,17 @@ def test_a_seeds_warp_among_more_than_2_to_the_27(tmp_path):
     for row in (0, 1, 7, 8, 2**27 - 1, 2**27, 2**27 + 9, 2**31 - 2):
         for lane in (0, 31):
             assert L.row(row // 8, 256, row % 8 * 32 + lane) == row
+
+
+@pytest.mark.parametrize("fp64", [0, 1])
+def test_lanes_of_the_rule_between_near_equal_hits(tmp_path, fp64):
+    """The lanes that a face's warps had when a block of eight warps held the rows of up to
+    eight faces (a power of two) in 73 KB of shared memory."""
+    L = rules(tmp_path, "int lanes(int fp64, int ALLP, int warps) { return hit_rule_lanes(fp64, ALLP, warps); }")
+    for allp in range(8, 12808, 8):
+        face = 32 * allp + 1120 if fp64 else 16 * allp + 1056
+        faces = 1
+        while 2 * faces <= 8 and 2 * faces * face <= 73 * 1024:
+            faces *= 2
+        assert L.lanes(fp64, allp, 0) == 32 * (8 // faces), allp
+        assert L.lanes(fp64, allp, 4) == 128
