@@ -76,6 +76,10 @@ def oracle_lib():
     return _ORACLE
 
 
+class ReferenceUnavailable(RuntimeError):
+    """The reference's sources are absent, and so is its CPU build."""
+
+
 def ref_available() -> bool:
     try:
         return ref_lib() is not None
@@ -201,7 +205,7 @@ def run_ref(net, states, points, iso=0.0, flip=False, dtype="float32", combine=N
     ``timing`` (a dict) receives the wall time of the marching call."""
     lib = ref_lib()
     if lib is None:
-        raise RuntimeError("reference CPU build unavailable")
+        raise ReferenceUnavailable("reference CPU build unavailable")
     lib.amref_set_threads(int(threads))
     lib.amref_set_region_budget(int(region_budget))
     p = _Packed(net, dtype)

@@ -25,3 +25,14 @@ def pytest_collection_modifyitems(config, items):
     for it in items:
         if "gpu" in it.keywords:
             it.add_marker(skip)
+
+
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_call(item):
+    """A test that runs the reference's own loop is skipped where that cannot be built."""
+    from oracle.oracle import ReferenceUnavailable
+
+    try:
+        return (yield)
+    except ReferenceUnavailable as ex:
+        pytest.skip(str(ex))
