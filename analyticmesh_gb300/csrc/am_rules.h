@@ -35,12 +35,13 @@ AM_RULE long long warp_row(unsigned block, unsigned block_threads, unsigned thre
 // `chunk`) and the history in which their regions find their parents.  A parent is at
 // most about one level of the breadth-first queue away, and a level held 28 to 39
 // regions per hidden unit on the benchmark networks (512 .. 4,096 units): 48 a unit.
-// Where memory is bounded -- the caller gave the wave's size, or many networks march
-// side by side -- two waves, which reach the parents while a wave holds a whole level.
-AM_RULE long long ring_slots(int wave, int chunk, int units, bool bounded)
+// Where memory is bounded, two waves, which reach the parents while a wave holds a
+// whole level: of the largest size at once where the caller gave it (a ring that grows
+// loses its history), of the present one in a batch, whose members' waves grow.
+AM_RULE long long ring_slots(int wave, int chunk, int units, bool batch, bool given)
 {
-    if (bounded) return 2ll * wave;
-    return (long long)(chunk > wave ? chunk : wave) + 48ll * units;
+    const long long most = chunk > wave ? chunk : wave;
+    return batch ? 2ll * wave : (given ? 2ll * most : most + 48ll * units);
 }
 
 // ---------------------------------------------------------------- near list

@@ -81,3 +81,18 @@ def test_lanes_of_the_rule_between_near_equal_hits(tmp_path, fp64):
             faces *= 2
         assert L.lanes(fp64, allp, 0) == 32 * (8 // faces), allp
         assert L.lanes(fp64, allp, 4) == 128
+
+
+def test_slots_of_the_ring_of_rows(tmp_path):
+    """Never less than a wave; a given wave size bounds it whatever the network, and the
+    ring then does not grow with the waves (a ring that grows loses its history)."""
+    L = rules(tmp_path, "long long slots(int wave, int chunk, int units, int batch, int given) {"
+                        " return ring_slots(wave, chunk, units, batch, given); }")
+    L.slots.restype = C.c_longlong
+    for units in (1, 512, 12800):
+        for chunk in (1, 1000, 524288):
+            for wave in {1, min(300, chunk), chunk}:
+                assert L.slots(wave, chunk, units, 0, 1) == 2 * chunk
+                assert L.slots(wave, chunk, units, 1, 0) == L.slots(wave, chunk, units, 1, 1) == 2 * wave
+                assert L.slots(wave, chunk, units, 0, 0) == chunk + 48 * units
+    assert L.slots(5000, 1000, 512, 0, 1) == 10000 and L.slots(5000, 1000, 512, 0, 0) == 5000 + 48 * 512
