@@ -53,22 +53,21 @@ REF_SAMPLE = {"sphere": 65536, "deep": 16384, "large_skip": 4096, "polytope": 65
 REF_SAMPLE_REGIONS = 65536
 ERROR_SAMPLE = 4096  # regions of the error report
 # DRAM bytes (read + write) per region of the two heavy kernels in the mixed
-# form, from one ncu capture each (--set full, dram__bytes_read.sum +
-# dram__bytes_write.sum): the sphere workload's wave of 12,672 regions, the
-# deep workload's wave of ~40,150 regions and the skip network's wave of ~12,030
-NCU_TRAFFIC_PER_REGION = {("sphere", "mixed"): {"compose": (1.214e6 + 45.631e6) / 12672,
-                                                "polygon": (109.571e6 + 4.067e6) / 12672},
-                          # a wave of ~12,030 regions of a bounded march (the full march is too
-                          # large to capture): per region, scaled to the step's regions
-                          ("large_skip", "mixed"): {"compose": (52.502e6 + 747.137e6) / 12030,
-                                                    "polygon": (806.011e6 + 16.420e6) / 12030},
-                          ("deep", "mixed"): {"compose": (27.491e6 + 957.757e6) / 40150,
-                                              "polygon": (1018.464e6 + 20.326e6) / 40150}}
+# form, from one ncu capture each (dram__bytes_read.sum + dram__bytes_write.sum) of
+# a bounded march (the full ones are too large to capture), the parents' rows in the
+# ring: the sphere workload's wave of 9,465 regions, the deep workload's of 9,721 and
+# the skip network's of 9,067 (profiles/); per region, scaled to the step's regions
+NCU_TRAFFIC_PER_REGION = {("sphere", "mixed"): {"compose": (12.839e6 + 0.237e6) / 9465,
+                                                "polygon": (65.960e6 + 25.613e6) / 9465},
+                          ("large_skip", "mixed"): {"compose": (433.124e6 + 664.776e6) / 9067,
+                                                    "polygon": (526.205e6 + 319.555e6) / 9067},
+                          ("deep", "mixed"): {"compose": (32.483e6 + 208.249e6) / 9721,
+                                              "polygon": (204.655e6 + 125.876e6) / 9721}}
 # the composition's tensor pipe (sm__pipe_tensor_cycles_active) in the same
 # captures: the mixed form issues six bf16 products per algorithmic product,
 # so `frac` (algorithmic FLOP/s over the bf16 peak) stays below 1/6 even with
 # the pipe saturated; this is the pipe's own share of the kernel's time
-NCU_TENSOR_ACTIVE = {("large_skip", "mixed"): 0.436, ("sphere", "mixed"): 0.152, ("deep", "mixed"): 0.257}
+NCU_TENSOR_ACTIVE = {("large_skip", "mixed"): 0.531, ("sphere", "mixed"): 0.144, ("deep", "mixed"): 0.347}
 
 
 def parse():
@@ -127,17 +126,32 @@ def max_over_ranks(value, device="cpu"):
     return float(t.item())
 
 
-def composition_flops(nodes, arc_table, tms):
+def composition_flops(nodes, arc_table, tms, first=1):
     """Algorithmic FLOPs of one region's composition: 4 columns x 2 flop per
     multiply-add over every layer product and every transformed connection
-    (the input's included: 8 (sum n_l n_l+1 + sum n_dst n_src))."""
-    macs = sum(nodes[i] * nodes[i + 1] for i in range(1, len(nodes) - 1))
-    for row in arc_table:
+    (the input's included: 8 (sum n_l n_l+1 + sum n_dst n_src)), of the linears
+    from ``first`` on: a region entered through a plane of hidden layer ``first``
+    shares the layers up to it with its parent."""
+    macs = sum(nodes[i] * nodes[i + 1] for i in range(first, len(nodes) - 1))
+    for i, row in enumerate(arc_table, 1):
+        if i < first:
+            continue
         for c in range(int(row[0])):
             t = int(row[2 + 2 * c])
             if tms[t].size:
                 macs += tms[t].shape[0] * tms[t].shape[1]
     return 8 * macs
+
+
+def marching_flops(net, starts):
+    """Algorithmic FLOPs of a marching's compositions; ``starts``: the plane each
+    region was entered through (-1: a seed, which composes every layer)."""
+    import numpy as np
+
+    ends = np.cumsum(net.nodes[1:-1])
+    layer = np.where(starts < 0, 1, 1 + np.searchsorted(ends, starts, side="right"))
+    return sum(int(n) * composition_flops(net.nodes, net.arc_table, net.tms, int(c))
+               for c, n in zip(*np.unique(layer, return_counts=True)))
 
 
 def workload(name, nseeds):
@@ -557,7 +571,9 @@ def main():
     hbm, tflops, peak_kind = measured_peaks()
     regions = sp["num_regions"]
     ALL = int(sum(net.nodes[1:-1])) + net.num_extra
-    flops = composition_flops(net.nodes, net.arc_table, net.tms) * regions
+    starts = np.zeros(regions, np.int32)
+    _lib.check(_lib.lib().am_get_regions(eng.h, None, None, None, None, None, None, starts.ctypes.data), eng.h)
+    flops = marching_flops(net, starts)
     elem = 8 if form == "float64" else 4
     poly_bytes = regions * (ALL * 4 * elem + 4 * elem + 12 * 6)
     per_region = NCU_TRAFFIC_PER_REGION.get((args.workload, form), {})
@@ -566,7 +582,8 @@ def main():
         tr = per_region.get("compose")
         roof = {"kernel": "compose", "bound": "tensor", "achieved": ach, "peak": tflops, "unit": "TFLOP/s",
                 "frac": ach / tflops, "traffic": tr * regions if tr else None, "peak_kind": peak_kind,
-                "algorithmic": "%d FLOP/region x %d regions" % (flops // max(regions, 1), regions),
+                "algorithmic": "%d FLOP/region (after the layer it was entered through) x %d regions"
+                               % (flops // max(regions, 1), regions),
                 "products_per_flop": 6, "tensor_pipe_active_ncu": NCU_TENSOR_ACTIVE.get((args.workload, form))}
     else:
         ach = poly_bytes / (phases["polygon_ms"] / 1e3) / 1e9
