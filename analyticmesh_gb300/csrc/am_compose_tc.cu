@@ -646,7 +646,8 @@ __global__ void __launch_bounds__(kThreads + 32, 1) compose_tc_kernel(NetDev net
 // for the first half's operand (8 K) and accumulators (4 K) around the passes'
 // ends, and lose about 400 cycles per weight block to barriers between blocks.
 // With the row warps rebuilding every block of every pass in shared memory from
-// the rows the composition took 308 ms of a marching, this way 275 ms; with six
+// the rows the composition took 308 ms of a marching, this way 275 ms (a weight
+// block copied once per CTA; shared by two CTAs 274); with six
 // layers of 256 units 16.5 and 15.4 ms.
 // The operand values, the order of the products into each accumulator and the
 // epilogue and face-plane arithmetic are those of compose_tc_kernel, so both

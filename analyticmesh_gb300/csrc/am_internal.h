@@ -72,8 +72,8 @@ struct HashDev {
 
 // Wave control block in device memory.  The host-driven loop reads tail and
 // err after every wave; the graph-driven loop keeps head and count here too,
-// so the kernels of a captured wave read their range from the device and a
-// one-thread step kernel advances the queue and decides whether to go on.
+// so the kernels of a captured wave read their range from the device and the last
+// block of the append advances the queue and decides whether to go on.
 struct WaveCtl {
     long long tail;     // regions in the store (appends advance it)
     int err;            // device error bits

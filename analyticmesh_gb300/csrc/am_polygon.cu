@@ -1379,7 +1379,7 @@ __device__ int insert_edges(const RegionsDev &reg, const HashDev &hs, long long 
 // that scans every row at every step from shared memory, because with the list a
 // step is four rows per lane and the rest of it (solve, decisions) is the same for
 // every warp of a group.  Measured on GB300, polygon phase of a whole marching:
-//   3-[512]x8-1 mixed (6.8 M faces)      378 ms -> 142 ms
+//   3-[512]x8-1 mixed (6.8 M faces)      378 ms -> 143 ms
 //   3-[256]x6-1 mixed (1.28 M)            29.4  -> 15.0
 //   3-[128]x4-1 mixed / fp32 / fp64 (265 K) 3.2 / 2.4 / 28.8 -> 2.7 / 1.7 / 8.5
 template <typename TC, typename TS>

@@ -224,8 +224,8 @@ def _fill_run_args(a, k, eng, net, st, pt, iso, flip_insideout):
 
 
 def autotune(eng, net, states, points, iso=0.0, flip_insideout=False, sample_regions=65536):
-    """am_autotune: choose the composition tile and the warps per face for
-    this engine's architecture from sample runs; returns (tile, warps)."""
+    """am_autotune: choose the composition tile for this engine's architecture
+    from sample runs; returns (tile, AM_OPT_FACE_WARPS' automatic value)."""
     k = _Keep()
     a = _lib.AmRunArgs()
     _fill_run_args(a, k, eng, net, states, points, iso, flip_insideout)
