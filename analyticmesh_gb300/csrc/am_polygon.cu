@@ -60,6 +60,7 @@ namespace {
 
 constexpr int kList = 128;      // rows of the near list (four per lane)
 constexpr int kTarget = 64;     // and how many it aims at (80 and 48 measured 1 to 7 % slower)
+constexpr int kDirect = 512;    // rows up to which a walk that left its ball goes on to every row (face_slow)
 constexpr int kFaceWarps = 4;   // faces per block
 constexpr int kBlocks = 8;      // blocks per SM
 constexpr int kUnroll = 4;      // FP32 rows per lane in flight (half as many FP64 ones)
@@ -730,10 +731,12 @@ struct Face {
 
 // One face walk from the start plane s: the scan in TC (kWide: FP64 predicates
 // near zero), vertices solved in TS.  kNear: `near` is set when some step's scan
-// met a row within 1e-6 of the current point.  False (list only): a point left
-// the ball, or the rule needs every row; the face is not valid.
+// met a row within 1e-6 of the current point.  kWalked, or (list only; the face is
+// not valid) kLeft: a point left the ball, kUndecided: the rule between near-equal
+// hits needs every row, whatever the ball's size.
+enum : int { kWalked = 0, kAgain = 1, kLeft = 2, kUndecided = 3 };
 template <typename TC, typename TS, bool kWide, bool kNear, typename Rows>
-__device__ bool walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *eqv, const TS *p,
+__device__ int walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *eqv, const TS *p,
                      int s, TC par_eps, TS same_eps, int lane, Face<TS> &f, bool &near)
 {
     TS last[3] = {0, 0, 0}, first[3] = {0, 0, 0}; // vertices appended last and first (every lane)
@@ -758,7 +761,7 @@ __device__ bool walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<
         l64.c1 = p[1];
         l64.c2 = p[2];
     }
-    if (!ball.in((float)ln.c0, (float)ln.c1, (float)ln.c2)) return false;
+    if (!ball.in((float)ln.c0, (float)ln.c1, (float)ln.c2)) return kLeft;
     for (int step = 0; step < kWalkSteps; ++step) {
         f.nsteps = step + 1;
         // direction of the edge line: w_eq x w_e (counter-clockwise about w_eq)
@@ -780,14 +783,14 @@ __device__ bool walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<
         } else {
             what = scan<TC, kNear>(rows, ln, ways, lane, bk, bt, near);
         }
-        if (what == kGiveUp) return false;
+        if (what == kGiveUp) return kUndecided;
         if (what == kNone) { // the edge line never leaves the region (or its ball)
-            if (ball.d2 != INFINITY) return false;
+            if (ball.d2 != INFINITY) return kLeft;
             f.status = kOpen;
             break;
         }
         if (!ball.in((float)ln.c0 + bt * (float)ln.d0, (float)ln.c1 + bt * (float)ln.d1, (float)ln.c2 + bt * (float)ln.d2))
-            return false;
+            return kLeft;
         // vertex = 3x3 solve of (edge plane, hit plane, face plane)
         TS V[3];
         TC Vc[3];
@@ -853,10 +856,10 @@ __device__ bool walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<
             l64.c1 = V[1];
             l64.c2 = V[2];
         }
-        if (!ball.in((float)ln.c0, (float)ln.c1, (float)ln.c2)) return false;
+        if (!ball.in((float)ln.c0, (float)ln.c1, (float)ln.c2)) return kLeft;
     }
     if (!f.closed && f.status == kOk) f.status = kTruncated;
-    return true;
+    return kWalked;
 }
 
 // Mixed form: the walk runs in the scan precision TC (solves included, as the
@@ -869,8 +872,7 @@ __device__ bool walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<
 // current point other than the two it lies on (a sign or feasibility test
 // near zero), when the TC walk did not close normally, took more than 32
 // steps or met a vertex that is not finite in TS, or when a decision comes
-// out differently in TS; kLeft when the walk left the list (see walk).
-enum : int { kRefined = 0, kAgain = 1, kLeft = 2 };
+// out differently in TS; kLeft and kUndecided as walk does.
 template <typename TC, typename TS, typename Rows>
 __device__ int walk_refined(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *eqv,
                             const TS *p, int s, TC par_eps, TS same_eps, int lane, Face<TS> &f)
@@ -880,7 +882,8 @@ __device__ int walk_refined(const Rows &rows, const Ball &ball, int ways, const 
     const TC pf[3] = {(TC)p[0], (TC)p[1], (TC)p[2]};
     Face<TC> w;
     bool near;
-    if (!walk<TC, TC, false, true>(rows, ball, ways, eqc, eqf, pf, s, par_eps, (TC)same_eps, lane, w, near)) return kLeft;
+    const int how = walk<TC, TC, false, true>(rows, ball, ways, eqc, eqf, pf, s, par_eps, (TC)same_eps, lane, w, near);
+    if (how != kWalked) return how;
     const int sbk = w.sbk, sdec = w.sdec, nsteps = w.nsteps;
     // a predicate near zero: the caller walks again with FP64 predicates
     if (near || w.status != kOk || !w.closed || nsteps < 1 || nsteps > 32) return kAgain;
@@ -962,11 +965,11 @@ __device__ int walk_refined(const Rows &rows, const Ball &ball, int ways, const 
     }
     f.closed = true;
     f.status = kOk;
-    return kRefined;
+    return kWalked;
 }
 
 template <typename TC, typename TS, typename Rows>
-__device__ bool walk_fp64(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *p,
+__device__ int walk_fp64(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *p,
                                        int s, TC par_eps, TS same_eps, int lane, Face<TS> &f)
 {
     const TS eqv[4] = {(TS)eqc.x, (TS)eqc.y, (TS)eqc.z, (TS)eqc.w};
@@ -974,16 +977,15 @@ __device__ bool walk_fp64(const Rows &rows, const Ball &ball, int ways, const ve
     return walk<TC, TS, true, false>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f, near);
 }
 
-// The whole walk of a form over one row source; false: the list does not do.
+// The whole walk of a form over one row source (kLeft, kUndecided: as walk).
 template <typename TC, typename TS, typename Rows>
-__device__ bool face_walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *eqv, const TS *p,
+__device__ int face_walk(const Rows &rows, const Ball &ball, int ways, const vec4_t<TC> &eqc, const TS *eqv, const TS *p,
                           int s, TC par_eps, TS same_eps, int lane, Face<TS> &f, bool &again)
 {
     again = false;
     if constexpr (sizeof(TS) > sizeof(TC)) { // scan-precision walk, vertices refined in the solve precision
         const int r = walk_refined<TC, TS>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f);
-        if (r == kRefined) return true;
-        if (r == kLeft) return false;
+        if (r != kAgain) return r;
         again = true; // FP64 predicates and FP64 solves
         return walk_fp64<TC, TS>(rows, ball, ways, eqc, p, s, par_eps, same_eps, lane, f);
     } else {
@@ -1191,11 +1193,19 @@ struct Result {
 
 // Everything but the common face (a region with a parent whose FP32 walk stays in
 // its list and needs no FP64 predicate): seeds, repeats with another radius, FP64
-// predicates, every row.  Kept out of the kernel's registers.  `again`: only
-// the FP64 predicates are asked for, on the list as it is.  `every_row`: no list.
+// predicates, every row.  Kept out of the kernel's registers.  `what`: kAgain, only
+// the FP64 predicates are asked for, on the list as it is; kLeft or kUndecided, the
+// walk over the list as it is (n rows within T) has failed.  `every_row`: no list.
+// A larger ball costs a pass over the rows and may fail again (an edge that never
+// ends does for certain), so it is tried only where a walk over every row costs
+// more: on up to kDirect rows a step of that takes a few rows per lane as the list's
+// does.  Measured on GB300, polygon phase in float64 / mixed / float32: 3-[50]x3-1 with
+// connections, 192 of 14,397 faces open, 2.5 / 0.98 / 0.73 ms with the failed walk made
+// again and larger balls tried, 1.8 / 0.76 / 0.53 this way; widths 8 to 87 with many
+// near-equal hits 10.4 / 3.4 / 2.8 and 6.2 / 2.2 / 1.8; the benchmark networks alike.
 template <typename TC, typename TS>
 __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *list, int ways, const vec4_t<TC> &eqc,
-                                       const TS *mid, int start, TC eps, TC par_eps, TS same_eps, int lane, bool again,
+                                       const TS *mid, int start, TC eps, TC par_eps, TS same_eps, int lane, int what,
                                        int n, float T, bool every_row, Result<TS> &out)
 {
     const bool is_seed = start < 0;
@@ -1203,7 +1213,7 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
     TS p[3] = {mid[0], mid[1], mid[2]};
     Ball ball{(float)p[0], (float)p[1], (float)p[2], -1.f};
     Face<TS> f;
-    bool done = false, wide = false;
+    bool done = false, wide = false, found = false;
     int s = start, s_plane = start;
     auto clear = [&] {
         f.vx = f.vy = f.vz = TS(0);
@@ -1217,12 +1227,20 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
         T = all.n > kList ? seed_radius<TC>(all, ball, lane) : INFINITY;
         n = -1;
     }
+    bool use_list = !every_row && what != kUndecided;
+    auto larger = [&](bool direct) { // a larger ball, if it is worth a pass
+        if (n > 3 * kList / 4 || T >= kReachMax || (direct && all.n <= kDirect)) return false;
+        T *= fminf((float)kList * 0.85f / (float)max(n, 1), 3.f);
+        n = -1;
+        return true;
+    };
+    if (use_list && !is_seed && what == kLeft && n <= kList) use_list = larger(true);
     if (n > kList) { // (only if dead units are in it is the same ball worth another pass)
         bool dead = false;
         for (int j = lane; j < kList; j += 32) dead = dead || list->row[j].w != list->row[j].w;
         if (__any_sync(kFull, dead)) n = -1;
     }
-    for (int tries = 0; tries < 5 && !done && !every_row; ++tries) {
+    for (int tries = 0; tries < 5 && !done && use_list; ++tries) {
         if (n < 0) n = collect<TC>(all, T, ball, list, lane);
         if (n > kList) { // a smaller ball
             T = clamp_reach(T * ((float)kTarget / (float)n));
@@ -1242,26 +1260,32 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
                 break;
             }
         }
+        int how = kLeft;
         if (s >= 0) {
             if constexpr (sizeof(TS) > sizeof(TC)) {
-                if (again) {
+                if (what == kAgain) {
                     wide = true;
-                    done = walk_fp64<TC, TS>(rows, ball, ways, eqc, q, s, par_eps, same_eps, lane, f);
+                    how = walk_fp64<TC, TS>(rows, ball, ways, eqc, q, s, par_eps, same_eps, lane, f);
                 } else {
-                    done = face_walk<TC, TS>(rows, ball, ways, eqc, eqv, q, s, par_eps, same_eps, lane, f, wide);
+                    how = face_walk<TC, TS>(rows, ball, ways, eqc, eqv, q, s, par_eps, same_eps, lane, f, wide);
                 }
             } else {
-                done = face_walk<TC, TS>(rows, ball, ways, eqc, eqv, q, s, par_eps, same_eps, lane, f, wide);
+                how = face_walk<TC, TS>(rows, ball, ways, eqc, eqv, q, s, par_eps, same_eps, lane, f, wide);
             }
-        }
-        again = false;
-        if (done) {
             s_plane = list->idx[s];
+        }
+        what = kLeft;
+        done = how == kWalked;
+        if (done) {
             if (f.ve >= 0) f.ve = list->idx[f.ve];
-        } else {
-            if (n > 3 * kList / 4 || T >= kReachMax) break;
-            T *= fminf((float)kList * 0.85f / (float)max(n, 1), 3.f); // a larger ball
-            n = -1;
+        } else if (how == kUndecided || !larger(s >= 0)) {
+            if (is_seed && s >= 0) { // the start vertex found is every row's too
+                found = true;
+                p[0] = q[0];
+                p[1] = q[1];
+                p[2] = q[2];
+            }
+            break;
         }
     }
     if (!done) { // every row
@@ -1269,7 +1293,8 @@ __device__ __noinline__ void face_slow(const GlobalRows<TC> &all, NearList<TC> *
         clear();
         wide = false;
         s = start;
-        if (is_seed) s = seed_start<TC, TS>(all, all, whole, INFINITY, eqv, p, eps, lane);
+        if (found) s = s_plane;
+        else if (is_seed) s = seed_start<TC, TS>(all, all, whole, INFINITY, eqv, p, eps, lane);
         if (s >= 0) face_walk<TC, TS>(all, whole, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f, wide);
         s_plane = s;
     }
@@ -1446,9 +1471,7 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
                         what = walk_refined<TC, TS>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f);
                     } else {
                         bool near;
-                        what = walk<TC, TS, false, false>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f, near)
-                                   ? kRefined
-                                   : kLeft;
+                        what = walk<TC, TS, false, false>(rows, ball, ways, eqc, eqv, p, s, par_eps, same_eps, lane, f, near);
                     }
                 }
                 r.vx = f.vx;
@@ -1457,14 +1480,14 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
                 r.n = f.n;
                 r.closed = f.closed;
                 r.status = f.status;
-                r.ve = what == kRefined && f.ve >= 0 ? (int)list->idx[f.ve] : -1;
+                r.ve = what == kWalked && f.ve >= 0 ? (int)list->idx[f.ve] : -1;
                 r.start = start;
             }
         }
-        if (what != kRefined) {
+        if (what != kWalked) {
             Result<TS> o;
             const vec4_t<TC> eqc = ld4<TC>((const TC *)ch.eq + (size_t)rl * 4);
-            face_slow<TC, TS>(all, list, ways, eqc, midp, start, eps, par_eps, same_eps, lane, what == kAgain, r.listed, r.T, every_row, o);
+            face_slow<TC, TS>(all, list, ways, eqc, midp, start, eps, par_eps, same_eps, lane, what, r.listed, r.T, every_row, o);
             r = o;
             if (r.again && lane == 0) atomicAdd(nfp64, 1ull);
         }
