@@ -410,7 +410,7 @@ struct am_engine {
     {
         const size_t per = tc * 4 * (size_t)ALLP;
         long long target = wave;
-        if (classes() && !ring_min) target = ring_slots(wave, run.chunk, N, run.lean, chunk_opt > 0);
+        if (classes() && !ring_min) target = ring_slots(wave, run.chunk, N, (long long)per, run.lean, chunk_opt > 0);
         if (wave <= ring && target <= ring_target) return;
         long long want = target;
         if (want > wave) {
@@ -940,7 +940,7 @@ void run_begin(am_engine *e, const RunArgs &a)
     const int chunk = e->default_chunk();
     e->ring_min = false;
     e->rows_from = 0;
-    if (e->chunk_opt > 0 && e->ring > ring_slots(chunk, chunk, e->N, false, true)) e->give_back_rows(); // (of earlier runs)
+    if (e->chunk_opt > 0 && e->ring > ring_slots(chunk, chunk, e->N, (long long)(tc * 4 * (size_t)e->ALLP), false, true)) e->give_back_rows(); // (of earlier runs)
     // the first stores hold the seeds' children of a first wave (a batch
     // member's, or a small network's, grow on demand from there)
     const long long first_wave = std::min<long long>(chunk, e->lean ? 4ll * S + 1024 : std::max(4ll * S + 1024, 65536ll));

@@ -37,11 +37,18 @@ AM_RULE long long warp_row(unsigned block, unsigned block_threads, unsigned thre
 // regions per hidden unit on the benchmark networks (512 .. 4,096 units): 48 a unit.
 // Where memory is bounded, two waves, which reach the parents while a wave holds a
 // whole level: of the largest size at once where the caller gave it (a ring that grows
-// loses its history), of the present one in a batch, whose members' waves grow.
-AM_RULE long long ring_slots(int wave, int chunk, int units, bool batch, bool given)
+// loses its history), of the present one in a batch, whose members' waves grow.  A
+// given size does not keep the history from 64 MiB: waves smaller than a level would
+// find no parent in two of them (3-42-10-12-92-125-246-1, mixed, 200 K regions in waves
+// of 64 on GB300: composition 130 ms without it, 124 with it).
+constexpr long long kRingBytes = 64ll << 20;
+AM_RULE long long ring_slots(int wave, int chunk, int units, long long row_bytes, bool batch, bool given)
 {
-    const long long most = chunk > wave ? chunk : wave;
-    return batch ? 2ll * wave : (given ? 2ll * most : most + 48ll * units);
+    const long long most = chunk > wave ? chunk : wave, all = most + 48ll * units;
+    if (batch) return 2ll * wave;
+    if (!given) return all;
+    const long long small = kRingBytes / row_bytes < all ? kRingBytes / row_bytes : all;
+    return 2ll * most > small ? 2ll * most : small;
 }
 
 // ---------------------------------------------------------------- near list

@@ -176,7 +176,7 @@ typedef enum {
                                  composition tiles, and beside them the rows of 48 earlier regions per
                                  hidden unit, in which regions find their parents': 13 GB at 4,096 units
                                  in FP32, at most an eighth of the free memory).  A given size bounds the
-                                 rows to those of two waves.  The rows stay with the engine between calls;
+                                 rows to those of two waves, or 64 MiB.  The rows stay with the engine between calls;
                                  where memory runs out they are given back before a call fails. */
     AM_OPT_PHASE_TIMING = 2,  /* 1: time compose / polygon / frontier separately */
     AM_OPT_WELD = 3,          /* CombineMesh vertex weld: 0 = topological (default: a vertex is named by

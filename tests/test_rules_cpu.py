@@ -86,13 +86,19 @@ def test_lanes_of_the_rule_between_near_equal_hits(tmp_path, fp64):
 def test_slots_of_the_ring_of_rows(tmp_path):
     """Never less than a wave; a given wave size bounds it whatever the network, and the
     ring then does not grow with the waves (a ring that grows loses its history)."""
-    L = rules(tmp_path, "long long slots(int wave, int chunk, int units, int batch, int given) {"
-                        " return ring_slots(wave, chunk, units, batch, given); }")
+    L = rules(tmp_path, "long long slots(int wave, int chunk, int units, long long row_bytes, int batch, int given) {"
+                        " return ring_slots(wave, chunk, units, row_bytes, batch, given); }")
     L.slots.restype = C.c_longlong
+    L.slots.argtypes = [C.c_int, C.c_int, C.c_int, C.c_longlong, C.c_int, C.c_int]
     for units in (1, 512, 12800):
+        row = 16 * ((units + 7) // 8 * 8)
         for chunk in (1, 1000, 524288):
+            full = chunk + 48 * units
             for wave in {1, min(300, chunk), chunk}:
-                assert L.slots(wave, chunk, units, 0, 1) == 2 * chunk
-                assert L.slots(wave, chunk, units, 1, 0) == L.slots(wave, chunk, units, 1, 1) == 2 * wave
-                assert L.slots(wave, chunk, units, 0, 0) == chunk + 48 * units
-    assert L.slots(5000, 1000, 512, 0, 1) == 10000 and L.slots(5000, 1000, 512, 0, 0) == 5000 + 48 * 512
+                given = L.slots(wave, chunk, units, row, 0, 1)
+                assert given == max(2 * chunk, min(full, (64 << 20) // row))
+                assert given * row <= max(2 * chunk * row, 64 << 20)
+                assert L.slots(wave, chunk, units, row, 1, 0) == L.slots(wave, chunk, units, row, 1, 1) == 2 * wave
+                assert L.slots(wave, chunk, units, row, 0, 0) == full
+    assert L.slots(50000, 1000, 4096, 65536, 0, 1) == 100000
+    assert L.slots(5000, 1000, 512, 8192, 0, 0) == 5000 + 48 * 512
