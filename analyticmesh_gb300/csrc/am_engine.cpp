@@ -215,12 +215,18 @@ struct am_engine {
     DevBuf tc_x; // the streamed composition's operand (TcNet::xbuf)
     TcNet tcnet{};
     // regions
-    DevBuf keys, hash, mid, start, parent, reach, nv, status, verts, edges;
+    DevBuf keys, hash, mid, start, parent, nv, status, verts, edges;
     long long cap = 0;
     DevBuf table;
     unsigned long long hcap = 0;
     // chunk
-    DevBuf cons, eq, rec, blocksum, order, split;
+    // (the wave buffers in one allocation: on the many engines of a batch each costs
+    // with the number of those there are)
+    DevBuf cons, blocksum, wave;
+    struct View {
+        void *p = nullptr;
+        template <typename T> T *as() const { return (T *)p; }
+    } eq, rec, order, split;
     int chunk_cap = 0;
     int append_cap = 0;       // blocks of blocksum (AppendScratch)
     int ring = 0;             // slots of cons (ChunkDev)
@@ -307,7 +313,6 @@ struct am_engine {
         r.mid = mid.p;
         r.start = start.as<int32_t>();
         r.parent = parent.as<int32_t>();
-        r.reach = reach.as<float>();
         r.nv = nv.as<int32_t>();
         r.status = status.as<int8_t>();
         r.verts = verts.p;
@@ -321,8 +326,8 @@ struct am_engine {
     void release_run_buffers()
     {
         drop_graph();
-        for (DevBuf *b : {&keys, &hash, &mid, &start, &parent, &reach, &nv, &status, &verts, &edges, &table, &cons, &eq, &rec,
-                          &blocksum, &order, &split, &tc_x})
+        for (DevBuf *b : {&keys, &hash, &mid, &start, &parent, &nv, &status, &verts, &edges, &table, &cons, &wave, &blocksum,
+                          &tc_x})
             b->reset();
         ring = 0;
         ring_target = 0;
@@ -343,7 +348,6 @@ struct am_engine {
         AM_CUDA(mid.grow(ts * 4 * nc, ts * 4 * keep, st));
         AM_CUDA(start.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
         AM_CUDA(parent.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
-        AM_CUDA(reach.grow(sizeof(float) * nc, sizeof(float) * keep, st));
         AM_CUDA(nv.grow(sizeof(int32_t) * nc, sizeof(int32_t) * keep, st));
         AM_CUDA(status.grow(sizeof(int8_t) * nc, sizeof(int8_t) * keep, st));
         AM_CUDA(verts.grow(ts * 3 * kVMax * nc, ts * 3 * kVMax * keep, st));
@@ -379,12 +383,21 @@ struct am_engine {
     {
         if (count <= chunk_cap) return;
         chunk_cap = 0; // (should one of the allocations fail, none is taken for there)
-        if (classes()) {
-            AM_CUDA(order.alloc(sizeof(int32_t) * (size_t)(n_lin - 1) * count, st));
-            AM_CUDA(split.alloc(sizeof(int32_t) * (size_t)count, st));
+        const size_t n = (size_t)count;
+        size_t bytes[4] = {tc * 4 * n, sizeof(int32_t) * kVMax * n, classes() ? sizeof(int32_t) * (n_lin - 1) * n : 0,
+                           classes() ? sizeof(int32_t) * n : 0};
+        size_t at = 0;
+        for (size_t &b : bytes) {
+            b = (b + 255) / 256 * 256;
+            at += b;
         }
-        AM_CUDA(eq.alloc(tc * 4 * (size_t)count, st));
-        AM_CUDA(rec.alloc(sizeof(int32_t) * (size_t)kVMax * count, st));
+        AM_CUDA(wave.alloc(at, st));
+        View *view[4] = {&eq, &rec, &order, &split};
+        at = 0;
+        for (int i = 0; i < 4; ++i) {
+            view[i]->p = bytes[i] ? wave.as<char>() + at : nullptr;
+            at += bytes[i];
+        }
         ensure_append(count);
         chunk_cap = count;
     }
@@ -413,7 +426,7 @@ struct am_engine {
         if (classes() && !ring_min) target = ring_slots(wave, run.chunk, N, (long long)per, run.lean, chunk_opt > 0);
         if (wave <= ring && target <= ring_target) return;
         long long want = target;
-        if (want > wave) {
+        if (want > wave && (size_t)want * per > kRingFree) {
             size_t fr = 0, all = 0;
             AM_CUDA(cudaMemGetInfo(&fr, &all));
             want = std::min<long long>(want, (long long)((fr + cons.bytes) / 8 / per));

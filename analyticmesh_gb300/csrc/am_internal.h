@@ -54,10 +54,9 @@ struct NetDev {
 struct RegionsDev {
     uint32_t *keys;     // [cap][W] packed activation bits
     uint64_t *hash;     // [cap]
-    void *mid;          // [cap][4] TS: seed point / edge midpoint
+    void *mid;          // [cap][4] TS: seed point / edge midpoint, radius of the near list for the region's children (am_polygon.cu)
     int32_t *start;     // [cap] start plane (-1 = seed)
     int32_t *parent;    // [cap] the region it was entered from (-1 = seed)
-    float *reach;       // [cap] radius of the near list for the region's children (am_polygon.cu)
     int32_t *nv;        // [cap] polygon vertex count
     int8_t *status;     // [cap]
     void *verts;        // [cap][kVMax][3] TS

@@ -1450,7 +1450,7 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
         r.T = INFINITY; // few rows: all of them
         int what = kLeft;
         if (start >= 0) {
-            if (ALL > kList) r.T = reg.reach[parent];
+            if (ALL > kList) r.T = (float)((const TS *)reg.mid)[(size_t)parent * 4 + 3];
             const Ball centre{(float)midp[0], (float)midp[1], (float)midp[2], -1.f};
             Sieve<TC> sv(centre, r.T, list, lane);
             stream_part<TC, true>(all.par, own, 0, all.nsplit, all.flip, sv);
@@ -1497,7 +1497,7 @@ __global__ void __launch_bounds__(32 * kFaceWarps, kBlocks) polygon_kernel(NetDe
         if (lane == 0) {
             reg.nv[rid] = nv;
             reg.status[rid] = r.status;
-            reg.reach[rid] = child_reach(r.T, r.listed, kTarget);
+            ((TS *)reg.mid)[(size_t)rid * 4 + 3] = (TS)child_reach(r.T, r.listed, kTarget);
         }
         if (lane < nv) {
             TS *vo = (TS *)reg.verts + ((size_t)rid * kVMax + lane) * 3;

@@ -2,6 +2,7 @@
 // so that they can be checked over their whole range on the CPU.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 
 #ifdef __CUDACC__
@@ -42,6 +43,7 @@ AM_RULE long long warp_row(unsigned block, unsigned block_threads, unsigned thre
 // find no parent in two of them (3-42-10-12-92-125-246-1, mixed, 200 K regions in waves
 // of 64 on GB300: composition 130 ms without it, 124 with it).
 constexpr long long kRingBytes = 64ll << 20;
+constexpr size_t kRingFree = size_t(256) << 20; // from here on a ring asks how much memory is free
 AM_RULE long long ring_slots(int wave, int chunk, int units, long long row_bytes, bool batch, bool given)
 {
     const long long most = chunk > wave ? chunk : wave, all = most + 48ll * units;
